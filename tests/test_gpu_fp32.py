@@ -295,3 +295,35 @@ def test_capture_without_scratch_reads_caller_tensors_with_same_bits(cglib, layo
         cg.check_device()
         assert torch.equal(y0.view(torch.int32), y1.view(torch.int32)), (layout, b, h, c, kn, k, st)
         assert torch.equal(dx0.view(torch.int32), dx1.view(torch.int32)), (layout, b, h, c, kn, k, st)
+
+
+@pytest.mark.parametrize("b,h,w,c,kn,kh,kw,stride,pad", [
+    (1, 9, 11, 5, 32, 3, 3, 1, 1),        # 128 x 32 tiles (forward, weight gradient), narrow input gradient
+    (2, 13, 9, 33, 33, 3, 3, 1, 1),       # one column past the narrow tile
+    (3, 17, 15, 40, 65, 1, 3, 2, 1),      # 64 x 64 tiles, one column past a tile; NCHW rows that are no vectors
+    (1, 40, 6, 4, 12, 17, 3, 1, 1),       # filter beyond the tap masks: range tests per element
+    (1, 6, 40, 3, 8, 1, 18, 2, 2),        # the same, wider than high, strided input gradient by phases
+    (1, 30, 30, 2, 6, 9, 9, 3, 4),        # more stride-phase taps than the phase table: gather form with masks
+    (8, 40, 40, 16, 136, 3, 3, 1, 1),     # 128 x 128 tiles with a ragged last column tile
+])
+def test_tiles_and_tap_forms_follow_reference_order(cglib, oracle_lib, b, h, w, c, kn, kh, kw, stride, pad):
+    """Every tile shape, store form and tap test of the FP32 kernels gives the reference order's bits
+    (forward and weight gradient; the input gradient within FP32 tolerance and reproducible)."""
+    g = C.geom(b, h, w, c, kn, kh, kw, vpad=pad, hpad=pad, vstr=stride, hstr=stride)
+    ho, wo = C.out_hw(g)
+    K = c * kh * kw
+    rng = np.random.default_rng(h * 100 + kn)
+    inp = {"x": rng.uniform(-1, 1, b * h * w * c).astype(np.float32),
+           "w": (rng.standard_normal(K * kn) * np.sqrt(2 / K)).astype(np.float32),
+           "dy": rng.uniform(-1, 1, b * ho * wo * kn).astype(np.float32),
+           "dx0": rng.uniform(-1, 1, b * h * w * c).astype(np.float32),
+           "epi": {"bias": rng.uniform(-.1, .1, kn).astype(np.float32), "relu": True}}
+    for layout in (C.NHWC, C.NCHW):
+        for op, n in (("fwd", b * ho * wo * kn), ("wgrad", K * kn)):
+            got = dropin(cglib, op, layout, g, inp, np.zeros(n, np.float32), to_dev=True)
+            assert bitexact(got, port(oracle_lib, op, layout, g, inp, n)), (layout, op)
+        got = dropin(cglib, "dgrad", layout, g, inp, inp["dx0"].copy(), to_dev=True)
+        want = port(oracle_lib, "dgrad", layout, g, inp, None)
+        assert errors(got, want)[0] <= FP32_TOL, layout
+        again = dropin(cglib, "dgrad", layout, g, inp, inp["dx0"].copy(), to_dev=True)
+        assert bitexact(got, again), layout
