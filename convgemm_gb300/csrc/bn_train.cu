@@ -19,50 +19,86 @@
 
 namespace {
 
-constexpr int BN_CHUNK = 256;   // statistics groups per block of the first pass
+constexpr int BN_CHUNK = CG_STAT_CHUNK;
 
 // Pass 1: block (x = 32 channels, y = a chunk of BN_CHUNK groups) sums its groups for
 // its channels in FP64, the 8 thread rows strided over the chunk, then in a fixed
-// order across the rows.  part: [ngroups][2][kn] FP32; out: [nchunks][2][kn] FP64.
+// order across the rows.  part: [ngroups][2][kn] FP32; out: [nchunks][2][kn] FP64 (PLANES = 1: the
+// sums alone). FP64 additions and conversions bound it (two per cycle and SM), so chunks are
+// small enough for every SM to have some (chunks of 256 groups left 56 blocks for 7168 groups x 64
+// channels: 22 us), and the conversions are done on the integer pipe (17 us with them on the FP64 pipe).
+__device__ __forceinline__ double widen(float f) {   // (double) f
+    const uint32_t u = __float_as_uint(f), e = u >> 23 & 255;
+    if (e - 1u < 254u) return __hiloint2double((int) ((u & 0x80000000u) | ((u & 0x7FFFFFFFu) >> 3) + 0x38000000u), (int) (u << 29));
+    return (u << 1) == 0 ? __hiloint2double((int) u, 0) : (double) f;   // zero; subnormal, infinite, NaN
+}
+template <int PLANES>
 __global__ void __launch_bounds__(256) bn_stats_pass1(const float *__restrict__ part, int ngroups, int kn,
                                                       double *__restrict__ out) {
-    __shared__ double red[2][8][33];
+    __shared__ double red[PLANES][8][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int c = blockIdx.x * 32 + tx;
-    const int g0 = blockIdx.y * BN_CHUNK, g1 = min(g0 + BN_CHUNK, ngroups);
-    double s = 0.0, q = 0.0;
-    if (c < kn)
-        for (int g = g0 + ty; g < g1; g += 8) {
-            s += (double) __ldg(part + (size_t) g * 2 * kn + c);
-            q += (double) __ldg(part + (size_t) g * 2 * kn + kn + c);
+    const int g0 = blockIdx.y * BN_CHUNK;
+    double s[PLANES] = {};
+    if (c < kn) {
+        float v[PLANES][BN_CHUNK / 8];   // all loads in flight, added in order
+#pragma unroll
+        for (int j = 0; j < BN_CHUNK / 8; j++) {
+            const int g = g0 + ty + 8 * j;
+#pragma unroll
+            for (int p = 0; p < PLANES; p++) v[p][j] = g < ngroups ? __ldg(part + ((size_t) g * 2 + p) * kn + c) : 0.0f;
         }
-    red[0][ty][tx] = s;
-    red[1][ty][tx] = q;
+#pragma unroll
+        for (int j = 0; j < BN_CHUNK / 8; j++)
+#pragma unroll
+            for (int p = 0; p < PLANES; p++) s[p] += widen(v[p][j]);
+    }
+#pragma unroll
+    for (int p = 0; p < PLANES; p++) red[p][ty][tx] = s[p];
     __syncthreads();
-    if (ty < 2 && c < kn) {
+    if (ty < PLANES && c < kn) {
         double a = 0.0;
         for (int r = 0; r < 8; r++) a += red[ty][r][tx];
         out[(size_t) blockIdx.y * 2 * kn + (size_t) ty * kn + c] = a;
     }
 }
 
-// Pass 2: stats[0][c] = sum, stats[1][c] = sum of squares, over the chunks in order.
-__global__ void bn_stats_pass2(const double *__restrict__ chunks, int nchunks, int kn, double *__restrict__ stats) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 2 * kn) return;
+// Pass 2, block = 32 columns: the chunks in order, eight thread rows strided over them, then the rows in
+// order. Returns the total to thread row 0.
+__device__ __forceinline__ double chunk_total(const double *__restrict__ chunks, int nchunks, int stride, int i, bool in) {
+    __shared__ double red[8][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     double a = 0.0;
-    for (int j = 0; j < nchunks; j++) a += chunks[(size_t) j * 2 * kn + i];
-    stats[i] = a;
+    if (in) {
+        int j = ty;
+        for (; j + 56 < nchunks; j += 64) {   // eight loads in flight, added in order
+            double v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = chunks[(size_t) (j + 8 * k) * stride + i];
+#pragma unroll
+            for (int k = 0; k < 8; k++) a += v[k];
+        }
+        for (; j < nchunks; j += 8) a += chunks[(size_t) j * stride + i];
+    }
+    red[ty][tx] = a;
+    __syncthreads();
+    a = 0.0;
+    if (ty == 0)
+        for (int r = 0; r < 8; r++) a += red[r][tx];
+    return a;
+}
+// stats[0][c] = sum, stats[1][c] = sum of squares.
+__global__ void __launch_bounds__(256) bn_stats_pass2(const double *__restrict__ chunks, int nchunks, int kn, double *__restrict__ stats) {
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+    const double a = chunk_total(chunks, nchunks, 2 * kn, i, i < 2 * kn);
+    if (threadIdx.x < 32 && i < 2 * kn) stats[i] = a;
 }
 
-// Column sums in FP32 from the chunk sums of pass 1: out[c] = sum over the chunks, in order,
-// of the first statistics plane.
-__global__ void colsum_pass2_f32(const double *__restrict__ chunks, int nchunks, int kn, float *__restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= kn) return;
-    double a = 0.0;
-    for (int j = 0; j < nchunks; j++) a += chunks[(size_t) j * 2 * kn + c];
-    out[c] = (float) a;
+// Column sums in FP32: out[c] = sum over the chunks of the first statistics plane.
+__global__ void __launch_bounds__(256) colsum_pass2_f32(const double *__restrict__ chunks, int nchunks, int kn, float *__restrict__ out) {
+    const int c = blockIdx.x * 32 + (threadIdx.x & 31);
+    const double a = chunk_total(chunks, nchunks, 2 * kn, c, c < kn);
+    if (threadIdx.x < 32 && c < kn) out[c] = (float) a;
 }
 
 __global__ void bn_fold_kernel(int kn, const double *__restrict__ stats, double inv_count, const float *gamma,
@@ -134,9 +170,9 @@ cudaError_t cg_colsum_reduce(void *workspace, int ngroups, int kn, float *out, c
     double *chunks = (double *) workspace;
     const float *part = (const float *) ((uint8_t *) workspace + (size_t) nchunks * 2 * kn * 8);
     dim3 g1((kn + 31) / 32, nchunks);
-    bn_stats_pass1<<<g1, 256, 0, st>>>(part, ngroups, kn, chunks);
+    bn_stats_pass1<1><<<g1, 256, 0, st>>>(part, ngroups, kn, chunks);
     cg_note_launch();
-    colsum_pass2_f32<<<(kn + 127) / 128, 128, 0, st>>>(chunks, nchunks, kn, out);
+    colsum_pass2_f32<<<(kn + 31) / 32, 256, 0, st>>>(chunks, nchunks, kn, out);
     cg_note_launch();
     return cudaGetLastError();
 }
@@ -181,9 +217,9 @@ extern "C" convgemm_status_t convgemm_fwd_bf16_stats(const convgemm_shape_t *sha
     }
     if (e) return e;
     dim3 g1((s.kn + 31) / 32, nchunks);
-    bn_stats_pass1<<<g1, 256, 0, st>>>(part, ng, s.kn, chunks);
+    bn_stats_pass1<2><<<g1, 256, 0, st>>>(part, ng, s.kn, chunks);
     cg_note_launch();
-    bn_stats_pass2<<<(2 * s.kn + 127) / 128, 128, 0, st>>>(chunks, nchunks, s.kn, stats);
+    bn_stats_pass2<<<(2 * s.kn + 31) / 32, 256, 0, st>>>(chunks, nchunks, s.kn, stats);
     cg_note_launch();
     return cg_cuda_check(cudaGetLastError(), "batch statistics reduction");
 }

@@ -8,6 +8,8 @@
 #include "prep.h"
 #include "tc_ptx.cuh"
 
+#include <algorithm>
+
 namespace {
 
 using bf16 = __nv_bfloat16;
@@ -116,6 +118,94 @@ __global__ void to_bf16_nhwc_kernel(const float *__restrict__ in, int nchw, int 
     }
 }
 
+__device__ __forceinline__ uint32_t bf16x2_of(float a, float b) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+__device__ __forceinline__ uint4 bf16x8_of(const float (&v)[8]) {
+    return make_uint4(bf16x2_of(v[0], v[1]), bf16x2_of(v[2], v[3]), bf16x2_of(v[4], v[5]), bf16x2_of(v[6], v[7]));
+}
+
+// The same cast for 16-byte aligned outputs. All three forms are HBM-bound and store whole
+// 16-byte groups of eight channels; the element form above divides per element, reads NCHW planes with
+// one value per lane and line, and ran at 1.0 TB/s (64 x 3 x 224 x 224: 87 us) to 1.5 TB/s.
+//
+// NCHW with c <= 8: a thread reads its pixel from every plane (neighbouring lanes, neighbouring pixels).
+__global__ void __launch_bounds__(256) nchw_few_to_bf16_kernel(const float *__restrict__ in, int C, long long HW, long long P,
+                                                               uint4 *__restrict__ out) {
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < P; i += gridDim.x * 256LL) {
+        const float *src = in + i / HW * C * HW + i % HW;
+        float v[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) v[c] = c < C ? __ldg(src + c * HW) : 0.0f;
+        out[i] = bf16x8_of(v);
+    }
+}
+
+// NCHW: 64 channels x 64 pixels per block through shared memory; planes read along the pixels (16-byte
+// vectors when HW % 4 == 0 and the input is aligned), pixels written along the channels.
+__global__ void __launch_bounds__(256) nchw_tiled_to_bf16_kernel(const float *__restrict__ in, int C, int HW, int Cp, int vec,
+                                                                 uint4 *__restrict__ out) {
+    __shared__ float t[64][65];
+    const int q0 = blockIdx.x * 64, c0 = blockIdx.y * 64, tid = threadIdx.x;
+    const float *src = in + (size_t) blockIdx.z * C * HW;
+    if (vec) {
+        float4 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int c = c0 + tid / 16 + 16 * k, q = q0 + 4 * (tid % 16);
+            v[k] = c < C && q < HW ? __ldg(reinterpret_cast<const float4 *>(src + (size_t) c * HW + q))
+                                   : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            float *o = &t[tid / 16 + 16 * k][4 * (tid % 16)];
+            o[0] = v[k].x;
+            o[1] = v[k].y;
+            o[2] = v[k].z;
+            o[3] = v[k].w;
+        }
+    } else {
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            const int c = c0 + tid / 64 + 4 * k, q = q0 + tid % 64;
+            v[k] = c < C && q < HW ? __ldg(src + (size_t) c * HW + q) : 0.0f;
+        }
+#pragma unroll
+        for (int k = 0; k < 16; k++) t[tid / 64 + 4 * k][tid % 64] = v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int q = tid / 8 + 32 * k, g = tid % 8;   // pixel, group of eight channels
+        if (q0 + q >= HW || c0 + 8 * g >= Cp) continue;
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = t[8 * g + j][q];
+        out[(((size_t) blockIdx.z * HW + q0 + q) * Cp + c0) / 8 + g] = bf16x8_of(v);
+    }
+}
+
+// NHWC: eight channels of a pixel per thread.
+__global__ void __launch_bounds__(256) nhwc_to_bf16_kernel(const float *__restrict__ in, int C, int Cp, long long n8, int vec,
+                                                           uint4 *__restrict__ out) {
+    const int k8 = Cp / 8;
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n8; i += gridDim.x * 256LL) {
+        float v[8];
+        if (vec) {   // C % 8 == 0, 16-byte aligned
+            const float4 a = __ldg(reinterpret_cast<const float4 *>(in) + 2 * i), b = __ldg(reinterpret_cast<const float4 *>(in) + 2 * i + 1);
+            v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        } else {
+            const long long pix = i / k8;
+            const int c = (int) (i - pix * k8) * 8;
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[j] = c + j < C ? __ldg(in + pix * C + c + j) : 0.0f;
+        }
+        out[i] = bf16x8_of(v);
+    }
+}
+
 // ------------------------------------------------------ FP8 and 3xBF16 forms
 constexpr float E4M3_MAX = 448.0f;
 
@@ -123,28 +213,82 @@ __device__ __forceinline__ uint8_t to_e4m3(float v) {
     return (uint8_t) __nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
 }
 
-// amax (as the bit pattern of a non-negative float, so atomicMax on unsigned orders it)
-__global__ void amax_kernel(const void *__restrict__ in, int in_bf16, long long n, unsigned *amax_bits) {
-    float m = 0.0f;
-    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
-        const float v = in_bf16 ? __bfloat162float(((const bf16 *) in)[i]) : ((const float *) in)[i];
-        m = fmaxf(m, fabsf(v));
+// Eight consecutive values from element 8 * i, both input types; 16-byte aligned.
+template <bool BF>
+__device__ __forceinline__ void load8(const void *in, long long i, float (&v)[8]) {
+    if (BF) {
+        const uint4 u = __ldg(reinterpret_cast<const uint4 *>(in) + i);
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            v[2 * j] = __uint_as_float(w[j] << 16);
+            v[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
+        }
+    } else {
+        const float4 a = __ldg(reinterpret_cast<const float4 *>(in) + 2 * i), b = __ldg(reinterpret_cast<const float4 *>(in) + 2 * i + 1);
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
     }
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(amax_bits, __float_as_uint(m));
+}
+template <bool BF>
+__device__ __forceinline__ float load1(const void *in, long long i) {
+    return BF ? __bfloat162float(((const bf16 *) in)[i]) : ((const float *) in)[i];
 }
 
-// per-tensor scale = amax / 448 (1 for an all-zero tensor); x_q = e4m3(x / scale)
-__global__ void quant_e4m3_kernel(const void *__restrict__ in, int in_bf16, long long n, const unsigned *amax_bits,
-                                  uint8_t *__restrict__ out, float *scale_out) {
+// amax (as the bit pattern of a non-negative float, so atomicMax on unsigned orders it). One atomic
+// per block: one per warp, 39k of them on one word, took longer than the reads (25 M values: 28 us).
+// n8: groups of eight read as vectors (0 when `in` is not 16-byte aligned).
+template <bool BF>
+__global__ void __launch_bounds__(256) amax_kernel(const void *__restrict__ in, long long n8, long long n, unsigned *amax_bits) {
+    __shared__ float red[8];
+    const long long step = gridDim.x * 256LL, i0 = blockIdx.x * 256LL + threadIdx.x;
+    float m = 0.0f;
+    long long i = i0;
+    for (; i + 3 * step < n8; i += 4 * step) {
+        float v[4][8];
+#pragma unroll
+        for (int k = 0; k < 4; k++) load8<BF>(in, i + k * step, v[k]);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) m = fmaxf(m, fabsf(v[k][j]));
+    }
+    for (; i < n8; i += step) {
+        float v[8];
+        load8<BF>(in, i, v);
+#pragma unroll
+        for (int j = 0; j < 8; j++) m = fmaxf(m, fabsf(v[j]));
+    }
+    for (long long k = 8 * n8 + i0; k < n; k += step) m = fmaxf(m, fabsf(load1<BF>(in, k)));
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 1; k < 8; k++) m = fmaxf(m, red[k]);
+        atomicMax(amax_bits, __float_as_uint(m));
+    }
+}
+
+// per-tensor scale = amax / 448 (1 for an all-zero tensor); x_q = e4m3(x / scale). Eight values per
+// thread and 8-byte stores where input (16) and output (8) are aligned (n8 as above).
+template <bool BF>
+__global__ void __launch_bounds__(256) quant_e4m3_kernel(const void *__restrict__ in, long long n8, long long n,
+                                                         const unsigned *amax_bits, uint8_t *__restrict__ out, float *scale_out) {
     const float amax = __uint_as_float(*amax_bits);
     const float sc = amax > 0.0f ? amax / E4M3_MAX : 1.0f;
     const float inv = 1.0f / sc;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = sc;
-    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
-        const float v = in_bf16 ? __bfloat162float(((const bf16 *) in)[i]) : ((const float *) in)[i];
-        out[i] = to_e4m3(v * inv);
+    const long long step = gridDim.x * 256LL, i0 = blockIdx.x * 256LL + threadIdx.x;
+    if (i0 == 0) *scale_out = sc;
+    for (long long i = i0; i < n8; i += step) {
+        float v[8];
+        load8<BF>(in, i, v);
+        uint32_t q[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            q[j] = __nv_cvt_float2_to_fp8x2(make_float2(v[2 * j] * inv, v[2 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
+        reinterpret_cast<uint2 *>(out)[i] = make_uint2(q[0] | q[1] << 16, q[2] | q[3] << 16);
     }
+    for (long long i = 8 * n8 + i0; i < n; i += step) out[i] = to_e4m3(load1<BF>(in, i) * inv);
 }
 
 // per-output-channel weight scale (NHWC-API weights [K][kn]: threads along co, loop over K)
@@ -179,9 +323,20 @@ __global__ void fp8_scales_kernel(int kn, const float *scale, const float *shift
     out_shift[n] = shift ? shift[n] : 0.0f;
 }
 
-// x = hi + lo with hi = bf16(x), lo = bf16(x - hi)
-__global__ void split_kernel(const float *__restrict__ in, long long n, bf16 *__restrict__ hi, bf16 *__restrict__ lo) {
-    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
+// x = hi + lo with hi = bf16(x), lo = bf16(x - hi); n8: groups of eight as 16-byte vectors (0 when a
+// tensor is not 16-byte aligned).
+__global__ void __launch_bounds__(256) split_kernel(const float *__restrict__ in, long long n8, long long n, bf16 *__restrict__ hi,
+                                                    bf16 *__restrict__ lo) {
+    const long long step = gridDim.x * 256LL, i0 = blockIdx.x * 256LL + threadIdx.x;
+    for (long long i = i0; i < n8; i += step) {
+        float v[8], r[8];
+        load8<false>(in, i, v);
+#pragma unroll
+        for (int j = 0; j < 8; j++) r[j] = v[j] - __bfloat162float(__float2bfloat16_rn(v[j]));
+        reinterpret_cast<uint4 *>(hi)[i] = bf16x8_of(v);
+        reinterpret_cast<uint4 *>(lo)[i] = bf16x8_of(r);
+    }
+    for (long long i = 8 * n8 + i0; i < n; i += step) {
         const float v = in[i];
         const bf16 h = __float2bfloat16_rn(v);
         hi[i] = h;
@@ -292,15 +447,24 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
             }
             return;
         }
-        case PREP_FWD_ELEM: {
-            // block = (row co, 256 columns of K): 32-bit index math, no division by the row length
-            const int nch = (J.Kpad + 255) / 256;
-            const int co = lb / nch, k = (lb % nch) * 256 + t;
-            if (k >= J.Kpad) return;
-            const int tap = k / J.Cp, ci = k - tap * J.Cp;
-            float v = 0.0f;
-            if (tap < J.kh * J.kw && ci < J.C) v = wref(J.w, J.nchw, J.C, J.kh, J.kw, J.kn, ci, tap / J.kw, tap % J.kw, co);
-            ((bf16 *) J.out)[(size_t) co * J.Kpad + k] = __float2bfloat16_rn(v);
+        case PREP_FWD_NCHW: {
+            // NCHW-API weights [co][ci][tap] -> out[co][tap*Cp + ci]: block = (row co, a chunk of its
+            // input channels), the chunk read contiguously into shared memory and written tap by tap
+            // (gathering single values from a stride of taps: 60 us for 512 x 512 x 3 x 3 with the
+            // input-gradient operand, 8 us staged)
+            const int khw = J.kh * J.kw, CH = prep_nchw_channels(khw), Cp = J.Cp, Kpad = J.Kpad, nch = (Cp + CH - 1) / CH;
+            const int co = lb / nch, ci0 = (lb % nch) * CH, n = min(CH, Cp - ci0);
+            float *buf = &tile[0][0];
+            const float *src = J.w + ((size_t) co * J.C + ci0) * khw;
+            const int have = max(0, min(n, J.C - ci0)) * khw;
+#pragma unroll 4
+            for (int i = t; i < n * khw; i += 256) buf[i] = i < have ? __ldg(src + i) : 0.0f;
+            __syncthreads();
+            bf16 *row = (bf16 *) J.out + (size_t) co * Kpad;
+            for (int tap = 0; tap < khw; tap++)
+                for (int ci = t; ci < n; ci += 256) row[tap * Cp + ci0 + ci] = __float2bfloat16_rn(buf[ci * khw + tap]);
+            if (ci0 == 0)
+                for (int k = khw * Cp + t; k < Kpad; k += 256) row[k] = __float2bfloat16_rn(0.0f);
             return;
         }
         case PREP_FWD_TAIL: {
@@ -309,6 +473,35 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
             if (i >= J.kn * width) return;
             const int co = i / width;
             ((bf16 *) J.out)[(size_t) co * J.Kpad + kbeg + (i - co * width)] = __float2bfloat16_rn(0.0f);
+            return;
+        }
+        case PREP_DGRAD_NCHW: {
+            // NCHW-API weights [co][ci][tap]: block = (4 input channels, one class, a run of output
+            // channels): the run's 4 x taps values, contiguous per output channel, staged through shared
+            // memory (odd pitch) and written along co
+            const int khw = J.kh * J.kw, Ktot = J.info.Ktot, knp = J.knp, C = J.C;
+            const int run = prep_nchw_run(khw), nrun = (knp + run - 1) / run;
+            const int c = (lb / nrun) % J.info.ncls, ci0 = lb / nrun / J.info.ncls * 4, co0 = lb % nrun * run;
+            const int beg = J.info.kbeg[c], end = c + 1 < J.info.ncls ? J.info.kbeg[c + 1] : Ktot;
+            const int nt = J.info.ntaps[c], nci = min(4, C - ci0), w4 = nci * khw, pitch = (4 * khw) | 1, nco = min(run, knp - co0);
+            float *buf = &tile[0][0];
+            __shared__ int taps[TC_MAXTAPS];
+            if (t < nt) taps[t] = J.info.kx[c][t] * J.kw + J.info.ky[c][t];
+            const float *src = J.w + ((size_t) co0 * C + ci0) * khw;
+            const int have = J.kn - co0;
+            for (int i = t; i < nco * w4; i += 256) {
+                const int co = i / w4, k = i - co * w4;
+                buf[co * pitch + k] = co < have ? __ldg(src + (size_t) co * C * khw + k) : 0.0f;
+            }
+            __syncthreads();
+            bf16 *dst = (bf16 *) J.out + (size_t) ci0 * Ktot + beg + co0;
+            for (int i = t; i < nci * nt * nco; i += 256) {
+                const int q = i / nco, co = i - q * nco, r = q / nt, g = q - r * nt;
+                dst[(size_t) r * Ktot + g * knp + co] = __float2bfloat16_rn(buf[co * pitch + r * khw + taps[g]]);
+            }
+            if (co0 == 0)   // the K padding after the class's taps
+                for (int r = 0; r < nci; r++)
+                    for (int k = nt * knp + t; k < end - beg; k += 256) dst[(size_t) r * Ktot + k] = __float2bfloat16_rn(0.0f);
             return;
         }
         default: {   // PREP_DGRAD: block = (4 input channels, one stride-phase class): the class's
@@ -396,7 +589,19 @@ cudaError_t prep_fold(int kn, const float *bias, const float *mean, const float 
 
 cudaError_t prep_to_bf16_nhwc(const float *in, int nchw, int B, int C, int H, int W, int Cp, void *out,
                               cudaStream_t st) {
-    to_bf16_nhwc_kernel<<<grid_for((long long) B * H * W * Cp), 256, 0, st>>>(in, nchw, B, C, H, W, Cp, (bf16 *) out); cg_note_launch();
+    const long long HW = (long long) H * W, P = B * HW;
+    const bool vin = ((uintptr_t) in & 15) == 0;
+    if ((uintptr_t) out & 15 || HW > (1LL << 30) || B > 65535 || Cp > 64 * 65535) {
+        to_bf16_nhwc_kernel<<<grid_for(P * Cp), 256, 0, st>>>(in, nchw, B, C, H, W, Cp, (bf16 *) out);
+    } else if (!nchw) {
+        nhwc_to_bf16_kernel<<<grid_for(P * (Cp / 8)), 256, 0, st>>>(in, C, Cp, P * (Cp / 8), vin && C == Cp, (uint4 *) out);
+    } else if (C <= 8) {
+        nchw_few_to_bf16_kernel<<<grid_for(P), 256, 0, st>>>(in, C, HW, P, (uint4 *) out);
+    } else {
+        const dim3 grid((unsigned) ((HW + 63) / 64), (unsigned) ((Cp + 63) / 64), (unsigned) B);
+        nchw_tiled_to_bf16_kernel<<<grid, 256, 0, st>>>(in, C, (int) HW, Cp, vin && HW % 4 == 0, (uint4 *) out);
+    }
+    cg_note_launch();
     return cudaGetLastError();
 }
 
@@ -404,8 +609,15 @@ cudaError_t prep_fp8_quantize(long long n, int in_bf16, const void *in, void *ou
                               cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(amax_tmp, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
-    amax_kernel<<<grid_for(n), 256, 0, st>>>(in, in_bf16, n, amax_tmp); cg_note_launch();
-    quant_e4m3_kernel<<<grid_for(n), 256, 0, st>>>(in, in_bf16, n, amax_tmp, (uint8_t *) out, scale); cg_note_launch();
+    const long long na = ((uintptr_t) in & 15) == 0 ? n / 8 : 0, nq = ((uintptr_t) out & 7) == 0 ? na : 0;
+    const int ga = (int) std::min<long long>(grid_for(na ? na : n), 152 * 8), gq = grid_for(nq ? nq : n);
+    if (in_bf16) {
+        amax_kernel<true><<<ga, 256, 0, st>>>(in, na, n, amax_tmp); cg_note_launch();
+        quant_e4m3_kernel<true><<<gq, 256, 0, st>>>(in, nq, n, amax_tmp, (uint8_t *) out, scale); cg_note_launch();
+    } else {
+        amax_kernel<false><<<ga, 256, 0, st>>>(in, na, n, amax_tmp); cg_note_launch();
+        quant_e4m3_kernel<false><<<gq, 256, 0, st>>>(in, nq, n, amax_tmp, (uint8_t *) out, scale); cg_note_launch();
+    }
     return cudaGetLastError();
 }
 
@@ -424,7 +636,8 @@ cudaError_t prep_fp8_scales(int kn, const float *scale, const float *shift, cons
 }
 
 cudaError_t prep_split(long long n, const float *in, void *hi, void *lo, cudaStream_t st) {
-    split_kernel<<<grid_for(n), 256, 0, st>>>(in, n, (bf16 *) hi, (bf16 *) lo); cg_note_launch();
+    const long long n8 = (((uintptr_t) in | (uintptr_t) hi | (uintptr_t) lo) & 15) == 0 ? n / 8 : 0;
+    split_kernel<<<grid_for(n8 ? n8 : n), 256, 0, st>>>(in, n8, n, (bf16 *) hi, (bf16 *) lo); cg_note_launch();
     return cudaGetLastError();
 }
 

@@ -1047,8 +1047,9 @@ extern "C" convgemm_status_t convgemm_prep_prepare(int n, const convgemm_prep_it
             f.out = it.packed_fwd;
             const int khw = s.kh * s.kw;
             if (j.nchw) {
-                f.type = PREP_FWD_ELEM;
-                add(f, (long long) s.kn * ((f.Kpad + 255) / 256));
+                f.type = PREP_FWD_NCHW;
+                const int ch = prep_nchw_channels(khw);
+                add(f, (long long) s.kn * ((f.Cp + ch - 1) / ch));
             } else {
                 f.type = PREP_FWD_TILED;
                 add(f, (long long) khw * ((f.Cp + 63) / 64) * ((s.kn + 63) / 64));
@@ -1066,12 +1067,13 @@ extern "C" convgemm_status_t convgemm_prep_prepare(int n, const convgemm_prep_it
                 return cg_set_error(CONVGEMM_ERROR_NOT_SUPPORTED, "%s: item %d: more than 16 stride-phase classes", fn, i);
             if (pl.Ktot > 0) {
                 PrepJob f = j;
-                f.type = PREP_DGRAD;
+                f.type = j.nchw ? PREP_DGRAD_NCHW : PREP_DGRAD;
                 f.knp = pl.Cin;
                 f.info = tc_pack_info(pl);
                 f.dknp = FastDiv((uint32_t) f.knp);
                 f.out = it.packed_dgrad;
-                add(f, (long long) ((s.c + 3) / 4) * f.info.ncls);
+                const int run = prep_nchw_run(s.kh * s.kw);
+                add(f, (long long) ((s.c + 3) / 4) * f.info.ncls * (j.nchw ? (f.knp + run - 1) / run : 1));
             }
         }
         if (blocks > (1LL << 31) - 1) return cg_set_error(CONVGEMM_ERROR_NOT_SUPPORTED, "%s: too many blocks", fn);
