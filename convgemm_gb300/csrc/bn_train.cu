@@ -21,12 +21,12 @@ namespace {
 
 constexpr int BN_CHUNK = CG_STAT_CHUNK;
 
-// Pass 1: block (x = 32 channels, y = a chunk of BN_CHUNK groups) sums its groups for
-// its channels in FP64, the 8 thread rows strided over the chunk, then in a fixed
+// Pass 1: block (x = 8 channels, y = a chunk of BN_CHUNK groups) sums its groups for
+// its channels in FP64, the 32 thread rows strided over the chunk, then in a fixed
 // order across the rows.  part: [ngroups][2][kn] FP32; out: [nchunks][2][kn] FP64 (PLANES = 1: the
-// sums alone). FP64 additions and conversions bound it (two per cycle and SM), so chunks are
-// small enough for every SM to have some (chunks of 256 groups left 56 blocks for 7168 groups x 64
-// channels: 22 us), and the conversions are done on the integer pipe (17 us with them on the FP64 pipe).
+// sums alone). FP64 arithmetic bounds it, so blocks are narrow enough for every SM to have some (32
+// channels wide, 7168 groups x 64 channels made 56 blocks: 22 us), and the conversions are done on the
+// integer pipe (17 us with them on the FP64 pipe, 12 us so).
 __device__ __forceinline__ double widen(float f) {   // (double) f
     const uint32_t u = __float_as_uint(f), e = u >> 23 & 255;
     if (e - 1u < 254u) return __hiloint2double((int) ((u & 0x80000000u) | ((u & 0x7FFFFFFFu) >> 3) + 0x38000000u), (int) (u << 29));
@@ -35,21 +35,21 @@ __device__ __forceinline__ double widen(float f) {   // (double) f
 template <int PLANES>
 __global__ void __launch_bounds__(256) bn_stats_pass1(const float *__restrict__ part, int ngroups, int kn,
                                                       double *__restrict__ out) {
-    __shared__ double red[PLANES][8][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int c = blockIdx.x * 32 + tx;
+    __shared__ double red[PLANES][32][9];
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    const int c = blockIdx.x * 8 + tx;
     const int g0 = blockIdx.y * BN_CHUNK;
     double s[PLANES] = {};
     if (c < kn) {
-        float v[PLANES][BN_CHUNK / 8];   // all loads in flight, added in order
+        float v[PLANES][BN_CHUNK / 32];   // all loads in flight, added in order
 #pragma unroll
-        for (int j = 0; j < BN_CHUNK / 8; j++) {
-            const int g = g0 + ty + 8 * j;
+        for (int j = 0; j < BN_CHUNK / 32; j++) {
+            const int g = g0 + ty + 32 * j;
 #pragma unroll
             for (int p = 0; p < PLANES; p++) v[p][j] = g < ngroups ? __ldg(part + ((size_t) g * 2 + p) * kn + c) : 0.0f;
         }
 #pragma unroll
-        for (int j = 0; j < BN_CHUNK / 8; j++)
+        for (int j = 0; j < BN_CHUNK / 32; j++)
 #pragma unroll
             for (int p = 0; p < PLANES; p++) s[p] += widen(v[p][j]);
     }
@@ -58,7 +58,8 @@ __global__ void __launch_bounds__(256) bn_stats_pass1(const float *__restrict__ 
     __syncthreads();
     if (ty < PLANES && c < kn) {
         double a = 0.0;
-        for (int r = 0; r < 8; r++) a += red[ty][r][tx];
+#pragma unroll
+        for (int r = 0; r < 32; r++) a += red[ty][r][tx];
         out[(size_t) blockIdx.y * 2 * kn + (size_t) ty * kn + c] = a;
     }
 }
@@ -169,7 +170,7 @@ cudaError_t cg_colsum_reduce(void *workspace, int ngroups, int kn, float *out, c
     const int nchunks = (ngroups + BN_CHUNK - 1) / BN_CHUNK;
     double *chunks = (double *) workspace;
     const float *part = (const float *) ((uint8_t *) workspace + (size_t) nchunks * 2 * kn * 8);
-    dim3 g1((kn + 31) / 32, nchunks);
+    dim3 g1((kn + 7) / 8, nchunks);
     bn_stats_pass1<1><<<g1, 256, 0, st>>>(part, ngroups, kn, chunks);
     cg_note_launch();
     colsum_pass2_f32<<<(kn + 31) / 32, 256, 0, st>>>(chunks, nchunks, kn, out);
@@ -216,7 +217,7 @@ extern "C" convgemm_status_t convgemm_fwd_bf16_stats(const convgemm_shape_t *sha
         e = tc_run(pl, s, x, wpacked, y, scale, shift, relu, st, 0, nullptr, nullptr, t.bn, t.splits, nullptr, part);
     }
     if (e) return e;
-    dim3 g1((s.kn + 31) / 32, nchunks);
+    dim3 g1((s.kn + 7) / 8, nchunks);
     bn_stats_pass1<2><<<g1, 256, 0, st>>>(part, ng, s.kn, chunks);
     cg_note_launch();
     bn_stats_pass2<<<(2 * s.kn + 31) / 32, 256, 0, st>>>(chunks, nchunks, s.kn, stats);

@@ -38,7 +38,7 @@ cudaError_t cg_fp32_dgrad(int nchw, const cg_shape &s, const float *w, const flo
 // workspace + the chunk bytes); out[c] = the sum of plane 0 over the groups, in FP32.
 size_t cg_colsum_ws_bytes(long long ngroups, int kn);
 cudaError_t cg_colsum_reduce(void *workspace, int ngroups, int kn, float *out, cudaStream_t st);
-constexpr int CG_STAT_CHUNK = 64;   // statistics groups per block of the first pass (bn_train.cu)
+constexpr int CG_STAT_CHUNK = 256;   // statistics groups per block of the first pass (bn_train.cu)
 inline size_t cg_colsum_part_offset(long long ngroups, int kn) {
     return (size_t) ((ngroups + CG_STAT_CHUNK - 1) / CG_STAT_CHUNK) * 2 * kn * 8;
 }
