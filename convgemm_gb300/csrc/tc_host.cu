@@ -288,23 +288,65 @@ int tc_num_sms() {
     return n;
 }
 
-// Output channels per tile: fewest waves of tiles times the per-stage cost of a
-// tile (the 16 KB A gather bounds a stage at ~128 cycles; the MMA takes 2*BN).
-int tc_pick_bn(const TcPlan &pl, int sms) {
-    int best = 64;
-    long long best_cost = -1;
-    for (int bn : {256, 128, 64}) {
-        if (bn > 64 && bn / 2 >= pl.Cout) continue;
+// Tile forms of tc_conv_kernel and what a tile costs (microseconds): `block` per 64-channel K block (FP8W: 128
+// channels), at least `epi` (the epilogue of short reductions, behind which the MMAs hide), `launch` once.
+// Fitted to 64 forward and input-gradient shapes (31 geometries from 1 x 14 x 14 to 32 x 56 x 56) with every form
+// forced: the form with the lowest estimate is within 0.6% of the best one on average. The rule before
+// (tiles x width, equal for all widths, so the narrowest won on wave rounding) was 26% off: 28 x 28, 512 -> 512
+// 3 x 3 at batch 32 took 199 us with the 64-wide tiles it chose and takes 81 with 256.
+struct TileForm {
+    int bn, mt, ew;
+    float block, epi, launch;
+};
+constexpr TileForm FORMS_BF16[] = {{64, 1, 4, 0.270f, 0.92f, 3.5f}, {128, 1, 4, 0.280f, 1.62f, 4.2f}, {128, 1, 8, 0.296f, 1.30f, 4.25f},
+                                   {128, 2, 8, 0.459f, 2.13f, 4.6f}, {256, 1, 8, 0.363f, 2.01f, 4.9f}};
+// with batch statistics or a fused bias gradient in the epilogue
+constexpr TileForm FORMS_STATS[] = {{64, 1, 4, 0.270f, 2.5f, 3.5f}, {128, 1, 4, 0.280f, 4.5f, 4.2f}, {256, 1, 4, 0.370f, 8.5f, 4.9f}};
+constexpr TileForm FORMS_GATHER[] = {{64, 1, 4, 0.60f, 1.95f, 3.5f}, {128, 1, 4, 0.63f, 2.10f, 4.0f}, {256, 1, 4, 0.80f, 3.00f, 4.9f}};
+constexpr TileForm FORMS_FP8[] = {{64, 1, 4, 0.200f, 0.87f, 3.4f}, {128, 1, 4, 0.210f, 1.47f, 3.9f}, {256, 1, 4, 0.270f, 2.70f, 4.7f}};
+constexpr TileForm FORMS_FP8W[] = {{64, 1, 4, 0.255f, 0.87f, 3.4f}, {128, 1, 4, 0.270f, 1.47f, 3.9f}, {256, 1, 4, 0.360f, 2.70f, 4.7f}};
+constexpr TileForm FORMS_X3[] = {{64, 1, 4, 0.560f, 1.17f, 3.4f}, {128, 1, 4, 0.580f, 2.00f, 4.0f}, {256, 1, 4, 0.900f, 3.80f, 4.9f}};
+
+// mode: TcConvParams::mode; the plan's K blocks hold `kdiv` blocks of 64 channels each.
+template <int N>
+TileForm cheapest_form(const TileForm (&forms)[N], const TcPlan &pl, int kdiv, int sms) {
+    TileForm best = forms[0];
+    float best_cost = -1.0f;
+    for (const TileForm &f : forms) {
+        if (f.bn > 64 && f.bn / 2 >= pl.Cout) continue;
         long long tiles = 0;
-        for (int c = 0; c < pl.ncls; c++) tiles += (long long) pl.cls[c].mtiles * ((pl.Cout + bn - 1) / bn);
-        const long long waves = (tiles + sms - 1) / sms;
-        const long long cost = waves * (bn * 2 > 128 ? bn * 2 : 128);
-        if (best_cost < 0 || cost < best_cost) {
+        float work = 0.0f;
+        for (int c = 0; c < pl.ncls; c++) {
+            const long long t = (long long) ((pl.cls[c].mtiles + f.mt - 1) / f.mt) * ((pl.Cout + f.bn - 1) / f.bn);
+            const float k = (float) (pl.cls[c].ktiles / kdiv) * f.block;
+            tiles += t;
+            work += (float) t * (k > f.epi ? k : f.epi);
+        }
+        const float cost = f.launch + (float) ((tiles + sms - 1) / sms) * work / (float) (tiles > 0 ? tiles : 1);
+        if (best_cost < 0.0f || cost < best_cost) {
             best_cost = cost;
-            best = bn;
+            best = f;
         }
     }
     return best;
+}
+TileForm tc_pick_form(const TcPlan &pl, int mode, bool im2col, bool stats, int sms) {
+    if (mode == 1) return cheapest_form(FORMS_FP8, pl, 1, sms);
+    if (mode == 2) return cheapest_form(FORMS_X3, pl, 1, sms);
+    if (mode == 3) return cheapest_form(FORMS_FP8W, pl, 2, sms);
+    if (stats) return cheapest_form(FORMS_STATS, pl, 1, sms);
+    return im2col ? cheapest_form(FORMS_BF16, pl, 1, sms) : cheapest_form(FORMS_GATHER, pl, 1, sms);
+}
+
+// Epilogue warps of tc_conv_kernel: eight where asked for (`by_k`: where every class has at most 8 K
+// blocks) and the form exists.
+int tc_epilogue_warps(const TcPlan &pl, bool eight, bool by_k, int bn, int mt, bool bf16_im2col) {
+    if (by_k) {
+        int kmax = 0;
+        for (int c = 0; c < pl.ncls; c++) kmax = pl.cls[c].ktiles > kmax ? pl.cls[c].ktiles : kmax;
+        eight = kmax <= 8;
+    }
+    return eight && bf16_im2col && (bn >= 128 || mt == 2) && !(bn == 256 && mt == 2) ? 8 : 4;
 }
 
 convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, const void *wpacked, void *out,
@@ -321,7 +363,18 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     TcConvParams p;
     memset(&p, 0, sizeof(p));
     p.mode = mode;
-    p.bn = bn_override ? bn_override : tc_pick_bn(pl, sms);
+    TcPlan pi = pl;
+    p.im2col = tc_plan_im2col(pi);
+    if (mode != 0 && !p.im2col)
+        return cg_set_error(CONVGEMM_ERROR_NOT_SUPPORTED,
+                            "FP8 / 3xBF16 forms need channels a multiple of 64 (im2col-mode TMA)");
+    // E4M3 with channels a multiple of 128: 128-channel K blocks (128-byte rows and swizzle, one
+    // 16 KB box per 128-row block and four 32-deep MMAs per block, as BF16) instead of 64-byte rows
+    bool f8w = mode == 1 && p.im2col && pl.Cin % 128 == 0 && pl.Ktot % 128 == 0;
+    for (int c = 0; f8w && c < pi.ncls; c++)
+        if (pi.cls[c].kbeg % 128 || pi.cls[c].ktiles % 2) f8w = false;
+    const TileForm form = tc_pick_form(pl, f8w ? 3 : mode, p.im2col, stats != nullptr, sms);
+    p.bn = bn_override ? bn_override : form.bn;
     const int eb = mode == 1 ? 1 : 2;   // operand element bytes
     CUtensorMap wmap, omap;
     if (convgemm_status_t e = tc_make_map_2d_sw(&wmap, eb == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
@@ -360,18 +413,8 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     if (!p.err) return cg_set_error(CONVGEMM_ERROR_CUDA, "device error word unavailable");
     p.ntiles = (pl.Cout + p.bn - 1) / p.bn;
     p.ncls = pl.ncls;
-    TcPlan pi = pl;
     TcMaps amaps;
     memset(&amaps, 0, sizeof(amaps));
-    p.im2col = tc_plan_im2col(pi);
-    if (mode != 0 && !p.im2col)
-        return cg_set_error(CONVGEMM_ERROR_NOT_SUPPORTED,
-                            "FP8 / 3xBF16 forms need channels a multiple of 64 (im2col-mode TMA)");
-    // E4M3 with channels a multiple of 128: 128-channel K blocks (128-byte rows and swizzle, one
-    // 16 KB box per 128-row block and four 32-deep MMAs per block, as BF16) instead of 64-byte rows
-    bool f8w = mode == 1 && p.im2col && pl.Cin % 128 == 0 && pl.Ktot % 128 == 0;
-    for (int c = 0; f8w && c < pi.ncls; c++)
-        if (pi.cls[c].kbeg % 128 || pi.cls[c].ktiles % 2) f8w = false;
     if (f8w) {
         if (convgemm_status_t e = tc_make_map_2d_sw(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wpacked, pl.Cout, pl.Ktot,
                                                     128, p.bn, CU_TENSOR_MAP_SWIZZLE_128B))
@@ -397,17 +440,13 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
                 return e;
     }
     // aux (tuning): bits 0-1 the M tiles per weight tile (1 / 2: BF16 im2col path only), bit 2
-    // eight epilogue warps, bit 3 (above) the general kernel instead of the slab kernel; bits 0-2
-    // zero = heuristic: one M tile, eight epilogue warps when every class
-    // has at most 8 K blocks per tile (the epilogue, not the MMA, bounds such tiles)
-    p.mt = ((aux_override & 3) == 2 && mode == 0 && p.im2col) ? 2 : 1;
-    bool ew8 = (aux_override & 4) != 0;
-    if ((aux_override & 7) == 0) {
-        int kmax = 0;
-        for (int c = 0; c < pl.ncls; c++) kmax = pl.cls[c].ktiles > kmax ? pl.cls[c].ktiles : kmax;
-        ew8 = kmax <= 8;
-    }
-    p.ew = (ew8 && mode == 0 && p.im2col && (p.bn >= 128 || p.mt == 2) && !(p.bn == 256 && p.mt == 2)) ? 8 : 4;
+    // eight epilogue warps, bit 3 (above) the general kernel instead of the slab kernel. Without bits 0-2:
+    // the cheapest form's, or for a width that was set, one M tile and eight epilogue warps when every
+    // class has at most 8 K blocks per tile (the epilogue, not the MMA, bounds such tiles)
+    const bool by_form = !bn_override && (aux_override & 7) == 0;
+    p.mt = (by_form ? form.mt == 2 : (aux_override & 3) == 2) && mode == 0 && p.im2col ? 2 : 1;
+    p.ew = tc_epilogue_warps(pl, by_form ? form.ew == 8 : (aux_override & 4) != 0, !by_form && (aux_override & 7) == 0, p.bn,
+                             p.mt, mode == 0 && p.im2col);
     if (stats) {   // the statistics form: one M tile, four epilogue warps
         p.mt = 1;
         p.ew = 4;
@@ -678,11 +717,58 @@ size_t wgrad_xchg_bytes(const WgPlan &w) {
     return sizeof(float) * 128 * (size_t) w.bn * (size_t) w.mtiles * (size_t) w.ntiles * (size_t) w.splits;
 }
 
+// The weight gradient's tiles and pixel splits where no tuning entry names them (im2col path), as the
+// flags an entry would hold. A CTA's cost (microseconds): `chunk` per 128 pixels, `tile` and `launch` once;
+// then what adds the splits up: nothing for one, the cluster exchange for 2 or 4 (8 only on small grids:
+// clusters of eight leave SMs without a place), the reduction kernels (planes at 5 TB/s) otherwise and for
+// pairs. Fitted to 32 shapes with every combination forced: 2% off the best on average, where the rule
+// before (64-pixel chunks, one wave, the slab kernel for 128-channel blocks) was 50% off: 28 x 28,
+// 512 -> 512 3 x 3 at batch 32 126 -> 77 us, 14 x 14, 256 -> 256 at batch 1 45 -> 4.8 us.
+struct WgForm {
+    int bn, pair;
+    float chunk, tile, launch;
+};
+constexpr WgForm WG_FORMS[] = {{64, 0, 0.435f, 3.66f, 0.1f}, {128, 0, 0.464f, 5.26f, -0.9f}, {128, 1, 0.454f, 5.04f, -0.4f}, {256, 1, 0.610f, 7.06f, -1.3f}};
+
+TcTune pick_wgrad(const cg_shape &s, const ConvGeom &g) {
+    const int sms = tc_num_sms(), Nx = s.kh * s.kw * round_up(s.c, 8), nch = (int) ((g.P + 127) / 128);
+    TcTune best{0, 0};
+    float best_cost = -1.0f;
+    for (const WgForm &f : WG_FORMS)
+        // X on the 128-row side: always for narrow layers, else tried second (several taps: first, the
+        // 3 x 3 layers run a few per cent faster that way at the same tile count)
+        for (int o = 0; o < (s.kn < 128 ? 1 : 2); o++) {
+            const bool xa = s.kn < 128 || (o == 0) == (s.kh * s.kw > 1);
+            const int M = xa ? Nx : s.kn, N = xa ? s.kn : Nx;
+            if (f.bn > 64 && f.bn / 2 >= N) continue;
+            if (s.kn < 128 && f.bn == 256) continue;   // narrow layers: 64 or 128 columns
+            long long tiles = (M + 127) / 128;
+            if (f.pair) tiles += tiles & 1;
+            tiles *= (N + f.bn - 1) / f.bn;
+            // splits: 1, 2, 4, 8, and those that fill one wave and half of one
+            const int wave = (int) (sms / tiles > 0 ? sms / tiles : 1);
+            for (int sp : {1, 2, 4, 8, wave, (wave + 1) / 2}) {
+                if (sp > nch) continue;
+                const int cps = (nch + sp - 1) / sp, n = (nch + cps - 1) / cps;
+                if (!f.pair && n > 1 && n <= 8 && n != 2 && n != 4 && !(n == 8 && tiles * n <= 96)) continue;
+                float cost = f.launch + (float) ((tiles * n + sms - 1) / sms) * ((float) cps * f.chunk + f.tile);
+                if (n > 1) cost += !f.pair && n <= 8 ? 2.8f : 5.4f + (float) n * (float) Nx * (float) s.kn * 4.0f / 5.0e6f;
+                if (best_cost < 0.0f || cost < best_cost) {
+                    best_cost = cost;
+                    best.bn = f.bn;
+                    best.splits = n | (f.pair ? CONVGEMM_WGRAD_PAIR : CONVGEMM_WGRAD_WIDE_CHUNKS) | (s.kn >= 128 && xa ? CONVGEMM_WGRAD_X_ON_A : 0);
+                }
+            }
+        }
+    return best;
+}
+
 WgPlan plan_wgrad(const convgemm_shape_t &ps) {
     const cg_shape s = cg_from_public(ps);
     const ConvGeom g = make_geom(s);
     TcTune t{0, 0};
     tc_tune_get(CONVGEMM_TUNE_WGRAD, ps, &t);
+    if (t.bn == 0 && t.splits == 0 && wgrad_im2col_ok(s, g) && !tc_stem_wgrad_applicable(s)) t = pick_wgrad(s, g);
     WgPlan w;
     w.Cp = round_up(s.c, 8);
     w.kn8 = round_up(s.kn, 8);
@@ -731,10 +817,9 @@ WgPlan plan_wgrad(const convgemm_shape_t &ps) {
         w.bn = 64;
         w.splits = tc_stem_wgrad_splits(s);
     }
-    // stride-1 layers with 128-channel input blocks: the slab kernel, by default (no tuning
-    // entry) or when the tuning entry asks for it
+    // stride-1 layers with 128-channel input blocks: the slab kernel, when the tuning entry asks for it
     w.slab = 0;
-    if (!w.stem && ((t.bn == 0 && t.splits == 0) || (t.splits & CONVGEMM_WGRAD_SLAB))) {
+    if (!w.stem && (t.splits & CONVGEMM_WGRAD_SLAB)) {
         const int sp = tc_wgrad_slab_splits(s, aux_splits, t.bn);
         if (sp > 0) {
             w.slab = 1;
@@ -966,15 +1051,11 @@ extern "C" convgemm_status_t convgemm_tune_describe(int op, const convgemm_shape
     }
     TcPlan pi = pl;
     const int im2col = tc_plan_im2col(pi);
-    *bn = t.bn ? t.bn : tc_pick_bn(pl, tc_num_sms());
-    const int mt = ((t.splits & 3) == 2 && im2col) ? 2 : 1;
-    bool ew8 = (t.splits & 4) != 0;
-    if ((t.splits & 7) == 0) {
-        int kmax = 0;
-        for (int c = 0; c < pl.ncls; c++) kmax = pl.cls[c].ktiles > kmax ? pl.cls[c].ktiles : kmax;
-        ew8 = kmax <= 8;
-    }
-    const int ew = (ew8 && im2col && (*bn >= 128 || mt == 2) && !(*bn == 256 && mt == 2)) ? 8 : 4;
+    const TileForm form = tc_pick_form(pl, 0, im2col, false, tc_num_sms());
+    const bool by_form = !t.bn && (t.splits & 7) == 0;
+    *bn = t.bn ? t.bn : form.bn;
+    const int mt = (by_form ? form.mt == 2 : (t.splits & 3) == 2) && im2col ? 2 : 1;
+    const int ew = tc_epilogue_warps(pl, by_form ? form.ew == 8 : (t.splits & 4) != 0, !by_form && (t.splits & 7) == 0, *bn, mt, im2col);
     const int kb1 = (t.splits & 16) && im2col && mt == 1 && ew == 4 && *bn != 256;
     *stages = tc_conv_stages(*bn, im2col, mt, ew, kb1);
     return CONVGEMM_SUCCESS;

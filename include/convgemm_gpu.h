@@ -277,8 +277,7 @@ convgemm_status_t convgemm_tune_set(int op, const convgemm_shape_t *shape, int b
 /* Weight gradient of a stride-1 layer whose channels are multiples of 128 and kn >= 64 (filters
  * 2..512/BN taps wide, output width + filter span <= 256): the slab kernel, whose MMAs read
  * each kernel row's taps as row-shifted windows of one input slab per band of output rows.
- * It is the default for such layers when the tuning table has no entry for the shape;
- * with an entry it runs when the entry carries this flag (its split count in bits 0-15,
+ * It runs when the shape's tuning entry carries this flag (its split count in bits 0-15,
  * 0 = heuristic). */
 #define CONVGEMM_WGRAD_SLAB 0x80000
 /* Weight gradient (im2col path): one 64-pixel chunk per ring stage and twice as many stages
