@@ -14,10 +14,12 @@
 //   k = tap * Cin + ci over the class's taps (64 per pipeline stage).
 // A comes straight from the NHWC activation into the 128-byte-swizzled K-major
 // layout the tensor core reads: by im2col-mode TMA (128 pixels x 64 channels of
-// one tap per load, out-of-range taps zero-filled) when the channels come in
-// blocks of 64, else by 16-byte cp.async gathers, zero-filled for padding — no
-// im2row buffer exists anywhere.  B is the packed weight matrix [Cout][K]
-// loaded by TMA.  The FP32 accumulator lives in TMEM.
+// one tap per load, out-of-range taps and channels zero-filled), or by 16-byte
+// cp.async gathers, zero-filled for padding, where channels are so few that
+// whole K blocks per tap would mostly be zeros — no im2row buffer exists
+// anywhere.  B is the packed weight matrix [Cout][K] loaded by TMA (as
+// (channel, tap, Cout) boxes where a tap's last K block is partly zeros).  The
+// FP32 accumulator lives in TMEM.
 //
 // The kernel is persistent: each CTA walks tiles blockIdx.x, +gridDim.x, ...
 // with two TMEM accumulators, so the epilogue of one tile runs while the MMAs
@@ -264,14 +266,15 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                         for (int mt = 0; mt < MT; mt++)
                             tc::tma_load_im2col_4d(ab + mt * C::A_BLOCK, am, ci0, w0[mt], h0[mt], bb0[mt], offx, offy,
                                                    &full[s]);
-                        tc::tma_load_2d(bb, &wmap, kcol, tl.n0, &full[s]);
+                        if (MODE == MODE_BF16 && p.wtail) tc::tma_load_3d(bb, &amaps.w[tl.cls], ci0, tap, tl.n0, &full[s]);
+                        else tc::tma_load_2d(bb, &wmap, kcol, tl.n0, &full[s]);
                         if (MODE == MODE_X3) {
                             tc::tma_load_im2col_4d(ab + C::A_TILE, &amaps.alo[tl.cls], ci0, w0[0], h0[0], bb0[0], offx,
                                                    offy, &full[s]);
                             tc::tma_load_2d(bb + C::B_TILE, &amaps.wlo, kcol, tl.n0, &full[s]);
                         }
                         ci0 += C::BK;
-                        if (ci0 == p.Cin) {
+                        if (ci0 >= p.Cin) {
                             ci0 = 0;
                             tap++;
                         }

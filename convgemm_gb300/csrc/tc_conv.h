@@ -47,8 +47,9 @@ struct TcConvParams {
     int ntiles;                // tiles along the output channels
     int ntiles_total;          // all tiles of all classes; tile t of a class: m = t / ntiles, n = t % ntiles
     int epi_tma;               // output pixels are the GEMM rows in order: stage in SMEM, TMA store
-    int im2col;                // A loaded by im2col-mode TMA (Cin % 64 == 0), else gathered by cp.async
-    int cpb;                   // 64-channel chunks per tap (Cin / 64) on the im2col path
+    int im2col;                // A loaded by im2col-mode TMA, else gathered by cp.async
+    int wtail;                 // im2col with Cin % 64 != 0: the classes count ceil(Cin / 64) K blocks per tap, the
+                               // last one's channels past Cin zero-filled by both operands' loads (TcMaps::w)
     int mode;                  // 0 BF16, 1 FP8-E4M3, 2 3xBF16 (FP32 output)
     int mt;                    // 128-row M tiles per tile (1, or 2 sharing each weight tile: BF16 im2col only)
     int ew;                    // epilogue warps: 4, or 8 (BF16 im2col, bn >= 128 or mt == 2, not bn 256 with mt 2)
@@ -64,6 +65,7 @@ struct TcMaps {
     CUtensorMap a[TC_MAXIM2COL];    // im2col maps of the gathered tensor, one per class
     CUtensorMap alo[TC_MAXIM2COL];  // 3xBF16: maps of the low parts
     CUtensorMap wlo;                // 3xBF16: packed low parts of the weights
+    CUtensorMap w[TC_MAXIM2COL];    // wtail: packed weights of a class as (channel, tap, output channel)
 };
 
 // wmap: packed weights [Cout][K] (box 64 x bn); omap: output [pixels][Cout] (box 64 x 128), used when epi_tma.

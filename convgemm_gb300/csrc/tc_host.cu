@@ -113,9 +113,9 @@ convgemm_status_t tc_make_im2col_map(CUtensorMap *map, const void *ptr, int B, i
 }
 
 // Fills the im2col fields of the plan's classes; false when some class cannot use
-// im2col-mode TMA (channels not a multiple of 64, too many classes, corners beyond +-128).
+// im2col-mode TMA (too many classes, corners beyond +-128).
 bool tc_plan_im2col(TcPlan &pl) {
-    if (pl.Cin % 64 || pl.ncls > TC_MAXIM2COL || pl.ncls < 1) return false;
+    if (pl.ncls > TC_MAXIM2COL || pl.ncls < 1) return false;
     for (int c = 0; c < pl.ncls; c++) {
         TcClass &cl = pl.cls[c];
         int my = 1 << 30, mx = 1 << 30, Xy = -(1 << 30), Xx = -(1 << 30);
@@ -307,9 +307,9 @@ constexpr TileForm FORMS_FP8[] = {{64, 1, 4, 0.200f, 0.87f, 3.4f}, {128, 1, 4, 0
 constexpr TileForm FORMS_FP8W[] = {{64, 1, 4, 0.255f, 0.87f, 3.4f}, {128, 1, 4, 0.270f, 1.47f, 3.9f}, {256, 1, 4, 0.360f, 2.70f, 4.7f}};
 constexpr TileForm FORMS_X3[] = {{64, 1, 4, 0.560f, 1.17f, 3.4f}, {128, 1, 4, 0.580f, 2.00f, 4.0f}, {256, 1, 4, 0.900f, 3.80f, 4.9f}};
 
-// mode: TcConvParams::mode; the plan's K blocks hold `kdiv` blocks of 64 channels each.
+// The plan's K blocks hold `kdiv` blocks of 64 channels each; *cost_out: the form's estimate.
 template <int N>
-TileForm cheapest_form(const TileForm (&forms)[N], const TcPlan &pl, int kdiv, int sms) {
+TileForm cheapest_form(const TileForm (&forms)[N], const TcPlan &pl, int kdiv, int sms, float *cost_out = nullptr) {
     TileForm best = forms[0];
     float best_cost = -1.0f;
     for (const TileForm &f : forms) {
@@ -328,8 +328,38 @@ TileForm cheapest_form(const TileForm (&forms)[N], const TcPlan &pl, int kdiv, i
             best = f;
         }
     }
+    if (cost_out) *cost_out = best_cost;
     return best;
 }
+
+// Whether the BF16 kernel loads the gathered operand by im2col TMA (pl's classes then count whole 64-channel K
+// blocks per tap). With channels in blocks of 64 always. Else each tap's last block is padded with zeros and
+// rows straddle cache lines, which makes a block TAIL_COST times as expensive, but still cheaper than one gathered
+// by threads (0.6 us against 0.27 for 64-wide tiles): it pays unless the blocks are mostly padding.
+// 14 x 14, 328 -> 200 3 x 3, batch 32 (54 blocks for 47): 31.7 -> 23.1 us; 56 x 56, 104 -> 312 1 x 1, batch 24 (2 for 2):
+// 44 -> 20 us; 28 x 28, 72 -> 72 3 x 3, batch 64 (18 for 11): 26.4 gathered, 42.8 by TMA. The rule depends on the
+// plan alone, so that every form of a layer adds its products in the same order.
+constexpr float TAIL_COST = 1.55f;
+bool tc_use_im2col(TcPlan &pl, int sms) {
+    TcPlan pi = pl;
+    if (!tc_plan_im2col(pi)) return false;
+    if (pl.Cin % 64) {
+        TileForm forms[sizeof(FORMS_BF16) / sizeof(FORMS_BF16[0])];
+        for (size_t i = 0; i < sizeof(forms) / sizeof(forms[0]); i++) {
+            forms[i] = FORMS_BF16[i];
+            forms[i].block *= TAIL_COST;
+        }
+        for (int c = 0; c < pi.ncls; c++) pi.cls[c].ktiles = pi.cls[c].ntaps * ((pl.Cin + 63) / 64);
+        float by_tma, gathered;
+        cheapest_form(forms, pi, 1, sms, &by_tma);
+        cheapest_form(FORMS_GATHER, pl, 1, sms, &gathered);
+        if (gathered < by_tma) return false;
+    }
+    pl = pi;
+    return true;
+}
+
+// mode: TcConvParams::mode.
 TileForm tc_pick_form(const TcPlan &pl, int mode, bool im2col, bool stats, int sms) {
     if (mode == 1) return cheapest_form(FORMS_FP8, pl, 1, sms);
     if (mode == 2) return cheapest_form(FORMS_X3, pl, 1, sms);
@@ -364,7 +394,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     memset(&p, 0, sizeof(p));
     p.mode = mode;
     TcPlan pi = pl;
-    p.im2col = tc_plan_im2col(pi);
+    p.im2col = mode == 0 ? tc_use_im2col(pi, sms) : pl.Cin % 64 == 0 && tc_plan_im2col(pi);
     if (mode != 0 && !p.im2col)
         return cg_set_error(CONVGEMM_ERROR_NOT_SUPPORTED,
                             "FP8 / 3xBF16 forms need channels a multiple of 64 (im2col-mode TMA)");
@@ -373,7 +403,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     bool f8w = mode == 1 && p.im2col && pl.Cin % 128 == 0 && pl.Ktot % 128 == 0;
     for (int c = 0; f8w && c < pi.ncls; c++)
         if (pi.cls[c].kbeg % 128 || pi.cls[c].ktiles % 2) f8w = false;
-    const TileForm form = tc_pick_form(pl, f8w ? 3 : mode, p.im2col, stats != nullptr, sms);
+    const TileForm form = tc_pick_form(pi, f8w ? 3 : mode, p.im2col, stats != nullptr, sms);
     p.bn = bn_override ? bn_override : form.bn;
     const int eb = mode == 1 ? 1 : 2;   // operand element bytes
     CUtensorMap wmap, omap;
@@ -421,9 +451,16 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
             return e;
     }
     if (p.im2col) {
-        p.cpb = pl.Cin / 64;
+        p.wtail = pl.Cin % 64 != 0;
         for (int c = 0; c < pi.ncls; c++) {
             const TcClass &cl = pi.cls[c];
+            if (p.wtail) {
+                const unsigned long long dims[3] = {(unsigned long long) pl.Cin, (unsigned long long) cl.ntaps, (unsigned long long) pl.Cout};
+                const unsigned long long str[2] = {(unsigned long long) pl.Cin * 2, (unsigned long long) pl.Ktot * 2};
+                const unsigned box[3] = {64, 1, (unsigned) p.bn}, estr[3] = {1, 1, 1};
+                if (convgemm_status_t e = tc_make_map_nd(&amaps.w[c], 3, (const uint16_t *) wpacked + cl.kbeg, dims, str, box, estr, 1))
+                    return e;
+            }
             const int up_y = cl.lo_y + (cl.Hg - 1) * cl.isy - (pl.Hin - 1);
             const int up_x = cl.lo_x + (cl.Wg - 1) * cl.isx - (pl.Win - 1);
             if (convgemm_status_t e = tc_make_im2col_map(&amaps.a[c], in, s.b, pl.Hin, pl.Win, pl.Cin, cl.lo_y,
@@ -445,7 +482,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     // class has at most 8 K blocks per tile (the epilogue, not the MMA, bounds such tiles)
     const bool by_form = !bn_override && (aux_override & 7) == 0;
     p.mt = (by_form ? form.mt == 2 : (aux_override & 3) == 2) && mode == 0 && p.im2col ? 2 : 1;
-    p.ew = tc_epilogue_warps(pl, by_form ? form.ew == 8 : (aux_override & 4) != 0, !by_form && (aux_override & 7) == 0, p.bn,
+    p.ew = tc_epilogue_warps(pi, by_form ? form.ew == 8 : (aux_override & 4) != 0, !by_form && (aux_override & 7) == 0, p.bn,
                              p.mt, mode == 0 && p.im2col);
     if (stats) {   // the statistics form: one M tile, four epilogue warps
         p.mt = 1;
@@ -704,11 +741,14 @@ struct WgPlan {
     size_t ws_bytes;
 };
 
-// Whether the weight gradient gathers X with im2col TMA (channels in 64-element atoms,
-// padding and far-edge offsets within the im2col map's signed 8-bit corners).
+// Whether the weight gradient gathers X with im2col TMA (padding and far-edge offsets within the im2col map's
+// signed 8-bit corners). Channels that are no multiple of 64 are padded to one with zeros by the loads; up to
+// 8 channels, nearly all padding, the cp.async gathers run instead. 14 x 14, 200 -> 328 3 x 3, batch 32: 52 us
+// gathered, 26 padded; 23 x 25, 24 -> 304, batch 1: 20 and 7 us; 37 x 45, 72 -> 136 stride 2, batch 12: 20 and 13 us
+// (28 x 28, 72 -> 72, batch 64, where the second block of every tap is nearly empty: 37.5 and 39.6).
 bool wgrad_im2col_ok(const cg_shape &s, const ConvGeom &g) {
     const int up_h = -s.vpad + (g.ho - 1) * s.vstride - (s.h - 1), up_w = -s.hpad + (g.wo - 1) * s.hstride - (s.w - 1);
-    return (round_up(s.c, 8) % 64) == 0 && s.vpad <= 128 && s.hpad <= 128 && up_h >= -128 && up_h <= 127 &&
+    return s.c > 8 && s.vpad <= 128 && s.hpad <= 128 && up_h >= -128 && up_h <= 127 &&
            up_w >= -128 && up_w <= 127 && s.vstride <= 8 && s.hstride <= 8;
 }
 
@@ -731,7 +771,7 @@ struct WgForm {
 constexpr WgForm WG_FORMS[] = {{64, 0, 0.435f, 3.66f, 0.1f}, {128, 0, 0.464f, 5.26f, -0.9f}, {128, 1, 0.454f, 5.04f, -0.4f}, {256, 1, 0.610f, 7.06f, -1.3f}};
 
 TcTune pick_wgrad(const cg_shape &s, const ConvGeom &g) {
-    const int sms = tc_num_sms(), Nx = s.kh * s.kw * round_up(s.c, 8), nch = (int) ((g.P + 127) / 128);
+    const int sms = tc_num_sms(), Nx = s.kh * s.kw * round_up(s.c, 64), nch = (int) ((g.P + 127) / 128);
     TcTune best{0, 0};
     float best_cost = -1.0f;
     for (const WgForm &f : WG_FORMS)
@@ -770,10 +810,10 @@ WgPlan plan_wgrad(const convgemm_shape_t &ps) {
     tc_tune_get(CONVGEMM_TUNE_WGRAD, ps, &t);
     if (t.bn == 0 && t.splits == 0 && wgrad_im2col_ok(s, g) && !tc_stem_wgrad_applicable(s)) t = pick_wgrad(s, g);
     WgPlan w;
-    w.Cp = round_up(s.c, 8);
+    const bool im2col = wgrad_im2col_ok(s, g);
+    w.Cp = round_up(s.c, im2col ? 64 : 8);
     w.kn8 = round_up(s.kn, 8);
     w.Nx = s.kh * s.kw * w.Cp;
-    const bool im2col = wgrad_im2col_ok(s, g);
     const int aux_splits = t.splits & 0xffff;
     w.pair = im2col && (t.splits & CONVGEMM_WGRAD_PAIR) ? 1 : 0;
     w.wide = im2col && (w.pair || (t.splits & CONVGEMM_WGRAD_WIDE_CHUNKS)) ? 1 : 0;
@@ -933,10 +973,10 @@ extern "C" convgemm_status_t convgemm_wgrad_bf16(convgemm_layout_t layout, const
         p.im2col = wgrad_im2col_ok(s, g);
         p.x2d = w.x2d;
         if (p.x2d) {
-            if (convgemm_status_t e = tc_make_map_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, g.P, p.Cp, 64, w.bk))
+            if (convgemm_status_t e = tc_make_map_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, g.P, round_up(s.c, 8), 64, w.bk))
                 return e;
         } else if (p.im2col) {
-            if (convgemm_status_t e = tc_make_im2col_map(&xmap, x, s.b, s.h, s.w, p.Cp, -s.vpad, -s.hpad, up_h, up_w,
+            if (convgemm_status_t e = tc_make_im2col_map(&xmap, x, s.b, s.h, s.w, round_up(s.c, 8), -s.vpad, -s.hpad, up_h, up_w,
                                                          s.vstride, s.hstride, w.bk, 2, 64))
                 return e;
         }
@@ -1049,8 +1089,7 @@ extern "C" convgemm_status_t convgemm_tune_describe(int op, const convgemm_shape
         *bn = 64;
         return CONVGEMM_SUCCESS;
     }
-    TcPlan pi = pl;
-    const int im2col = tc_plan_im2col(pi);
+    const int im2col = tc_use_im2col(pl, tc_num_sms());
     const TileForm form = tc_pick_form(pl, 0, im2col, false, tc_num_sms());
     const bool by_form = !t.bn && (t.splits & 7) == 0;
     *bn = t.bn ? t.bn : form.bn;
