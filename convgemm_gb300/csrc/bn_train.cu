@@ -32,27 +32,32 @@ __device__ __forceinline__ double widen(float f) {   // (double) f
     if (e - 1u < 254u) return __hiloint2double((int) ((u & 0x80000000u) | ((u & 0x7FFFFFFFu) >> 3) + 0x38000000u), (int) (u << 29));
     return (u << 1) == 0 ? __hiloint2double((int) u, 0) : (double) f;   // zero; subnormal, infinite, NaN
 }
-template <int PLANES>
-__global__ void __launch_bounds__(256) bn_stats_pass1(const float *__restrict__ part, int ngroups, int kn,
-                                                      double *__restrict__ out) {
+// With one chunk of all groups (at most BN_ONE_PASS: a few batches of loads per thread) its sums are the
+// result, and the second kernel is not needed: OUT double writes them like the chunk sums, OUT float the
+// first plane's.
+constexpr int BN_ONE_PASS = 1024;
+template <int PLANES, class OUT>
+__global__ void __launch_bounds__(256) bn_stats_pass1(const float *__restrict__ part, int ngroups, int chunk, int kn,
+                                                      OUT *__restrict__ out) {
     __shared__ double red[PLANES][32][9];
     const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
     const int c = blockIdx.x * 8 + tx;
-    const int g0 = blockIdx.y * BN_CHUNK;
+    const int g1 = min(ngroups, (int) (blockIdx.y + 1) * chunk);
     double s[PLANES] = {};
-    if (c < kn) {
-        float v[PLANES][BN_CHUNK / 32];   // all loads in flight, added in order
+    if (c < kn)
+        for (int g0 = blockIdx.y * chunk; g0 < g1; g0 += BN_CHUNK) {
+            float v[PLANES][BN_CHUNK / 32];   // eight groups in flight, added in order
 #pragma unroll
-        for (int j = 0; j < BN_CHUNK / 32; j++) {
-            const int g = g0 + ty + 32 * j;
+            for (int j = 0; j < BN_CHUNK / 32; j++) {
+                const int g = g0 + ty + 32 * j;
 #pragma unroll
-            for (int p = 0; p < PLANES; p++) v[p][j] = g < ngroups ? __ldg(part + ((size_t) g * 2 + p) * kn + c) : 0.0f;
+                for (int p = 0; p < PLANES; p++) v[p][j] = g < g1 ? __ldg(part + ((size_t) g * 2 + p) * kn + c) : 0.0f;
+            }
+#pragma unroll
+            for (int j = 0; j < BN_CHUNK / 32; j++)
+#pragma unroll
+                for (int p = 0; p < PLANES; p++) s[p] += widen(v[p][j]);
         }
-#pragma unroll
-        for (int j = 0; j < BN_CHUNK / 32; j++)
-#pragma unroll
-            for (int p = 0; p < PLANES; p++) s[p] += widen(v[p][j]);
-    }
 #pragma unroll
     for (int p = 0; p < PLANES; p++) red[p][ty][tx] = s[p];
     __syncthreads();
@@ -60,7 +65,7 @@ __global__ void __launch_bounds__(256) bn_stats_pass1(const float *__restrict__ 
         double a = 0.0;
 #pragma unroll
         for (int r = 0; r < 32; r++) a += red[ty][r][tx];
-        out[(size_t) blockIdx.y * 2 * kn + (size_t) ty * kn + c] = a;
+        out[(size_t) blockIdx.y * 2 * kn + (size_t) ty * kn + c] = (OUT) a;
     }
 }
 
@@ -170,8 +175,13 @@ cudaError_t cg_colsum_reduce(void *workspace, int ngroups, int kn, float *out, c
     const int nchunks = (ngroups + BN_CHUNK - 1) / BN_CHUNK;
     double *chunks = (double *) workspace;
     const float *part = (const float *) ((uint8_t *) workspace + (size_t) nchunks * 2 * kn * 8);
+    if (ngroups <= BN_ONE_PASS) {
+        bn_stats_pass1<1, float><<<(kn + 7) / 8, 256, 0, st>>>(part, ngroups, BN_ONE_PASS, kn, out);
+        cg_note_launch();
+        return cudaGetLastError();
+    }
     dim3 g1((kn + 7) / 8, nchunks);
-    bn_stats_pass1<1><<<g1, 256, 0, st>>>(part, ngroups, kn, chunks);
+    bn_stats_pass1<1, double><<<g1, 256, 0, st>>>(part, ngroups, BN_CHUNK, kn, chunks);
     cg_note_launch();
     colsum_pass2_f32<<<(kn + 31) / 32, 256, 0, st>>>(chunks, nchunks, kn, out);
     cg_note_launch();
@@ -217,11 +227,16 @@ extern "C" convgemm_status_t convgemm_fwd_bf16_stats(const convgemm_shape_t *sha
         e = tc_run(pl, s, x, wpacked, y, scale, shift, relu, st, 0, nullptr, nullptr, t.bn, t.splits, nullptr, part);
     }
     if (e) return e;
-    dim3 g1((s.kn + 7) / 8, nchunks);
-    bn_stats_pass1<2><<<g1, 256, 0, st>>>(part, ng, s.kn, chunks);
-    cg_note_launch();
-    bn_stats_pass2<<<(2 * s.kn + 31) / 32, 256, 0, st>>>(chunks, nchunks, s.kn, stats);
-    cg_note_launch();
+    if (ng <= BN_ONE_PASS) {
+        bn_stats_pass1<2, double><<<(s.kn + 7) / 8, 256, 0, st>>>(part, ng, BN_ONE_PASS, s.kn, stats);
+        cg_note_launch();
+    } else {
+        dim3 g1((s.kn + 7) / 8, nchunks);
+        bn_stats_pass1<2, double><<<g1, 256, 0, st>>>(part, ng, BN_CHUNK, s.kn, chunks);
+        cg_note_launch();
+        bn_stats_pass2<<<(2 * s.kn + 31) / 32, 256, 0, st>>>(chunks, nchunks, s.kn, stats);
+        cg_note_launch();
+    }
     return cg_cuda_check(cudaGetLastError(), "batch statistics reduction");
 }
 

@@ -42,6 +42,11 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 
+// What the epilogue does beside scale, shift and ReLU (BF16 forms): nothing (or adding into the output);
+// masking by the activation of a ReLU; column sums of its output, masked when a mask is given (input
+// gradient); column sums of its output and of the squares (forward).
+constexpr int EXTRA_NONE = 0, EXTRA_MASK = 1, EXTRA_SUMS = 2, EXTRA_STATS = 3;
+
 // Operand forms of the kernel.
 constexpr int MODE_BF16 = 0;  // BF16 x BF16, kind::f16
 constexpr int MODE_FP8 = 1;   // E4M3 x E4M3, kind::f8f6f4 (64-byte K rows, 64-byte swizzle)
@@ -78,11 +83,12 @@ struct TcCfg {
     // MMA run ahead of the arrivals (LAG = STAGES - 1 would lock the two in step)
     static constexpr int LAG = STAGES / 2;
     // shared tables: tap offsets, the class table, scale/shift (whole vectors up to 1024 channels)
+    static constexpr size_t BAR_BYTES = 512;                   // mbarriers
     static constexpr size_t TAB_BYTES = TC_MAXCLS * TC_MAXTAPS * 4 + TC_MAXCLS * 128 + 2 * 1024 * 4;
     // output staging buffers: two when they fit beside the stage ring, else one
     static constexpr int EPI_BUFS =
-        (1024 + (size_t) STAGES * STAGE_BYTES + 2 * EPI_BYTES + 256 + TAB_BYTES <= 232448) ? 2 : 1;
-    static constexpr size_t SMEM = 1024 + (size_t) STAGES * STAGE_BYTES + EPI_BUFS * EPI_BYTES + 256 + TAB_BYTES;
+        (1024 + (size_t) STAGES * STAGE_BYTES + 2 * EPI_BYTES + BAR_BYTES + TAB_BYTES <= 232448) ? 2 : 1;
+    static constexpr size_t SMEM = 1024 + (size_t) STAGES * STAGE_BYTES + EPI_BUFS * EPI_BYTES + BAR_BYTES + TAB_BYTES;
     static_assert(SMEM <= 232448, "shared memory above the 227 KB per-block limit");
     static_assert(EW == 4 || EW == 8, "four or eight epilogue warps");
     // warps: 0 producer (0-3 on the cp.async path), 4..4+EW-1 epilogue, the MMA issuer in
@@ -103,9 +109,9 @@ __device__ __forceinline__ uint64_t op_desc(uint32_t saddr, uint32_t sbo, uint32
     return d | ((uint64_t) layout << 61);
 }
 
-__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t *>(&v);
+// 0xFFFF in each half where the BF16 value is positive (not zero, not NaN).
+__device__ __forceinline__ uint32_t positive_mask(uint32_t v) {
+    return __hgt2_mask(*reinterpret_cast<const __nv_bfloat162 *>(&v), __floats2bfloat162_rn(0.0f, 0.0f));
 }
 
 template <int N>
@@ -147,12 +153,19 @@ __device__ __forceinline__ Tile decode_tile(const ClsS *cls, int ncls, int ntile
     return tl;
 }
 
-template <int BN, int STAGES, int KB, bool IM2C, int MODE, int MT, int EW, bool STATS>
+template <int BN, int STAGES, int KB, bool IM2C, int MODE, int MT, int EW, int EXTRA>
 __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
     tc_conv_kernel(const __grid_constant__ TcConvParams p, const __grid_constant__ CUtensorMap wmap,
                    const __grid_constant__ CUtensorMap omap, const __grid_constant__ TcMaps amaps) {
     using C = TcCfg<BN, STAGES, KB, MODE, MT, EW>;
-    static_assert(EW == 4 || (IM2C && MT * C::NCH >= 2), "eight epilogue warps: im2col path, two chunks or more");
+    static_assert(EW == 4 || IM2C, "eight epilogue warps: im2col path");
+    static_assert(EXTRA == EXTRA_NONE || (MODE == MODE_BF16 && C::EPI_BUFS == 2), "masks and sums: BF16, two staging buffers");
+    // items of a tile: (accumulator mt, 64-column chunk). Eight warps: the two warps of a TMEM lane quarter
+    // take alternate items, or alternate tiles where a tile has one item (each tile's accumulator is then
+    // released by four warps)
+    constexpr int NIT = MT * C::NCH;
+    constexpr bool ALT = EW == 8 && NIT == 1;
+    constexpr int STEP = ALT ? 1 : EW / 4, TSTEP = ALT ? 2 : 1;
     // Two MMA-issuing threads on the BF16 im2col path: one per M tile (MT = 2), or one per N half
     // (MT = 1, BN >= 128).  One thread's instruction stream issues N <= 128 MMAs more slowly than the
     // tensor core runs them; both wait for the same stage and commit to it.
@@ -167,9 +180,11 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
     uint64_t *acc_full = empty + STAGES;
     uint64_t *acc_empty = acc_full + 4;
     uint32_t *tmem_holder = (uint32_t *) (acc_empty + 4);
+    uint64_t *mask_full = acc_empty + 5;   // [epilogue warp][staging buffer]
+    static_assert((2 * STAGES + 9 + 2 * EW) * 8 <= C::BAR_BYTES, "mbarriers");
     // per-class tap offsets (packed y:16 | x:16) and the tile's epilogue scale/shift, in shared
     // memory: indexing the kernel parameters with runtime values would go through slow generic loads
-    int32_t *tap_tab = (int32_t *) (epi_smem + C::EPI_BUFS * C::EPI_BYTES + 256);
+    int32_t *tap_tab = (int32_t *) (epi_smem + C::EPI_BUFS * C::EPI_BYTES + C::BAR_BYTES);
     ClsS *cls_tab = (ClsS *) (tap_tab + TC_MAXCLS * TC_MAXTAPS);
     float *sc_tab = (float *) (cls_tab + TC_MAXCLS);   // [1024]: all channels, or the tile's BN
     float *sh_tab = sc_tab + 1024;
@@ -182,9 +197,11 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
             tc::mbar_init(&full[s], IM2C ? 1 : 128 + 1);
             tc::mbar_init(&empty[s], SPLIT ? 2 : 1);
         }
+        if (EXTRA == EXTRA_MASK || EXTRA == EXTRA_SUMS)
+            for (int b = 0; b < 2 * EW; b++) tc::mbar_init(&mask_full[b], 1);
         for (int b = 0; b < C::ACC_BUFS; b++) {
             tc::mbar_init(&acc_full[b], SPLIT ? 2 : 1);
-            tc::mbar_init(&acc_empty[b], 32 * EW);
+            tc::mbar_init(&acc_empty[b], ALT ? 128 : 32 * EW);
         }
         tc::fence_mbar_init();
         tc::prefetch_tmap(&wmap);
@@ -351,13 +368,58 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
     } else if (warp >= 4 && warp < 4 + EW) {
         // ------------------------------------------------ epilogue
         const int ew = (warp - 4) & 3;    // TMEM lane quarter (a warp reads lanes 32 * (warp % 4) ..)
-        const int half = (warp - 4) >> 2; // EW = 8: which alternate chunks this warp takes
+        const int half = (warp - 4) >> 2; // EW = 8: which alternate items (ALT: tiles) this warp takes
         const int row = ew * 32 + lane;   // tile row = TMEM lane
         const int et = threadIdx.x - 128; // 0 .. 32 * EW - 1
         uint8_t *const stg_warp = epi_smem + (warp - 4) * 4096;   // this warp's 32 x 128-byte staging
-        uint32_t lt = 0;                  // local tile count
+        const int first_item = ALT ? 0 : half;
+        uint32_t lt = ALT ? half : 0;     // local tile count
         int ebuf = 0;                     // staging buffer toggle
-        for (int tile = blockIdx.x; tile < p.ntiles_total && ok; tile += gridDim.x, lt++) {
+        // The mask's 32 x 64 values of an item, loaded into the staging buffer the item will use: by TMA, or where
+        // the rows are scattered (stride-phase classes) by 16-byte pieces, eight lanes to a row. (Read by
+        // their own lanes, one cache line of another row per lane, the masked form of 56 x 56, 256 -> 64 took 60 us,
+        // 27 without a mask.) The load is issued during the item before, off the critical path. Returns whether
+        // the mask_full barrier will tell of its arrival.
+        uint64_t *const mbar = mask_full + 2 * (warp - 4);
+        auto prefetch_mask = [&](int tile, int item, int buf) {
+            const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, BN, tile, MT);
+            const ClsS &cl = cls_tab[tl.cls];
+            const int M = p.B * cl.Hg * cl.Wg;
+            const int r0 = tl.m0 + (item / C::NCH) * 128 + ew * 32, nb = tl.n0 + (item % C::NCH) * C::CW;
+            const uint32_t dst = tc::smem_u32(stg_warp + buf * C::EPI_BYTES);
+            if (p.epi_tma) {
+                if (r0 >= M || nb >= p.Cout) return false;
+                if (lane == 0) {
+                    tc::mbar_arrive_expect_tx(&mbar[buf], 4096);
+                    tc::tma_load_2d(dst, &amaps.mask, nb, r0, &mbar[buf]);
+                }
+                return true;
+            }
+            int pix = r0 + lane;
+            uint32_t q, jw, j, b;
+            cl.dwg.divmod(pix < M ? pix : 0, q, jw);
+            cl.dhg.divmod(q, b, j);
+            pix = ((int) b * p.Hout + cl.oy0 + cl.osy * (int) j) * p.Wout + cl.ox0 + cl.osx * (int) jw;
+            const int ch = lane & 7;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int r = i * 4 + (lane >> 3);
+                const int px = __shfl_sync(0xFFFFFFFFu, pix, r);
+                const bool v = r0 + r < M && nb + ch * 8 < p.Cout;
+                const __nv_bfloat16 *src = v ? p.mask + ((size_t) px * p.Cout + nb + ch * 8) : p.mask;
+                tc::cp_async_16(dst + r * 128 + ((ch ^ (r & 7)) << 4), src, v ? 16u : 0u);
+            }
+            tc::cp_async_commit();
+            return false;
+        };
+        constexpr bool MASKED = EXTRA == EXTRA_MASK || EXTRA == EXTRA_SUMS;
+        bool by_tma = false;       // this item's mask arrives at mbar[ebuf]
+        uint32_t mphase = 0;       // bit b: parity of the next arrival at mbar[b]
+        if constexpr (MASKED) {
+            const int t0 = blockIdx.x + (int) (lt * gridDim.x);
+            if (p.mask && t0 < p.ntiles_total && first_item < NIT) by_tma = prefetch_mask(t0, first_item, 0);
+        }
+        for (int tile = blockIdx.x + (int) (lt * gridDim.x); tile < p.ntiles_total && ok; tile += TSTEP * gridDim.x, lt += TSTEP) {
             const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, BN, tile, MT);
             const ClsS &cl = cls_tab[tl.cls];
             const int M = p.B * cl.Hg * cl.Wg;
@@ -367,23 +429,26 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                 scp += tl.n0;
                 shp += tl.n0;
             } else {
-                // this tile's scale/shift (the previous tile's readers passed the barrier below)
-                epi_bar<32 * EW>();
-                for (int j = et; j < BN; j += 32 * EW) {
+                // this tile's scale/shift (the previous tile's readers passed the barrier below;
+                // ALT: the two groups of warps keep their own copies)
+                float *sc = sc_tab + (ALT ? half * 64 : 0), *sh = sh_tab + (ALT ? half * 64 : 0);
+                if (ALT) tc::named_bar_sync(1 + half, 128);
+                else epi_bar<32 * EW>();
+                for (int j = ALT ? (et & 127) : et; j < BN; j += ALT ? 128 : 32 * EW) {
                     const int n = min(tl.n0 + j, p.Cout - 1);
-                    sc_tab[j] = p.scale ? __ldg(p.scale + n) : 1.0f;
-                    sh_tab[j] = p.shift ? __ldg(p.shift + n) : 0.0f;
+                    sc[j] = p.scale ? __ldg(p.scale + n) : 1.0f;
+                    sh[j] = p.shift ? __ldg(p.shift + n) : 0.0f;
                 }
-                epi_bar<32 * EW>();
+                if (ALT) tc::named_bar_sync(1 + half, 128);
+                else epi_bar<32 * EW>();
+                scp = sc;
+                shp = sh;
             }
             ok = tc::mbar_wait(&acc_full[buf], (lt / C::ACC_BUFS) & 1, p.err, 3);
             if (!ok) break;
             tc::tc_fence_after();
-            // items: (accumulator mt, chunk c0) in order; with eight warps the two warps of a
-            // lane quarter take alternate items
-            constexpr int NIT = MT * C::NCH, STEP = EW / 4;
 #pragma unroll 1
-            for (int item = half; item < NIT; item += STEP) {
+            for (int item = first_item; item < NIT; item += STEP) {
                 const int mt = item / C::NCH, c0 = (item % C::NCH) * C::CW;
                 const int m0 = tl.m0 + mt * 128;   // this accumulator's first output row
                 const int m = m0 + row;
@@ -408,48 +473,110 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                     tc::mbar_arrive(&acc_empty[buf]);
                 }
                 const int nb = tl.n0 + c0;
-                if constexpr (STATS) if (m0 + ew * 32 < M) {
-                    // column statistics of this chunk's 64 columns over the warp's 32 rows (group
-                    // gbase + (m0 + 32 ew) / 32 of the class; the classes' groups are concatenated):
-                    // the forward's batch-norm sums, or, for the masked input gradient, the sums of
-                    // the masked output (the bias gradient of the layer that produced the mask)
-                    if (p.mask && m < M && nb < p.Cout) {
-                        size_t pix = (size_t) m;
-                        if (!p.epi_tma) {
-                            uint32_t q, jw, j, b;
-                            cl.dwg.divmod(m, q, jw);
-                            cl.dhg.divmod(q, b, j);
-                            pix = ((size_t) b * p.Hout + cl.oy0 + cl.osy * (int) j) * p.Wout + cl.ox0 + cl.osx * (int) jw;
+                bool next_by_tma = false;
+                if constexpr (MASKED) {
+                    if (p.mask) {
+                        if (by_tma) {
+                            if (!(ok = tc::mbar_wait(&mbar[ebuf], mphase >> ebuf & 1, p.err, 5))) break;
+                            mphase ^= 1u << ebuf;
+                        } else {
+                            tc::cp_async_wait<0>();
                         }
-                        const __nv_bfloat16 *mrow = p.mask + pix * p.Cout + nb;
-#pragma unroll
-                        for (int q = 0; q < 8; q++) {
-                            uint4 mv = make_uint4(0, 0, 0, 0);
-                            if (nb + 8 * q + 8 <= p.Cout) mv = __ldg(reinterpret_cast<const uint4 *>(mrow) + q);
-                            const uint32_t mw[4] = {mv.x, mv.y, mv.z, mv.w};
-#pragma unroll
-                            for (int e = 0; e < 4; e++) {
-                                const int jj = 8 * q + 2 * e;
-                                uint32_t &lo = jj < 32 ? v0[jj] : v1[jj - 32];
-                                uint32_t &hi = jj + 1 < 32 ? v0[jj + 1] : v1[jj - 31];
-                                if ((mw[e] & 0xFFFFu) - 1u >= 0x7F80u) lo = 0u;   // mask <= 0 (or NaN)
-                                if ((mw[e] >> 16) - 1u >= 0x7F80u) hi = 0u;
-                            }
+                        __syncwarp();
+                        // the next item's mask goes to the other buffer, once the store of the item before
+                        // this one has read it
+                        int nt = tile, ni = item + STEP;
+                        if (ni >= NIT) {
+                            ni = first_item;
+                            nt += TSTEP * gridDim.x;
                         }
-                    }
-                    float *part = p.stats + (size_t) (cl.gbase + (m0 >> 5) + ew) * 2 * p.Cout;
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        float sum, sq;
-                        tc::stats_cols32(h ? v1 : v0, scp + c0 + 32 * h, shp + c0 + 32 * h, m < M, sum, sq);
-                        const int col = nb + 32 * h + lane;
-                        if (col < p.Cout) {
-                            part[col] = sum;
-                            part[p.Cout + col] = sq;
+                        if (nt < p.ntiles_total) {
+                            if (lane == 0) bulk_wait_read<0>();
+                            __syncwarp();
+                            next_by_tma = prefetch_mask(nt, ni, ebuf ^ 1);
                         }
                     }
                 }
-                if (!C::OUTF32 && p.accum && m < M && nb < p.Cout) {
+                if constexpr (EXTRA == EXTRA_SUMS || EXTRA == EXTRA_STATS) {
+                    // Column sums of this item's 64 columns over the warp's 32 rows, to group
+                    // gbase + m0 / 32 + ew of the class (the classes' groups are concatenated): the forward's
+                    // batch-norm sums of z and z^2, or the sums of the masked input gradient (the bias
+                    // gradient of the layer that produced the mask). Each half of the columns passes through
+                    // the staging buffer, rows in, columns out: lane l adds up columns 2 (l % 16), + 1 of the rows
+                    // of its parity l / 16, two running sums each. (Exchanged by shuffles the same sums were about
+                    // a thousand instructions of straight-line code per item and bound by instruction
+                    // fetches: 56 x 56, 64 -> 256 forward with statistics 111 us, 27 without.)
+                    if (m0 + ew * 32 < M) {
+                        uint8_t *stg = stg_warp + ebuf * C::EPI_BYTES;
+                        if (EXTRA == EXTRA_SUMS && p.mask) {
+                            // rows past M arrived as zeros, which keep nothing
+#pragma unroll
+                            for (int q = 0; q < 8; q++) {
+                                const uint4 mv = *reinterpret_cast<const uint4 *>(stg + lane * 128 + ((q ^ (lane & 7)) << 4));
+                                const uint32_t mw[4] = {mv.x, mv.y, mv.z, mv.w};
+#pragma unroll
+                                for (int e = 0; e < 4; e++) {
+                                    const uint32_t k = positive_mask(mw[e]);
+                                    const int jj = 8 * q + 2 * e;
+                                    (jj < 32 ? v0[jj] : v1[jj - 32]) &= __byte_perm(k, 0, 0x1010);
+                                    (jj < 32 ? v0[jj + 1] : v1[jj - 31]) &= __byte_perm(k, 0, 0x3232);
+                                }
+                            }
+                            __syncwarp();
+                        } else {   // the buffer's last store has read it (masked: waited for above)
+                            if (lane == 0) bulk_wait_read<1>();
+                            __syncwarp();
+                        }
+                        float *part = p.stats + (size_t) (cl.gbase + (m0 >> 5) + ew) * 2 * p.Cout + nb;
+                        const bool in = m < M;
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+#pragma unroll
+                            for (int q = 0; q < 8; q++) {
+                                float z[4];
+#pragma unroll
+                                for (int e = 0; e < 4; e++) z[e] = __uint_as_float(h ? v1[4 * q + e] : v0[4 * q + e]);
+                                if (EXTRA == EXTRA_STATS) {   // (the input gradient has no scale and shift)
+                                    const float4 sc = *reinterpret_cast<const float4 *>(scp + c0 + 32 * h + 4 * q);
+                                    const float4 sh = *reinterpret_cast<const float4 *>(shp + c0 + 32 * h + 4 * q);
+                                    z[0] = fmaf(z[0], sc.x, sh.x);
+                                    z[1] = fmaf(z[1], sc.y, sh.y);
+                                    z[2] = fmaf(z[2], sc.z, sh.z);
+                                    z[3] = fmaf(z[3], sc.w, sh.w);
+                                }
+                                *reinterpret_cast<float4 *>(stg + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+                                    in ? make_float4(z[0], z[1], z[2], z[3]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                            }
+                            __syncwarp();
+                            const int l16 = lane & 15;
+                            float2 s2[2] = {}, q2[2] = {};
+#pragma unroll 2
+                            for (int r = lane >> 4; r < 32; r += 4)
+#pragma unroll
+                                for (int e = 0; e < 2; e++) {
+                                    const int rr = r + 2 * e;
+                                    const float2 z = *reinterpret_cast<const float2 *>(
+                                        stg + rr * 128 + (((l16 >> 1) ^ (rr & 7)) << 4) + (l16 & 1) * 8);
+                                    s2[e].x += z.x;
+                                    s2[e].y += z.y;
+                                    if (EXTRA == EXTRA_STATS) q2[e] = __ffma2_rn(z, z, q2[e]);
+                                }
+                            float2 sum = make_float2(s2[0].x + s2[1].x, s2[0].y + s2[1].y);
+                            sum.x += __shfl_xor_sync(0xFFFFFFFFu, sum.x, 16);
+                            sum.y += __shfl_xor_sync(0xFFFFFFFFu, sum.y, 16);
+                            const bool col = nb + 32 * h + 2 * l16 < p.Cout;   // Cout is a multiple of 8
+                            if (lane < 16 && col) *reinterpret_cast<float2 *>(part + 32 * h + 2 * l16) = sum;
+                            if (EXTRA == EXTRA_STATS) {
+                                sum = make_float2(q2[0].x + q2[1].x, q2[0].y + q2[1].y);
+                                sum.x += __shfl_xor_sync(0xFFFFFFFFu, sum.x, 16);
+                                sum.y += __shfl_xor_sync(0xFFFFFFFFu, sum.y, 16);
+                                if (lane < 16 && col) *reinterpret_cast<float2 *>(part + p.Cout + 32 * h + 2 * l16) = sum;
+                            }
+                            __syncwarp();
+                        }
+                    }
+                }
+                if ((EXTRA == EXTRA_NONE || EXTRA == EXTRA_MASK) && !C::OUTF32 && p.accum && m < M && nb < p.Cout) {
                     // accumulate (the reference's dx += ...): add the output's current 64 values in FP32
                     size_t pix = (size_t) m;
                     if (!p.epi_tma) {
@@ -487,32 +614,21 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                 } else {
                     tc::epi_bf16_64<false>(v0, v1, scp + c0, shp + c0, pk);
                 }
-                if (!C::OUTF32 && p.mask && m < M && nb < p.Cout) {
-                    // ReLU backward: keep the outputs where the mask (the activation the ReLU
-                    // produced, laid out like the output) is positive
-                    size_t pix = (size_t) m;
-                    if (!p.epi_tma) {
-                        uint32_t q, jw, j, b;
-                        cl.dwg.divmod(m, q, jw);
-                        cl.dhg.divmod(q, b, j);
-                        pix = ((size_t) b * p.Hout + cl.oy0 + cl.osy * (int) j) * p.Wout + cl.ox0 + cl.osx * (int) jw;
-                    }
-                    const __nv_bfloat16 *mrow = p.mask + pix * p.Cout + nb;
+                if constexpr (EXTRA == EXTRA_MASK) {
+                    // ReLU backward: the outputs where the mask is positive; this lane's row of the mask lies
+                    // where its row of the output goes
+                    const uint8_t *mrow = stg_warp + ebuf * C::EPI_BYTES + lane * 128;
 #pragma unroll
                     for (int q = 0; q < 8; q++) {
-                        uint4 mv = make_uint4(0, 0, 0, 0);
-                        if (nb + 8 * q + 8 <= p.Cout) mv = __ldg(reinterpret_cast<const uint4 *>(mrow) + q);
-                        const uint32_t mw[4] = {mv.x, mv.y, mv.z, mv.w};
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const uint32_t lo = mw[e] & 0xFFFFu, hi = mw[e] >> 16;
-                            // positive: sign clear, not zero, not NaN
-                            const uint32_t klo = (lo - 1u) < 0x7F80u ? 0x0000FFFFu : 0u;
-                            const uint32_t khi = (hi - 1u) < 0x7F80u ? 0xFFFF0000u : 0u;
-                            pk[4 * q + e] &= klo | khi;
-                        }
+                        const uint4 mv = *reinterpret_cast<const uint4 *>(mrow + ((q ^ (lane & 7)) << 4));
+                        pk[4 * q] &= positive_mask(mv.x);
+                        pk[4 * q + 1] &= positive_mask(mv.y);
+                        pk[4 * q + 2] &= positive_mask(mv.z);
+                        pk[4 * q + 3] &= positive_mask(mv.w);
                     }
+                    __syncwarp();
                 }
+                by_tma = next_by_tma;
                 if (p.epi_tma) {
                     // each warp stages its 32 rows (4 KB) and stores them with its own TMA
                     // store: no barrier across the epilogue warps (out-of-range rows/columns
@@ -530,11 +646,10 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                     }
                     tc::fence_proxy_async_smem();
                     __syncwarp();
-                    if (lane == 0 && nb < p.Cout && m0 + ew * 32 < M) {
-                        tma_store_2d(&omap, tc::smem_u32(stg), nb, m0 + ew * 32);
-                        bulk_commit();
+                    if (lane == 0) {
+                        if (nb < p.Cout && m0 + ew * 32 < M) tma_store_2d(&omap, tc::smem_u32(stg), nb, m0 + ew * 32);
+                        bulk_commit();   // a group per item, so that waiting for all but the last frees the other buffer
                     }
-                    if (C::EPI_BUFS == 2) ebuf ^= 1;
                 } else if (!C::OUTF32 && nb + C::CW <= p.Cout && __any_sync(0xFFFFFFFFu, orow != nullptr)) {
                     // rows scattered over the output (stride-phase classes): staged through this warp's
                     // buffer, then each store instruction writes four whole 128-byte rows (eight lanes
@@ -557,7 +672,6 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                         if (dst) *reinterpret_cast<uint4 *>((uint8_t *) dst + ch * 16) = u;
                     }
                     __syncwarp();
-                    if (C::EPI_BUFS == 2) ebuf ^= 1;
                 } else if (orow && nb < p.Cout) {
                     if (nb + C::CW <= p.Cout) {
                         uint4 *dst = reinterpret_cast<uint4 *>(orow + (size_t) nb * (C::OUTF32 ? 4 : 2));
@@ -578,6 +692,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                         }
                     }
                 }
+                if (C::EPI_BUFS == 2) ebuf ^= 1;
             }
         }
         if (lane == 0) bulk_wait_all();
@@ -657,12 +772,11 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
     if (warp == C::MMA_WARP) tc::tmem_dealloc(tmem, C::TMEM_COLS);
 }
 
-template <int BN, int STAGES, int KB, bool IM2C, int MODE, int MT = 1, int EW = 4, bool STATS = false>
+template <int BN, int STAGES, int KB, bool IM2C, int MODE, int MT = 1, int EW = 4, int EXTRA = EXTRA_NONE>
 cudaError_t launch_bn(const TcConvParams &p, const CUtensorMap &wmap, const CUtensorMap &omap, const TcMaps &amaps,
                       int grid, cudaStream_t st) {
-    static_assert(!STATS || (MODE == MODE_BF16 && MT == 1 && EW == 4), "statistics: BF16, one M tile, four warps");
     using C = TcCfg<BN, STAGES, KB, MODE, MT, EW>;
-    auto kern = tc_conv_kernel<BN, STAGES, KB, IM2C, MODE, MT, EW, STATS>;
+    auto kern = tc_conv_kernel<BN, STAGES, KB, IM2C, MODE, MT, EW, EXTRA>;
     static bool attr = false;
     if (!attr) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM);
@@ -685,6 +799,30 @@ int tc_conv_stages(int bn, int im2col, int mt, int ew, int kb1) {
     if (kb1 && bn != 256) return bn == 64 ? 8 : 6;
     return bn == 64 ? 4 : 3;
 }
+
+namespace {
+// The forms with a mask or column sums: one M tile, eight epilogue warps (four beside the gathers), two
+// staging buffers.
+template <int EXTRA>
+cudaError_t launch_extra(const TcConvParams &p, const CUtensorMap &wmap, const CUtensorMap &omap, const TcMaps &amaps,
+                         int grid, cudaStream_t st) {
+    if (p.mode != MODE_BF16 || p.mt != 1 || p.ew != (p.im2col ? 8 : 4)) return cudaErrorInvalidValue;
+    if (p.im2col) {
+        switch (p.bn) {
+            case 64: return launch_bn<64, 3, 2, true, MODE_BF16, 1, 8, EXTRA>(p, wmap, omap, amaps, grid, st);
+            case 128: return launch_bn<128, 4, 1, true, MODE_BF16, 1, 8, EXTRA>(p, wmap, omap, amaps, grid, st);
+            case 256: return launch_bn<256, 3, 1, true, MODE_BF16, 1, 8, EXTRA>(p, wmap, omap, amaps, grid, st);
+            default: return cudaErrorInvalidValue;
+        }
+    }
+    switch (p.bn) {
+        case 64: return launch_bn<64, 6, 1, false, MODE_BF16, 1, 4, EXTRA>(p, wmap, omap, amaps, grid, st);
+        case 128: return launch_bn<128, 5, 1, false, MODE_BF16, 1, 4, EXTRA>(p, wmap, omap, amaps, grid, st);
+        case 256: return launch_bn<256, 3, 1, false, MODE_BF16, 1, 4, EXTRA>(p, wmap, omap, amaps, grid, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+}  // namespace
 
 cudaError_t tc_conv_launch(const TcConvParams &p, const CUtensorMap &wmap, const CUtensorMap &omap,
                            const TcMaps &amaps, int grid, cudaStream_t st) {
@@ -712,24 +850,9 @@ cudaError_t tc_conv_launch(const TcConvParams &p, const CUtensorMap &wmap, const
             default: return cudaErrorInvalidValue;
         }
     }
-    if (p.stats) {
-        // forward with batch statistics (tc_conv_kernel's STATS form): one M tile, four epilogue warps
-        if (p.mode != MODE_BF16 || p.mt != 1 || p.ew != 4) return cudaErrorInvalidValue;
-        if (p.im2col) {
-            switch (p.bn) {
-                case 64: return launch_bn<64, 4, 2, true, MODE_BF16, 1, 4, true>(p, wmap, omap, amaps, grid, st);
-                case 128: return launch_bn<128, 3, 2, true, MODE_BF16, 1, 4, true>(p, wmap, omap, amaps, grid, st);
-                case 256: return launch_bn<256, 3, 1, true, MODE_BF16, 1, 4, true>(p, wmap, omap, amaps, grid, st);
-                default: return cudaErrorInvalidValue;
-            }
-        }
-        switch (p.bn) {
-            case 64: return launch_bn<64, 8, 1, false, MODE_BF16, 1, 4, true>(p, wmap, omap, amaps, grid, st);
-            case 128: return launch_bn<128, 6, 1, false, MODE_BF16, 1, 4, true>(p, wmap, omap, amaps, grid, st);
-            case 256: return launch_bn<256, 4, 1, false, MODE_BF16, 1, 4, true>(p, wmap, omap, amaps, grid, st);
-            default: return cudaErrorInvalidValue;
-        }
-    }
+    if (p.stats && p.sums_only) return launch_extra<EXTRA_SUMS>(p, wmap, omap, amaps, grid, st);
+    if (p.stats) return launch_extra<EXTRA_STATS>(p, wmap, omap, amaps, grid, st);
+    if (p.mask) return launch_extra<EXTRA_MASK>(p, wmap, omap, amaps, grid, st);
     if (p.im2col && p.ew == 8) {
         // eight epilogue warps (short-K tiles): one K block per stage, two staging buffers
         if (p.mt == 2) {

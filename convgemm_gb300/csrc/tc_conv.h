@@ -40,6 +40,7 @@ struct TcConvParams {
                                // rounding), then the mask; 0: out overwritten
     float *stats;              // BF16 forward: per 32-row group g of the output pixels, [g][0][Cout] the sum
                                // and [g][1][Cout] the sum of squares of z = acc * scale + shift; or NULL
+    int sums_only;             // stats without the squares (bias gradient)
     int B, Hin, Win, Cin, Hout, Wout, Cout;
     FastDiv dcin;
     int *err;                  // device error word for timed-out waits
@@ -52,7 +53,7 @@ struct TcConvParams {
                                // last one's channels past Cin zero-filled by both operands' loads (TcMaps::w)
     int mode;                  // 0 BF16, 1 FP8-E4M3, 2 3xBF16 (FP32 output)
     int mt;                    // 128-row M tiles per tile (1, or 2 sharing each weight tile: BF16 im2col only)
-    int ew;                    // epilogue warps: 4, or 8 (BF16 im2col, bn >= 128 or mt == 2, not bn 256 with mt 2)
+    int ew;                    // epilogue warps: 4, or 8 (BF16 im2col, not bn 256 with mt 2; with a mask or sums always)
     int kb1;                   // BF16 im2col, one M tile, four epilogue warps, bn 64 / 128: one K block per ring
                                // stage and twice the stages (8 / 6) instead of two blocks per stage (4 / 3)
     int ncls;
@@ -65,6 +66,7 @@ struct TcMaps {
     CUtensorMap a[TC_MAXIM2COL];    // im2col maps of the gathered tensor, one per class
     CUtensorMap alo[TC_MAXIM2COL];  // 3xBF16: maps of the low parts
     CUtensorMap wlo;                // 3xBF16: packed low parts of the weights
+    CUtensorMap mask;               // epi_tma with a mask: the mask, laid out and boxed like the output
     CUtensorMap w[TC_MAXIM2COL];    // wtail: packed weights of a class as (channel, tap, output channel)
 };
 

@@ -300,8 +300,9 @@ struct TileForm {
 };
 constexpr TileForm FORMS_BF16[] = {{64, 1, 4, 0.270f, 0.92f, 3.5f}, {128, 1, 4, 0.280f, 1.62f, 4.2f}, {128, 1, 8, 0.296f, 1.30f, 4.25f},
                                    {128, 2, 8, 0.459f, 2.13f, 4.6f}, {256, 1, 8, 0.363f, 2.01f, 4.9f}};
-// with batch statistics or a fused bias gradient in the epilogue
-constexpr TileForm FORMS_STATS[] = {{64, 1, 4, 0.270f, 2.5f, 3.5f}, {128, 1, 4, 0.280f, 4.5f, 4.2f}, {256, 1, 4, 0.370f, 8.5f, 4.9f}};
+// with a ReLU mask, or with column sums (batch statistics, a fused bias gradient) in the epilogue
+constexpr TileForm FORMS_MASK[] = {{64, 1, 8, 0.270f, 0.95f, 3.5f}, {128, 1, 8, 0.296f, 1.85f, 4.25f}, {256, 1, 8, 0.363f, 3.50f, 4.9f}};
+constexpr TileForm FORMS_SUMS[] = {{64, 1, 8, 0.270f, 1.30f, 3.5f}, {128, 1, 8, 0.296f, 2.80f, 4.25f}, {256, 1, 8, 0.363f, 5.00f, 4.9f}};
 constexpr TileForm FORMS_GATHER[] = {{64, 1, 4, 0.60f, 1.95f, 3.5f}, {128, 1, 4, 0.63f, 2.10f, 4.0f}, {256, 1, 4, 0.80f, 3.00f, 4.9f}};
 constexpr TileForm FORMS_FP8[] = {{64, 1, 4, 0.200f, 0.87f, 3.4f}, {128, 1, 4, 0.210f, 1.47f, 3.9f}, {256, 1, 4, 0.270f, 2.70f, 4.7f}};
 constexpr TileForm FORMS_FP8W[] = {{64, 1, 4, 0.255f, 0.87f, 3.4f}, {128, 1, 4, 0.270f, 1.47f, 3.9f}, {256, 1, 4, 0.360f, 2.70f, 4.7f}};
@@ -360,12 +361,13 @@ bool tc_use_im2col(TcPlan &pl, int sms) {
 }
 
 // mode: TcConvParams::mode.
-TileForm tc_pick_form(const TcPlan &pl, int mode, bool im2col, bool stats, int sms) {
+TileForm tc_pick_form(const TcPlan &pl, int mode, bool im2col, bool mask, bool sums, int sms) {
     if (mode == 1) return cheapest_form(FORMS_FP8, pl, 1, sms);
     if (mode == 2) return cheapest_form(FORMS_X3, pl, 1, sms);
     if (mode == 3) return cheapest_form(FORMS_FP8W, pl, 2, sms);
-    if (stats) return cheapest_form(FORMS_STATS, pl, 1, sms);
-    return im2col ? cheapest_form(FORMS_BF16, pl, 1, sms) : cheapest_form(FORMS_GATHER, pl, 1, sms);
+    if (!im2col) return cheapest_form(FORMS_GATHER, pl, 1, sms);
+    if (sums) return cheapest_form(FORMS_SUMS, pl, 1, sms);
+    return mask ? cheapest_form(FORMS_MASK, pl, 1, sms) : cheapest_form(FORMS_BF16, pl, 1, sms);
 }
 
 // Epilogue warps of tc_conv_kernel: eight where asked for (`by_k`: where every class has at most 8 K
@@ -382,7 +384,7 @@ int tc_epilogue_warps(const TcPlan &pl, bool eight, bool by_k, int bn, int mt, b
 convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, const void *wpacked, void *out,
                          const float *scale, const float *shift, int relu, cudaStream_t st, int mode,
                          const void *in_lo, const void *w_lo, int bn_override, int aux_override,
-                         const void *mask, float *stats, int accum) {
+                         const void *mask, float *stats, int accum, int sums_only) {
     if (pl.ncls == 0) return CONVGEMM_SUCCESS;
     // stride-1 layers with 64-channel blocks and several taps: operands from input slabs, unless the
     // tuning entry asks for the general kernel (aux bit 8)
@@ -403,7 +405,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     bool f8w = mode == 1 && p.im2col && pl.Cin % 128 == 0 && pl.Ktot % 128 == 0;
     for (int c = 0; f8w && c < pi.ncls; c++)
         if (pi.cls[c].kbeg % 128 || pi.cls[c].ktiles % 2) f8w = false;
-    const TileForm form = tc_pick_form(pi, f8w ? 3 : mode, p.im2col, stats != nullptr, sms);
+    const TileForm form = tc_pick_form(pi, f8w ? 3 : mode, p.im2col, mask != nullptr, stats != nullptr, sms);
     p.bn = bn_override ? bn_override : form.bn;
     const int eb = mode == 1 ? 1 : 2;   // operand element bytes
     CUtensorMap wmap, omap;
@@ -431,6 +433,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     p.mask = (const __nv_bfloat16 *) mask;
     p.accum = accum;
     p.stats = stats;
+    p.sums_only = sums_only;
     p.B = s.b;
     p.Hin = pl.Hin;
     p.Win = pl.Win;
@@ -445,6 +448,10 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     p.ncls = pl.ncls;
     TcMaps amaps;
     memset(&amaps, 0, sizeof(amaps));
+    if (mask && p.epi_tma)
+        if (convgemm_status_t e = tc_make_map_2d(&amaps.mask, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, mask,
+                                                 (long long) s.b * pl.Hout * pl.Wout, pl.Cout, 64, 32))
+            return e;
     if (f8w) {
         if (convgemm_status_t e = tc_make_map_2d_sw(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wpacked, pl.Cout, pl.Ktot,
                                                     128, p.bn, CU_TENSOR_MAP_SWIZZLE_128B))
@@ -484,9 +491,9 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     p.mt = (by_form ? form.mt == 2 : (aux_override & 3) == 2) && mode == 0 && p.im2col ? 2 : 1;
     p.ew = tc_epilogue_warps(pi, by_form ? form.ew == 8 : (aux_override & 4) != 0, !by_form && (aux_override & 7) == 0, p.bn,
                              p.mt, mode == 0 && p.im2col);
-    if (stats) {   // the statistics form: one M tile, four epilogue warps
+    if (stats || mask) {   // the forms with column sums or a mask: one M tile, eight epilogue warps beside TMA loads
         p.mt = 1;
-        p.ew = 4;
+        p.ew = p.im2col ? 8 : 4;
     }
     // aux bit 4 (tuning): one K block per ring stage, twice the stages (BF16 im2col, one M tile,
     // four epilogue warps, 64 / 128-wide tiles)
@@ -711,7 +718,7 @@ extern "C" convgemm_status_t convgemm_dgrad_bf16_bias_grad(const convgemm_shape_
     tc_tune_get(CONVGEMM_TUNE_DGRAD, *shape, &t);
     float *part = (float *) ((uint8_t *) workspace + cg_colsum_part_offset(ng, s.c));
     if (convgemm_status_t e = tc_run(pl, s, dy, wpacked, dx, nullptr, nullptr, 0, st, 0, nullptr, nullptr, t.bn,
-                                     t.splits, relu_x, part, 0))
+                                     t.splits, relu_x, part, 0, 1))
         return e;
     return cg_cuda_check(cg_colsum_reduce(workspace, (int) ng, s.c, db, st), "bias-gradient column sums");
 }
@@ -1090,7 +1097,7 @@ extern "C" convgemm_status_t convgemm_tune_describe(int op, const convgemm_shape
         return CONVGEMM_SUCCESS;
     }
     const int im2col = tc_use_im2col(pl, tc_num_sms());
-    const TileForm form = tc_pick_form(pl, 0, im2col, false, tc_num_sms());
+    const TileForm form = tc_pick_form(pl, 0, im2col, false, false, tc_num_sms());
     const bool by_form = !t.bn && (t.splits & 7) == 0;
     *bn = t.bn ? t.bn : form.bn;
     const int mt = (by_form ? form.mt == 2 : (t.splits & 3) == 2) && im2col ? 2 : 1;

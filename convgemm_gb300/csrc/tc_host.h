@@ -81,4 +81,4 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
                          const float *scale, const float *shift, int relu, cudaStream_t st, int mode = 0,
                          const void *in_lo = nullptr, const void *w_lo = nullptr, int bn_override = 0,
                          int aux_override = 0, const void *mask = nullptr,
-                         float *stats = nullptr, int accum = 0);
+                         float *stats = nullptr, int accum = 0, int sums_only = 0);
