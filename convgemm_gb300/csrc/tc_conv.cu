@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
     float *sh_tab = sc_tab + 1024;
     const bool sc_all = p.Cout <= 1024;              // whole scale/shift vectors fit
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = tc::w::warp_index(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
             // im2col: the one expect_tx arrival; gather: 128 producer threads + the expect_tx
@@ -245,15 +245,15 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
     bool ok = true;
 
     if (IM2C && warp < 4 && warp != C::MMA_WARP && !(SPLIT && warp == C::ISS2_WARP)) {
-        // ------------------------------------------------ producer: one thread, im2col TMA for A, TMA for B
-        if (threadIdx.x == 0) {
+        // ------------------------------------------------ producer: one warp, im2col TMA for A, TMA for B
+        if (warp == 0) {
             uint32_t it = 0;
             for (int tile = blockIdx.x; tile < p.ntiles_total && ok; tile += gridDim.x) {
                 if (tile + (int) gridDim.x >= p.ntiles_total) tc::pdl_trigger();   // this CTA's last tile
                 const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, BN, tile, MT);
                 const ClsS &cl = cls_tab[tl.cls];
                 const int32_t *taps = tap_tab + tl.cls * TC_MAXTAPS;
-                const int ktiles = cl.ktiles, kbeg = cl.kbeg, mint_y = cl.mint_y, mint_x = cl.mint_x;
+                const int ktiles = __shfl_sync(0xFFFFFFFFu, cl.ktiles, 0), kbeg = cl.kbeg, mint_y = cl.mint_y, mint_x = cl.mint_x;
                 int h0[MT], w0[MT], bb0[MT];   // im2col start of each M tile (beyond the class: zero-filled)
 #pragma unroll
                 for (int mt = 0; mt < MT; mt++) {
@@ -269,10 +269,10 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                 for (int kt = 0; kt < ktiles; kt += KB, it++) {
                     const int s = it % STAGES;
                     const uint32_t ph = (it / STAGES) & 1;
-                    if (it >= (uint32_t) STAGES && !(ok = tc::mbar_wait(&empty[s], ph ^ 1, p.err, 1))) break;
+                    if (it >= (uint32_t) STAGES && !(ok = tc::w::mbar_wait(&empty[s], ph ^ 1, p.err, 1))) break;
                     const int nkb = min(KB, ktiles - kt);
                     const uint32_t sa = tc::smem_u32(base + s * C::STAGE_BYTES);
-                    tc::mbar_arrive_expect_tx(&full[s], nkb * (MT * C::A_BLOCK + C::B_BLOCK));
+                    tc::w::mbar_arrive_expect_tx(&full[s], nkb * (MT * C::A_BLOCK + C::B_BLOCK));
                     for (int kb = 0; kb < nkb; kb++) {
                         const int32_t to = taps[tap];
                         const uint16_t offy = (uint16_t) ((to >> 16) - mint_y);
@@ -281,14 +281,14 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                         const int kcol = kbeg + (kt + kb) * C::BK;
 #pragma unroll
                         for (int mt = 0; mt < MT; mt++)
-                            tc::tma_load_im2col_4d(ab + mt * C::A_BLOCK, am, ci0, w0[mt], h0[mt], bb0[mt], offx, offy,
+                            tc::w::tma_load_im2col_4d(ab + mt * C::A_BLOCK, am, ci0, w0[mt], h0[mt], bb0[mt], offx, offy,
                                                    &full[s]);
-                        if (MODE == MODE_BF16 && p.wtail) tc::tma_load_3d(bb, &amaps.w[tl.cls], ci0, tap, tl.n0, &full[s]);
-                        else tc::tma_load_2d(bb, &wmap, kcol, tl.n0, &full[s]);
+                        if (MODE == MODE_BF16 && p.wtail) tc::w::tma_load_3d(bb, &amaps.w[tl.cls], ci0, tap, tl.n0, &full[s]);
+                        else tc::w::tma_load_2d(bb, &wmap, kcol, tl.n0, &full[s]);
                         if (MODE == MODE_X3) {
-                            tc::tma_load_im2col_4d(ab + C::A_TILE, &amaps.alo[tl.cls], ci0, w0[0], h0[0], bb0[0], offx,
+                            tc::w::tma_load_im2col_4d(ab + C::A_TILE, &amaps.alo[tl.cls], ci0, w0[0], h0[0], bb0[0], offx,
                                                    offy, &full[s]);
-                            tc::tma_load_2d(bb + C::B_TILE, &amaps.wlo, kcol, tl.n0, &full[s]);
+                            tc::w::tma_load_2d(bb + C::B_TILE, &amaps.wlo, kcol, tl.n0, &full[s]);
                         }
                         ci0 += C::BK;
                         if (ci0 >= p.Cin) {
@@ -698,7 +698,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
         if (lane == 0) bulk_wait_all();
     } else {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
             // issuer `me`: its M tile (MT = 2) or N half (MT = 1) when SPLIT, else everything
             const int me = (SPLIT && warp == C::ISS2_WARP) ? 1 : 0;
             constexpr int NI = (SPLIT && MT == 1) ? BN / 2 : BN;   // N of one MMA instruction
@@ -709,10 +709,10 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
             uint32_t it = 0, lt = 0;
             for (int tile = blockIdx.x; tile < p.ntiles_total && ok; tile += gridDim.x, lt++) {
                 const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, BN, tile, MT);
-                const int KT = cls_tab[tl.cls].ktiles;
+                const int KT = __shfl_sync(0xFFFFFFFFu, cls_tab[tl.cls].ktiles, 0);   // warp-uniform loop bounds
                 const int buf = lt % C::ACC_BUFS;
                 if (lt >= (uint32_t) C::ACC_BUFS) {
-                    ok = tc::mbar_wait(&acc_empty[buf], ((lt / C::ACC_BUFS) - 1) & 1, p.err, 4);
+                    ok = tc::w::mbar_wait(&acc_empty[buf], ((lt / C::ACC_BUFS) - 1) & 1, p.err, 4);
                     if (!ok) break;
                     tc::tc_fence_after();
                 }
@@ -720,7 +720,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                 for (int kt = 0; kt < KT; kt += KB, it++) {
                     const int s = it % STAGES;
                     const uint32_t ph = (it / STAGES) & 1;
-                    if (!tc::mbar_wait(&full[s], ph, p.err, 2)) {
+                    if (!tc::w::mbar_wait(&full[s], ph, p.err, 2)) {
                         ok = false;
                         break;
                     }
@@ -745,22 +745,22 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                             const uint64_t ad = ad0 + (((kb * MT + mt) * C::A_BLOCK + k * 32) >> 4);
                             const uint32_t dtm = dt + (uint32_t) (mt * BN) + n_off;
                             if (F8) {
-                                tc::mma_f8(dtm, ad, bd, idesc, acc);
+                                tc::w::mma_f8(dtm, ad, bd, idesc, acc);
                             } else {
-                                tc::mma_f16(dtm, ad, bd, idesc, acc);
+                                tc::w::mma_f16(dtm, ad, bd, idesc, acc);
                                 if (MODE == MODE_X3) {
                                     const uint64_t adl = ad + (C::A_TILE >> 4);
                                     const uint64_t bdl = bd + (C::B_TILE >> 4);
-                                    tc::mma_f16(dtm, ad, bdl, idesc, 1);   // hi * lo
-                                    tc::mma_f16(dtm, adl, bd, idesc, 1);   // lo * hi
+                                    tc::w::mma_f16(dtm, ad, bdl, idesc, 1);   // hi * lo
+                                    tc::w::mma_f16(dtm, adl, bd, idesc, 1);   // lo * hi
                                 }
                             }
                           }
                         }
                     }
-                    tc::mma_commit(&empty[s]);
+                    tc::w::mma_commit(&empty[s]);
                 }
-                tc::mma_commit(&acc_full[buf]);
+                tc::w::mma_commit(&acc_full[buf]);
             }
         }
         __syncwarp();

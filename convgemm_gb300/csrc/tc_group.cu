@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(288, 1)
     float *sc_tab = (float *) (epi + EPI_BYTES + 256);
     float *sh_tab = sc_tab + GBN;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = tc::w::warp_index(), lane = threadIdx.x & 31;
     tc::pdl_wait();   // pdl_trigger: when the producer starts this CTA's last tile
     // a table prepared for another count, or a tile count beyond the table: run nothing
     if (__ldg(&probs[0].count) != nprob) {
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(288, 1)
     bool ok = true;
 
     if (warp < 4) {
-        if (threadIdx.x == 0) {
+        if (warp == 0) {
             // ---------------------------------------------- producer
             uint32_t it = 0;
             int pi = 0;
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(288, 1)
                 const GroupProblem *P = probs + pi;
                 const int local = tile - __ldg(&P->tile0), ntn = __ldg(&P->ntiles_n), bn = __ldg(&P->bn);
                 const int m0 = (local / ntn) * 128, n0 = (local % ntn) * bn;
-                const int ktiles = __ldg(&P->ktiles), cpb = __ldg(&P->cpb);
+                const int ktiles = __shfl_sync(0xFFFFFFFFu, __ldg(&P->ktiles), 0), cpb = __ldg(&P->cpb);
                 const FastDiv dwg = P->dwg, dhg = P->dhg;
                 uint32_t q, jw, j, b;
                 dwg.divmod(m0, q, jw);
@@ -121,19 +121,21 @@ __global__ void __launch_bounds__(288, 1)
                 const int w0 = (int) jw * __ldg(&P->isx) + __ldg(&P->lo_x);
                 const uint32_t tx_bytes = A_BYTES + (uint32_t) bn * 128;
                 int tap = 0, cc = 0;
+                int32_t to = __ldg(&P->taps[0]), to_next = __ldg(&P->taps[1]);   // the next tap's offsets, loaded ahead
                 for (int kt = 0; kt < ktiles; kt++, it++) {
                     const int s = it % GSTAGES;
                     const uint32_t ph = (it / GSTAGES) & 1;
-                    if (it >= (uint32_t) GSTAGES && !(ok = tc::mbar_wait(&empty[s], ph ^ 1, err, 21))) break;
-                    const int32_t to = __ldg(&P->taps[tap]);
+                    if (it >= (uint32_t) GSTAGES && !(ok = tc::w::mbar_wait(&empty[s], ph ^ 1, err, 21))) break;
                     const uint32_t sa = tc::smem_u32(base + s * STAGE_BYTES);
-                    tc::mbar_arrive_expect_tx(&full[s], tx_bytes);
-                    tc::tma_load_im2col_4d(sa, &P->amap, cc * 64, w0, h0, (int) b, (uint16_t) (to & 0xFFFF),
+                    tc::w::mbar_arrive_expect_tx(&full[s], tx_bytes);
+                    tc::w::tma_load_im2col_4d(sa, &P->amap, cc * 64, w0, h0, (int) b, (uint16_t) (to & 0xFFFF),
                                            (uint16_t) (to >> 16), &full[s]);
-                    tc::tma_load_2d(sa + A_BYTES, &P->wmap, kt * 64, n0, &full[s]);
+                    tc::w::tma_load_2d(sa + A_BYTES, &P->wmap, kt * 64, n0, &full[s]);
                     if (++cc == cpb) {
                         cc = 0;
                         tap++;
+                        to = to_next;
+                        to_next = __ldg(&P->taps[min(tap + 1, TC_MAXTAPS - 1)]);
                     }
                 }
             }
@@ -199,17 +201,17 @@ __global__ void __launch_bounds__(288, 1)
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else {
         // -------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        {
             uint32_t it = 0, lt = 0;
             int pi = 0;
             for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, lt++) {
                 pi = advance(probs, nprob, pi, tile);
                 const GroupProblem *P = probs + pi;
-                const int ktiles = __ldg(&P->ktiles);
+                const int ktiles = __shfl_sync(0xFFFFFFFFu, __ldg(&P->ktiles), 0);   // warp-uniform loop bounds
                 const uint32_t idesc = __ldg(&P->idesc);
                 const int buf = lt & 1;
                 if (lt >= 2) {
-                    ok = tc::mbar_wait(&acc_empty[buf], ((lt >> 1) - 1) & 1, err, 24);
+                    ok = tc::w::mbar_wait(&acc_empty[buf], ((lt >> 1) - 1) & 1, err, 24);
                     if (!ok) break;
                     tc::tc_fence_after();
                 }
@@ -217,7 +219,7 @@ __global__ void __launch_bounds__(288, 1)
                 for (int kt = 0; kt < ktiles; kt++, it++) {
                     const int s = it % GSTAGES;
                     const uint32_t ph = (it / GSTAGES) & 1;
-                    if (!tc::mbar_wait(&full[s], ph, err, 22)) {
+                    if (!tc::w::mbar_wait(&full[s], ph, err, 22)) {
                         ok = false;
                         break;
                     }
@@ -226,10 +228,10 @@ __global__ void __launch_bounds__(288, 1)
                     const uint64_t ad = tc::sw128_desc(tc::smem_u32(base + s * STAGE_BYTES), 16, 1024);
                     const uint64_t bd = ad + (A_BYTES >> 4);
 #pragma unroll
-                    for (int k = 0; k < 4; k++) tc::mma_f16(dt, ad + 2 * k, bd + 2 * k, idesc, (kt | k) != 0);
-                    tc::mma_commit(&empty[s]);
+                    for (int k = 0; k < 4; k++) tc::w::mma_f16(dt, ad + 2 * k, bd + 2 * k, idesc, (kt | k) != 0);
+                    tc::w::mma_commit(&empty[s]);
                 }
-                tc::mma_commit(&acc_full[buf]);
+                tc::w::mma_commit(&acc_full[buf]);
             }
         }
         __syncwarp();

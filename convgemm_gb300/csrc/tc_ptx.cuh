@@ -248,6 +248,109 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// ------------------------------------------------ issue by a whole warp
+// The producer and MMA loops run on all 32 lanes of a warp with warp-uniform control flow, and one elected
+// lane issues each TMA load, MMA, commit and expect_tx. These instructions take their operands from uniform
+// registers: in a loop that a single thread runs (`if (lane == 0)`) the compiler has to move every operand
+// there from that thread's registers first, which made an MMA cost 60-150 cycles to issue.
+namespace w {
+
+#define TC_ELECT "{\n\t.reg .pred e;\n\telect.sync _|e, 0xFFFFFFFF;\n\t@e "
+
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xFFFFFFFFu, (int) (threadIdx.x >> 5), 0); }
+
+// mbar_wait by the whole warp; the result is the same in every lane.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *err, int code) {
+    uint64_t t0 = 0;
+    for (uint32_t i = 1;; i++) {
+        if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+        if ((i & 1023) == 0) {
+            const uint64_t now = globaltimer();
+            if (t0 == 0) t0 = now;
+            if (__any_sync(0xFFFFFFFFu, now - t0 > WAIT_BUDGET_NS)) {
+                if (err && (threadIdx.x & 31) == 0) atomicCAS(err, 0, code);
+                return false;
+            }
+        }
+    }
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes) {
+    asm volatile(TC_ELECT "mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
+                 "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
+    asm volatile(TC_ELECT
+                 "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}" ::
+                     "r"(dst), "l"((uint64_t) map), "r"(x), "r"(y), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, uint64_t *bar) {
+    asm volatile(TC_ELECT
+                 "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+                 "[%5];\n\t}" ::"r"(dst), "l"((uint64_t) map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, uint64_t *bar) {
+    asm volatile(TC_ELECT
+                 "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+                 "[%6];\n\t}" ::"r"(dst), "l"((uint64_t) map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void tma_load_im2col_4d(uint32_t dst, const CUtensorMap *map, int c, int w, int h, int n,
+                                                   uint16_t ow, uint16_t oh, uint64_t *bar) {
+    asm volatile(TC_ELECT
+                 "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+                 " [%0], [%1, {%2, %3, %4, %5}], [%6], {%7, %8};\n\t}" ::"r"(dst), "l"((uint64_t) map), "r"(c), "r"(w), "r"(h),
+                 "r"(n), "r"(smem_u32(bar)), "h"(ow), "h"(oh)
+                 : "memory");
+}
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|e, 0xFFFFFFFF;\n\t"
+                 "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), "l"(adesc), "l"(bdesc),
+                 "r"(idesc), "r"(accumulate)
+                 : "memory");
+}
+__device__ __forceinline__ void mma_f8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|e, 0xFFFFFFFF;\n\t"
+                 "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), "l"(adesc), "l"(bdesc),
+                 "r"(idesc), "r"(accumulate)
+                 : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t *bar) {
+    asm volatile(TC_ELECT "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
+                 : "memory");
+}
+
+__device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|e, 0xFFFFFFFF;\n\t"
+                 "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), "l"(adesc), "l"(bdesc),
+                 "r"(idesc), "r"(accumulate)
+                 : "memory");
+}
+__device__ __forceinline__ void mma_commit_pair(uint64_t *bar, uint16_t mask) {
+    asm volatile(TC_ELECT
+                 "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::
+                     "r"(smem_u32(bar)), "h"(mask)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar_cluster) {
+    asm volatile(TC_ELECT
+                 "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
+                 "[%4];\n\t}" ::"r"(dst), "l"((uint64_t) map), "r"(x), "r"(y), "r"(bar_cluster)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_load_im2col_4d_pair(uint32_t dst, const CUtensorMap *map, int c, int w, int h, int n,
+                                                        uint16_t ow, uint16_t oh, uint32_t bar_cluster) {
+    asm volatile(TC_ELECT
+                 "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+                 " [%0], [%1, {%2, %3, %4, %5}], [%6], {%7, %8};\n\t}" ::"r"(dst), "l"((uint64_t) map), "r"(c), "r"(w), "r"(h),
+                 "r"(n), "r"(bar_cluster), "h"(ow), "h"(oh)
+                 : "memory");
+}
+
+}  // namespace w
+
 // 32 lanes x 32 consecutive 32-bit columns: thread i of the warp gets lane
 // (base lane + i), columns col..col+31.
 __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[32]) {

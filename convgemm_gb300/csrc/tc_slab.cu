@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(288, 1)
     float *sc_tab = (float *) (bars + 32);                  // 256 bytes of barriers above
     float *sh_tab = sc_tab + SLAB_BN;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = tc::w::warp_index(), lane = threadIdx.x & 31;
     const int n0 = (blockIdx.x % p.ntn) * SLAB_BN;          // this CTA's N tile
     const int m_first = blockIdx.x / p.ntn, m_step = gridDim.x / p.ntn;
     if (threadIdx.x == 0) {
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(288, 1)
 
     if (warp == 0) {
         // ------------------------------------------------ producer: one slab load per (tile, channel block)
-        if (lane == 0) {
+        {
             uint32_t it = 0;
             for (int m = m_first; m < p.mtiles && ok; m += m_step) {
                 if (m + m_step >= p.mtiles) tc::pdl_trigger();   // this CTA's last tile
@@ -130,9 +130,9 @@ __global__ void __launch_bounds__(288, 1)
                 for (int cb = 0; cb < p.cblocks; cb++, it++) {
                     const int s = it % p.nbuf;
                     const uint32_t ph = (it / p.nbuf) & 1;
-                    if (it >= (uint32_t) p.nbuf && !(ok = tc::mbar_wait(&slab_free[s], ph ^ 1, p.err, 51))) break;
-                    tc::mbar_arrive_expect_tx(&slab_full[s], p.slab_tx);
-                    tc::tma_load_4d(tc::smem_u32(slab + (size_t) s * p.buf_bytes), &xmap, cb * 64, ox0 + p.tx0,
+                    if (it >= (uint32_t) p.nbuf && !(ok = tc::w::mbar_wait(&slab_free[s], ph ^ 1, p.err, 51))) break;
+                    tc::w::mbar_arrive_expect_tx(&slab_full[s], p.slab_tx);
+                    tc::w::tma_load_4d(tc::smem_u32(slab + (size_t) s * p.buf_bytes), &xmap, cb * 64, ox0 + p.tx0,
                                    oy0 + p.ty0, b, &slab_full[s]);
                 }
             }
@@ -185,25 +185,25 @@ __global__ void __launch_bounds__(288, 1)
         }
         if (et == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else if (warp == 8 || (warp >= 1 && warp < p.niss)) {
-        // ------------------------------------------------ MMA issuers: lane 0 of warp 8 (issuer 0) and
-        // of warps 1 .. niss-1; issuer k takes this CTA's tiles k, k + niss, ..., each into its own
+        // ------------------------------------------------ MMA issuers: warp 8 (issuer 0) and warps
+        // 1 .. niss-1; issuer k takes this CTA's tiles k, k + niss, ..., each into its own
         // accumulator buffer (one thread's instruction stream cannot issue N = 64 MMAs as fast as
         // the tensor core runs them)
-        if (lane == 0) {
+        {
             const uint32_t me = warp == 8 ? 0u : (uint32_t) warp;
             constexpr uint32_t idesc = tc::idesc_bf16(128, SLAB_BN, 0, 0);
             const uint32_t wbase = tc::smem_u32(wres);
             uint32_t ao[SLAB_MAXTAPS];   // tap row offsets in registers (no table loads between the MMAs)
 #pragma unroll
             for (int t = 0; t < SLAB_MAXTAPS; t++) ao[t] = p.aoff[t];
-            if (!(ok = tc::mbar_wait(wfull, 0, p.err, 50))) ok = false;
+            if (!(ok = tc::w::mbar_wait(wfull, 0, p.err, 50))) ok = false;
             tc::tc_fence_after();
             for (uint32_t lt = me, m = m_first + me * m_step; (int) m < p.mtiles && ok;
                  lt += p.niss, m += p.niss * m_step) {
                 const uint32_t it = lt * p.cblocks;   // the producer's slab index of this tile's first block
                 const int buf = lt % SLAB_ACC;
                 if (lt >= (uint32_t) SLAB_ACC) {
-                    if (!(ok = tc::mbar_wait(&acc_empty[buf], ((lt / SLAB_ACC) + 1) & 1, p.err, 54))) break;
+                    if (!(ok = tc::w::mbar_wait(&acc_empty[buf], ((lt / SLAB_ACC) + 1) & 1, p.err, 54))) break;
                     tc::tc_fence_after();
                 }
                 const uint32_t dt = tmem + (uint32_t) (buf * SLAB_BN);
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(288, 1)
                 int sbuf[SLAB_MAXBUF];
                 for (int cb = 0; cb < p.cblocks && ok; cb++) {
                     sbuf[cb] = (it + cb) % p.nbuf;
-                    ok = tc::mbar_wait(&slab_full[sbuf[cb]], ((it + cb) / p.nbuf) & 1, p.err, 52);
+                    ok = tc::w::mbar_wait(&slab_full[sbuf[cb]], ((it + cb) / p.nbuf) & 1, p.err, 52);
                 }
                 if (!ok) break;
                 tc::tc_fence_after();
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(288, 1)
                         if (t >= p.ntaps) break;
                         const uint64_t ad = a0 + (ao[t] >> 4), bd = b0 + (uint64_t) t * (8192 >> 4);
 #pragma unroll
-                        for (int k = 0; k < 4; k++) tc::mma_f16(dt, ad + 2 * k, bd + 2 * k, idesc, (t | k) != 0);
+                        for (int k = 0; k < 4; k++) tc::w::mma_f16(dt, ad + 2 * k, bd + 2 * k, idesc, (t | k) != 0);
                     }
                 } else {
                     uint64_t ab[SLAB_MAXBUF];
@@ -240,12 +240,12 @@ __global__ void __launch_bounds__(288, 1)
                             const uint64_t bd = b0 + (uint64_t) (t * p.cblocks + cb) * (8192 >> 4);
 #pragma unroll
                             for (int k = 0; k < 4; k++)
-                                tc::mma_f16(dt, ad + 2 * k, bd + 2 * k, idesc, (cb | t | k) != 0);
+                                tc::w::mma_f16(dt, ad + 2 * k, bd + 2 * k, idesc, (cb | t | k) != 0);
                         }
                     }
                 }
-                for (int cb = 0; cb < p.cblocks; cb++) tc::mma_commit(&slab_free[sbuf[cb]]);
-                tc::mma_commit(&acc_full[buf]);
+                for (int cb = 0; cb < p.cblocks; cb++) tc::w::mma_commit(&slab_free[sbuf[cb]]);
+                tc::w::mma_commit(&acc_full[buf]);
             }
         }
         __syncwarp();

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(288, 1)
     uint32_t *aoff_tab = (uint32_t *) (sh_tab + BN);
     uint32_t *alead_tab = aoff_tab + STEM_MAXPAIRS;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = tc::w::warp_index(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int b = 0; b < 2; b++) {
             tc::mbar_init(&slab_full[b], 1);
@@ -169,18 +169,18 @@ __global__ void __launch_bounds__(288, 1)
 
     if (warp == 0) {
         // ------------------------------------------------ producer: the slab TMA loads of each tile
-        if (lane == 0) {
+        {
             uint32_t lt = 0;
             for (int tile = blockIdx.x; tile < p.total && ok; tile += gridDim.x, lt++) {
                 if (tile + (int) gridDim.x >= p.total) tc::pdl_trigger();   // this CTA's last tile
                 const int sb = lt & 1;
-                if (lt >= 2 && !(ok = tc::mbar_wait(&slab_free[sb], ((lt >> 1) + 1) & 1, p.err, 41))) break;
+                if (lt >= 2 && !(ok = tc::w::mbar_wait(&slab_free[sb], ((lt >> 1) + 1) & 1, p.err, 41))) break;
                 const int row = tile / p.nwc, wc = tile % p.nwc;
                 const int b = row / p.Ho, oy = row % p.Ho;
                 const uint32_t dst = tc::smem_u32(slab + sb * p.buf_bytes);
-                tc::mbar_arrive_expect_tx(&slab_full[sb], p.slab_tx);
+                tc::w::mbar_arrive_expect_tx(&slab_full[sb], p.slab_tx);
                 for (int rho = 0; rho < p.sw; rho++)
-                    tc::tma_load_4d(dst + rho * p.rho_bytes, &xmap, 0, p.sw * (128 * wc + p.qmin) + rho,
+                    tc::w::tma_load_4d(dst + rho * p.rho_bytes, &xmap, 0, p.sw * (128 * wc + p.qmin) + rho,
                                 oy * p.sh - p.pad_h, b, &slab_full[sb]);
             }
         }
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(288, 1)
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else if (warp == 8) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc = tc::idesc_bf16(128, BN, 0, 0);
             const uint32_t wbase = tc::smem_u32(wres);
             // the low descriptor words of every pair's A operand (start within a slab buffer,
@@ -259,20 +259,20 @@ __global__ void __launch_bounds__(288, 1)
             for (int tile = blockIdx.x; tile < p.total && ok; tile += gridDim.x, lt++) {
                 const int sb = lt & 1, buf = lt & 1;
                 if (lt >= 2) {
-                    if (!(ok = tc::mbar_wait(&acc_empty[buf], ((lt >> 1) + 1) & 1, p.err, 44))) break;
+                    if (!(ok = tc::w::mbar_wait(&acc_empty[buf], ((lt >> 1) + 1) & 1, p.err, 44))) break;
                     tc::tc_fence_after();
                 }
-                if (!(ok = tc::mbar_wait(&slab_full[sb], (lt >> 1) & 1, p.err, 45))) break;
+                if (!(ok = tc::w::mbar_wait(&slab_full[sb], (lt >> 1) & 1, p.err, 45))) break;
                 tc::tc_fence_after();
                 const uint32_t a0 = tc::smem_u32(slab + sb * p.buf_bytes);
                 const uint32_t dt = tmem + (uint32_t) (buf * BN);
 #pragma unroll
                 for (int q = 0; q < STEM_MAXPAIRS; q++)
                     if (q < p.npairs)
-                        tc::mma_f16(dt, dhi | (uint64_t) (alo[q] + ((a0 & 0x3FFFF) >> 4)),
+                        tc::w::mma_f16(dt, dhi | (uint64_t) (alo[q] + ((a0 & 0x3FFFF) >> 4)),
                                     kmajor_desc(wbase + q * C::PAIR_W, BN * 16), idesc, q > 0);
-                tc::mma_commit(&slab_free[sb]);
-                tc::mma_commit(&acc_full[buf]);
+                tc::w::mma_commit(&slab_free[sb]);
+                tc::w::mma_commit(&acc_full[buf]);
             }
         }
         __syncwarp();

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(320, 1)
     uint64_t *accum = dy_empty + SW_DYB;
     uint32_t *tmem_holder = (uint32_t *) (accum + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = tc::w::warp_index(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         // one MMA issuer per tap pair (warps 1, 7, 8, 9) commits to every consumer barrier
         for (int s = 0; s < 2; s++) {
@@ -98,25 +98,25 @@ __global__ void __launch_bounds__(320, 1)
 
     if (warp == 0) {
         // ------------------------------------------------ producer: the slab rows of each band
-        if (lane == 0) {
+        {
             for (int k = 0; k < nb; k++) {
                 const int s = k & 1;
-                if (k >= 2 && !(ok = tc::mbar_wait(&empty[s], ((k >> 1) + 1) & 1, p.err, 61))) break;
+                if (k >= 2 && !(ok = tc::w::mbar_wait(&empty[s], ((k >> 1) + 1) & 1, p.err, 61))) break;
                 const int band = (int) blockIdx.x + k * (int) gridDim.x;
                 const int b = band / p.bands_per_img, oy0 = (band - b * p.bands_per_img) * SW_R;
                 const uint32_t st = tc::smem_u32(base + s * SW_SLAB_MAX);
-                tc::mbar_arrive_expect_tx(&full[s], p.tx);
+                tc::w::mbar_arrive_expect_tx(&full[s], p.tx);
                 for (int y = 0; y < p.nyl; y++)
 #pragma unroll
                     for (int sm = 0; sm < 2; sm++)
-                        tc::tma_load_4d(st + (2 * y + sm) * p.pitch, &xmap, 0, p.col0[sm], 2 * oy0 - p.pad_h + y, b,
+                        tc::w::tma_load_4d(st + (2 * y + sm) * p.pitch, &xmap, 0, p.col0[sm], 2 * oy0 - p.pad_h + y, b,
                                         &full[s]);
             }
         }
         __syncwarp();
     } else if (warp == 6) {
         // ------------------------------------------------ producer: dY, one output row per buffer
-        if (lane == 0) {
+        {
             int dq = 0;
             for (int k = 0; k < nb && ok; k++) {
                 const int band = (int) blockIdx.x + k * (int) gridDim.x;
@@ -124,10 +124,10 @@ __global__ void __launch_bounds__(320, 1)
                 const int rows = min(SW_R, p.Ho - oy0);
                 for (int r = 0; r < rows; r++, dq++) {
                     const int d = dq % SW_DYB;
-                    if (dq >= SW_DYB && !(ok = tc::mbar_wait(&dy_empty[d], ((dq / SW_DYB) + 1) & 1, p.err, 64)))
+                    if (dq >= SW_DYB && !(ok = tc::w::mbar_wait(&dy_empty[d], ((dq / SW_DYB) + 1) & 1, p.err, 64)))
                         break;
-                    tc::mbar_arrive_expect_tx(&dy_full[d], (uint32_t) p.wpad * 128);
-                    tc::tma_load_3d(tc::smem_u32(dyb + d * SW_DY_MAX), &dymap, 0, 0, b * p.Ho + oy0 + r, &dy_full[d]);
+                    tc::w::mbar_arrive_expect_tx(&dy_full[d], (uint32_t) p.wpad * 128);
+                    tc::w::tma_load_3d(tc::smem_u32(dyb + d * SW_DY_MAX), &dymap, 0, 0, b * p.Ho + oy0 + r, &dy_full[d]);
                 }
             }
         }
@@ -135,13 +135,13 @@ __global__ void __launch_bounds__(320, 1)
     } else if (warp == 1 || warp >= 7) {
         // ------------------------------------------------ MMA issuers: one per tap pair, warp 1 pair 0,
         // warps 7-9 pairs 1-3 (one thread's loop overhead between MMAs bounds its issue rate)
-        if (lane == 0) {
+        {
             const int m = warp == 1 ? 0 : warp - 6;
             constexpr uint32_t idesc = tc::idesc_bf16(128, 64, 1, 1);
             int dq = 0;
             for (int k = 0; k < nb && ok; k++) {
                 const int s = k & 1;
-                if (!(ok = tc::mbar_wait(&full[s], (k >> 1) & 1, p.err, 62))) break;
+                if (!(ok = tc::w::mbar_wait(&full[s], (k >> 1) & 1, p.err, 62))) break;
                 tc::tc_fence_after();
                 const int band = (int) blockIdx.x + k * (int) gridDim.x;
                 const int b = band / p.bands_per_img, oy0 = (band - b * p.bands_per_img) * SW_R;
@@ -152,20 +152,20 @@ __global__ void __launch_bounds__(320, 1)
                 const uint64_t a0 = tc::mn_interleave_desc(sa, 128, p.pitch);
                 for (int r = 0; r < rows; r++, dq++) {
                     const int d = dq % SW_DYB;
-                    if (!(ok = tc::mbar_wait(&dy_full[d], (dq / SW_DYB) & 1, p.err, 65))) break;
+                    if (!(ok = tc::w::mbar_wait(&dy_full[d], (dq / SW_DYB) & 1, p.err, 65))) break;
                     tc::tc_fence_after();
                     const uint64_t b0 = tc::sw128_desc(tc::smem_u32(dyb + d * SW_DY_MAX), 8192, 1024);
                     for (int ks = 0; ks < p.nks; ks++) {
                         const uint64_t bd = b0 + (uint64_t) (ks * 128);
                         const uint64_t ar = a0 + (uint64_t) ((4 * r * p.pitch + 256 * ks) >> 4);
                         if (m < p.npairs)
-                            tc::mma_f16(tmem + (uint32_t) (64 * m), ar + (uint64_t) m, bd, idesc, (k | r | ks) != 0);
+                            tc::w::mma_f16(tmem + (uint32_t) (64 * m), ar + (uint64_t) m, bd, idesc, (k | r | ks) != 0);
                     }
-                    tc::mma_commit(&dy_empty[d]);
+                    tc::w::mma_commit(&dy_empty[d]);
                 }
-                tc::mma_commit(&empty[s]);
+                tc::w::mma_commit(&empty[s]);
             }
-            tc::mma_commit(accum);
+            tc::w::mma_commit(accum);
         }
         __syncwarp();
     } else if (warp < 6) {

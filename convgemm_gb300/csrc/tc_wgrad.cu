@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(WgWarps<IM2C, ISS2>::THREADS, 1)
     uint64_t *xbar = accum + 2;   // four: the epilogue warps' copies of the exchanged blocks
 
     constexpr int GW = WgWarps<IM2C>::GW;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = tc::w::warp_index(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
             tc::mbar_init(&full[s], IM2C ? 1 : 32 * GW + 1);
@@ -243,9 +243,9 @@ __global__ void __launch_bounds__(WgWarps<IM2C, ISS2>::THREADS, 1)
     const bool push = !PAIR && PUSH_FITS && p.cluster && p.xchg;
 
     if (IM2C && warp < 4) {
-        // one thread: im2col TMA for each 64-channel X atom (a fixed tap and channel chunk
+        // warp 0: im2col TMA for each 64-channel X atom (a fixed tap and channel chunk
         // for the CTA, 64 consecutive pixels per stage) and tiled TMA for dY
-        if (threadIdx.x == 0) {
+        if (warp == 0) {
             int a_ci[C::X_ATOMS];
             uint16_t a_oy[C::X_ATOMS], a_ox[C::X_ATOMS];
 #pragma unroll
@@ -264,10 +264,10 @@ __global__ void __launch_bounds__(WgWarps<IM2C, ISS2>::THREADS, 1)
             for (int g = 0; g < NG; g++) {
                 const int s = g % STAGES;
                 const uint32_t ph = (g / STAGES) & 1;
-                if (g >= STAGES && !(ok = tc::mbar_wait(&empty[s], ph ^ 1, p.err, 11))) break;
+                if (g >= STAGES && !(ok = tc::w::mbar_wait(&empty[s], ph ^ 1, p.err, 11))) break;
                 const int nch = min(KB, KT - g * KB);
                 if (!PAIR || prank == 0)
-                    tc::mbar_arrive_expect_tx(&full[s], (PAIR ? 2 : 1) * nch * (C::X_ATOMS * C::ATOM_BYTES + C::DY_BYTES));
+                    tc::w::mbar_arrive_expect_tx(&full[s], (PAIR ? 2 : 1) * nch * (C::X_ATOMS * C::ATOM_BYTES + C::DY_BYTES));
                 const uint32_t fb = lead_full + (uint32_t) s * 8u;
                 for (int c = 0; c < nch; c++) {
                     const int pbase = (chunk0 + g * KB + c) * C::BK;
@@ -281,21 +281,21 @@ __global__ void __launch_bounds__(WgWarps<IM2C, ISS2>::THREADS, 1)
                         const uint32_t d = st0 + xoff + a * C::ATOM_BYTES;
                         if (PAIR) {
                             if (p.x2d)
-                                tc::tma_load_2d_pair(d, &xmap, a_ci[a], pbase, fb);
+                                tc::w::tma_load_2d_pair(d, &xmap, a_ci[a], pbase, fb);
                             else
-                                tc::tma_load_im2col_4d_pair(d, &xmap, a_ci[a], w0, h0, (int) b, a_ox[a], a_oy[a], fb);
+                                tc::w::tma_load_im2col_4d_pair(d, &xmap, a_ci[a], w0, h0, (int) b, a_ox[a], a_oy[a], fb);
                         } else if (p.x2d) {   // one tap: the atom's channels are columns a_ci of the [P][Cp] matrix
-                            tc::tma_load_2d(d, &xmap, a_ci[a], pbase, &full[s]);
+                            tc::w::tma_load_2d(d, &xmap, a_ci[a], pbase, &full[s]);
                         } else {
-                            tc::tma_load_im2col_4d(d, &xmap, a_ci[a], w0, h0, (int) b, a_ox[a], a_oy[a], &full[s]);
+                            tc::w::tma_load_im2col_4d(d, &xmap, a_ci[a], w0, h0, (int) b, a_ox[a], a_oy[a], &full[s]);
                         }
                     }
 #pragma unroll
                     for (int a = 0; a < C::DY_ATOMS; a++) {
                         if (PAIR)
-                            tc::tma_load_2d_pair(st0 + dyoff + a * C::ATOM_BYTES, &dymap, co0 + 64 * a, pbase, fb);
+                            tc::w::tma_load_2d_pair(st0 + dyoff + a * C::ATOM_BYTES, &dymap, co0 + 64 * a, pbase, fb);
                         else
-                            tc::tma_load_2d(st0 + dyoff + a * C::ATOM_BYTES, &dymap, co0 + 64 * a, pbase, &full[s]);
+                            tc::w::tma_load_2d(st0 + dyoff + a * C::ATOM_BYTES, &dymap, co0 + 64 * a, pbase, &full[s]);
                     }
                 }
             }
@@ -487,14 +487,14 @@ __global__ void __launch_bounds__(WgWarps<IM2C, ISS2>::THREADS, 1)
             }
         }
     } else if (warp == GW || (ISS2 && warp == GW + 1)) {
-        if (lane == 0 && (!PAIR || prank == 0)) {
+        if (!PAIR || prank == 0) {
             constexpr uint32_t idesc = tc::idesc_bf16(PAIR ? 256 : 128, BN, 1, 1);
             const int j = warp - GW;   // issuer: chunk parity it takes (ISS2), accumulator
             const uint32_t dt = tmem + (uint32_t) (j * BN);
             for (int g = 0; g < NG; g++) {
                 const int s = g % STAGES;
                 const uint32_t ph = (g / STAGES) & 1;
-                if (!tc::mbar_wait(&full[s], ph, p.err, 12)) {
+                if (!tc::w::mbar_wait(&full[s], ph, p.err, 12)) {
                     ok = false;
                     break;
                 }
@@ -510,20 +510,20 @@ __global__ void __launch_bounds__(WgWarps<IM2C, ISS2>::THREADS, 1)
 #pragma unroll
                     for (int k = 0; k < C::BK / 16; k++) {
                         if constexpr (PAIR)
-                            tc::mma_f16_pair(dt, ad + 128 * k, bd + 128 * k, idesc, (g | c | k) != 0);
+                            tc::w::mma_f16_pair(dt, ad + 128 * k, bd + 128 * k, idesc, (g | c | k) != 0);
                         else
-                            tc::mma_f16(dt, ad + 128 * k, bd + 128 * k, idesc, (g | (ISS2 ? 0 : c) | k) != 0);
+                            tc::w::mma_f16(dt, ad + 128 * k, bd + 128 * k, idesc, (g | (ISS2 ? 0 : c) | k) != 0);
                     }
                 }
                 if constexpr (PAIR)
-                    tc::mma_commit_pair(&empty[s], (uint16_t) 3);   // both CTAs' stage s is free
+                    tc::w::mma_commit_pair(&empty[s], (uint16_t) 3);   // both CTAs' stage s is free
                 else
-                    tc::mma_commit(&empty[s]);
+                    tc::w::mma_commit(&empty[s]);
             }
             if constexpr (PAIR)
-                tc::mma_commit_pair(accum, (uint16_t) 3);
+                tc::w::mma_commit_pair(accum, (uint16_t) 3);
             else
-                tc::mma_commit(accum);
+                tc::w::mma_commit(accum);
         }
         __syncwarp();
     }

@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(128, 2)
     uint64_t *empty = full + WS_MAXST;
     uint64_t *accum = empty + WS_MAXST;
     uint32_t *tmem_holder = (uint32_t *) (accum + 1);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = tc::w::warp_index(), lane = threadIdx.x & 31;
 
     // unit: (kernel row dy, input-block pair cp, output-channel tile ct); split: a band range
     const int unit = blockIdx.x;
@@ -110,26 +110,26 @@ __global__ void __launch_bounds__(128, 2)
     const uint32_t tmem = *tmem_holder;
     bool ok = true;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // producer: per band two input slabs and DYA dY atoms
         const uint32_t tx = 2 * p.x_box_rows * 128 + DYA * p.x_box_rows * 128;
         for (int i = 0; i < nb; i++) {
             const int s = i % p.stages;
             const uint32_t ph = (i / p.stages) & 1;
-            if (i >= p.stages && !(ok = tc::mbar_wait(&empty[s], ph ^ 1, p.err, 41))) break;
+            if (i >= p.stages && !(ok = tc::w::mbar_wait(&empty[s], ph ^ 1, p.err, 41))) break;
             const int band = band0 + i;
             const int b = band / p.bands_per_img, oy0 = (band % p.bands_per_img) * p.R;
             const uint32_t st = tc::smem_u32(base + (size_t) s * p.stage_bytes);
-            tc::mbar_arrive_expect_tx(&full[s], tx);
+            tc::w::mbar_arrive_expect_tx(&full[s], tx);
 #pragma unroll
             for (int a = 0; a < 2; a++)
-                tc::tma_load_4d(st + a * p.x_bytes, &xmap, cp * 128 + 64 * a, -p.padw, oy0 + dy * p.vdil - p.padh, b,
+                tc::w::tma_load_4d(st + a * p.x_bytes, &xmap, cp * 128 + 64 * a, -p.padw, oy0 + dy * p.vdil - p.padh, b,
                                 &full[s]);
 #pragma unroll
             for (int a = 0; a < DYA; a++)
-                tc::tma_load_4d(st + 2 * p.x_bytes + a * p.dy_bytes, &dymap, ct * BN + 64 * a, 0, oy0, b, &full[s]);
+                tc::w::tma_load_4d(st + 2 * p.x_bytes + a * p.dy_bytes, &dymap, ct * BN + 64 * a, 0, oy0, b, &full[s]);
         }
-    } else if (warp >= 1 && warp <= p.niss && lane == 0) {
+    } else if (warp >= 1 && warp <= p.niss) {
         // MMA issuers (warps 1..niss): issuer j takes the accumulators dx = j, j + niss, ...;
         // each waits for the band, issues its MMAs and commits once to the band's empty barrier
         // (count niss).  One thread's tcgen05 issue, barrier wait and commit cost tens of cycles
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(128, 2)
         for (int i = 0; i < nb; i++) {
             const int s = i % p.stages;
             const uint32_t ph = (i / p.stages) & 1;
-            if (!(ok = tc::mbar_wait(&full[s], ph, p.err, 42))) break;
+            if (!(ok = tc::w::mbar_wait(&full[s], ph, p.err, 42))) break;
             tc::tc_fence_after();
             const uint32_t st = tc::smem_u32(base + (size_t) s * p.stage_bytes);
             const uint64_t a0 = tc::sw128_desc(st, p.x_bytes, 1024);
@@ -148,12 +148,12 @@ __global__ void __launch_bounds__(128, 2)
                 // 16 rows of 128 B = 2048 B = 128 units of the descriptor's start field
                 const uint64_t bd = b0 + (uint64_t) (128 * k);
                 for (int dx = j; dx < p.kw; dx += p.niss)
-                    tc::mma_f16(tmem + (uint32_t) (dx * BN), a0 + (uint64_t) (128 * k + 8 * dx * p.hdil), bd, idesc,
+                    tc::w::mma_f16(tmem + (uint32_t) (dx * BN), a0 + (uint64_t) (128 * k + 8 * dx * p.hdil), bd, idesc,
                                 (i | k) != 0);
             }
-            tc::mma_commit(&empty[s]);
+            tc::w::mma_commit(&empty[s]);
         }
-        tc::mma_commit(&accum[0]);
+        tc::w::mma_commit(&accum[0]);
     }
     __syncwarp();
 
