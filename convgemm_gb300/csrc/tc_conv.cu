@@ -95,7 +95,6 @@ struct TcCfg {
     // warp 8 (EW = 4) or in the otherwise idle warp 1 (EW = 8)
     static constexpr int THREADS = EW == 8 ? 384 : 288;
     static constexpr int MMA_WARP = EW == 8 ? 1 : 8;
-    static constexpr int ISS2_WARP = EW == 8 ? 2 : 1;   // the second MMA issuer (an otherwise idle warp)
     static constexpr int NCH = BN / CW;   // output chunks of one accumulator
     // TMEM: MT accumulators of BN columns, double-buffered when 512 columns allow (four buffers
     // for tiles of <= 128 columns)
@@ -163,13 +162,13 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
     // items of a tile: (accumulator mt, 64-column chunk). Eight warps: the two warps of a TMEM lane quarter
     // take alternate items, or alternate tiles where a tile has one item (each tile's accumulator is then
     // released by four warps)
-    constexpr int NIT = MT * C::NCH;
-    constexpr bool ALT = EW == 8 && NIT == 1;
+    constexpr bool ALT = EW == 8 && MT * C::NCH == 1;
     constexpr int STEP = ALT ? 1 : EW / 4, TSTEP = ALT ? 2 : 1;
-    // Two MMA-issuing threads on the BF16 im2col path: one per M tile (MT = 2), or one per N half
-    // (MT = 1, BN >= 128).  One thread's instruction stream issues N <= 128 MMAs more slowly than the
-    // tensor core runs them; both wait for the same stage and commit to it.
-    constexpr bool SPLIT = IM2C && MODE == MODE_BF16 && (MT == 2 || BN >= 128);
+    // A tile covers p.nn <= BN output channels (a multiple of 16): the width that divides the channels into
+    // equal tiles, so that 192 or 272 channels do not pay for 256 and 512. The last of its nch 64-column
+    // chunks starts at nn - 64 and repeats columns of the one before (same values, stored twice).
+    const int nn = p.nn, nch = (nn + C::CW - 1) / C::CW, NIT = MT * nch;
+    auto chunk_col = [&](int chunk) { return max(0, min(chunk * C::CW, nn - C::CW)); };
     static_assert(IM2C || (KB == 1 && MODE == MODE_BF16), "the cp.async gather fills one BF16 K block per stage");
     static_assert(MT == 1 || (IM2C && MODE == MODE_BF16), "two M tiles per weight tile: BF16 im2col path only");
     extern __shared__ uint8_t smem_raw[];
@@ -195,12 +194,12 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
         for (int s = 0; s < STAGES; s++) {
             // im2col: the one expect_tx arrival; gather: 128 producer threads + the expect_tx
             tc::mbar_init(&full[s], IM2C ? 1 : 128 + 1);
-            tc::mbar_init(&empty[s], SPLIT ? 2 : 1);
+            tc::mbar_init(&empty[s], 1);
         }
         if (EXTRA == EXTRA_MASK || EXTRA == EXTRA_SUMS)
             for (int b = 0; b < 2 * EW; b++) tc::mbar_init(&mask_full[b], 1);
         for (int b = 0; b < C::ACC_BUFS; b++) {
-            tc::mbar_init(&acc_full[b], SPLIT ? 2 : 1);
+            tc::mbar_init(&acc_full[b], 1);
             tc::mbar_init(&acc_empty[b], ALT ? 128 : 32 * EW);
         }
         tc::fence_mbar_init();
@@ -244,13 +243,14 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
     const uint32_t tmem = *tmem_holder;
     bool ok = true;
 
-    if (IM2C && warp < 4 && warp != C::MMA_WARP && !(SPLIT && warp == C::ISS2_WARP)) {
+    if (IM2C && warp < 4 && warp != C::MMA_WARP) {
         // ------------------------------------------------ producer: one warp, im2col TMA for A, TMA for B
         if (warp == 0) {
             uint32_t it = 0;
+            const uint32_t b_bytes = (uint32_t) (C::NOPS * nn * C::ROWB);
             for (int tile = blockIdx.x; tile < p.ntiles_total && ok; tile += gridDim.x) {
                 if (tile + (int) gridDim.x >= p.ntiles_total) tc::pdl_trigger();   // this CTA's last tile
-                const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, BN, tile, MT);
+                const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, nn, tile, MT);
                 const ClsS &cl = cls_tab[tl.cls];
                 const int32_t *taps = tap_tab + tl.cls * TC_MAXTAPS;
                 const int ktiles = __shfl_sync(0xFFFFFFFFu, cl.ktiles, 0), kbeg = cl.kbeg, mint_y = cl.mint_y, mint_x = cl.mint_x;
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                     if (it >= (uint32_t) STAGES && !(ok = tc::w::mbar_wait(&empty[s], ph ^ 1, p.err, 1))) break;
                     const int nkb = min(KB, ktiles - kt);
                     const uint32_t sa = tc::smem_u32(base + s * C::STAGE_BYTES);
-                    tc::w::mbar_arrive_expect_tx(&full[s], nkb * (MT * C::A_BLOCK + C::B_BLOCK));
+                    tc::w::mbar_arrive_expect_tx(&full[s], nkb * (MT * C::A_BLOCK + b_bytes));
                     for (int kb = 0; kb < nkb; kb++) {
                         const int32_t to = taps[tap];
                         const uint16_t offy = (uint16_t) ((to >> 16) - mint_y);
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
         uint32_t it = 0;
         for (int tile = blockIdx.x; tile < p.ntiles_total && ok; tile += gridDim.x) {
             if (t == 0 && tile + (int) gridDim.x >= p.ntiles_total) tc::pdl_trigger();   // this CTA's last tile
-            const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, BN, tile);
+            const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, nn, tile);
             const ClsS &cl = cls_tab[tl.cls];
             const int32_t *taps = tap_tab + tl.cls * TC_MAXTAPS;
             const int M = p.B * cl.Hg * cl.Wg;
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                 }
                 tc::cp_async_commit();
                 if (t == 0) {
-                    tc::mbar_arrive_expect_tx(&full[s], C::B_BYTES);
+                    tc::mbar_arrive_expect_tx(&full[s], (uint32_t) (nn * C::ROWB));
                     tc::tma_load_2d(tc::smem_u32(base + s * C::STAGE_BYTES + C::A_BYTES), &wmap,
                                     cl.kbeg + kt * C::BK, tl.n0, &full[s]);
                 }
@@ -382,10 +382,10 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
         // the mask_full barrier will tell of its arrival.
         uint64_t *const mbar = mask_full + 2 * (warp - 4);
         auto prefetch_mask = [&](int tile, int item, int buf) {
-            const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, BN, tile, MT);
+            const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, nn, tile, MT);
             const ClsS &cl = cls_tab[tl.cls];
             const int M = p.B * cl.Hg * cl.Wg;
-            const int r0 = tl.m0 + (item / C::NCH) * 128 + ew * 32, nb = tl.n0 + (item % C::NCH) * C::CW;
+            const int r0 = tl.m0 + (item / nch) * 128 + ew * 32, nb = tl.n0 + chunk_col(item % nch);
             const uint32_t dst = tc::smem_u32(stg_warp + buf * C::EPI_BYTES);
             if (p.epi_tma) {
                 if (r0 >= M || nb >= p.Cout) return false;
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
             if (p.mask && t0 < p.ntiles_total && first_item < NIT) by_tma = prefetch_mask(t0, first_item, 0);
         }
         for (int tile = blockIdx.x + (int) (lt * gridDim.x); tile < p.ntiles_total && ok; tile += TSTEP * gridDim.x, lt += TSTEP) {
-            const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, BN, tile, MT);
+            const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, nn, tile, MT);
             const ClsS &cl = cls_tab[tl.cls];
             const int M = p.B * cl.Hg * cl.Wg;
             const int buf = lt % C::ACC_BUFS;
@@ -447,9 +447,13 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
             ok = tc::mbar_wait(&acc_full[buf], (lt / C::ACC_BUFS) & 1, p.err, 3);
             if (!ok) break;
             tc::tc_fence_after();
+            if (first_item >= NIT) {   // nothing for this warp in the tile: its share of the buffer is free
+                tc::tc_fence_before();
+                tc::mbar_arrive(&acc_empty[buf]);
+            }
 #pragma unroll 1
             for (int item = first_item; item < NIT; item += STEP) {
-                const int mt = item / C::NCH, c0 = (item % C::NCH) * C::CW;
+                const int mt = item / nch, c0 = chunk_col(item % nch);
                 const int m0 = tl.m0 + mt * 128;   // this accumulator's first output row
                 const int m = m0 + row;
                 uint8_t *orow = nullptr;   // this row of the output (BF16, or FP32 for MODE_X3)
@@ -650,10 +654,10 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                         if (nb < p.Cout && m0 + ew * 32 < M) tma_store_2d(&omap, tc::smem_u32(stg), nb, m0 + ew * 32);
                         bulk_commit();   // a group per item, so that waiting for all but the last frees the other buffer
                     }
-                } else if (!C::OUTF32 && nb + C::CW <= p.Cout && __any_sync(0xFFFFFFFFu, orow != nullptr)) {
+                } else if (!C::OUTF32) {
                     // rows scattered over the output (stride-phase classes): staged through this warp's
                     // buffer, then each store instruction writes four whole 128-byte rows (eight lanes
-                    // per row) instead of 16 bytes of 32 rows
+                    // per row, Cout a multiple of their 8 channels) instead of 16 bytes of 32 rows
                     uint8_t *stg = stg_warp + ebuf * C::EPI_BYTES;
                     if (lane == 0 && C::EPI_BUFS == 2) bulk_wait_read<1>();
                     else if (lane == 0) bulk_wait_read<0>();
@@ -669,27 +673,19 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                         const int r = q * 4 + (lane >> 3), ch = lane & 7;
                         const unsigned long long dst = __shfl_sync(0xFFFFFFFFu, my, r);
                         const uint4 u = *reinterpret_cast<const uint4 *>(stg + r * 128 + ((ch ^ (r & 7)) << 4));
-                        if (dst) *reinterpret_cast<uint4 *>((uint8_t *) dst + ch * 16) = u;
+                        if (dst && nb + ch * 8 < p.Cout) *reinterpret_cast<uint4 *>((uint8_t *) dst + ch * 16) = u;
                     }
                     __syncwarp();
                 } else if (orow && nb < p.Cout) {
+                    float *o = reinterpret_cast<float *>(orow) + nb;
                     if (nb + C::CW <= p.Cout) {
-                        uint4 *dst = reinterpret_cast<uint4 *>(orow + (size_t) nb * (C::OUTF32 ? 4 : 2));
 #pragma unroll
-                        for (int q = 0; q < 8; q++) dst[q] = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-                    } else if (C::OUTF32) {
-                        float *o = reinterpret_cast<float *>(orow);
+                        for (int q = 0; q < 8; q++)
+                            reinterpret_cast<uint4 *>(o)[q] = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
+                    } else {
 #pragma unroll
                         for (int jj = 0; jj < 32; jj++)
-                            if (nb + jj < p.Cout) o[nb + jj] = __uint_as_float(pk[jj]);
-                    } else {
-                        bf16 *o = reinterpret_cast<bf16 *>(orow);
-#pragma unroll
-                        for (int jj = 0; jj < 32; jj++) {
-                            __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162 *>(&pk[jj]);
-                            if (nb + 2 * jj < p.Cout) o[nb + 2 * jj] = h.x;
-                            if (nb + 2 * jj + 1 < p.Cout) o[nb + 2 * jj + 1] = h.y;
-                        }
+                            if (nb + jj < p.Cout) o[jj] = __uint_as_float(pk[jj]);
                     }
                 }
                 if (C::EPI_BUFS == 2) ebuf ^= 1;
@@ -699,16 +695,11 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
     } else {
         // ------------------------------------------------ MMA issuer
         {
-            // issuer `me`: its M tile (MT = 2) or N half (MT = 1) when SPLIT, else everything
-            const int me = (SPLIT && warp == C::ISS2_WARP) ? 1 : 0;
-            constexpr int NI = (SPLIT && MT == 1) ? BN / 2 : BN;   // N of one MMA instruction
             constexpr bool F8 = MODE == MODE_FP8 || MODE == MODE_FP8W;
-            constexpr uint32_t idesc = F8 ? tc::idesc_e4m3(128, BN) : tc::idesc_bf16(128, NI, 0, 0);
-            const uint32_t n_off = (SPLIT && MT == 1) ? (uint32_t) (me * NI) : 0u;   // accumulator column
-            const uint64_t b_off = (SPLIT && MT == 1) ? (uint64_t) (me * NI * C::ROWB) >> 4 : 0u;   // B rows
+            const uint32_t idesc = (F8 ? tc::idesc_e4m3(128, 0) : tc::idesc_bf16(128, 0, 0, 0)) | (uint32_t) (nn >> 3) << 17;
             uint32_t it = 0, lt = 0;
             for (int tile = blockIdx.x; tile < p.ntiles_total && ok; tile += gridDim.x, lt++) {
-                const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, BN, tile, MT);
+                const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, nn, tile, MT);
                 const int KT = __shfl_sync(0xFFFFFFFFu, cls_tab[tl.cls].ktiles, 0);   // warp-uniform loop bounds
                 const int buf = lt % C::ACC_BUFS;
                 if (lt >= (uint32_t) C::ACC_BUFS) {
@@ -738,24 +729,23 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
 #pragma unroll
                         for (int k = 0; k < C::ROWB / 32; k++) {
                             const uint32_t acc = (kt | kb | k) != 0;
-                            const uint64_t bd = bd0 + ((kb * C::B_BLOCK + k * 32) >> 4) + b_off;
+                            const uint64_t bd = bd0 + ((kb * C::B_BLOCK + k * 32) >> 4);
 #pragma unroll
-                          for (int mt = 0; mt < MT; mt++) {
-                            if (SPLIT && MT == 2 && mt != me) continue;
-                            const uint64_t ad = ad0 + (((kb * MT + mt) * C::A_BLOCK + k * 32) >> 4);
-                            const uint32_t dtm = dt + (uint32_t) (mt * BN) + n_off;
-                            if (F8) {
-                                tc::w::mma_f8(dtm, ad, bd, idesc, acc);
-                            } else {
-                                tc::w::mma_f16(dtm, ad, bd, idesc, acc);
-                                if (MODE == MODE_X3) {
-                                    const uint64_t adl = ad + (C::A_TILE >> 4);
-                                    const uint64_t bdl = bd + (C::B_TILE >> 4);
-                                    tc::w::mma_f16(dtm, ad, bdl, idesc, 1);   // hi * lo
-                                    tc::w::mma_f16(dtm, adl, bd, idesc, 1);   // lo * hi
+                            for (int mt = 0; mt < MT; mt++) {
+                                const uint64_t ad = ad0 + (((kb * MT + mt) * C::A_BLOCK + k * 32) >> 4);
+                                const uint32_t dtm = dt + (uint32_t) (mt * BN);
+                                if (F8) {
+                                    tc::w::mma_f8(dtm, ad, bd, idesc, acc);
+                                } else {
+                                    tc::w::mma_f16(dtm, ad, bd, idesc, acc);
+                                    if (MODE == MODE_X3) {
+                                        const uint64_t adl = ad + (C::A_TILE >> 4);
+                                        const uint64_t bdl = bd + (C::B_TILE >> 4);
+                                        tc::w::mma_f16(dtm, ad, bdl, idesc, 1);   // hi * lo
+                                        tc::w::mma_f16(dtm, adl, bd, idesc, 1);   // lo * hi
+                                    }
                                 }
                             }
-                          }
                         }
                     }
                     tc::w::mma_commit(&empty[s]);

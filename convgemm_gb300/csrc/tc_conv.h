@@ -46,6 +46,7 @@ struct TcConvParams {
     int *err;                  // device error word for timed-out waits
     int bn;                    // output channels per tile (64, 128, 256)
     int ntiles;                // tiles along the output channels
+    int nn;                    // output channels per tile in use: Cout / ntiles rounded up to 16, at most bn
     int ntiles_total;          // all tiles of all classes; tile t of a class: m = t / ntiles, n = t % ntiles
     int epi_tma;               // output pixels are the GEMM rows in order: stage in SMEM, TMA store
     int im2col;                // A loaded by im2col-mode TMA, else gathered by cp.async

@@ -6,15 +6,23 @@
 // width and epilogue.  The tiles of all problems are numbered consecutively
 // (problem-major; inside a problem, pixel tiles x channel tiles with the
 // channel tile fastest); persistent CTAs walk them blockIdx.x, +gridDim.x, ...
-// The tile width (64/128/256 output channels) is a per-problem runtime value:
-// shared memory and TMEM are sized for 256 and the MMA instruction descriptor
-// carries N, so one launch mixes tile shapes chosen per shape by the autotuner.
+// The tile width is a per-problem runtime value: at most 64 / 128 / 256 output
+// channels (chosen per shape by the autotuner), divided into equal tiles of whole
+// 16-column MMA widths, so that 272 channels make two tiles of 144 and not two of
+// 256.  Shared memory and TMEM are sized for 256 and the MMA instruction
+// descriptor carries N, so one launch mixes tile shapes.
 //
-// Warp roles as in tc_conv.cu: warp 0 lane 0 issues the im2col TMA for the
-// activations and the tiled TMA for the weights; warps 4-7 drain TMEM through
-// the fused scale/shift/ReLU epilogue and TMA-store BF16; warp 8 owns TMEM and
-// issues tcgen05.mma.  Channels that are not a multiple of 64 are read as
-// 64-channel boxes whose tail TMA zero-fills; the packed weights carry zeros there.
+// Warp roles as in tc_conv.cu's form with eight epilogue warps: warp 0 issues the
+// im2col TMA for the activations and the tiled TMA for the weights, warp 1 owns
+// TMEM and issues tcgen05.mma, warps 4-11 drain TMEM through the fused
+// scale/shift/ReLU epilogue and TMA-store BF16 (the two warps of a lane quarter
+// take alternate 64-column chunks).  Each role keeps its problem's fields in
+// registers while its tiles stay in one problem.  Channels that are not a multiple
+// of 64 are read as 64-channel boxes whose tail TMA zero-fills; the packed weights
+// carry zeros there.
+//
+// What bounds it: the tensor cores at the power-limited clock on the long
+// reductions, and padding: 16 k channels fill whole 64-channel blocks.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -33,9 +41,9 @@ using bf16 = __nv_bfloat16;
 
 struct alignas(64) GroupProblem {
     CUtensorMap amap;   // im2col map of x: 128 pixels x 64 channels per load
-    CUtensorMap wmap;   // packed weights [kn][taps * c64]: box 64 x bn
+    CUtensorMap wmap;   // packed weights [kn][taps * c64]: box 64 x nn
     CUtensorMap omap;   // y as [pixels][kn]: box 64 x 32 (one epilogue warp's rows)
-    int tile0, tile_end, count, ntiles_n, bn, M;   // count: convolutions in the table
+    int tile0, tile_end, count, ntiles_n, nn, M;   // count: convolutions in the table; nn: channels per tile
     int ktiles, cpb, isy, isx, lo_y, lo_x, Cout, relu;
     uint32_t idesc;
     FastDiv dwg, dhg;
@@ -44,32 +52,38 @@ struct alignas(64) GroupProblem {
 };
 
 constexpr int GBN = 256;
-constexpr int GSTAGES = 4;
+constexpr int GSTAGES = 3, GEW = 8;
+constexpr int GTHREADS = 32 * (4 + GEW);
 constexpr uint32_t A_BYTES = 128 * 128;
 constexpr uint32_t B_MAX = GBN * 128;
 constexpr uint32_t STAGE_BYTES = A_BYTES + B_MAX;
-constexpr uint32_t EPI_BYTES = 128 * 128;   // one 64-column chunk of a tile (4 KB per epilogue warp)
-constexpr size_t GSMEM = 1024 + GSTAGES * STAGE_BYTES + EPI_BYTES + 256 + 2 * GBN * 4;
+constexpr uint32_t EPI_BYTES = GEW * 4096;   // one 32 x 64 staging chunk per epilogue warp; two buffers
+constexpr size_t GSMEM = 1024 + GSTAGES * STAGE_BYTES + 2 * EPI_BYTES + 256 + 2 * GBN * 4;
 static_assert(GSMEM <= 232448, "shared memory above the 227 KB per-block limit");
 
-__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(32 * GEW) : "memory"); }
 
-__device__ __forceinline__ int advance(const GroupProblem *probs, int nprob, int pi, int tile) {
-    while (pi + 1 < nprob && tile >= __ldg(&probs[pi + 1].tile0)) pi++;
-    return pi;
+// The problem of a tile and its tile range; true when it changed.
+__device__ __forceinline__ bool advance(const GroupProblem *probs, int nprob, int tile, int &pi, int &end) {
+    if (pi >= 0 && tile < end) return false;
+    do {
+        pi++;
+        end = __ldg(&probs[pi].tile_end);
+    } while (tile >= end && pi + 1 < nprob);
+    return true;
 }
 
-__global__ void __launch_bounds__(288, 1)
+__global__ void __launch_bounds__(GTHREADS, 1)
     tc_group_kernel(const GroupProblem *__restrict__ probs, int nprob, int total, int *err) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *base = (uint8_t *) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023);
     uint8_t *epi = base + GSTAGES * STAGE_BYTES;
-    uint64_t *full = (uint64_t *) (epi + EPI_BYTES);
+    uint64_t *full = (uint64_t *) (epi + 2 * EPI_BYTES);
     uint64_t *empty = full + GSTAGES;
     uint64_t *acc_full = empty + GSTAGES;
     uint64_t *acc_empty = acc_full + 2;
     uint32_t *tmem_holder = (uint32_t *) (acc_empty + 2);
-    float *sc_tab = (float *) (epi + EPI_BYTES + 256);
+    float *sc_tab = (float *) (epi + 2 * EPI_BYTES + 256);
     float *sh_tab = sc_tab + GBN;
 
     const int warp = tc::w::warp_index(), lane = threadIdx.x & 31;
@@ -87,11 +101,11 @@ __global__ void __launch_bounds__(288, 1)
         }
         for (int b = 0; b < 2; b++) {
             tc::mbar_init(&acc_full[b], 1);
-            tc::mbar_init(&acc_empty[b], 128);
+            tc::mbar_init(&acc_empty[b], 32 * GEW);
         }
         tc::fence_mbar_init();
     }
-    if (warp == 8) {
+    if (warp == 1) {
         tc::tmem_alloc(tmem_holder, 2 * GBN);
         tc::tmem_relinquish();
     }
@@ -100,76 +114,101 @@ __global__ void __launch_bounds__(288, 1)
     tc::tc_fence_after();
     const uint32_t tmem = *tmem_holder;
     bool ok = true;
+    int pi = -1, pend = 0;
 
-    if (warp < 4) {
-        if (warp == 0) {
-            // ---------------------------------------------- producer
-            uint32_t it = 0;
-            int pi = 0;
-            for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
-                if (tile + (int) gridDim.x >= total) tc::pdl_trigger();   // this CTA's last tile
-                pi = advance(probs, nprob, pi, tile);
-                const GroupProblem *P = probs + pi;
-                const int local = tile - __ldg(&P->tile0), ntn = __ldg(&P->ntiles_n), bn = __ldg(&P->bn);
-                const int m0 = (local / ntn) * 128, n0 = (local % ntn) * bn;
-                const int ktiles = __shfl_sync(0xFFFFFFFFu, __ldg(&P->ktiles), 0), cpb = __ldg(&P->cpb);
-                const FastDiv dwg = P->dwg, dhg = P->dhg;
-                uint32_t q, jw, j, b;
-                dwg.divmod(m0, q, jw);
-                dhg.divmod(q, b, j);
-                const int h0 = (int) j * __ldg(&P->isy) + __ldg(&P->lo_y);
-                const int w0 = (int) jw * __ldg(&P->isx) + __ldg(&P->lo_x);
-                const uint32_t tx_bytes = A_BYTES + (uint32_t) bn * 128;
-                int tap = 0, cc = 0;
-                int32_t to = __ldg(&P->taps[0]), to_next = __ldg(&P->taps[1]);   // the next tap's offsets, loaded ahead
-                for (int kt = 0; kt < ktiles; kt++, it++) {
-                    const int s = it % GSTAGES;
-                    const uint32_t ph = (it / GSTAGES) & 1;
-                    if (it >= (uint32_t) GSTAGES && !(ok = tc::w::mbar_wait(&empty[s], ph ^ 1, err, 21))) break;
-                    const uint32_t sa = tc::smem_u32(base + s * STAGE_BYTES);
-                    tc::w::mbar_arrive_expect_tx(&full[s], tx_bytes);
-                    tc::w::tma_load_im2col_4d(sa, &P->amap, cc * 64, w0, h0, (int) b, (uint16_t) (to & 0xFFFF),
-                                           (uint16_t) (to >> 16), &full[s]);
-                    tc::w::tma_load_2d(sa + A_BYTES, &P->wmap, kt * 64, n0, &full[s]);
-                    if (++cc == cpb) {
-                        cc = 0;
-                        tap++;
-                        to = to_next;
-                        to_next = __ldg(&P->taps[min(tap + 1, TC_MAXTAPS - 1)]);
-                    }
+    if (warp == 0) {
+        // ---------------------------------------------- producer
+        uint32_t it = 0, tx_bytes = 0;
+        const GroupProblem *P = nullptr;
+        int tile0 = 0, ntn = 1, nn = 0, ktiles = 0, cpb = 1, isy = 0, isx = 0, lo_y = 0, lo_x = 0;
+        FastDiv dwg, dhg;
+        for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
+            if (tile + (int) gridDim.x >= total) tc::pdl_trigger();   // this CTA's last tile
+            if (advance(probs, nprob, tile, pi, pend)) {
+                P = probs + pi;
+                tile0 = __ldg(&P->tile0);
+                ntn = __ldg(&P->ntiles_n);
+                nn = __ldg(&P->nn);
+                ktiles = __shfl_sync(0xFFFFFFFFu, __ldg(&P->ktiles), 0);   // warp-uniform loop bounds
+                cpb = __ldg(&P->cpb);
+                isy = __ldg(&P->isy);
+                isx = __ldg(&P->isx);
+                lo_y = __ldg(&P->lo_y);
+                lo_x = __ldg(&P->lo_x);
+                dwg = P->dwg;
+                dhg = P->dhg;
+                tx_bytes = A_BYTES + (uint32_t) nn * 128;
+            }
+            const int local = tile - tile0, mt = local / ntn, n0 = (local - mt * ntn) * nn;
+            uint32_t q, jw, j, b;
+            dwg.divmod(mt * 128, q, jw);
+            dhg.divmod(q, b, j);
+            const int h0 = (int) j * isy + lo_y, w0 = (int) jw * isx + lo_x;
+            int tap = 0, cc = 0;
+            int32_t to = __ldg(&P->taps[0]), to_next = __ldg(&P->taps[1]);   // the next tap's offsets, loaded ahead
+            for (int kt = 0; kt < ktiles; kt++, it++) {
+                const int s = it % GSTAGES;
+                const uint32_t ph = (it / GSTAGES) & 1;
+                if (it >= (uint32_t) GSTAGES && !(ok = tc::w::mbar_wait(&empty[s], ph ^ 1, err, 21))) break;
+                const uint32_t sa = tc::smem_u32(base + s * STAGE_BYTES);
+                tc::w::mbar_arrive_expect_tx(&full[s], tx_bytes);
+                tc::w::tma_load_im2col_4d(sa, &P->amap, cc * 64, w0, h0, (int) b, (uint16_t) (to & 0xFFFF),
+                                          (uint16_t) (to >> 16), &full[s]);
+                tc::w::tma_load_2d(sa + A_BYTES, &P->wmap, kt * 64, n0, &full[s]);
+                if (++cc == cpb) {
+                    cc = 0;
+                    tap++;
+                    to = to_next;
+                    to_next = __ldg(&P->taps[min(tap + 1, TC_MAXTAPS - 1)]);
                 }
             }
         }
-    } else if (warp < 8) {
+    } else if (warp >= 4) {
         // -------------------------------------------------- epilogue
-        const int ew = warp - 4, row = ew * 32 + lane, et = threadIdx.x - 128;
+        const int ew = (warp - 4) & 3, half = (warp - 4) >> 2, et = threadIdx.x - 128;
         uint32_t lt = 0;
-        int pi = 0;
+        int ebuf = 0;
+        const GroupProblem *P = nullptr;
+        int tile0 = 0, ntn = 1, nn = 0, Cout = 0, relu = 0, M = 0;
+        const float *scale = nullptr, *shift = nullptr;
         for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, lt++) {
-            pi = advance(probs, nprob, pi, tile);
-            const GroupProblem *P = probs + pi;
-            const int local = tile - __ldg(&P->tile0), ntn = __ldg(&P->ntiles_n), bn = __ldg(&P->bn);
-            const int m0 = (local / ntn) * 128, n0 = (local % ntn) * bn;
-            const int Cout = __ldg(&P->Cout), relu = __ldg(&P->relu), M = __ldg(&P->M);
-            const float *scale = P->scale, *shift = P->shift;
+            if (advance(probs, nprob, tile, pi, pend)) {
+                P = probs + pi;
+                tile0 = __ldg(&P->tile0);
+                ntn = __ldg(&P->ntiles_n);
+                nn = __ldg(&P->nn);
+                Cout = __ldg(&P->Cout);
+                relu = __ldg(&P->relu);
+                M = __ldg(&P->M);
+                scale = P->scale;
+                shift = P->shift;
+            }
+            const int local = tile - tile0, mt = local / ntn, m0 = mt * 128, n0 = (local - mt * ntn) * nn;
+            const int nch = (nn + 63) / 64;
             epi_bar();   // the previous tile's readers of the tables are done
-            for (int jj = et; jj < bn; jj += 128) {
-                const int n = min(n0 + jj, Cout - 1);
-                sc_tab[jj] = scale ? __ldg(scale + n) : 1.0f;
-                sh_tab[jj] = shift ? __ldg(shift + n) : 0.0f;
+            if (et < nn) {
+                const int n = min(n0 + et, Cout - 1);
+                sc_tab[et] = scale ? __ldg(scale + n) : 1.0f;
+                sh_tab[et] = shift ? __ldg(shift + n) : 0.0f;
             }
             epi_bar();
             const int buf = lt & 1;
             ok = tc::mbar_wait(&acc_full[buf], (lt >> 1) & 1, err, 23);
             if (!ok) break;
             tc::tc_fence_after();
-            for (int c0 = 0; c0 < bn; c0 += 64) {
+            if (half >= nch) {   // one chunk: the other four warps take it
+                tc::tc_fence_before();
+                tc::mbar_arrive(&acc_empty[buf]);
+            }
+#pragma unroll 1
+            for (int ch = half; ch < nch; ch += 2) {
+                const int c0 = max(0, min(ch * 64, nn - 64));   // the last chunk repeats columns of the one before
                 uint32_t v0[32], v1[32];
                 const uint32_t ta = tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * GBN + c0);
                 tc::tmem_ld_32x32b_x32(ta, v0);
                 tc::tmem_ld_32x32b_x32(ta + 32, v1);
                 tc::tmem_ld_wait();
-                if (c0 + 64 >= bn) {
+                if (ch + 2 >= nch) {
                     tc::tc_fence_before();
                     tc::mbar_arrive(&acc_empty[buf]);
                 }
@@ -179,67 +218,66 @@ __global__ void __launch_bounds__(288, 1)
                 else
                     tc::epi_bf16_64<false>(v0, v1, sc_tab + c0, sh_tab + c0, pk);
                 // each warp stages its 32 rows and stores them itself: no barrier across warps
-                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                 __syncwarp();
-                uint8_t *stg = epi + ew * (EPI_BYTES / 4);
+                uint8_t *stg = epi + ebuf * EPI_BYTES + (warp - 4) * 4096;
 #pragma unroll
                 for (int qq = 0; qq < 8; qq++)
                     *reinterpret_cast<uint4 *>(stg + lane * 128 + ((qq ^ (lane & 7)) << 4)) =
                         make_uint4(pk[4 * qq], pk[4 * qq + 1], pk[4 * qq + 2], pk[4 * qq + 3]);
                 tc::fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0 && n0 + c0 < Cout && m0 + ew * 32 < M) {
-                    asm volatile(
-                        "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                            (uint64_t) &P->omap),
-                        "r"(tc::smem_u32(stg)), "r"(n0 + c0), "r"(m0 + ew * 32)
-                        : "memory");
-                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                if (lane == 0) {
+                    if (n0 + c0 < Cout && m0 + ew * 32 < M)
+                        asm volatile(
+                            "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+                                (uint64_t) &P->omap),
+                            "r"(tc::smem_u32(stg)), "r"(n0 + c0), "r"(m0 + ew * 32)
+                            : "memory");
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");   // a group per chunk: the waits count them
                 }
+                ebuf ^= 1;
             }
         }
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-    } else {
+    } else if (warp == 1) {
         // -------------------------------------------------- MMA issuer
-        {
-            uint32_t it = 0, lt = 0;
-            int pi = 0;
-            for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, lt++) {
-                pi = advance(probs, nprob, pi, tile);
-                const GroupProblem *P = probs + pi;
-                const int ktiles = __shfl_sync(0xFFFFFFFFu, __ldg(&P->ktiles), 0);   // warp-uniform loop bounds
-                const uint32_t idesc = __ldg(&P->idesc);
-                const int buf = lt & 1;
-                if (lt >= 2) {
-                    ok = tc::w::mbar_wait(&acc_empty[buf], ((lt >> 1) - 1) & 1, err, 24);
-                    if (!ok) break;
-                    tc::tc_fence_after();
-                }
-                const uint32_t dt = tmem + (uint32_t) (buf * GBN);
-                for (int kt = 0; kt < ktiles; kt++, it++) {
-                    const int s = it % GSTAGES;
-                    const uint32_t ph = (it / GSTAGES) & 1;
-                    if (!tc::w::mbar_wait(&full[s], ph, err, 22)) {
-                        ok = false;
-                        break;
-                    }
-                    tc::tc_fence_after();
-                    // descriptors built once per stage; a 32-byte K step adds 2 to the start field
-                    const uint64_t ad = tc::sw128_desc(tc::smem_u32(base + s * STAGE_BYTES), 16, 1024);
-                    const uint64_t bd = ad + (A_BYTES >> 4);
-#pragma unroll
-                    for (int k = 0; k < 4; k++) tc::w::mma_f16(dt, ad + 2 * k, bd + 2 * k, idesc, (kt | k) != 0);
-                    tc::w::mma_commit(&empty[s]);
-                }
-                tc::w::mma_commit(&acc_full[buf]);
+        uint32_t it = 0, lt = 0, idesc = 0;
+        int ktiles = 0;
+        for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, lt++) {
+            if (advance(probs, nprob, tile, pi, pend)) {
+                ktiles = __shfl_sync(0xFFFFFFFFu, __ldg(&probs[pi].ktiles), 0);
+                idesc = __shfl_sync(0xFFFFFFFFu, __ldg(&probs[pi].idesc), 0);
             }
+            const int buf = lt & 1;
+            if (lt >= 2) {
+                ok = tc::w::mbar_wait(&acc_empty[buf], ((lt >> 1) - 1) & 1, err, 24);
+                if (!ok) break;
+                tc::tc_fence_after();
+            }
+            const uint32_t dt = tmem + (uint32_t) (buf * GBN);
+            for (int kt = 0; kt < ktiles; kt++, it++) {
+                const int s = it % GSTAGES;
+                const uint32_t ph = (it / GSTAGES) & 1;
+                if (!tc::w::mbar_wait(&full[s], ph, err, 22)) {
+                    ok = false;
+                    break;
+                }
+                tc::tc_fence_after();
+                // descriptors built once per stage; a 32-byte K step adds 2 to the start field
+                const uint64_t ad = tc::sw128_desc(tc::smem_u32(base + s * STAGE_BYTES), 16, 1024);
+                const uint64_t bd = ad + (A_BYTES >> 4);
+#pragma unroll
+                for (int k = 0; k < 4; k++) tc::w::mma_f16(dt, ad + 2 * k, bd + 2 * k, idesc, (kt | k) != 0);
+                tc::w::mma_commit(&empty[s]);
+            }
+            tc::w::mma_commit(&acc_full[buf]);
         }
-        __syncwarp();
     }
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
-    if (warp == 8) tc::tmem_dealloc(tmem, 2 * GBN);
+    if (warp == 1) tc::tmem_dealloc(tmem, 2 * GBN);
 }
 
 inline int rup(int v, int m) { return (v + m - 1) / m * m; }
@@ -295,6 +333,15 @@ extern "C" convgemm_status_t convgemm_group_prepare(int n, const convgemm_group_
         return (long long) s.kh * s.kw * rup(s.c > 0 ? s.c : 1, 64);
     };
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return klen(a) > klen(b); });
+    // width where the caller names none: 256 channels, or 128 / 64 by the channel count where tiles that wide
+    // would not give every SM two
+    long long wide = 0;
+    for (int i = 0; i < n; i++) {
+        const convgemm_shape_t &s = convs[i].shape;
+        if (check_group_shape(s, fn)) continue;   // reported below
+        wide += (make_geom(cg_from_public(s)).P + 127) / 128 * ((s.kn + 255) / 256);
+    }
+    const bool wide_ok = wide >= 2LL * tc_num_sms();
     std::vector<GroupProblem> host(n);
     int t0 = 0;
     for (int oi = 0; oi < n; oi++) {
@@ -304,7 +351,10 @@ extern "C" convgemm_status_t convgemm_group_prepare(int n, const convgemm_group_
         if (!cv.x || !cv.w || !cv.y) return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "%s: conv %d has a NULL tensor", fn, i);
         const cg_shape s = cg_from_public(cv.shape);
         const ConvGeom g = make_geom(s);
-        const int bn = cv.bn == 64 || cv.bn == 128 || cv.bn == 256 ? cv.bn : (s.kn >= 256 ? 256 : (s.kn > 64 ? 128 : 64));
+        const int bn = cv.bn == 64 || cv.bn == 128 || cv.bn == 256 ? cv.bn : (s.kn >= 256 || wide_ok ? 256 : (s.kn > 64 ? 128 : 64));
+        const int ntn = (s.kn + bn - 1) / bn;
+        int nn = rup((s.kn + ntn - 1) / ntn, 16);   // equal tiles; two tiles never share a 64-column chunk
+        if (nn < 64 && ntn > 1) nn = 64;
         const int c64 = rup(s.c, 64);
         GroupProblem &P = host[oi];
         memset(&P, 0, sizeof(P));
@@ -316,7 +366,7 @@ extern "C" convgemm_status_t convgemm_group_prepare(int n, const convgemm_group_
                                                      s.vstride, s.hstride, 128, 2))
             return e;
         if (convgemm_status_t e = tc_make_map_2d(&P.wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, cv.w, s.kn,
-                                                 s.kh * s.kw * c64, 64, bn))
+                                                 s.kh * s.kw * c64, 64, nn))
             return e;
         if (convgemm_status_t e = tc_make_map_2d(&P.omap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, cv.y, g.P, s.kn, 64, 32))
             return e;
@@ -324,8 +374,8 @@ extern "C" convgemm_status_t convgemm_group_prepare(int n, const convgemm_group_
             return cg_set_error(CONVGEMM_ERROR_NOT_SUPPORTED, "%s: conv %d has more than 2^31 elements", fn, i);
         P.tile0 = t0;
         P.count = n;
-        P.ntiles_n = (s.kn + bn - 1) / bn;
-        P.bn = bn;
+        P.ntiles_n = ntn;
+        P.nn = nn;
         P.M = (int) g.P;
         P.cpb = c64 / 64;
         P.ktiles = s.kh * s.kw * P.cpb;
@@ -335,7 +385,7 @@ extern "C" convgemm_status_t convgemm_group_prepare(int n, const convgemm_group_
         P.lo_x = lo_x;
         P.Cout = s.kn;
         P.relu = cv.relu;
-        P.idesc = tc::idesc_bf16(128, bn, 0, 0);
+        P.idesc = tc::idesc_bf16(128, nn, 0, 0);
         P.dwg = FastDiv(g.wo);
         P.dhg = FastDiv(g.ho);
         P.scale = cv.scale;
@@ -368,7 +418,7 @@ extern "C" convgemm_status_t convgemm_group_launch(const void *table, int n, int
     }
     const int sms = tc_num_sms();
     const int grid = total_tiles < sms ? total_tiles : sms;
-    return cg_cuda_check(cg_launch_pdl(tc_group_kernel, dim3(grid), dim3(288), GSMEM, (cudaStream_t) stream,
+    return cg_cuda_check(cg_launch_pdl(tc_group_kernel, dim3(grid), dim3(GTHREADS), GSMEM, (cudaStream_t) stream,
                                        (const GroupProblem *) table, n, total_tiles, err),
                          "grouped kernel launch");
 }

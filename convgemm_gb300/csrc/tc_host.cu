@@ -291,22 +291,22 @@ int tc_num_sms() {
 // Tile forms of tc_conv_kernel and what a tile costs (microseconds): `block` per 64-channel K block (FP8W: 128
 // channels), at least `epi` (the epilogue of short reductions, behind which the MMAs hide), `launch` once.
 // Fitted to 64 forward and input-gradient shapes (31 geometries from 1 x 14 x 14 to 32 x 56 x 56) with every form
-// forced: the form with the lowest estimate is within 0.6% of the best one on average. The rule before
+// forced: the form with the lowest estimate is within 1% of the best one on average. The rule before
 // (tiles x width, equal for all widths, so the narrowest won on wave rounding) was 26% off: 28 x 28, 512 -> 512
-// 3 x 3 at batch 32 took 199 us with the 64-wide tiles it chose and takes 81 with 256.
+// 3 x 3 at batch 32 takes 132 us with the 64-wide tiles it chose and 67 with 256.
 struct TileForm {
     int bn, mt, ew;
     float block, epi, launch;
 };
-constexpr TileForm FORMS_BF16[] = {{64, 1, 4, 0.270f, 0.92f, 3.5f}, {128, 1, 4, 0.280f, 1.62f, 4.2f}, {128, 1, 8, 0.296f, 1.30f, 4.25f},
-                                   {128, 2, 8, 0.459f, 2.13f, 4.6f}, {256, 1, 8, 0.363f, 2.01f, 4.9f}};
+constexpr TileForm FORMS_BF16[] = {{64, 1, 4, 0.180f, 1.10f, 3.2f}, {128, 1, 4, 0.203f, 1.95f, 3.6f}, {128, 1, 8, 0.230f, 1.20f, 3.8f},
+                                   {128, 2, 8, 0.332f, 2.05f, 4.6f}, {256, 1, 8, 0.313f, 1.95f, 4.6f}};
 // with a ReLU mask, or with column sums (batch statistics, a fused bias gradient) in the epilogue
-constexpr TileForm FORMS_MASK[] = {{64, 1, 8, 0.270f, 0.95f, 3.5f}, {128, 1, 8, 0.296f, 1.85f, 4.25f}, {256, 1, 8, 0.363f, 3.50f, 4.9f}};
-constexpr TileForm FORMS_SUMS[] = {{64, 1, 8, 0.270f, 1.30f, 3.5f}, {128, 1, 8, 0.296f, 2.80f, 4.25f}, {256, 1, 8, 0.363f, 5.00f, 4.9f}};
-constexpr TileForm FORMS_GATHER[] = {{64, 1, 4, 0.60f, 1.95f, 3.5f}, {128, 1, 4, 0.63f, 2.10f, 4.0f}, {256, 1, 4, 0.80f, 3.00f, 4.9f}};
-constexpr TileForm FORMS_FP8[] = {{64, 1, 4, 0.200f, 0.87f, 3.4f}, {128, 1, 4, 0.210f, 1.47f, 3.9f}, {256, 1, 4, 0.270f, 2.70f, 4.7f}};
-constexpr TileForm FORMS_FP8W[] = {{64, 1, 4, 0.255f, 0.87f, 3.4f}, {128, 1, 4, 0.270f, 1.47f, 3.9f}, {256, 1, 4, 0.360f, 2.70f, 4.7f}};
-constexpr TileForm FORMS_X3[] = {{64, 1, 4, 0.560f, 1.17f, 3.4f}, {128, 1, 4, 0.580f, 2.00f, 4.0f}, {256, 1, 4, 0.900f, 3.80f, 4.9f}};
+constexpr TileForm FORMS_MASK[] = {{64, 1, 8, 0.190f, 0.95f, 3.2f}, {128, 1, 8, 0.230f, 1.85f, 3.8f}, {256, 1, 8, 0.313f, 3.50f, 4.6f}};
+constexpr TileForm FORMS_SUMS[] = {{64, 1, 8, 0.190f, 1.30f, 3.2f}, {128, 1, 8, 0.230f, 2.80f, 3.8f}, {256, 1, 8, 0.313f, 5.00f, 4.6f}};
+constexpr TileForm FORMS_GATHER[] = {{64, 1, 4, 0.58f, 1.95f, 3.2f}, {128, 1, 4, 0.61f, 2.10f, 3.8f}, {256, 1, 4, 0.75f, 3.00f, 4.6f}};
+constexpr TileForm FORMS_FP8[] = {{64, 1, 4, 0.107f, 0.92f, 3.2f}, {128, 1, 4, 0.130f, 1.50f, 3.6f}, {256, 1, 4, 0.185f, 2.75f, 4.6f}};
+constexpr TileForm FORMS_FP8W[] = {{64, 1, 4, 0.150f, 0.92f, 3.2f}, {128, 1, 4, 0.200f, 1.50f, 3.6f}, {256, 1, 4, 0.306f, 2.75f, 4.6f}};
+constexpr TileForm FORMS_X3[] = {{64, 1, 4, 0.335f, 1.43f, 3.2f}, {128, 1, 4, 0.440f, 2.60f, 3.6f}, {256, 1, 4, 0.870f, 4.90f, 4.6f}};
 
 // The plan's K blocks hold `kdiv` blocks of 64 channels each; *cost_out: the form's estimate.
 template <int N>
@@ -336,11 +336,11 @@ TileForm cheapest_form(const TileForm (&forms)[N], const TcPlan &pl, int kdiv, i
 // Whether the BF16 kernel loads the gathered operand by im2col TMA (pl's classes then count whole 64-channel K
 // blocks per tap). With channels in blocks of 64 always. Else each tap's last block is padded with zeros and
 // rows straddle cache lines, which makes a block TAIL_COST times as expensive, but still cheaper than one gathered
-// by threads (0.6 us against 0.27 for 64-wide tiles): it pays unless the blocks are mostly padding.
+// by threads (0.6 us against 0.36 for 64-wide tiles): it pays unless the blocks are mostly padding.
 // 14 x 14, 328 -> 200 3 x 3, batch 32 (54 blocks for 47): 31.7 -> 23.1 us; 56 x 56, 104 -> 312 1 x 1, batch 24 (2 for 2):
 // 44 -> 20 us; 28 x 28, 72 -> 72 3 x 3, batch 64 (18 for 11): 26.4 gathered, 42.8 by TMA. The rule depends on the
 // plan alone, so that every form of a layer adds its products in the same order.
-constexpr float TAIL_COST = 1.55f;
+constexpr float TAIL_COST = 2.0f;
 bool tc_use_im2col(TcPlan &pl, int sms) {
     TcPlan pi = pl;
     if (!tc_plan_im2col(pi)) return false;
@@ -407,10 +407,15 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
         if (pi.cls[c].kbeg % 128 || pi.cls[c].ktiles % 2) f8w = false;
     const TileForm form = tc_pick_form(pi, f8w ? 3 : mode, p.im2col, mask != nullptr, stats != nullptr, sms);
     p.bn = bn_override ? bn_override : form.bn;
+    p.ntiles = (pl.Cout + p.bn - 1) / p.bn;
+    // equal tiles of whole 16-column MMA widths; a single chunk of 64 columns is never shared by two tiles,
+    // and an accumulating call, which must not add a repeated column twice, keeps whole chunks
+    p.nn = round_up((pl.Cout + p.ntiles - 1) / p.ntiles, accum ? 64 : 16);
+    if (p.nn < 64 && p.ntiles > 1) p.nn = 64;
     const int eb = mode == 1 ? 1 : 2;   // operand element bytes
     CUtensorMap wmap, omap;
     if (convgemm_status_t e = tc_make_map_2d_sw(&wmap, eb == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
-                                                eb, wpacked, pl.Cout, pl.Ktot, 64, p.bn,
+                                                eb, wpacked, pl.Cout, pl.Ktot, 64, p.nn,
                                                 eb == 1 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B))
         return e;
     const TcClass &c0 = pl.cls[0];
@@ -444,7 +449,6 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     p.dcin = FastDiv(pl.Cin);
     p.err = cg_device_error_word();
     if (!p.err) return cg_set_error(CONVGEMM_ERROR_CUDA, "device error word unavailable");
-    p.ntiles = (pl.Cout + p.bn - 1) / p.bn;
     p.ncls = pl.ncls;
     TcMaps amaps;
     memset(&amaps, 0, sizeof(amaps));
@@ -454,7 +458,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
             return e;
     if (f8w) {
         if (convgemm_status_t e = tc_make_map_2d_sw(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wpacked, pl.Cout, pl.Ktot,
-                                                    128, p.bn, CU_TENSOR_MAP_SWIZZLE_128B))
+                                                    128, p.nn, CU_TENSOR_MAP_SWIZZLE_128B))
             return e;
     }
     if (p.im2col) {
@@ -464,7 +468,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
             if (p.wtail) {
                 const unsigned long long dims[3] = {(unsigned long long) pl.Cin, (unsigned long long) cl.ntaps, (unsigned long long) pl.Cout};
                 const unsigned long long str[2] = {(unsigned long long) pl.Cin * 2, (unsigned long long) pl.Ktot * 2};
-                const unsigned box[3] = {64, 1, (unsigned) p.bn}, estr[3] = {1, 1, 1};
+                const unsigned box[3] = {64, 1, (unsigned) p.nn}, estr[3] = {1, 1, 1};
                 if (convgemm_status_t e = tc_make_map_nd(&amaps.w[c], 3, (const uint16_t *) wpacked + cl.kbeg, dims, str, box, estr, 1))
                     return e;
             }
@@ -480,7 +484,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
         }
         if (mode == 2)
             if (convgemm_status_t e =
-                    tc_make_map_2d(&amaps.wlo, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w_lo, pl.Cout, pl.Ktot, 64, p.bn))
+                    tc_make_map_2d(&amaps.wlo, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w_lo, pl.Cout, pl.Ktot, 64, p.nn))
                 return e;
     }
     // aux (tuning): bits 0-1 the M tiles per weight tile (1 / 2: BF16 im2col path only), bit 2
@@ -767,15 +771,15 @@ size_t wgrad_xchg_bytes(const WgPlan &w) {
 // The weight gradient's tiles and pixel splits where no tuning entry names them (im2col path), as the
 // flags an entry would hold. A CTA's cost (microseconds): `chunk` per 128 pixels, `tile` and `launch` once;
 // then what adds the splits up: nothing for one, the cluster exchange for 2 or 4 (8 only on small grids:
-// clusters of eight leave SMs without a place), the reduction kernels (planes at 5 TB/s) otherwise and for
+// clusters of eight leave SMs without a place), the reduction kernels (planes at 4.5 TB/s) otherwise and for
 // pairs. Fitted to 32 shapes with every combination forced: 2% off the best on average, where the rule
 // before (64-pixel chunks, one wave, the slab kernel for 128-channel blocks) was 50% off: 28 x 28,
-// 512 -> 512 3 x 3 at batch 32 126 -> 77 us, 14 x 14, 256 -> 256 at batch 1 45 -> 4.8 us.
+// 512 -> 512 3 x 3 at batch 32 126 -> 73 us, 14 x 14, 256 -> 256 at batch 1 45 -> 4.4 us.
 struct WgForm {
     int bn, pair;
     float chunk, tile, launch;
 };
-constexpr WgForm WG_FORMS[] = {{64, 0, 0.435f, 3.66f, 0.1f}, {128, 0, 0.464f, 5.26f, -0.9f}, {128, 1, 0.454f, 5.04f, -0.4f}, {256, 1, 0.610f, 7.06f, -1.3f}};
+constexpr WgForm WG_FORMS[] = {{64, 0, 0.257f, 4.34f, -0.7f}, {128, 0, 0.375f, 5.67f, -1.8f}, {128, 1, 0.347f, 4.89f, -0.7f}, {256, 1, 0.584f, 6.46f, -1.1f}};
 
 TcTune pick_wgrad(const cg_shape &s, const ConvGeom &g) {
     const int sms = tc_num_sms(), Nx = s.kh * s.kw * round_up(s.c, 64), nch = (int) ((g.P + 127) / 128);
@@ -799,7 +803,7 @@ TcTune pick_wgrad(const cg_shape &s, const ConvGeom &g) {
                 const int cps = (nch + sp - 1) / sp, n = (nch + cps - 1) / cps;
                 if (!f.pair && n > 1 && n <= 8 && n != 2 && n != 4 && !(n == 8 && tiles * n <= 96)) continue;
                 float cost = f.launch + (float) ((tiles * n + sms - 1) / sms) * ((float) cps * f.chunk + f.tile);
-                if (n > 1) cost += !f.pair && n <= 8 ? 2.8f : 5.4f + (float) n * (float) Nx * (float) s.kn * 4.0f / 5.0e6f;
+                if (n > 1) cost += !f.pair && n <= 8 ? 2.4f : 5.6f + (float) n * (float) Nx * (float) s.kn * 4.0f / 4.5e6f;
                 if (best_cost < 0.0f || cost < best_cost) {
                     best_cost = cost;
                     best.bn = f.bn;

@@ -1,0 +1,88 @@
+"""GPU tests of output tiles that are not a power of two wide: the output channels are divided into equal
+tiles of whole 16-column MMA widths, whose last 64-column chunk repeats columns of the chunk before (BF16
+stores) and is cut to whole chunks where the output is accumulated.
+
+Reference: FP64 convolutions of the same BF16 tensors.  BF16 outputs: one rounding (2^-9 of the value, two
+where the output is accumulated) plus FP32 accumulation, 6e-3 of the largest value as for the other forms.
+FP32 outputs of the 3xBF16 form: products to 2^-16, 1e-4 of the largest value."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+WIDTHS = [16, 48, 72, 80, 144, 192, 272, 400]
+
+
+def nmax(got, want):
+    return ((got.double() - want).abs().max() / want.abs().max()).item()
+
+
+def tensors(cg, kn, stride, seed):
+    s = cg.Shape.of(3, 15, 13, 64, kn, 3, 3, 1, 1, stride, stride)
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(3, 15, 13, 64, device="cuda", generator=g)
+    wt = torch.randn(64, 3, 3, kn, device="cuda", generator=g) * (2 / 576) ** 0.5
+    return s, x, wt, g
+
+
+@pytest.mark.parametrize("bn", [0, 64, 128, 256])
+@pytest.mark.parametrize("kn", WIDTHS)
+def test_forward_widths(cglib, kn, bn):
+    from convgemm_gb300 import tc
+    cg = cglib
+    s, x, wt, g = tensors(cg, kn, 1, kn)
+    xb, wb = x.to(torch.bfloat16), wt.to(torch.bfloat16)
+    z = torch.nn.functional.conv2d(xb.double().permute(0, 3, 1, 2), wb.double().permute(3, 0, 1, 2), padding=1)
+    z = z.permute(0, 2, 3, 1)
+    wp = torch.empty(tc.weights_size(s, tc.OPERAND_FWD) // 2, dtype=torch.bfloat16, device="cuda")
+    tc.pack_weights(cg.NHWC, s, tc.OPERAND_FWD, wb.float(), wp)
+    try:
+        tc.tune_set(tc.TUNE_FWD, s, bn, 1 if bn else 0)
+        y = torch.full((3, 15, 13, kn), float("nan"), dtype=torch.bfloat16, device="cuda")
+        tc.fwd_bf16(s, xb, wp, y)
+    finally:
+        tc.tune_set(tc.TUNE_FWD, s, 0, 0)
+    assert nmax(y, z) <= 6e-3
+
+    # grouped: the same tiles; the packing of 64 channels is the same
+    yg = torch.full_like(y, float("nan"))
+    tc.Group([{"shape": s, "x": xb, "w": wp, "y": yg, "bn": bn}]).launch()
+    assert nmax(yg, z) <= 6e-3
+
+    # 3xBF16, FP32 output
+    hi, lo = torch.empty_like(xb), torch.empty_like(xb)
+    tc.split_bf16x2(x, hi, lo)
+    wh, wl = torch.empty_like(wp), torch.empty_like(wp)
+    tc.bf16x3_pack_weights(cg.NHWC, s, wt, wh, wl)
+    y32 = torch.full((3, 15, 13, kn), float("nan"), device="cuda")
+    tc.fwd_bf16x3(s, hi, lo, wh, wl, y32)
+    z = torch.nn.functional.conv2d(x.double().permute(0, 3, 1, 2), wt.double().permute(3, 0, 1, 2), padding=1)
+    torch.cuda.synchronize()
+    cg.check_device()
+    assert nmax(y32, z.permute(0, 2, 3, 1)) <= 1e-4
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+@pytest.mark.parametrize("c", [16, 72, 144, 272])
+def test_input_gradient_widths(cglib, c, stride):
+    from convgemm_gb300 import tc
+    cg = cglib
+    s = cg.Shape.of(3, 15, 13, c, 64, 3, 3, 1, 1, stride, stride)
+    g = torch.Generator(device="cuda").manual_seed(c + stride)
+    x = torch.randn(3, 15, 13, c, device="cuda", generator=g).to(torch.bfloat16)
+    wt = (torch.randn(c, 3, 3, 64, device="cuda", generator=g) * (2 / 576) ** 0.5).to(torch.bfloat16).float()
+    dy = torch.randn(3, s.ho, s.wo, 64, device="cuda", generator=g).to(torch.bfloat16)
+    want = torch.nn.grad.conv2d_input((3, c, 15, 13), wt.double().permute(3, 0, 1, 2),
+                                      dy.double().permute(0, 3, 1, 2), stride=stride, padding=1).permute(0, 2, 3, 1)
+    wpd = torch.empty(tc.weights_size(s, tc.OPERAND_DGRAD) // 2, dtype=torch.bfloat16, device="cuda")
+    tc.pack_weights(cg.NHWC, s, tc.OPERAND_DGRAD, wt, wpd)
+    dx = torch.full_like(x, float("nan"))
+    tc.dgrad_bf16(s, dy, wpd, dx)
+    assert nmax(dx, want) <= 6e-3
+    tc.dgrad_bf16_ex(s, dy, wpd, dx, accumulate=True)
+    assert nmax(dx, 2 * want) <= 6e-3
+    masked = torch.full_like(x, float("nan"))
+    tc.dgrad_bf16_relu(s, dy, wpd, masked, x)
+    torch.cuda.synchronize()
+    cg.check_device()
+    assert nmax(masked, torch.where(x > 0, want, torch.zeros_like(want))) <= 6e-3
