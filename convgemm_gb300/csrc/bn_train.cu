@@ -148,6 +148,36 @@ __global__ void bn_apply_kernel(long long n8, int kn, const __nv_bfloat16 *z, co
     }
 }
 
+// dz = bf16(gy * (y > 0) * scale), 8 channels per thread step. One pass over memory (6 bytes per value) and one
+// launch for the five of the same expression in tensor operations; the products in their order, so that a NaN or
+// an infinity under the mask and the sign of a zero stay what they were.
+__global__ void epilogue_grad_kernel(uint32_t n8, uint32_t k8, const uint4 *__restrict__ gy, const uint4 *__restrict__ y,
+                                     const float *__restrict__ scale, uint4 *__restrict__ dz) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += gridDim.x * blockDim.x) {
+        const uint4 ug = gy[i], uy = y ? y[i] : ug;
+        const uint32_t wg[4] = {ug.x, ug.y, ug.z, ug.w}, wy[4] = {uy.x, uy.y, uy.z, uy.w};
+        const float *sc = scale ? scale + i % k8 * 8 : nullptr;
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const __nv_bfloat162 g = *reinterpret_cast<const __nv_bfloat162 *>(&wg[j]);
+            const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162 *>(&wy[j]);
+            float a = __bfloat162float(g.x), b = __bfloat162float(g.y);
+            if (y) {
+                a = __fmul_rn(a, __bfloat162float(v.x) > 0.0f ? 1.0f : 0.0f);
+                b = __fmul_rn(b, __bfloat162float(v.y) > 0.0f ? 1.0f : 0.0f);
+            }
+            if (sc) {
+                a = __fmul_rn(a, __ldg(sc + 2 * j));
+                b = __fmul_rn(b, __ldg(sc + 2 * j + 1));
+            }
+            const __nv_bfloat162 r = __floats2bfloat162_rn(a, b);
+            o[j] = *reinterpret_cast<const uint32_t *>(&r);
+        }
+        dz[i] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
+
 // statistics groups of the forward's path for this shape: the small-channel kernel
 // groups per (output row, 128-pixel chunk), the general kernel per 32 output pixels
 int stat_groups(const cg_shape &s, bool *stem) {
@@ -264,4 +294,17 @@ extern "C" convgemm_status_t convgemm_bn_apply_bf16(long long npix, int kn, cons
                                                                      relu, (__nv_bfloat16 *) y);
     cg_note_launch();
     return cg_cuda_check(cudaGetLastError(), "convgemm_bn_apply_bf16");
+}
+
+extern "C" convgemm_status_t convgemm_epilogue_grad_bf16(long long npix, int kn, const void *gy, const void *y,
+                                                         const float *scale, void *dz, void *stream) {
+    if (npix < 1 || kn < 8 || kn % 8 || !gy || !dz || npix > ((1LL << 31) - 1) / kn)
+        return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "convgemm_epilogue_grad_bf16: bad arguments (kn %% 8 == 0)");
+    if (((uintptr_t) gy & 15) || ((uintptr_t) y & 15) || ((uintptr_t) dz & 15))
+        return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "convgemm_epilogue_grad_bf16: tensors must be 16-byte aligned");
+    const uint32_t n8 = (uint32_t) (npix * (kn / 8)), blocks = (n8 + 255) / 256;
+    epilogue_grad_kernel<<<blocks < 152 * 16 ? blocks : 152 * 16, 256, 0, (cudaStream_t) stream>>>(
+        n8, (uint32_t) kn / 8, (const uint4 *) gy, (const uint4 *) y, scale, (uint4 *) dz);
+    cg_note_launch();
+    return cg_cuda_check(cudaGetLastError(), "convgemm_epilogue_grad_bf16");
 }

@@ -76,7 +76,7 @@ __global__ void pack_dgrad_kernel(const float *__restrict__ w, int nchw, int C, 
         const int k = col - info.kbeg[c];
         const int t = k / knp, co = k % knp;
         float v = 0.0f;
-        if (t < info.ntaps[c] && co < kn) v = wref(w, nchw, C, kh, kw, kn, ci, info.kx[c][t], info.ky[c][t], co);
+        if (t < info.ntaps[c] && co < kn) v = wref(w, nchw, C, kh, kw, kn, ci, info.kx[info.tap0[c] + t], info.ky[info.tap0[c] + t], co);
         out[i] = __float2bfloat16_rn(v);
     }
 }
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
             const int nt = J.info.ntaps[c], nci = min(4, C - ci0), w4 = nci * khw, pitch = (4 * khw) | 1, nco = min(run, knp - co0);
             float *buf = &tile[0][0];
             __shared__ int taps[TC_MAXTAPS];
-            if (t < nt) taps[t] = J.info.kx[c][t] * J.kw + J.info.ky[c][t];
+            if (t < nt) taps[t] = J.info.kx[J.info.tap0[c] + t] * J.kw + J.info.ky[J.info.tap0[c] + t];
             const float *src = J.w + ((size_t) co0 * C + ci0) * khw;
             const int have = J.kn - co0;
             for (int i = t; i < nco * w4; i += 256) {
@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
                         const int g = (int) J.dknp.div((uint32_t) idx), co = idx - g * J.knp;
                         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                         if (g < nt && co < J.kn) {
-                            const int tap = J.info.kx[c][g] * J.kw + J.info.ky[c][g];
+                            const int tap = J.info.kx[J.info.tap0[c] + g] * J.kw + J.info.ky[J.info.tap0[c] + g];
                             v = __ldg(reinterpret_cast<const float4 *>(J.w + ((size_t) ci * J.kh * J.kw + tap) * J.kn + co));
                         }
                         __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
                 for (int idx = t; idx < end - beg; idx += 256) {
                     const int g = (int) J.dknp.div((uint32_t) idx), co = idx - g * J.knp;
                     float v = 0.0f;
-                    if (g < nt && co < J.kn) v = wref(J.w, J.nchw, J.C, J.kh, J.kw, J.kn, ci, J.info.kx[c][g], J.info.ky[c][g], co);
+                    if (g < nt && co < J.kn) v = wref(J.w, J.nchw, J.C, J.kh, J.kw, J.kn, ci, J.info.kx[J.info.tap0[c] + g], J.info.ky[J.info.tap0[c] + g], co);
                     row[idx] = __float2bfloat16_rn(v);
                 }
             }

@@ -7,8 +7,8 @@
 // Where each stride-phase class of the input gradient sits in the packed operand.
 struct PackDgradInfo {
     int ncls, Ktot;
-    int kbeg[TC_MAXCLS], ntaps[TC_MAXCLS];
-    int8_t kx[TC_MAXCLS][TC_MAXTAPS], ky[TC_MAXCLS][TC_MAXTAPS];
+    int kbeg[TC_MAXCLS], tap0[TC_MAXCLS], ntaps[TC_MAXCLS];
+    int8_t kx[TC_MAXTAPS], ky[TC_MAXTAPS];   // taps of all classes, class c's from tap0[c]
 };
 
 // One job of the grouped preparation launch (prep_group_launch): a block range of

@@ -84,7 +84,7 @@ struct TcCfg {
     static constexpr int LAG = STAGES / 2;
     // shared tables: tap offsets, the class table, scale/shift (whole vectors up to 1024 channels)
     static constexpr size_t BAR_BYTES = 512;                   // mbarriers
-    static constexpr size_t TAB_BYTES = TC_MAXCLS * TC_MAXTAPS * 4 + TC_MAXCLS * 128 + 2 * 1024 * 4;
+    static constexpr size_t TAB_BYTES = TC_TAPTAB * 4 + TC_MAXCLS * 128 + 2 * 1024 * 4;
     // output staging buffers: two when they fit beside the stage ring, else one
     static constexpr int EPI_BUFS =
         (1024 + (size_t) STAGES * STAGE_BYTES + 2 * EPI_BYTES + BAR_BYTES + TAB_BYTES <= 232448) ? 2 : 1;
@@ -136,7 +136,7 @@ struct Tile {
 // kernel parameters with a runtime class index would cost generic-memory loads
 // on every tile).
 struct ClsS {
-    int Hg, Wg, oy0, ox0, osy, osx, isy, isx, iby, ibx, ntaps, kbeg, ktiles, tile0, lo_y, lo_x, mint_y, mint_x, gbase;
+    int Hg, Wg, oy0, ox0, osy, osx, isy, isx, iby, ibx, tap0, ntaps, kbeg, ktiles, tile0, lo_y, lo_x, mint_y, mint_x, gbase;
     FastDiv dwg, dhg;
 };
 static_assert(sizeof(ClsS) <= 128, "class table entry");
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
     // per-class tap offsets (packed y:16 | x:16) and the tile's epilogue scale/shift, in shared
     // memory: indexing the kernel parameters with runtime values would go through slow generic loads
     int32_t *tap_tab = (int32_t *) (epi_smem + C::EPI_BUFS * C::EPI_BYTES + C::BAR_BYTES);
-    ClsS *cls_tab = (ClsS *) (tap_tab + TC_MAXCLS * TC_MAXTAPS);
+    ClsS *cls_tab = (ClsS *) (tap_tab + TC_TAPTAB);
     float *sc_tab = (float *) (cls_tab + TC_MAXCLS);   // [1024]: all channels, or the tile's BN
     float *sh_tab = sc_tab + 1024;
     const bool sc_all = p.Cout <= 1024;              // whole scale/shift vectors fit
@@ -208,19 +208,17 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
         if (IM2C)
             for (int c = 0; c < p.ncls; c++) {
                 tc::prefetch_tmap(&amaps.a[c]);
-                if (MODE == MODE_X3) tc::prefetch_tmap(&amaps.alo[c]);
+                if (MODE == MODE_X3) tc::prefetch_tmap(&amaps.b[c]);
             }
         if (MODE == MODE_X3) tc::prefetch_tmap(&amaps.wlo);
     }
-    for (int i = threadIdx.x; i < p.ncls * TC_MAXTAPS; i += blockDim.x) {
-        const int c = i / TC_MAXTAPS, t = i % TC_MAXTAPS;
-        tap_tab[i] = ((int32_t) p.cls[c].toy[t] << 16) | ((int32_t) p.cls[c].tox[t] & 0xFFFF);
-    }
+    for (int i = threadIdx.x; i < TC_MAXTAPS; i += blockDim.x)
+        tap_tab[i] = ((int32_t) p.toy[i] << 16) | ((int32_t) p.tox[i] & 0xFFFF);
     if (threadIdx.x < (unsigned) p.ncls) {
         const TcClass &c = p.cls[threadIdx.x];
         ClsS &d = cls_tab[threadIdx.x];
         d.Hg = c.Hg; d.Wg = c.Wg; d.oy0 = c.oy0; d.ox0 = c.ox0; d.osy = c.osy; d.osx = c.osx;
-        d.isy = c.isy; d.isx = c.isx; d.iby = c.iby; d.ibx = c.ibx; d.ntaps = c.ntaps; d.kbeg = c.kbeg;
+        d.isy = c.isy; d.isx = c.isx; d.iby = c.iby; d.ibx = c.ibx; d.tap0 = c.tap0; d.ntaps = c.ntaps; d.kbeg = c.kbeg;
         d.ktiles = c.ktiles; d.tile0 = c.tile0; d.lo_y = c.lo_y; d.lo_x = c.lo_x; d.mint_y = c.mint_y;
         d.mint_x = c.mint_x; d.gbase = c.gbase; d.dwg = c.dwg; d.dhg = c.dhg;
     }
@@ -252,7 +250,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                 if (tile + (int) gridDim.x >= p.ntiles_total) tc::pdl_trigger();   // this CTA's last tile
                 const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, nn, tile, MT);
                 const ClsS &cl = cls_tab[tl.cls];
-                const int32_t *taps = tap_tab + tl.cls * TC_MAXTAPS;
+                const int32_t *taps = tap_tab + cl.tap0;
                 const int ktiles = __shfl_sync(0xFFFFFFFFu, cl.ktiles, 0), kbeg = cl.kbeg, mint_y = cl.mint_y, mint_x = cl.mint_x;
                 int h0[MT], w0[MT], bb0[MT];   // im2col start of each M tile (beyond the class: zero-filled)
 #pragma unroll
@@ -283,10 +281,10 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                         for (int mt = 0; mt < MT; mt++)
                             tc::w::tma_load_im2col_4d(ab + mt * C::A_BLOCK, am, ci0, w0[mt], h0[mt], bb0[mt], offx, offy,
                                                    &full[s]);
-                        if (MODE == MODE_BF16 && p.wtail) tc::w::tma_load_3d(bb, &amaps.w[tl.cls], ci0, tap, tl.n0, &full[s]);
+                        if (MODE == MODE_BF16 && p.wtail) tc::w::tma_load_3d(bb, &amaps.b[tl.cls], ci0, tap, tl.n0, &full[s]);
                         else tc::w::tma_load_2d(bb, &wmap, kcol, tl.n0, &full[s]);
                         if (MODE == MODE_X3) {
-                            tc::w::tma_load_im2col_4d(ab + C::A_TILE, &amaps.alo[tl.cls], ci0, w0[0], h0[0], bb0[0], offx,
+                            tc::w::tma_load_im2col_4d(ab + C::A_TILE, &amaps.b[tl.cls], ci0, w0[0], h0[0], bb0[0], offx,
                                                    offy, &full[s]);
                             tc::w::tma_load_2d(bb + C::B_TILE, &amaps.wlo, kcol, tl.n0, &full[s]);
                         }
@@ -309,7 +307,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
             if (t == 0 && tile + (int) gridDim.x >= p.ntiles_total) tc::pdl_trigger();   // this CTA's last tile
             const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, nn, tile);
             const ClsS &cl = cls_tab[tl.cls];
-            const int32_t *taps = tap_tab + tl.cls * TC_MAXTAPS;
+            const int32_t *taps = tap_tab + cl.tap0;
             const int M = p.B * cl.Hg * cl.Wg;
             int rb[8], ry[8], rx[8];
 #pragma unroll

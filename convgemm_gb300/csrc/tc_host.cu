@@ -120,10 +120,10 @@ bool tc_plan_im2col(TcPlan &pl) {
         TcClass &cl = pl.cls[c];
         int my = 1 << 30, mx = 1 << 30, Xy = -(1 << 30), Xx = -(1 << 30);
         for (int t = 0; t < cl.ntaps; t++) {
-            my = cl.toy[t] < my ? cl.toy[t] : my;
-            mx = cl.tox[t] < mx ? cl.tox[t] : mx;
-            Xy = cl.toy[t] > Xy ? cl.toy[t] : Xy;
-            Xx = cl.tox[t] > Xx ? cl.tox[t] : Xx;
+            my = pl.toy[cl.tap0 + t] < my ? pl.toy[cl.tap0 + t] : my;
+            mx = pl.tox[cl.tap0 + t] < mx ? pl.tox[cl.tap0 + t] : mx;
+            Xy = pl.toy[cl.tap0 + t] > Xy ? pl.toy[cl.tap0 + t] : Xy;
+            Xx = pl.tox[cl.tap0 + t] > Xx ? pl.tox[cl.tap0 + t] : Xx;
         }
         cl.mint_y = my;
         cl.mint_x = mx;
@@ -171,6 +171,8 @@ bool tc_plan_fwd(const cg_shape &s, TcPlan &pl) {
     pl.Hout = g.ho;
     pl.Wout = g.wo;
     pl.ncls = 1;
+    memset(pl.toy, 0, sizeof(pl.toy));
+    memset(pl.tox, 0, sizeof(pl.tox));
     TcClass &c = pl.cls[0];
     memset(&c, 0, sizeof(c));
     c.Hg = g.ho;
@@ -184,10 +186,10 @@ bool tc_plan_fwd(const cg_shape &s, TcPlan &pl) {
     c.ntaps = s.kh * s.kw;
     for (int kx = 0; kx < s.kh; kx++)
         for (int ky = 0; ky < s.kw; ky++) {
-            c.toy[kx * s.kw + ky] = (int16_t) (kx * s.vdil);
-            c.tox[kx * s.kw + ky] = (int16_t) (ky * s.hdil);
-            pl.kx[0][kx * s.kw + ky] = (int8_t) kx;
-            pl.ky[0][kx * s.kw + ky] = (int8_t) ky;
+            pl.toy[kx * s.kw + ky] = (int16_t) (kx * s.vdil);
+            pl.tox[kx * s.kw + ky] = (int16_t) (ky * s.hdil);
+            pl.kx[kx * s.kw + ky] = (int8_t) kx;
+            pl.ky[kx * s.kw + ky] = (int8_t) ky;
         }
     c.kbeg = 0;
     c.ktiles = (c.ntaps * pl.Cin + 63) / 64;
@@ -212,9 +214,11 @@ bool tc_plan_dgrad(const cg_shape &s, TcPlan &pl) {
     pl.Hout = s.h;
     pl.Wout = s.w;
     pl.ncls = 0;
+    memset(pl.toy, 0, sizeof(pl.toy));
+    memset(pl.tox, 0, sizeof(pl.tox));
     pl.has_empty_class = false;
     pl.mtiles_max = 0;
-    int kb = 0;
+    int kb = 0, tap0 = 0;
     for (int cy = 0; cy < sy; cy++)
         for (int cx = 0; cx < sx; cx++) {
             const int Hg = s.h > cy ? (s.h - cy + sy - 1) / sy : 0;
@@ -229,10 +233,10 @@ bool tc_plan_dgrad(const cg_shape &s, TcPlan &pl) {
                 for (int ky = 0; ky < s.kw; ky++) {
                     const int tx = cx + s.hpad - ky * s.hdil;
                     if (((tx % sx) + sx) % sx) continue;
-                    c.toy[nt] = (int16_t) (ty / sy);
-                    c.tox[nt] = (int16_t) (tx / sx);
-                    pl.kx[pl.ncls][nt] = (int8_t) kx;
-                    pl.ky[pl.ncls][nt] = (int8_t) ky;
+                    pl.toy[tap0 + nt] = (int16_t) (ty / sy);
+                    pl.tox[tap0 + nt] = (int16_t) (tx / sx);
+                    pl.kx[tap0 + nt] = (int8_t) kx;
+                    pl.ky[tap0 + nt] = (int8_t) ky;
                     nt++;
                 }
             }
@@ -248,7 +252,9 @@ bool tc_plan_dgrad(const cg_shape &s, TcPlan &pl) {
             c.osx = sx;
             c.isy = c.isx = 1;
             c.iby = c.ibx = 0;
+            c.tap0 = tap0;
             c.ntaps = nt;
+            tap0 += nt;
             c.kbeg = kb;
             c.ktiles = (nt * pl.Cin + 63) / 64;
             kb += c.ktiles * 64;
@@ -270,10 +276,11 @@ PackDgradInfo tc_pack_info(const TcPlan &pl) {
     info.Ktot = pl.Ktot;
     for (int c = 0; c < pl.ncls; c++) {
         info.kbeg[c] = pl.cls[c].kbeg;
+        info.tap0[c] = pl.cls[c].tap0;
         info.ntaps[c] = pl.cls[c].ntaps;
-        memcpy(info.kx[c], pl.kx[c], TC_MAXTAPS);
-        memcpy(info.ky[c], pl.ky[c], TC_MAXTAPS);
     }
+    memcpy(info.kx, pl.kx, sizeof(info.kx));
+    memcpy(info.ky, pl.ky, sizeof(info.ky));
     return info;
 }
 
@@ -450,6 +457,8 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     p.err = cg_device_error_word();
     if (!p.err) return cg_set_error(CONVGEMM_ERROR_CUDA, "device error word unavailable");
     p.ncls = pl.ncls;
+    memcpy(p.toy, pl.toy, sizeof(p.toy));
+    memcpy(p.tox, pl.tox, sizeof(p.tox));
     TcMaps amaps;
     memset(&amaps, 0, sizeof(amaps));
     if (mask && p.epi_tma)
@@ -469,7 +478,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
                 const unsigned long long dims[3] = {(unsigned long long) pl.Cin, (unsigned long long) cl.ntaps, (unsigned long long) pl.Cout};
                 const unsigned long long str[2] = {(unsigned long long) pl.Cin * 2, (unsigned long long) pl.Ktot * 2};
                 const unsigned box[3] = {64, 1, (unsigned) p.nn}, estr[3] = {1, 1, 1};
-                if (convgemm_status_t e = tc_make_map_nd(&amaps.w[c], 3, (const uint16_t *) wpacked + cl.kbeg, dims, str, box, estr, 1))
+                if (convgemm_status_t e = tc_make_map_nd(&amaps.b[c], 3, (const uint16_t *) wpacked + cl.kbeg, dims, str, box, estr, 1))
                     return e;
             }
             const int up_y = cl.lo_y + (cl.Hg - 1) * cl.isy - (pl.Hin - 1);
@@ -478,7 +487,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
                                                          cl.lo_x, up_y, up_x, cl.isy, cl.isx, 128, eb, f8w ? 128 : 64))
                 return e;
             if (mode == 2)
-                if (convgemm_status_t e = tc_make_im2col_map(&amaps.alo[c], in_lo, s.b, pl.Hin, pl.Win, pl.Cin,
+                if (convgemm_status_t e = tc_make_im2col_map(&amaps.b[c], in_lo, s.b, pl.Hin, pl.Win, pl.Cin,
                                                              cl.lo_y, cl.lo_x, up_y, up_x, cl.isy, cl.isx, 128, 2, 64))
                     return e;
         }

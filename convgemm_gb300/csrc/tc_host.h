@@ -13,7 +13,8 @@ struct TcPlan {
     int ncls, Ktot, mtiles_max, bn;
     bool has_empty_class;
     TcClass cls[TC_MAXCLS];
-    int8_t kx[TC_MAXCLS][TC_MAXTAPS], ky[TC_MAXCLS][TC_MAXTAPS];
+    int16_t toy[TC_MAXTAPS], tox[TC_MAXTAPS];   // taps of all classes (TcClass::tap0): offsets in the gathered tensor
+    int8_t kx[TC_MAXTAPS], ky[TC_MAXTAPS];      // and in the filter
 };
 
 bool tc_plan_fwd(const cg_shape &s, TcPlan &pl);

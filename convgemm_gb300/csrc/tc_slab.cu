@@ -274,7 +274,7 @@ bool slab_geom(const TcPlan &pl, SlabParams &p) {
     if (p.w_bytes > SLAB_W_MAX) return false;
     int dymin = 1 << 20, dymax = -(1 << 20), dxmin = 1 << 20, dxmax = -(1 << 20);
     for (int t = 0; t < c.ntaps; t++) {
-        const int dy = c.iby + c.toy[t], dx = c.ibx + c.tox[t];
+        const int dy = c.iby + pl.toy[t], dx = c.ibx + pl.tox[t];
         dymin = std::min(dymin, dy);
         dymax = std::max(dymax, dy);
         dxmin = std::min(dxmin, dx);
@@ -305,7 +305,7 @@ bool slab_geom(const TcPlan &pl, SlabParams &p) {
     p.tx0 = dxmin;
     uint32_t rows = (uint32_t) p.Hs * p.Wp;
     for (int t = 0; t < c.ntaps; t++) {
-        const uint32_t r0 = (uint32_t) ((c.iby + c.toy[t] - dymin) * p.Wp + (c.ibx + c.tox[t] - dxmin));
+        const uint32_t r0 = (uint32_t) ((c.iby + pl.toy[t] - dymin) * p.Wp + (c.ibx + pl.tox[t] - dxmin));
         p.aoff[t] = r0 * 128;
         rows = std::max(rows, r0 + 128);   // the operand reads 128 rows (the rows past the tile's are dropped)
     }

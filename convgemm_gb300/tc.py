@@ -108,6 +108,11 @@ def bn_apply_bf16(npix: int, kn: int, z, scale, shift, y, relu=True, stream=None
                                            _stream(stream)))
 
 
+def epilogue_grad_bf16(npix: int, kn: int, gy, y, scale, dz, stream=None):
+    """dz = bf16(gy * (y > 0) * scale): the gradient before the epilogue (y None: no ReLU, scale None: 1)."""
+    _raise_if(lib().convgemm_epilogue_grad_bf16(npix, kn, ptr(gy), ptr(y), ptr(scale), ptr(dz), _stream(stream)))
+
+
 def wgrad_bf16_workspace_size(shape: Shape) -> int:
     return lib().convgemm_wgrad_bf16_workspace_size(ctypes.byref(shape))
 

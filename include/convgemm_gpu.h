@@ -402,6 +402,10 @@ convgemm_status_t convgemm_bn_stats_fold(int kn, const double *stats, long long 
  * z == y allowed). */
 convgemm_status_t convgemm_bn_apply_bf16(long long npix, int kn, const void *z, const float *scale,
                                          const float *shift, int relu, void *y, void *stream);
+/* The gradient before the epilogue y = relu?(z * scale + shift): dz = bf16(gy * (y > 0) * scale), each product
+ * in FP32, BF16 NHWC [npix][kn] (kn % 8 == 0, 16-byte aligned; y NULL: no ReLU, scale NULL: 1). */
+convgemm_status_t convgemm_epilogue_grad_bf16(long long npix, int kn, const void *gy, const void *y,
+                                              const float *scale, void *dz, void *stream);
 
 /* Workspace of convgemm_wgrad_bf16 in bytes: FP32 partial tiles of the pixel splits. */
 size_t convgemm_wgrad_bf16_workspace_size(const convgemm_shape_t *shape);
