@@ -503,11 +503,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                     // Column sums of this item's 64 columns over the warp's 32 rows, to group
                     // gbase + m0 / 32 + ew of the class (the classes' groups are concatenated): the forward's
                     // batch-norm sums of z and z^2, or the sums of the masked input gradient (the bias
-                    // gradient of the layer that produced the mask). Each half of the columns passes through
-                    // the staging buffer, rows in, columns out: lane l adds up columns 2 (l % 16), + 1 of the rows
-                    // of its parity l / 16, two running sums each. (Exchanged by shuffles the same sums were about
-                    // a thousand instructions of straight-line code per item and bound by instruction
-                    // fetches: 56 x 56, 64 -> 256 forward with statistics 111 us, 27 without.)
+                    // gradient of the layer that produced the mask), through the staging buffer.
                     if (m0 + ew * 32 < M) {
                         uint8_t *stg = stg_warp + ebuf * C::EPI_BYTES;
                         if (EXTRA == EXTRA_SUMS && p.mask) {
@@ -533,48 +529,14 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                         const bool in = m < M;
 #pragma unroll
                         for (int h = 0; h < 2; h++) {
-#pragma unroll
-                            for (int q = 0; q < 8; q++) {
-                                float z[4];
-#pragma unroll
-                                for (int e = 0; e < 4; e++) z[e] = __uint_as_float(h ? v1[4 * q + e] : v0[4 * q + e]);
-                                if (EXTRA == EXTRA_STATS) {   // (the input gradient has no scale and shift)
-                                    const float4 sc = *reinterpret_cast<const float4 *>(scp + c0 + 32 * h + 4 * q);
-                                    const float4 sh = *reinterpret_cast<const float4 *>(shp + c0 + 32 * h + 4 * q);
-                                    z[0] = fmaf(z[0], sc.x, sh.x);
-                                    z[1] = fmaf(z[1], sc.y, sh.y);
-                                    z[2] = fmaf(z[2], sc.z, sh.z);
-                                    z[3] = fmaf(z[3], sc.w, sh.w);
-                                }
-                                *reinterpret_cast<float4 *>(stg + lane * 128 + ((q ^ (lane & 7)) << 4)) =
-                                    in ? make_float4(z[0], z[1], z[2], z[3]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                            float2 sum, sq;   // (the input gradient has no scale and shift)
+                            tc::staged_col_sums32<EXTRA == EXTRA_STATS, EXTRA == EXTRA_STATS>(
+                                stg, h ? v1 : v0, scp + c0 + 32 * h, shp + c0 + 32 * h, in, sum, sq);
+                            const int col = 32 * h + 2 * (lane & 15);
+                            if (lane < 16 && nb + col < p.Cout) {   // Cout is a multiple of 8
+                                *reinterpret_cast<float2 *>(part + col) = sum;
+                                if (EXTRA == EXTRA_STATS) *reinterpret_cast<float2 *>(part + p.Cout + col) = sq;
                             }
-                            __syncwarp();
-                            const int l16 = lane & 15;
-                            float2 s2[2] = {}, q2[2] = {};
-#pragma unroll 2
-                            for (int r = lane >> 4; r < 32; r += 4)
-#pragma unroll
-                                for (int e = 0; e < 2; e++) {
-                                    const int rr = r + 2 * e;
-                                    const float2 z = *reinterpret_cast<const float2 *>(
-                                        stg + rr * 128 + (((l16 >> 1) ^ (rr & 7)) << 4) + (l16 & 1) * 8);
-                                    s2[e].x += z.x;
-                                    s2[e].y += z.y;
-                                    if (EXTRA == EXTRA_STATS) q2[e] = __ffma2_rn(z, z, q2[e]);
-                                }
-                            float2 sum = make_float2(s2[0].x + s2[1].x, s2[0].y + s2[1].y);
-                            sum.x += __shfl_xor_sync(0xFFFFFFFFu, sum.x, 16);
-                            sum.y += __shfl_xor_sync(0xFFFFFFFFu, sum.y, 16);
-                            const bool col = nb + 32 * h + 2 * l16 < p.Cout;   // Cout is a multiple of 8
-                            if (lane < 16 && col) *reinterpret_cast<float2 *>(part + 32 * h + 2 * l16) = sum;
-                            if (EXTRA == EXTRA_STATS) {
-                                sum = make_float2(q2[0].x + q2[1].x, q2[0].y + q2[1].y);
-                                sum.x += __shfl_xor_sync(0xFFFFFFFFu, sum.x, 16);
-                                sum.y += __shfl_xor_sync(0xFFFFFFFFu, sum.y, 16);
-                                if (lane < 16 && col) *reinterpret_cast<float2 *>(part + p.Cout + 32 * h + 2 * l16) = sum;
-                            }
-                            __syncwarp();
                         }
                     }
                 }

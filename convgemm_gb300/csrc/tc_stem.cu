@@ -48,7 +48,10 @@ constexpr int STEM_MAXPAIRS = STEM_MAXTAPS / 2;
 constexpr uint32_t STEM_SLAB_MAX = 48 * 1024;    // the residue slabs of one buffer
 constexpr uint32_t STEM_ZERO = 2048;             // zero region behind each slab buffer: 128 rows x 16 B
 constexpr uint32_t STEM_W_MAX = 64 * 1024;       // resident weights
-constexpr uint32_t STEM_EPI = 4 * 4096;          // per-warp output staging, 32 rows x 128 B
+// Eight epilogue warps, two sets of four that take alternate tiles: a tile's 25 MMAs (7 x 7, 64 channels) take half a
+// microsecond, one set's epilogue (with statistics) twice that.
+constexpr int STEM_EW = 8, STEM_MMA_WARP = 4 + STEM_EW, STEM_THREADS = 32 * (STEM_MMA_WARP + 1);
+constexpr uint32_t STEM_EPI = STEM_EW * 4096;    // per-warp output staging, 32 rows x 128 B
 
 struct StemParams {
     const __nv_bfloat16 *w;   // packed weights [kn][Kpad], K = tap * 8 + channel
@@ -68,7 +71,7 @@ template <int BN>
 struct StemCfg {
     static constexpr uint32_t PAIR_W = 2 * BN * 16;   // one pair of taps of the resident weights
     static constexpr size_t SMEM = 1024 + (size_t) STEM_W_MAX + 2 * ((size_t) STEM_SLAB_MAX + STEM_ZERO) +
-                                   2 * STEM_EPI + 256 + 2 * BN * 4 + 2 * STEM_MAXPAIRS * 4;
+                                   STEM_EPI + 256 + 2 * BN * 4 + 2 * STEM_MAXPAIRS * 4;
     static_assert(SMEM <= 232448, "shared memory");
 };
 
@@ -97,7 +100,7 @@ __device__ __forceinline__ void bulk_wait_read() {
 }
 
 template <int BN>
-__global__ void __launch_bounds__(288, 1)
+__global__ void __launch_bounds__(STEM_THREADS, 1)
     tc_stem_kernel(const __grid_constant__ StemParams p, const __grid_constant__ CUtensorMap xmap,
                    const __grid_constant__ CUtensorMap omap) {
     using C = StemCfg<BN>;
@@ -106,13 +109,13 @@ __global__ void __launch_bounds__(288, 1)
     uint8_t *base = (uint8_t *) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023);
     uint8_t *wres = base;                                   // resident weights, pair p at p * PAIR_W
     uint8_t *slab = wres + STEM_W_MAX;                      // two buffers of p.buf_bytes (1024-aligned)
-    uint8_t *epi = slab + 2 * (STEM_SLAB_MAX + STEM_ZERO);  // 2 x 4 warps x 4 KB of output staging
-    uint64_t *slab_full = (uint64_t *) (epi + 2 * STEM_EPI);
+    uint8_t *epi = slab + 2 * (STEM_SLAB_MAX + STEM_ZERO);  // 8 warps x 4 KB of output staging
+    uint64_t *slab_full = (uint64_t *) (epi + STEM_EPI);
     uint64_t *slab_free = slab_full + 2;
     uint64_t *acc_full = slab_free + 2;
     uint64_t *acc_empty = acc_full + 2;
     uint32_t *tmem_holder = (uint32_t *) (acc_empty + 2);
-    float *sc_tab = (float *) (epi + 2 * STEM_EPI + 256);
+    float *sc_tab = (float *) (epi + STEM_EPI + 256);
     float *sh_tab = sc_tab + BN;
     uint32_t *aoff_tab = (uint32_t *) (sh_tab + BN);
     uint32_t *alead_tab = aoff_tab + STEM_MAXPAIRS;
@@ -146,14 +149,14 @@ __global__ void __launch_bounds__(288, 1)
                 *reinterpret_cast<uint4 *>(slab + b * p.buf_bytes + p.sw * p.rho_bytes + i * 16) =
                     make_uint4(0, 0, 0, 0);
         tc::fence_proxy_async_smem();
-    } else if (warp < 8) {
+    } else if (warp < STEM_MMA_WARP) {
         const int et = threadIdx.x - 128;
-        for (int n = et; n < BN; n += 128) {
+        for (int n = et; n < BN; n += 32 * STEM_EW) {
             const int nn = min(n, p.kn - 1);
             sc_tab[n] = p.scale ? __ldg(p.scale + nn) : 1.0f;
             sh_tab[n] = p.shift ? __ldg(p.shift + nn) : 0.0f;
         }
-        for (int i = et; i < p.npairs; i += 128) {
+        for (int i = et; i < p.npairs; i += 32 * STEM_EW) {
             aoff_tab[i] = p.aoff[i];
             alead_tab[i] = p.alead[i];
         }
@@ -185,15 +188,13 @@ __global__ void __launch_bounds__(288, 1)
             }
         }
         __syncwarp();
-    } else if (warp >= 4 && warp < 8) {
+    } else if (warp >= 4 && warp < STEM_MMA_WARP) {
         // ------------------------------------------------ epilogue
-        const int ew = warp - 4;
-        uint8_t *stg_warp = epi + ew * 4096;
-        uint32_t lt = 0;
-        int ebuf = 0;
-        for (int tile = blockIdx.x; tile < p.total && ok; tile += gridDim.x, lt++) {
+        const int ew = warp & 3, buf = (warp - 4) >> 2;   // the set's accumulator: every other tile of the CTA
+        uint8_t *stg = epi + (warp - 4) * 4096;
+        uint32_t lt = buf;
+        for (int tile = blockIdx.x + buf * gridDim.x; tile < p.total && ok; tile += 2 * gridDim.x, lt += 2) {
             const int row = tile / p.nwc, wc = tile % p.nwc;
-            const int buf = lt & 1;
             if (!(ok = tc::mbar_wait(&acc_full[buf], (lt >> 1) & 1, p.err, 43))) break;
             tc::tc_fence_after();
             for (int c0 = 0; c0 < BN; c0 += 64) {
@@ -206,18 +207,21 @@ __global__ void __launch_bounds__(288, 1)
                     tc::tc_fence_before();
                     tc::mbar_arrive(&acc_empty[buf]);
                 }
+                if (lane == 0) bulk_wait_read<0>();   // the store that last read the staging buffer
+                __syncwarp();
                 if (p.stats) {
                     // batch-norm statistics of the 64 columns over this warp's 32 pixels
-                    float *part = p.stats + ((size_t) tile * 4 + ew) * 2 * p.kn;
+                    float *part = p.stats + ((size_t) tile * 4 + ew) * 2 * p.kn + c0;
                     const bool valid = 128 * wc + ew * 32 + lane < p.Wo;
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        float sum, sq;
-                        tc::stats_cols32(h ? v1 : v0, sc_tab + c0 + 32 * h, sh_tab + c0 + 32 * h, valid, sum, sq);
-                        const int col = c0 + 32 * h + lane;
-                        if (col < p.kn) {
-                            part[col] = sum;
-                            part[p.kn + col] = sq;
+                        float2 sum, sq;
+                        tc::staged_col_sums32<true, true>(stg, h ? v1 : v0, sc_tab + c0 + 32 * h, sh_tab + c0 + 32 * h,
+                                                          valid, sum, sq);
+                        const int col = 32 * h + 2 * (lane & 15);
+                        if (lane < 16 && c0 + col < p.kn) {   // kn is a multiple of 8
+                            *reinterpret_cast<float2 *>(part + col) = sum;
+                            *reinterpret_cast<float2 *>(part + p.kn + col) = sq;
                         }
                     }
                 }
@@ -226,9 +230,6 @@ __global__ void __launch_bounds__(288, 1)
                     tc::epi_bf16_64<true>(v0, v1, sc_tab + c0, sh_tab + c0, pk);
                 else
                     tc::epi_bf16_64<false>(v0, v1, sc_tab + c0, sh_tab + c0, pk);
-                if (lane == 0) bulk_wait_read<1>();   // the store that last read this staging buffer
-                __syncwarp();
-                uint8_t *stg = stg_warp + ebuf * STEM_EPI;
 #pragma unroll
                 for (int q = 0; q < 8; q++) {
                     const uint4 u = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
@@ -238,11 +239,10 @@ __global__ void __launch_bounds__(288, 1)
                 __syncwarp();
                 const int ox0 = 128 * wc + ew * 32;
                 if (lane == 0 && ox0 < p.Wo && c0 < p.kn) tma_store_3d(&omap, tc::smem_u32(stg), c0, ox0, row);
-                ebuf ^= 1;
             }
         }
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-    } else if (warp == 8) {
+    } else if (warp == STEM_MMA_WARP) {
         // ------------------------------------------------ MMA issuer
         {
             constexpr uint32_t idesc = tc::idesc_bf16(128, BN, 0, 0);
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(288, 1)
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
-    if (warp == 8) tc::tmem_dealloc(tmem, 2 * BN);
+    if (warp == STEM_MMA_WARP) tc::tmem_dealloc(tmem, 2 * BN);
 }
 
 template <int BN>
@@ -292,7 +292,7 @@ cudaError_t launch_stem(const StemParams &p, const CUtensorMap &x, const CUtenso
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    return cg_launch_pdl(tc_stem_kernel<BN>, dim3(grid), dim3(288), StemCfg<BN>::SMEM, st, p, x, o);
+    return cg_launch_pdl(tc_stem_kernel<BN>, dim3(grid), dim3(STEM_THREADS), StemCfg<BN>::SMEM, st, p, x, o);
 }
 
 int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
