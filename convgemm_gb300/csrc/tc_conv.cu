@@ -371,6 +371,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
         const int et = threadIdx.x - 128; // 0 .. 32 * EW - 1
         uint8_t *const stg_warp = epi_smem + (warp - 4) * 4096;   // this warp's 32 x 128-byte staging
         const int first_item = ALT ? 0 : half;
+        const bool affine = p.scale || p.shift;
         uint32_t lt = ALT ? half : 0;     // local tile count
         int ebuf = 0;                     // staging buffer toggle
         // The mask's 32 x 64 values of an item, loaded into the staging buffer the item will use: by TMA, or where
@@ -463,11 +464,9 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                     orow = (uint8_t *) p.out +
                            ((((size_t) b * p.Hout + oy) * p.Wout + ox) * p.Cout) * (C::OUTF32 ? 4 : 2);
                 }
-                uint32_t v0[32], v1[32];
-                const uint32_t ta = tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) ((buf * MT + mt) * BN + c0);
-                tc::tmem_ld_32x32b_x32(ta, v0);
-                if (C::CW == 64) tc::tmem_ld_32x32b_x32(ta + 32, v1);
-                tc::tmem_ld_wait();
+                constexpr int NQ = C::CW / 8;
+                uint32_t v[2][4 * NQ];
+                tc::frag_load<NQ>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) ((buf * MT + mt) * BN + c0), v);
                 if (item + STEP >= NIT) {
                     // this warp's last read of the accumulator: its share of the TMEM buffer
                     // goes back to the MMA warp
@@ -499,99 +498,99 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                         }
                     }
                 }
+                if constexpr (EXTRA == EXTRA_SUMS) {
+                    if (p.mask) {   // rows past M arrived as zeros, which keep nothing
+                        uint8_t *stg = stg_warp + ebuf * C::EPI_BYTES;
+#pragma unroll
+                        for (int q = 0; q < 8; q++)
+#pragma unroll
+                            for (int k = 0; k < 4; k++) {
+                                const uint32_t w = positive_mask(*reinterpret_cast<const uint32_t *>(tc::frag_word(stg, q, k)));
+                                v[k >> 1][4 * q + 2 * (k & 1)] &= __byte_perm(w, 0, 0x1010);
+                                v[k >> 1][4 * q + 2 * (k & 1) + 1] &= __byte_perm(w, 0, 0x3232);
+                            }
+                    }
+                }
+                if ((EXTRA == EXTRA_NONE || EXTRA == EXTRA_MASK) && !C::OUTF32 && p.accum) {
+                    // accumulate (the reference's dx += ...): add the output's current values in FP32
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const int mr = m0 + ew * 32 + (lane >> 2) + 8 * k;
+                        size_t pix = (size_t) mr;
+                        if (!p.epi_tma) {
+                            uint32_t q, jw, j, b;
+                            cl.dwg.divmod(mr < M ? mr : 0, q, jw);
+                            cl.dhg.divmod(q, b, j);
+                            pix = ((size_t) b * p.Hout + cl.oy0 + cl.osy * (int) j) * p.Wout + cl.ox0 + cl.osx * (int) jw;
+                        }
+                        const int col = nb + 2 * (lane & 3);
+                        const uint32_t *old = reinterpret_cast<const uint32_t *>(p.out + pix * p.Cout + col);
+                        uint32_t ow[NQ];
+#pragma unroll
+                        for (int q = 0; q < NQ; q++) ow[q] = mr < M && col + 8 * q < p.Cout ? old[4 * q] : 0u;
+#pragma unroll
+                        for (int q = 0; q < NQ; q++) {
+                            uint32_t *w = &v[k >> 1][4 * q + 2 * (k & 1)];
+                            w[0] = __float_as_uint(__uint_as_float(w[0]) + __uint_as_float(ow[q] << 16));
+                            w[1] = __float_as_uint(__uint_as_float(w[1]) + __uint_as_float(ow[q] & 0xFFFF0000u));
+                        }
+                    }
+                }
+                tc::frag_affine<NQ>(v, affine, scp + c0, shp + c0);
                 if constexpr (EXTRA == EXTRA_SUMS || EXTRA == EXTRA_STATS) {
                     // Column sums of this item's 64 columns over the warp's 32 rows, to group
                     // gbase + m0 / 32 + ew of the class (the classes' groups are concatenated): the forward's
                     // batch-norm sums of z and z^2, or the sums of the masked input gradient (the bias
-                    // gradient of the layer that produced the mask), through the staging buffer.
-                    if (m0 + ew * 32 < M) {
-                        uint8_t *stg = stg_warp + ebuf * C::EPI_BYTES;
-                        if (EXTRA == EXTRA_SUMS && p.mask) {
-                            // rows past M arrived as zeros, which keep nothing
-#pragma unroll
-                            for (int q = 0; q < 8; q++) {
-                                const uint4 mv = *reinterpret_cast<const uint4 *>(stg + lane * 128 + ((q ^ (lane & 7)) << 4));
-                                const uint32_t mw[4] = {mv.x, mv.y, mv.z, mv.w};
-#pragma unroll
-                                for (int e = 0; e < 4; e++) {
-                                    const uint32_t k = positive_mask(mw[e]);
-                                    const int jj = 8 * q + 2 * e;
-                                    (jj < 32 ? v0[jj] : v1[jj - 32]) &= __byte_perm(k, 0, 0x1010);
-                                    (jj < 32 ? v0[jj + 1] : v1[jj - 31]) &= __byte_perm(k, 0, 0x3232);
-                                }
-                            }
-                            __syncwarp();
-                        } else {   // the buffer's last store has read it (masked: waited for above)
-                            if (lane == 0) bulk_wait_read<1>();
-                            __syncwarp();
-                        }
-                        float *part = p.stats + (size_t) (cl.gbase + (m0 >> 5) + ew) * 2 * p.Cout + nb;
-                        const bool in = m < M;
-#pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            float2 sum, sq;   // (the input gradient has no scale and shift)
-                            tc::staged_col_sums32<EXTRA == EXTRA_STATS, EXTRA == EXTRA_STATS>(
-                                stg, h ? v1 : v0, scp + c0 + 32 * h, shp + c0 + 32 * h, in, sum, sq);
-                            const int col = 32 * h + 2 * (lane & 15);
-                            if (lane < 16 && nb + col < p.Cout) {   // Cout is a multiple of 8
-                                *reinterpret_cast<float2 *>(part + col) = sum;
-                                if (EXTRA == EXTRA_STATS) *reinterpret_cast<float2 *>(part + p.Cout + col) = sq;
-                            }
+                    // gradient of the layer that produced the mask).
+                    const int rows = M - (m0 + ew * 32);
+                    if (rows > 0) {
+                        if (rows < 32) tc::frag_clear_rows(v, rows);
+                        float2 sum, sq;
+                        tc::frag_col_sums<EXTRA == EXTRA_STATS>(v, sum, sq);
+                        float *part = p.stats + (size_t) (cl.gbase + (m0 >> 5) + ew) * 2 * p.Cout + nb + 2 * lane;
+                        if (nb + 2 * lane < p.Cout) {   // Cout is a multiple of 8
+                            *reinterpret_cast<float2 *>(part) = sum;
+                            if (EXTRA == EXTRA_STATS) *reinterpret_cast<float2 *>(part + p.Cout) = sq;
                         }
                     }
                 }
-                if ((EXTRA == EXTRA_NONE || EXTRA == EXTRA_MASK) && !C::OUTF32 && p.accum && m < M && nb < p.Cout) {
-                    // accumulate (the reference's dx += ...): add the output's current 64 values in FP32
-                    size_t pix = (size_t) m;
-                    if (!p.epi_tma) {
-                        uint32_t q, jw, j, b;
-                        cl.dwg.divmod(m, q, jw);
-                        cl.dhg.divmod(q, b, j);
-                        pix = ((size_t) b * p.Hout + cl.oy0 + cl.osy * (int) j) * p.Wout + cl.ox0 + cl.osx * (int) jw;
-                    }
-                    const uint4 *orow4 = reinterpret_cast<const uint4 *>(p.out + pix * p.Cout + nb);
+                uint32_t pk[32];   // 128 bytes of each of the 32 rows, over the warp
+                if constexpr (C::OUTF32) {
 #pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        uint4 ov = make_uint4(0, 0, 0, 0);
-                        if (nb + 8 * q + 8 <= p.Cout) ov = orow4[q];
-                        const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w};
+                    for (int h = 0; h < 2; h++)
 #pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const int jj = 8 * q + 2 * e;   // column of the low half
-                            uint32_t &lo = jj < 32 ? v0[jj] : v1[jj - 32];
-                            uint32_t &hi = jj + 1 < 32 ? v0[jj + 1] : v1[jj - 31];
-                            lo = __float_as_uint(__uint_as_float(lo) + __uint_as_float(ow[e] << 16));
-                            hi = __float_as_uint(__uint_as_float(hi) + __uint_as_float(ow[e] & 0xFFFF0000u));
-                        }
-                    }
-                }
-                uint32_t pk[32];   // one 128-byte output row chunk
-                if (C::OUTF32) {
-#pragma unroll
-                    for (int jj = 0; jj < 32; jj++) {
-                        float a = fmaf(__uint_as_float(v0[jj]), scp[c0 + jj], shp[c0 + jj]);
-                        if (p.relu) a = fmaxf(a, 0.0f);
-                        pk[jj] = __float_as_uint(a);
-                    }
-                } else if (p.relu) {
-                    tc::epi_bf16_64<true>(v0, v1, scp + c0, shp + c0, pk);
+                        for (int j = 0; j < 16; j++)
+                            pk[16 * h + j] = p.relu ? __float_as_uint(fmaxf(__uint_as_float(v[h][j]), 0.0f)) : v[h][j];
                 } else {
-                    tc::epi_bf16_64<false>(v0, v1, scp + c0, shp + c0, pk);
+                    tc::frag_pack(v, p.relu != 0, pk);
                 }
                 if constexpr (EXTRA == EXTRA_MASK) {
-                    // ReLU backward: the outputs where the mask is positive; this lane's row of the mask lies
-                    // where its row of the output goes
-                    const uint8_t *mrow = stg_warp + ebuf * C::EPI_BYTES + lane * 128;
+                    // ReLU backward: the outputs where the mask is positive; each word of the mask lies where the
+                    // word of the output goes
+                    uint8_t *stg = stg_warp + ebuf * C::EPI_BYTES;
 #pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        const uint4 mv = *reinterpret_cast<const uint4 *>(mrow + ((q ^ (lane & 7)) << 4));
-                        pk[4 * q] &= positive_mask(mv.x);
-                        pk[4 * q + 1] &= positive_mask(mv.y);
-                        pk[4 * q + 2] &= positive_mask(mv.z);
-                        pk[4 * q + 3] &= positive_mask(mv.w);
-                    }
-                    __syncwarp();
+                    for (int q = 0; q < 8; q++)
+#pragma unroll
+                        for (int k = 0; k < 4; k++)
+                            pk[4 * q + k] &= positive_mask(*reinterpret_cast<const uint32_t *>(tc::frag_word(stg, q, k)));
                 }
+                // to the staging buffer of the warp
+                auto stage = [&](uint8_t *stg) {
+                    if constexpr (C::OUTF32) {
+                        const int fr = lane >> 2, fc = lane & 3;
+#pragma unroll
+                        for (int h = 0; h < 2; h++)
+#pragma unroll
+                            for (int q = 0; q < 4; q++)
+#pragma unroll
+                                for (int k = 0; k < 2; k++)
+                                    *reinterpret_cast<uint2 *>(stg + (16 * h + 8 * k + fr) * 128 +
+                                                               (((2 * q + (fc >> 1)) ^ fr) << 4) + (fc & 1) * 8) =
+                                        make_uint2(pk[16 * h + 4 * q + 2 * k], pk[16 * h + 4 * q + 2 * k + 1]);
+                    } else {
+                        tc::frag_stage(stg, pk);
+                    }
+                };
                 by_tma = next_by_tma;
                 if (p.epi_tma) {
                     // each warp stages its 32 rows (4 KB) and stores them with its own TMA
@@ -603,11 +602,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                     }
                     __syncwarp();
                     uint8_t *stg = stg_warp + ebuf * C::EPI_BYTES;
-#pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        uint4 u = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-                        *reinterpret_cast<uint4 *>(stg + lane * 128 + ((q ^ (lane & 7)) << 4)) = u;
-                    }
+                    stage(stg);
                     tc::fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
@@ -622,10 +617,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                     if (lane == 0 && C::EPI_BUFS == 2) bulk_wait_read<1>();
                     else if (lane == 0) bulk_wait_read<0>();
                     __syncwarp();
-#pragma unroll
-                    for (int q = 0; q < 8; q++)
-                        *reinterpret_cast<uint4 *>(stg + lane * 128 + ((q ^ (lane & 7)) << 4)) =
-                            make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
+                    stage(stg);
                     __syncwarp();
                     const unsigned long long my = (unsigned long long) (orow ? orow + (size_t) nb * 2 : nullptr);
 #pragma unroll
@@ -636,16 +628,22 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                         if (dst && nb + ch * 8 < p.Cout) *reinterpret_cast<uint4 *>((uint8_t *) dst + ch * 16) = u;
                     }
                     __syncwarp();
-                } else if (orow && nb < p.Cout) {
-                    float *o = reinterpret_cast<float *>(orow) + nb;
-                    if (nb + C::CW <= p.Cout) {
+                } else {
+                    // FP32 rows that TMA cannot store (an output off the 16-byte grid)
+                    uint8_t *stg = stg_warp + ebuf * C::EPI_BYTES;
+                    __syncwarp();
+                    stage(stg);
+                    __syncwarp();
+                    if (orow) {
+                        float *o = reinterpret_cast<float *>(orow) + nb;
+#pragma unroll 1
+                        for (int q = 0; q < 8; q++) {
+                            const float4 u = *reinterpret_cast<const float4 *>(stg + lane * 128 + ((q ^ (lane & 7)) << 4));
+                            const float e[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-                        for (int q = 0; q < 8; q++)
-                            reinterpret_cast<uint4 *>(o)[q] = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-                    } else {
-#pragma unroll
-                        for (int jj = 0; jj < 32; jj++)
-                            if (nb + jj < p.Cout) o[jj] = __uint_as_float(pk[jj]);
+                            for (int j = 0; j < 4; j++)
+                                if (nb + 4 * q + j < p.Cout) o[4 * q + j] = e[j];
+                        }
                     }
                 }
                 if (C::EPI_BUFS == 2) ebuf ^= 1;

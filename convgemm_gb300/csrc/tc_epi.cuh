@@ -1,11 +1,17 @@
-// Fused epilogue arithmetic of the tensor-core kernels: one thread turns 64
-// FP32 accumulators of its output row into 32 packed BF16 pairs,
-//   y = relu?(acc * scale + shift),
-// with two-wide FMAs (fma.rn.f32x2: each lane rounds exactly as fmaf) and the
-// ReLU folded into the BF16 conversion (cvt.rn.relu.bf16x2.f32).
+// Fused epilogue of the tensor-core kernels, by fragments: a warp reads its 32 accumulator rows 16 x 256 bits at a
+// time (tcgen05.ld.16x256b), so that lane l holds columns 8q + 2 (l % 4), + 1 of rows l / 4 + 8k, the words of row
+// l / 4 + 8k being v[k / 2][4q + 2 (k % 2)], + 1. Then
+//   y = relu?(acc * scale + shift)
+// with two-wide FMAs (fma.rn.f32x2: each lane rounds exactly as fmaf) and the ReLU folded into the BF16 conversion.
+// What bounds it is the shared-memory pipe: with a row per lane (32x32b) each lane needs the scale and shift of all 64
+// columns, 128 wavefronts per warp and 64 columns beside 32 for the staging; here of 16 columns, and column sums take
+// 28 exchanges instead of a pass through the staging buffer. Batch 64: 56 x 56, 64 -> 256 1 x 1 forward 28.5 -> 23.8 us
+// (19 at the memory's rate), the 224 x 224 stem's forward with statistics 71 -> 57.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include "tc_ptx.cuh"
 
 namespace tc {
 
@@ -19,76 +25,119 @@ __device__ __forceinline__ uint32_t cvt_bf16x2(float lo, float hi) {
     return d;
 }
 
-// v0: columns 0-31, v1: columns 32-63 (tcgen05.ld 32x32b.x32 results); sc/sh:
-// the 64 columns' scale and shift, 16-byte aligned (shared memory).
-template <bool RELU>
-__device__ __forceinline__ void epi_bf16_64(const uint32_t (&v0)[32], const uint32_t (&v1)[32],
-                                            const float *__restrict__ sc, const float *__restrict__ sh,
-                                            uint32_t (&pk)[32]) {
-    const float4 *s4 = reinterpret_cast<const float4 *>(sc);
-    const float4 *t4 = reinterpret_cast<const float4 *>(sh);
+// 32 rows x 8 * NQ columns of FP32 accumulators; ta: the warp's lane quarter and the first column.
+template <int NQ>
+__device__ __forceinline__ void frag_load(uint32_t ta, uint32_t (&v)[2][4 * NQ]) {
+    static_assert(NQ == 8 || NQ == 4, "64 or 32 columns");
+    if constexpr (NQ == 8) {
+        tmem_ld_16x256b_x8(ta, v[0]);
+        tmem_ld_16x256b_x8(ta + (16u << 16), v[1]);
+    } else {
+        tmem_ld_16x256b_x4(ta, v[0]);
+        tmem_ld_16x256b_x4(ta + (16u << 16), v[1]);
+    }
+    tmem_ld_wait();
+}
+
+// v = v * sc + sh (sc, sh: the first column's, 8-byte aligned); without either v + 0, which is the same for 1 and 0.
+template <int NQ>
+__device__ __forceinline__ void frag_affine(uint32_t (&v)[2][4 * NQ], bool affine, const float *__restrict__ sc,
+                                            const float *__restrict__ sh) {
+    const int fc = 2 * (threadIdx.x & 3);
 #pragma unroll
-    for (int q = 0; q < 16; q++) {
-        const float4 s = s4[q], t = t4[q];
-        const int j = 4 * q;
-        float2 a = make_float2(__uint_as_float(j < 32 ? v0[j] : v1[j - 32]),
-                               __uint_as_float(j < 32 ? v0[j + 1] : v1[j - 31]));
-        float2 b = make_float2(__uint_as_float(j < 32 ? v0[j + 2] : v1[j - 30]),
-                               __uint_as_float(j < 32 ? v0[j + 3] : v1[j - 29]));
-        a = __ffma2_rn(a, make_float2(s.x, s.y), make_float2(t.x, t.y));
-        b = __ffma2_rn(b, make_float2(s.z, s.w), make_float2(t.z, t.w));
-        pk[2 * q] = cvt_bf16x2<RELU>(a.x, a.y);
-        pk[2 * q + 1] = cvt_bf16x2<RELU>(b.x, b.y);
+    for (int q = 0; q < NQ; q++) {
+        float2 s = make_float2(1.0f, 1.0f), t = make_float2(0.0f, 0.0f);
+        if (affine) {
+            s = *reinterpret_cast<const float2 *>(sc + 8 * q + fc);
+            t = *reinterpret_cast<const float2 *>(sh + 8 * q + fc);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            uint32_t *w = &v[k >> 1][4 * q + 2 * (k & 1)];
+            const float2 z = __ffma2_rn(make_float2(__uint_as_float(w[0]), __uint_as_float(w[1])), s, t);
+            w[0] = __float_as_uint(z.x);
+            w[1] = __float_as_uint(z.y);
+        }
     }
 }
 
-// Column sums (SQ: and sums of squares) of z = v * sc + sh (AFFINE; else v) over a warp's 32 rows and 32 columns:
-// lane l returns them for columns 2 (l % 16), + 1. The values pass through the warp's 4 KB staging buffer, rows in
-// (rows that do not count, `in` false, as zeros), columns out: each lane adds up two columns of the rows of its
-// parity l / 16, in two running sums. Exchanged by shuffles the same sums were about a thousand instructions of
-// straight-line code per 64 columns and bound by instruction fetches: 56 x 56, 64 -> 256 forward with statistics
-// 111 us, 27 this way; 224 x 224 stem forward with statistics 93 us, STEMNOW this way and with eight epilogue warps.
-template <bool AFFINE, bool SQ>
-__device__ __forceinline__ void staged_col_sums32(uint8_t *stg, const uint32_t (&v)[32], const float *sc, const float *sh,
-                                                  bool in, float2 &sum, float2 &sq) {
-    const int lane = threadIdx.x & 31, l16 = lane & 15;
+// Packed BF16 pairs, pk[4q + k]: row l / 4 + 8k, columns 8q + 2 (l % 4), + 1.
+template <bool RELU>
+__device__ __forceinline__ void frag_pack(const uint32_t (&v)[2][32], uint32_t (&pk)[32]) {
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t *w = &v[k >> 1][4 * q + 2 * (k & 1)];
+            pk[4 * q + k] = cvt_bf16x2<RELU>(__uint_as_float(w[0]), __uint_as_float(w[1]));
+        }
+}
+__device__ __forceinline__ void frag_pack(const uint32_t (&v)[2][32], bool relu, uint32_t (&pk)[32]) {
+    if (relu) frag_pack<true>(v, pk);
+    else frag_pack<false>(v, pk);
+}
+
+// This lane's word of packed pair (q, k) in a staging buffer of 32 rows x 128 bytes, 128-byte swizzle.
+__device__ __forceinline__ uint8_t *frag_word(uint8_t *stg, int q, int k) {
+    const int lane = threadIdx.x & 31, fr = lane >> 2;
+    return stg + fr * 128 + k * 1024 + ((q ^ fr) << 4) + (lane & 3) * 4;
+}
+__device__ __forceinline__ void frag_stage(uint8_t *stg, const uint32_t (&pk)[32]) {
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) *reinterpret_cast<uint32_t *>(frag_word(stg, q, k)) = pk[4 * q + k];
+}
+
+// The rows from `rows` on become zeros.
+__device__ __forceinline__ void frag_clear_rows(uint32_t (&v)[2][32], int rows) {
+    const int fr = (threadIdx.x & 31) >> 2;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (fr + 8 * k >= rows)
+#pragma unroll
+            for (int q = 0; q < 8; q++) v[k >> 1][4 * q + 2 * (k & 1)] = v[k >> 1][4 * q + 2 * (k & 1) + 1] = 0u;
+}
+
+// One exchange of the column sums: lanes with bit 4N set keep the upper half of s, the others the lower half.
+template <int N>
+__device__ __forceinline__ void frag_round(float2 (&s)[8]) {
+    const bool up = (threadIdx.x & (4 * N)) != 0;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const float2 keep = up ? s[i + N] : s[i], send = up ? s[i] : s[i + N];
+        s[i].x = keep.x + __shfl_xor_sync(0xFFFFFFFFu, send.x, 4 * N);
+        s[i].y = keep.y + __shfl_xor_sync(0xFFFFFFFFu, send.y, 4 * N);
+    }
+}
+// Sums (SQ: and sums of squares) of the 64 columns over the 32 rows; lane l gets columns 2l, 2l + 1. Four rows are
+// added up by each lane, then eight lanes' sums in three exchanges of halves.
+template <bool SQ>
+__device__ __forceinline__ void frag_col_sums(const uint32_t (&v)[2][32], float2 &sum, float2 &sq) {
+    float2 s[8], p[8];
 #pragma unroll
     for (int q = 0; q < 8; q++) {
-        float z[4];
+        float2 z[4];
 #pragma unroll
-        for (int e = 0; e < 4; e++) z[e] = __uint_as_float(v[4 * q + e]);
-        if (AFFINE) {
-            const float4 a = *reinterpret_cast<const float4 *>(sc + 4 * q);
-            const float4 b = *reinterpret_cast<const float4 *>(sh + 4 * q);
-            z[0] = fmaf(z[0], a.x, b.x);
-            z[1] = fmaf(z[1], a.y, b.y);
-            z[2] = fmaf(z[2], a.z, b.z);
-            z[3] = fmaf(z[3], a.w, b.w);
+        for (int k = 0; k < 4; k++)
+            z[k] = make_float2(__uint_as_float(v[k >> 1][4 * q + 2 * (k & 1)]), __uint_as_float(v[k >> 1][4 * q + 2 * (k & 1) + 1]));
+        s[q] = make_float2((z[0].x + z[1].x) + (z[2].x + z[3].x), (z[0].y + z[1].y) + (z[2].y + z[3].y));
+        if (SQ) {
+            p[q] = make_float2(z[0].x * z[0].x, z[0].y * z[0].y);
+#pragma unroll
+            for (int k = 1; k < 4; k++) p[q] = __ffma2_rn(z[k], z[k], p[q]);
         }
-        *reinterpret_cast<float4 *>(stg + lane * 128 + ((q ^ (lane & 7)) << 4)) =
-            in ? make_float4(z[0], z[1], z[2], z[3]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
-    __syncwarp();
-    float2 s2[2] = {}, q2[2] = {};
-#pragma unroll 2
-    for (int r = lane >> 4; r < 32; r += 4)
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-            const int rr = r + 2 * e;
-            const float2 z = *reinterpret_cast<const float2 *>(stg + rr * 128 + (((l16 >> 1) ^ (rr & 7)) << 4) + (l16 & 1) * 8);
-            s2[e].x += z.x;
-            s2[e].y += z.y;
-            if (SQ) q2[e] = __ffma2_rn(z, z, q2[e]);
-        }
-    sum = make_float2(s2[0].x + s2[1].x, s2[0].y + s2[1].y);
-    sum.x += __shfl_xor_sync(0xFFFFFFFFu, sum.x, 16);
-    sum.y += __shfl_xor_sync(0xFFFFFFFFu, sum.y, 16);
+    frag_round<4>(s);
+    frag_round<2>(s);
+    frag_round<1>(s);
+    sum = s[0];
     if (SQ) {
-        sq = make_float2(q2[0].x + q2[1].x, q2[0].y + q2[1].y);
-        sq.x += __shfl_xor_sync(0xFFFFFFFFu, sq.x, 16);
-        sq.y += __shfl_xor_sync(0xFFFFFFFFu, sq.y, 16);
+        frag_round<4>(p);
+        frag_round<2>(p);
+        frag_round<1>(p);
+        sq = p[0];
     }
-    __syncwarp();
 }
 
 }  // namespace tc

@@ -203,28 +203,20 @@ __global__ void __launch_bounds__(GTHREADS, 1)
 #pragma unroll 1
             for (int ch = half; ch < nch; ch += 2) {
                 const int c0 = max(0, min(ch * 64, nn - 64));   // the last chunk repeats columns of the one before
-                uint32_t v0[32], v1[32];
-                const uint32_t ta = tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * GBN + c0);
-                tc::tmem_ld_32x32b_x32(ta, v0);
-                tc::tmem_ld_32x32b_x32(ta + 32, v1);
-                tc::tmem_ld_wait();
+                uint32_t v[2][32];
+                tc::frag_load<8>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * GBN + c0), v);
                 if (ch + 2 >= nch) {
                     tc::tc_fence_before();
                     tc::mbar_arrive(&acc_empty[buf]);
                 }
+                tc::frag_affine<8>(v, scale || shift, sc_tab + c0, sh_tab + c0);
                 uint32_t pk[32];
-                if (relu)
-                    tc::epi_bf16_64<true>(v0, v1, sc_tab + c0, sh_tab + c0, pk);
-                else
-                    tc::epi_bf16_64<false>(v0, v1, sc_tab + c0, sh_tab + c0, pk);
+                tc::frag_pack(v, relu != 0, pk);
                 // each warp stages its 32 rows and stores them itself: no barrier across warps
                 if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                 __syncwarp();
                 uint8_t *stg = epi + ebuf * EPI_BYTES + (warp - 4) * 4096;
-#pragma unroll
-                for (int qq = 0; qq < 8; qq++)
-                    *reinterpret_cast<uint4 *>(stg + lane * 128 + ((qq ^ (lane & 7)) << 4)) =
-                        make_uint4(pk[4 * qq], pk[4 * qq + 1], pk[4 * qq + 2], pk[4 * qq + 3]);
+                tc::frag_stage(stg, pk);
                 tc::fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {

@@ -139,30 +139,28 @@ __global__ void __launch_bounds__(288, 1)
         }
         __syncwarp();
     } else if (warp >= 4 && warp < 8) {
-        // ------------------------------------------------ epilogue: this thread's tile row, compacted
+        // ------------------------------------------------ epilogue: the tile's rows, compacted
         // into the staging box [R][Wc][64 channels] (128-byte swizzle) of one TMA store per tile
-        const int ew = warp - 4, r = ew * 32 + lane, et = threadIdx.x - 128;
-        const int i = r / p.Wp, jj = r % p.Wp;
-        const bool inbox = i < p.R && jj < p.Wc;
-        const int drow = i * p.Wc + jj;
+        const int ew = warp - 4, et = threadIdx.x - 128;
+        int drow[4];   // where this lane's four rows go; -1: past a row of pixels
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int r = ew * 32 + (lane >> 2) + 8 * k, i = r / p.Wp, jj = r % p.Wp;
+            drow[k] = i < p.R && jj < p.Wc ? i * p.Wc + jj : -1;
+        }
         uint32_t lt = 0;
         for (int m = m_first; m < p.mtiles && ok; m += m_step, lt++) {
             const int wc = m % p.nwc, q = m / p.nwc, rg = q % p.nrg, b = q / p.nrg;
             const int buf = lt % SLAB_ACC;
             if (!(ok = tc::mbar_wait(&acc_full[buf], (lt / SLAB_ACC) & 1, p.err, 53))) break;
             tc::tc_fence_after();
-            uint32_t v0[32], v1[32];
-            const uint32_t ta = tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * SLAB_BN);
-            tc::tmem_ld_32x32b_x32(ta, v0);
-            tc::tmem_ld_32x32b_x32(ta + 32, v1);
-            tc::tmem_ld_wait();
+            uint32_t v[2][32];
+            tc::frag_load<8>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * SLAB_BN), v);
             tc::tc_fence_before();
             tc::mbar_arrive(&acc_empty[buf]);
+            tc::frag_affine<8>(v, p.scale || p.shift, sc_tab, sh_tab);
             uint32_t pk[32];
-            if (p.relu)
-                tc::epi_bf16_64<true>(v0, v1, sc_tab, sh_tab, pk);
-            else
-                tc::epi_bf16_64<false>(v0, v1, sc_tab, sh_tab, pk);
+            tc::frag_pack(v, p.relu != 0, pk);
             uint8_t *stg = stage + (size_t) (p.nstage == 2 ? (lt & 1) : 0) * SLAB_STAGE;
             // the store that last read this staging buffer is done reading it
             if (et == 0) {
@@ -172,12 +170,13 @@ __global__ void __launch_bounds__(288, 1)
                     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             }
             asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (inbox) {
 #pragma unroll
-                for (int c = 0; c < 8; c++)
-                    *reinterpret_cast<uint4 *>(stg + drow * 128 + ((c ^ (drow & 7)) << 4)) =
-                        make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
-            }
+            for (int k = 0; k < 4; k++)
+                if (drow[k] >= 0)
+#pragma unroll
+                    for (int q = 0; q < 8; q++)
+                        *reinterpret_cast<uint32_t *>(stg + drow[k] * 128 + ((q ^ (drow[k] & 7)) << 4) + (lane & 3) * 4) =
+                            pk[4 * q + k];
             tc::fence_proxy_async_smem();
             asm volatile("bar.sync 1, 128;" ::: "memory");
             // rows and columns past the output (partial row groups, column chunks, N tiles) are clipped

@@ -7,11 +7,11 @@
 // A tiles by threads, bound by shared-memory copies.  Here the tensor core reads
 // its A operand straight out of input slabs:
 //   * a tile is a chunk of up to 128 output pixels of one output row (b, oy,
-//     columns 128*wc ..);
+//     columns 128*wc ..); up to four rows' tiles share their slabs;
 //   * for each residue rho of the input column modulo the horizontal stride sw,
 //     one TMA load (traversal stride sw along W) brings the slab
 //     S_rho[i][j] = x[b][oy*sh - pad_h + i][sw*(128*wc + qmin + j) + rho][0..7]
-//     for i < Hbox = (kh-1)*dh + 1 input rows: tap (ky, kx), whose input column
+//     for i < Hbox = (R-1)*sh + (kh-1)*dh + 1 input rows (R output rows): tap (ky, kx), whose input column
 //     for output column ox is sw*(ox + q) + rho with kx*dw - pad_w = sw*q + rho,
 //     reads rows j = r + q - qmin of S_rho[ky*dh] for the tile's pixels r -- 128
 //     consecutive 16-byte rows, i.e. a K-major operand of 8 K elements in the
@@ -25,8 +25,8 @@
 //   * the packed weights of the single N tile are resident in shared memory in the
 //     same pair order: pair p holds [BN][8] BF16 for its first tap, then for its
 //     second (zero for the zero region);
-//   * slab buffers are double-buffered across tiles: the MMA commit of a tile frees
-//     its slab, the next-but-one tile's TMA loads refill it;
+//   * slab buffers are double-buffered: the MMA commit of a group's last row frees its
+//     slab, the next-but-one group's TMA loads refill it;
 //   * the epilogue applies scale / shift / ReLU and stores through per-warp TMA
 //     stores of a 3-D output map [B*Ho][Wo][kn] (rows past Wo are clipped).
 // There is no K pipeline: the whole reduction of a tile (kh*kw*8 <= 512 deep) is
@@ -56,14 +56,17 @@ constexpr uint32_t STEM_EPI = STEM_EW * 4096;    // per-warp output staging, 32 
 struct StemParams {
     const __nv_bfloat16 *w;   // packed weights [kn][Kpad], K = tap * 8 + channel
     const float *scale, *shift;
-    int relu, B, Ho, Wo, kn, Kpad, nwc, total, sh, sw, pad_h, qmin, npairs;
+    int relu, B, Ho, Wo, kn, Kpad, nwc, units, sh, sw, pad_h, qmin, npairs;
+    int R, nrg;               // output rows that share a slab; such groups per image
     uint32_t buf_bytes;       // one slab buffer: sw residue slabs (rho_bytes apart) + the zero region
     uint32_t rho_bytes;       // one residue slab, 1024-aligned
     uint32_t slab_tx;         // bytes the TMA loads of one tile deliver
     int *err;
     float *stats;             // per (tile, epilogue warp) group g: [g][0][kn] sum, [g][1][kn] sum of squares, or NULL
-    uint32_t aoff[STEM_MAXPAIRS];   // byte offset of the pair's first tap rows within a slab buffer
-    uint32_t alead[STEM_MAXPAIRS];  // bytes from the first to the second tap's rows (or to the zero region)
+    // low descriptor word of the pair's A operand (first tap's rows within a slab buffer, distance to the second
+    // tap's), and what the next output row adds to it; read at fixed indexes, so that the MMAs find their operands in
+    // uniform registers
+    uint32_t adesc[STEM_MAXPAIRS], astep[STEM_MAXPAIRS];
     int16_t wtap[2 * STEM_MAXPAIRS];   // the pair's taps (ky * kw + kx) in the packed weights; -1 = zero
 };
 
@@ -71,13 +74,13 @@ template <int BN>
 struct StemCfg {
     static constexpr uint32_t PAIR_W = 2 * BN * 16;   // one pair of taps of the resident weights
     static constexpr size_t SMEM = 1024 + (size_t) STEM_W_MAX + 2 * ((size_t) STEM_SLAB_MAX + STEM_ZERO) +
-                                   STEM_EPI + 256 + 2 * BN * 4 + 2 * STEM_MAXPAIRS * 4;
+                                   STEM_EPI + 256 + 2 * BN * 4;
     static_assert(SMEM <= 232448, "shared memory");
 };
 
 // No-swizzle K-major descriptor: core matrices of 8 rows x 16 bytes; `lead` = bytes
 // between the core matrices of K elements 0-7 and 8-15, 8-row groups 128 bytes apart.
-__device__ __forceinline__ uint64_t kmajor_desc(uint32_t saddr, uint32_t lead) {
+__host__ __device__ __forceinline__ uint64_t kmajor_desc(uint32_t saddr, uint32_t lead) {
     uint64_t d = 0;
     d |= (uint64_t) ((saddr & 0x3FFFF) >> 4);
     d |= (uint64_t) ((lead >> 4) & 0x3FFF) << 16;
@@ -117,8 +120,6 @@ __global__ void __launch_bounds__(STEM_THREADS, 1)
     uint32_t *tmem_holder = (uint32_t *) (acc_empty + 2);
     float *sc_tab = (float *) (epi + STEM_EPI + 256);
     float *sh_tab = sc_tab + BN;
-    uint32_t *aoff_tab = (uint32_t *) (sh_tab + BN);
-    uint32_t *alead_tab = aoff_tab + STEM_MAXPAIRS;
 
     const int warp = tc::w::warp_index(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -132,33 +133,35 @@ __global__ void __launch_bounds__(STEM_THREADS, 1)
         tc::prefetch_tmap(&xmap);
         tc::prefetch_tmap(&omap);
     }
-    if (warp < 4) {
-        // the resident weights in pair order, and the zero regions
+    if (warp < STEM_MMA_WARP) {
+        // the resident weights in pair order, several 16-byte loads in flight per thread, and the zero regions
+        constexpr int NT = 32 * STEM_MMA_WARP, BATCH = 5;
         const int t = threadIdx.x;
         const int nrow = p.npairs * 2 * BN;   // 16-byte rows
-        for (int i = t; i < nrow; i += 128) {
-            const int half = i / BN, n = i % BN;   // half = 2 * pair + (second tap)
-            const int tap = p.wtap[half];
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (tap >= 0 && n < p.kn)
-                v = __ldg(reinterpret_cast<const uint4 *>(p.w + (size_t) n * p.Kpad + tap * 8));
-            *reinterpret_cast<uint4 *>(wres + (size_t) i * 16) = v;
+        for (int i0 = t; i0 < nrow; i0 += BATCH * NT) {
+            uint4 v[BATCH];
+#pragma unroll
+            for (int j = 0; j < BATCH; j++) {
+                const int i = i0 + j * NT, half = i / BN, n = i % BN;   // half = 2 * pair + (second tap)
+                v[j] = make_uint4(0, 0, 0, 0);
+                if (i < nrow && n < p.kn) {
+                    const int tap = p.wtap[half];
+                    if (tap >= 0) v[j] = __ldg(reinterpret_cast<const uint4 *>(p.w + (size_t) n * p.Kpad + tap * 8));
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < BATCH; j++)
+                if (i0 + j * NT < nrow) *reinterpret_cast<uint4 *>(wres + (size_t) (i0 + j * NT) * 16) = v[j];
         }
         for (int b = 0; b < 2; b++)
-            for (int i = t; i < (int) (STEM_ZERO / 16); i += 128)
+            for (int i = t; i < (int) (STEM_ZERO / 16); i += NT)
                 *reinterpret_cast<uint4 *>(slab + b * p.buf_bytes + p.sw * p.rho_bytes + i * 16) =
                     make_uint4(0, 0, 0, 0);
         tc::fence_proxy_async_smem();
-    } else if (warp < STEM_MMA_WARP) {
-        const int et = threadIdx.x - 128;
-        for (int n = et; n < BN; n += 32 * STEM_EW) {
+        for (int n = t; n < BN; n += NT) {
             const int nn = min(n, p.kn - 1);
             sc_tab[n] = p.scale ? __ldg(p.scale + nn) : 1.0f;
             sh_tab[n] = p.shift ? __ldg(p.shift + nn) : 0.0f;
-        }
-        for (int i = et; i < p.npairs; i += 32 * STEM_EW) {
-            aoff_tab[i] = p.aoff[i];
-            alead_tab[i] = p.alead[i];
         }
     } else {
         tc::tmem_alloc(tmem_holder, 2 * BN);
@@ -174,12 +177,12 @@ __global__ void __launch_bounds__(STEM_THREADS, 1)
         // ------------------------------------------------ producer: the slab TMA loads of each tile
         {
             uint32_t lt = 0;
-            for (int tile = blockIdx.x; tile < p.total && ok; tile += gridDim.x, lt++) {
-                if (tile + (int) gridDim.x >= p.total) tc::pdl_trigger();   // this CTA's last tile
+            for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x, lt++) {
+                if (u + (int) gridDim.x >= p.units) tc::pdl_trigger();   // this CTA's last group
                 const int sb = lt & 1;
                 if (lt >= 2 && !(ok = tc::w::mbar_wait(&slab_free[sb], ((lt >> 1) + 1) & 1, p.err, 41))) break;
-                const int row = tile / p.nwc, wc = tile % p.nwc;
-                const int b = row / p.Ho, oy = row % p.Ho;
+                const int g = u / p.nwc, wc = u % p.nwc;
+                const int b = g / p.nrg, oy = g % p.nrg * p.R;
                 const uint32_t dst = tc::smem_u32(slab + sb * p.buf_bytes);
                 tc::w::mbar_arrive_expect_tx(&slab_full[sb], p.slab_tx);
                 for (int rho = 0; rho < p.sw; rho++)
@@ -192,53 +195,43 @@ __global__ void __launch_bounds__(STEM_THREADS, 1)
         // ------------------------------------------------ epilogue
         const int ew = warp & 3, buf = (warp - 4) >> 2;   // the set's accumulator: every other tile of the CTA
         uint8_t *stg = epi + (warp - 4) * 4096;
-        uint32_t lt = buf;
-        for (int tile = blockIdx.x + buf * gridDim.x; tile < p.total && ok; tile += 2 * gridDim.x, lt += 2) {
-            const int row = tile / p.nwc, wc = tile % p.nwc;
-            if (!(ok = tc::mbar_wait(&acc_full[buf], (lt >> 1) & 1, p.err, 43))) break;
-            tc::tc_fence_after();
-            for (int c0 = 0; c0 < BN; c0 += 64) {
-                uint32_t v0[32], v1[32];
-                const uint32_t ta = tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * BN + c0);
-                tc::tmem_ld_32x32b_x32(ta, v0);
-                tc::tmem_ld_32x32b_x32(ta + 32, v1);
-                tc::tmem_ld_wait();
-                if (c0 + 64 >= BN) {
-                    tc::tc_fence_before();
-                    tc::mbar_arrive(&acc_empty[buf]);
-                }
-                if (lane == 0) bulk_wait_read<0>();   // the store that last read the staging buffer
-                __syncwarp();
-                if (p.stats) {
-                    // batch-norm statistics of the 64 columns over this warp's 32 pixels
-                    float *part = p.stats + ((size_t) tile * 4 + ew) * 2 * p.kn + c0;
-                    const bool valid = 128 * wc + ew * 32 + lane < p.Wo;
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
+        uint32_t lt = 0;
+        for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
+            const int g = u / p.nwc, wc = u % p.nwc, b = g / p.nrg, oy0 = g % p.nrg * p.R;
+            const int rows = min(p.R, p.Ho - oy0);
+            for (int r = 0; r < rows; r++, lt++) {
+                if ((int) (lt & 1) != buf) continue;
+                const int row = b * p.Ho + oy0 + r, tile = row * p.nwc + wc, ox0 = 128 * wc + ew * 32;
+                if (!(ok = tc::mbar_wait(&acc_full[buf], (lt >> 1) & 1, p.err, 43))) break;
+                tc::tc_fence_after();
+                for (int c0 = 0; c0 < BN; c0 += 64) {
+                    uint32_t v[2][32];
+                    tc::frag_load<8>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * BN + c0), v);
+                    if (c0 + 64 >= BN) {
+                        tc::tc_fence_before();
+                        tc::mbar_arrive(&acc_empty[buf]);
+                    }
+                    tc::frag_affine<8>(v, p.scale || p.shift, sc_tab + c0, sh_tab + c0);
+                    if (p.stats) {
+                        // batch-norm statistics of the 64 columns over this warp's 32 pixels
+                        if (ox0 + 32 > p.Wo) tc::frag_clear_rows(v, p.Wo - ox0);
                         float2 sum, sq;
-                        tc::staged_col_sums32<true, true>(stg, h ? v1 : v0, sc_tab + c0 + 32 * h, sh_tab + c0 + 32 * h,
-                                                          valid, sum, sq);
-                        const int col = 32 * h + 2 * (lane & 15);
-                        if (lane < 16 && c0 + col < p.kn) {   // kn is a multiple of 8
-                            *reinterpret_cast<float2 *>(part + col) = sum;
-                            *reinterpret_cast<float2 *>(part + p.kn + col) = sq;
+                        tc::frag_col_sums<true>(v, sum, sq);
+                        float *part = p.stats + ((size_t) tile * 4 + ew) * 2 * p.kn + c0 + 2 * lane;
+                        if (c0 + 2 * lane < p.kn) {   // kn is a multiple of 8
+                            *reinterpret_cast<float2 *>(part) = sum;
+                            *reinterpret_cast<float2 *>(part + p.kn) = sq;
                         }
                     }
+                    uint32_t pk[32];
+                    tc::frag_pack(v, p.relu != 0, pk);
+                    if (lane == 0) bulk_wait_read<0>();   // the store that last read the staging buffer
+                    __syncwarp();
+                    tc::frag_stage(stg, pk);
+                    tc::fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0 && ox0 < p.Wo && c0 < p.kn) tma_store_3d(&omap, tc::smem_u32(stg), c0, ox0, row);
                 }
-                uint32_t pk[32];
-                if (p.relu)
-                    tc::epi_bf16_64<true>(v0, v1, sc_tab + c0, sh_tab + c0, pk);
-                else
-                    tc::epi_bf16_64<false>(v0, v1, sc_tab + c0, sh_tab + c0, pk);
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    const uint4 u = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-                    *reinterpret_cast<uint4 *>(stg + lane * 128 + ((q ^ (lane & 7)) << 4)) = u;
-                }
-                tc::fence_proxy_async_smem();
-                __syncwarp();
-                const int ox0 = 128 * wc + ew * 32;
-                if (lane == 0 && ox0 < p.Wo && c0 < p.kn) tma_store_3d(&omap, tc::smem_u32(stg), c0, ox0, row);
             }
         }
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -246,33 +239,29 @@ __global__ void __launch_bounds__(STEM_THREADS, 1)
         // ------------------------------------------------ MMA issuer
         {
             constexpr uint32_t idesc = tc::idesc_bf16(128, BN, 0, 0);
-            const uint32_t wbase = tc::smem_u32(wres);
-            // the low descriptor words of every pair's A operand (start within a slab buffer,
-            // lead) in registers: table loads between the MMAs would queue behind the TMA and
-            // tensor-core shared-memory traffic
-            uint32_t alo[STEM_MAXPAIRS];
-#pragma unroll
-            for (int q = 0; q < STEM_MAXPAIRS; q++)
-                alo[q] = q < p.npairs ? (uint32_t) kmajor_desc(aoff_tab[q], alead_tab[q]) : 0u;
-            const uint64_t dhi = kmajor_desc(0, 0) & 0xFFFFFFFF00000000ull;   // SBO, version, layout
-            uint32_t lt = 0;
-            for (int tile = blockIdx.x; tile < p.total && ok; tile += gridDim.x, lt++) {
-                const int sb = lt & 1, buf = lt & 1;
-                if (lt >= 2) {
-                    if (!(ok = tc::w::mbar_wait(&acc_empty[buf], ((lt >> 1) + 1) & 1, p.err, 44))) break;
-                    tc::tc_fence_after();
-                }
-                if (!(ok = tc::w::mbar_wait(&slab_full[sb], (lt >> 1) & 1, p.err, 45))) break;
+            const uint64_t b0 = kmajor_desc(tc::smem_u32(wres), BN * 16);
+            constexpr uint32_t dhi = (uint32_t) (128 >> 4) | 1u << 14;   // kmajor_desc's high word
+            uint32_t lt = 0, ut = 0;
+            for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x, ut++) {
+                const int sb = ut & 1, rows = min(p.R, p.Ho - u / p.nwc % p.nrg * p.R);
+                if (!(ok = tc::w::mbar_wait(&slab_full[sb], (ut >> 1) & 1, p.err, 45))) break;
                 tc::tc_fence_after();
-                const uint32_t a0 = tc::smem_u32(slab + sb * p.buf_bytes);
-                const uint32_t dt = tmem + (uint32_t) (buf * BN);
+                const uint32_t a0 = (tc::smem_u32(slab + sb * p.buf_bytes) & 0x3FFFF) >> 4;
+                for (int r = 0; r < rows; r++, lt++) {
+                    const int buf = lt & 1;
+                    if (lt >= 2) {
+                        if (!(ok = tc::w::mbar_wait(&acc_empty[buf], ((lt >> 1) + 1) & 1, p.err, 44))) break;
+                        tc::tc_fence_after();
+                    }
+                    const uint32_t dt = tmem + (uint32_t) (buf * BN);
 #pragma unroll
-                for (int q = 0; q < STEM_MAXPAIRS; q++)
-                    if (q < p.npairs)
-                        tc::w::mma_f16(dt, dhi | (uint64_t) (alo[q] + ((a0 & 0x3FFFF) >> 4)),
-                                    kmajor_desc(wbase + q * C::PAIR_W, BN * 16), idesc, q > 0);
-                tc::w::mma_commit(&slab_free[sb]);
-                tc::w::mma_commit(&acc_full[buf]);
+                    for (int q = 0; q < STEM_MAXPAIRS; q++)
+                        if (q < p.npairs)
+                            tc::w::mma_f16(dt, (uint64_t) dhi << 32 | (p.adesc[q] + a0 + r * p.astep[q]),
+                                           b0 + (uint64_t) (q * (C::PAIR_W >> 4)), idesc, q > 0);
+                    if (r == rows - 1) tc::w::mma_commit(&slab_free[sb]);
+                    tc::w::mma_commit(&acc_full[buf]);
+                }
             }
         }
         __syncwarp();
@@ -299,7 +288,7 @@ int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
 // The slab geometry of a shape; false when the path does not apply.
 struct StemGeom {
-    int bn, wc, qmin, qmax, nj, hbox, npairs;
+    int bn, wc, qmin, qmax, nj, hbox, npairs, R;
     uint32_t rho_bytes, buf_bytes;
 };
 
@@ -321,9 +310,29 @@ bool stem_geom(const cg_shape &s, StemGeom &sg) {
     sg.hbox = (s.kh - 1) * s.vdil + 1;
     sg.npairs = (s.kh * s.kw + 1) / 2;
     sg.rho_bytes = (uint32_t) ((sg.hbox * sg.nj * 16 + 1023) / 1024 * 1024);
+    if (sg.nj * s.hstride > 256 || sg.hbox > 256 || (uint32_t) s.hstride * sg.rho_bytes > STEM_SLAB_MAX ||
+        (uint32_t) sg.npairs * 2 * sg.bn * 16 > STEM_W_MAX)
+        return false;
+    // Output rows per slab, as many as the buffer holds: neighbouring rows share most of their input rows (7 x 7
+    // at stride 2: 7 per row alone, 11 for three). A group costs its pixel loads (a clock each) or its tiles' MMAs
+    // and epilogues (some 850 clocks each), the SMs take groups in waves.
+    long long best = 0;
+    const int hbox1 = sg.hbox, sms = tc_num_sms();
+    for (int R = 1; R <= 4; R++) {
+        const int hbox = hbox1 + (R - 1) * s.vstride;
+        const uint32_t rho_bytes = (uint32_t) ((hbox * sg.nj * 16 + 1023) / 1024 * 1024);
+        if (hbox > 256 || (uint32_t) s.hstride * rho_bytes > STEM_SLAB_MAX || R > g.ho) break;
+        const long long units = (long long) s.b * ((g.ho + R - 1) / R) * ((g.wo + 127) / 128);
+        const long long cost = (units + sms - 1) / sms * std::max(R * 850, hbox * sg.nj * s.hstride);
+        if (R == 1 || cost < best) {
+            best = cost;
+            sg.R = R;
+            sg.hbox = hbox;
+            sg.rho_bytes = rho_bytes;
+        }
+    }
     sg.buf_bytes = (uint32_t) s.hstride * sg.rho_bytes + STEM_ZERO;
-    return sg.nj * s.hstride <= 256 && sg.hbox <= 256 && (uint32_t) s.hstride * sg.rho_bytes <= STEM_SLAB_MAX &&
-           (uint32_t) sg.npairs * 2 * sg.bn * 16 <= STEM_W_MAX;
+    return true;
 }
 
 }  // namespace
@@ -357,7 +366,9 @@ convgemm_status_t tc_stem_run(const cg_shape &s, const void *x, const void *wpac
     p.kn = s.kn;
     p.Kpad = Kpad;
     p.nwc = (g.wo + 127) / 128;
-    p.total = s.b * g.ho * p.nwc;
+    p.R = sg.R;
+    p.nrg = (g.ho + sg.R - 1) / sg.R;
+    p.units = s.b * p.nrg * p.nwc;
     p.sh = s.vstride;
     p.sw = s.hstride;
     p.pad_h = s.vpad;
@@ -385,15 +396,12 @@ convgemm_status_t tc_stem_run(const cg_shape &s, const void *x, const void *wpac
     const uint32_t zero_off = (uint32_t) s.hstride * sg.rho_bytes;
     for (int q = 0; q < sg.npairs; q++) {
         const TapAt &t1 = taps[2 * q];
-        p.aoff[q] = t1.off;
+        const bool two = 2 * q + 1 < ntaps;
+        const uint32_t lead = (two ? taps[2 * q + 1].off : zero_off) - t1.off, row4 = (uint32_t) (s.vstride * sg.nj);
+        p.adesc[q] = (uint32_t) kmajor_desc(t1.off, lead);
+        p.astep[q] = two ? row4 : row4 - (row4 << 16);   // the zero region stays where it is
         p.wtap[2 * q] = (int16_t) t1.tap;
-        if (2 * q + 1 < ntaps) {
-            p.alead[q] = taps[2 * q + 1].off - t1.off;
-            p.wtap[2 * q + 1] = (int16_t) taps[2 * q + 1].tap;
-        } else {
-            p.alead[q] = zero_off - t1.off;
-            p.wtap[2 * q + 1] = -1;
-        }
+        p.wtap[2 * q + 1] = two ? (int16_t) taps[2 * q + 1].tap : (int16_t) -1;
     }
     // input [B][H][W][8]: box {8, nj * sw (traversal stride sw: nj pixels), hbox rows, 1 image}
     CUtensorMap xmap, omap;
@@ -415,7 +423,7 @@ convgemm_status_t tc_stem_run(const cg_shape &s, const void *x, const void *wpac
         if (convgemm_status_t e = tc_make_map_nd(&omap, 3, y, dims, str, box, estr, 1)) return e;
     }
     const int sms = tc_num_sms();
-    const int grid = p.total < sms ? p.total : sms;
+    const int grid = p.units < sms ? p.units : sms;
     return cg_cuda_check(sg.bn == 64 ? launch_stem<64>(p, xmap, omap, grid, st) : launch_stem<128>(p, xmap, omap, grid, st),
                          "small-channel forward launch");
 }
