@@ -1259,7 +1259,7 @@ def main():
     alg_bytes = sum(layer_bytes(l, batch, dominant) for d, l in zip(net.L, layers)
                     if not (dominant == "dgrad" and d["first"]))
     traffic = profile_traffic(("tc_wgrad_kernel", "tc_stem_wgrad_kernel", "wgrad_reduce_kernel",
-                               "wgrad_group_sum_kernel")) \
+                               "wgrad_reduce_groups_kernel", "wgrad_group_sum_kernel")) \
         if dominant == "wgrad" else None
     roofline = {"bound": "tensor", "kernel": kern_of[dominant], "achieved": dom["tflops"],
                 "peak": peaks["bf16_tflops_sustained"], "unit": "TFLOP/s",
