@@ -359,10 +359,26 @@ __global__ void pack_split_kernel(const float *__restrict__ w, int nchw, int C, 
     }
 }
 
+// n values by 256 threads, B loads in flight per thread.
+template <int B, class T, class Load, class Store>
+__device__ __forceinline__ void batched(int n, Load load, Store store) {
+    for (int i0 = threadIdx.x; i0 < n; i0 += 256 * B) {
+        T v[B];
+#pragma unroll
+        for (int j = 0; j < B; j++)
+            if (i0 + 256 * j < n) v[j] = load(i0 + 256 * j);
+#pragma unroll
+        for (int j = 0; j < B; j++)
+            if (i0 + 256 * j < n) store(i0 + 256 * j, v[j]);
+    }
+}
+
 // Grouped preparation: every block finds its job by binary search over the jobs'
 // first blocks and runs that job's body for its block (256 threads).
-// The jobs' first blocks (b0, njobs ints) are staged in shared memory first, so the
-// search costs one global round trip.
+// What bounds it is the chain of latencies within a block: the jobs' first blocks (b0, njobs ints) are staged in
+// shared memory, so the search costs one global round trip, then the job itself (read field by field from memory,
+// each access a round trip again behind the stores), and the weights are read several at a time. Both operands of
+// 512 x 512 x 3 x 3 (NCHW) 20.6 us, 14.4 so; of a 1024 / 256-channel bottleneck 12.9, 10.4.
 __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restrict__ jobs, const int *__restrict__ b0,
                                                          int njobs) {
     __shared__ float tile[64][65];
@@ -377,9 +393,14 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
         if (s_b0[mid] <= (int) blockIdx.x) lo = mid;
         else hi = mid - 1;
     }
-    const PrepJob &J = jobs[lo];
-    const int lb = blockIdx.x - J.block0;
     const int t = threadIdx.x;
+    __shared__ alignas(16) uint32_t job[sizeof(PrepJob) / 4];
+    __shared__ int taps[TC_MAXTAPS];   // the class's filter taps (input-gradient jobs)
+    static_assert(sizeof(PrepJob) % 4 == 0, "job copied by words");
+    for (int i = t; i < (int) (sizeof(PrepJob) / 4); i += 256) job[i] = __ldg(reinterpret_cast<const uint32_t *>(jobs + lo) + i);
+    __syncthreads();
+    const PrepJob &J = *reinterpret_cast<const PrepJob *>(job);
+    const int lb = blockIdx.x - J.block0;
     switch (J.type) {
         case PREP_FOLD: {
             const int n = lb * 256 + t;
@@ -457,12 +478,32 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
             float *buf = &tile[0][0];
             const float *src = J.w + ((size_t) co * J.C + ci0) * khw;
             const int have = max(0, min(n, J.C - ci0)) * khw;
-#pragma unroll 4
-            for (int i = t; i < n * khw; i += 256) buf[i] = i < have ? __ldg(src + i) : 0.0f;
+            if (((uintptr_t) src & 15) == 0 && (have & 3) == 0 && (n * khw & 3) == 0)
+                batched<4, float4>(
+                    n * khw >> 2,
+                    [&](int i) { return 4 * i < have ? __ldg(reinterpret_cast<const float4 *>(src) + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f); },
+                    [&](int i, float4 v) {
+                        buf[4 * i] = v.x;
+                        buf[4 * i + 1] = v.y;
+                        buf[4 * i + 2] = v.z;
+                        buf[4 * i + 3] = v.w;
+                    });
+            else
+                batched<8, float>(n * khw, [&](int i) { return i < have ? __ldg(src + i) : 0.0f; }, [&](int i, float v) { buf[i] = v; });
             __syncthreads();
+            // a warp per tap, two channels per store where the chunk's ends are even
             bf16 *row = (bf16 *) J.out + (size_t) co * Kpad;
-            for (int tap = 0; tap < khw; tap++)
-                for (int ci = t; ci < n; ci += 256) row[tap * Cp + ci0 + ci] = __float2bfloat16_rn(buf[ci * khw + tap]);
+            const int lane = t & 31;
+            if ((n & 1) == 0 && (ci0 & 1) == 0 && ((uintptr_t) row & 3) == 0) {
+                for (int tap = t >> 5; tap < khw; tap += 8)
+#pragma unroll 4
+                    for (int ci = 2 * lane; ci < n; ci += 64)
+                        *reinterpret_cast<__nv_bfloat162 *>(row + tap * Cp + ci0 + ci) =
+                            __floats2bfloat162_rn(buf[ci * khw + tap], buf[(ci + 1) * khw + tap]);
+            } else {
+                for (int tap = t >> 5; tap < khw; tap += 8)
+                    for (int ci = lane; ci < n; ci += 32) row[tap * Cp + ci0 + ci] = __float2bfloat16_rn(buf[ci * khw + tap]);
+            }
             if (ci0 == 0)
                 for (int k = khw * Cp + t; k < Kpad; k += 256) row[k] = __float2bfloat16_rn(0.0f);
             return;
@@ -485,19 +526,41 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
             const int beg = J.info.kbeg[c], end = c + 1 < J.info.ncls ? J.info.kbeg[c + 1] : Ktot;
             const int nt = J.info.ntaps[c], nci = min(4, C - ci0), w4 = nci * khw, pitch = (4 * khw) | 1, nco = min(run, knp - co0);
             float *buf = &tile[0][0];
-            __shared__ int taps[TC_MAXTAPS];
             if (t < nt) taps[t] = J.info.kx[J.info.tap0[c] + t] * J.kw + J.info.ky[J.info.tap0[c] + t];
             const float *src = J.w + ((size_t) co0 * C + ci0) * khw;
             const int have = J.kn - co0;
-            for (int i = t; i < nco * w4; i += 256) {
-                const int co = i / w4, k = i - co * w4;
-                buf[co * pitch + k] = co < have ? __ldg(src + (size_t) co * C * khw + k) : 0.0f;
+            const int lane = t & 31;
+            if ((w4 & 3) == 0 && (C * khw & 3) == 0 && ((uintptr_t) src & 15) == 0) {
+                // 16 lanes per output channel
+#pragma unroll 4
+                for (int co = t >> 4; co < nco; co += 16)
+                    for (int k = 4 * (t & 15); k < w4; k += 64) {
+                        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        if (co < have) v = __ldg(reinterpret_cast<const float4 *>(src + (size_t) co * C * khw + k));
+                        float *d = buf + co * pitch + k;
+                        d[0] = v.x;
+                        d[1] = v.y;
+                        d[2] = v.z;
+                        d[3] = v.w;
+                    }
+            } else {
+                for (int co = t >> 5; co < nco; co += 8)
+                    for (int k = lane; k < w4; k += 32)
+                        buf[co * pitch + k] = co < have ? __ldg(src + (size_t) co * C * khw + k) : 0.0f;
             }
             __syncthreads();
+            // a warp per (input channel, tap), two output channels per store
             bf16 *dst = (bf16 *) J.out + (size_t) ci0 * Ktot + beg + co0;
-            for (int i = t; i < nci * nt * nco; i += 256) {
-                const int q = i / nco, co = i - q * nco, r = q / nt, g = q - r * nt;
-                dst[(size_t) r * Ktot + g * knp + co] = __float2bfloat16_rn(buf[co * pitch + r * khw + taps[g]]);
+            const bool two = (nco & 1) == 0 && (knp & 1) == 0 && (Ktot & 1) == 0 && ((uintptr_t) dst & 3) == 0;
+            for (int q = t >> 5; q < nci * nt; q += 8) {
+                const int r = q / nt, g = q - r * nt;
+                const float *v = buf + r * khw + taps[g];
+                bf16 *o = dst + (size_t) r * Ktot + g * knp;
+                if (two)
+                    for (int co = 2 * lane; co < nco; co += 64)
+                        *reinterpret_cast<__nv_bfloat162 *>(o + co) = __floats2bfloat162_rn(v[co * pitch], v[(co + 1) * pitch]);
+                else
+                    for (int co = lane; co < nco; co += 32) o[co] = __float2bfloat16_rn(v[co * pitch]);
             }
             if (co0 == 0)   // the K padding after the class's taps
                 for (int r = 0; r < nci; r++)
@@ -512,28 +575,29 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
             if (!J.nchw && (J.kn & 3) == 0 && (J.knp & 3) == 0 && ((beg | end | J.info.Ktot) & 3) == 0 &&
                 ((uintptr_t) J.w & 15) == 0 && ((uintptr_t) J.out & 7) == 0) {
                 // NHWC-API weights: four consecutive output channels per 16-byte load and 8-byte
-                // store, unrolled for several loads in flight
-                const int nq = (end - beg) >> 2;
-                for (int r = 0; r < 4; r++) {
-                    const int ci = ci0 + r;
-                    if (ci >= J.C) break;
-                    bf16 *row = (bf16 *) J.out + (size_t) ci * J.info.Ktot + beg;
-#pragma unroll 4
-                    for (int q = t; q < nq; q += 256) {
-                        const int idx = q * 4;
-                        const int g = (int) J.dknp.div((uint32_t) idx), co = idx - g * J.knp;
-                        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        if (g < nt && co < J.kn) {
-                            const int tap = J.info.kx[J.info.tap0[c] + g] * J.kw + J.info.ky[J.info.tap0[c] + g];
-                            v = __ldg(reinterpret_cast<const float4 *>(J.w + ((size_t) ci * J.kh * J.kw + tap) * J.kn + co));
-                        }
+                // store, four loads in flight
+                if (t < nt) taps[t] = J.info.kx[J.info.tap0[c] + t] * J.kw + J.info.ky[J.info.tap0[c] + t];
+                __syncthreads();
+                const int nq = (end - beg) >> 2, khw = J.kh * J.kw, kn = J.kn, knp = J.knp, Ktot = J.info.Ktot;
+                const FastDiv dknp = J.dknp;
+                const float *w = J.w + (size_t) ci0 * khw * kn;
+                bf16 *out = (bf16 *) J.out + (size_t) ci0 * Ktot + beg;
+                batched<4, float4>(
+                    min(4, J.C - ci0) * nq,
+                    [&](int i) {
+                        const int r = i / nq, idx = (i - r * nq) * 4;
+                        const int g = (int) dknp.div((uint32_t) idx), co = idx - g * knp;
+                        if (g >= nt || co >= kn) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        return __ldg(reinterpret_cast<const float4 *>(w + ((size_t) r * khw + taps[g]) * kn + co));
+                    },
+                    [&](int i, float4 v) {
+                        const int r = i / nq, idx = (i - r * nq) * 4;
                         __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
                         uint2 u;
                         u.x = *reinterpret_cast<uint32_t *>(&lo);
                         u.y = *reinterpret_cast<uint32_t *>(&hi);
-                        *reinterpret_cast<uint2 *>(row + idx) = u;
-                    }
-                }
+                        *reinterpret_cast<uint2 *>(out + (size_t) r * Ktot + idx) = u;
+                    });
                 return;
             }
             for (int r = 0; r < 4; r++) {

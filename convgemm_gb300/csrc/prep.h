@@ -15,7 +15,7 @@ struct PackDgradInfo {
 // one batch-norm fold or one weight packing.
 enum { PREP_FOLD = 0, PREP_FWD_TILED = 1, PREP_FWD_NCHW = 2, PREP_FWD_TAIL = 3, PREP_DGRAD = 4, PREP_DGRAD_NCHW = 5 };
 // Input channels per block of a PREP_FWD_NCHW job: their taps fill the 64 x 65 float staging tile.
-__host__ __device__ constexpr int prep_nchw_channels(int khw) { return 4160 / khw < 512 ? 4160 / khw : 512; }
+__host__ __device__ constexpr int prep_nchw_channels(int khw) { return 4160 / khw < 512 ? 4160 / khw & ~3 : 512; }
 // Output channels per block of a PREP_DGRAD_NCHW job: four input channels' taps of each in the same tile.
 __host__ __device__ constexpr int prep_nchw_run(int khw) { return 4160 / ((4 * khw) | 1) < 64 ? 4160 / ((4 * khw) | 1) : 64; }
 struct PrepJob {

@@ -305,8 +305,8 @@ struct TileForm {
     int bn, mt, ew;
     float block, epi, launch;
 };
-constexpr TileForm FORMS_BF16[] = {{64, 1, 4, 0.180f, 1.10f, 3.2f}, {128, 1, 4, 0.203f, 1.95f, 3.6f}, {128, 1, 8, 0.230f, 1.20f, 3.8f},
-                                   {128, 2, 8, 0.332f, 2.05f, 4.6f}, {256, 1, 8, 0.313f, 1.95f, 4.6f}};
+constexpr TileForm FORMS_BF16[] = {{64, 1, 4, 0.178f, 1.01f, 3.1f}, {128, 1, 4, 0.210f, 1.45f, 3.7f}, {128, 1, 8, 0.231f, 1.11f, 3.5f},
+                                   {128, 2, 8, 0.335f, 1.86f, 4.1f}, {256, 1, 8, 0.315f, 1.77f, 4.1f}};
 // with a ReLU mask, or with column sums (batch statistics, a fused bias gradient) in the epilogue
 constexpr TileForm FORMS_MASK[] = {{64, 1, 8, 0.190f, 0.95f, 3.2f}, {128, 1, 8, 0.230f, 1.85f, 3.8f}, {256, 1, 8, 0.313f, 3.50f, 4.6f}};
 constexpr TileForm FORMS_SUMS[] = {{64, 1, 8, 0.190f, 1.30f, 3.2f}, {128, 1, 8, 0.230f, 2.80f, 3.8f}, {256, 1, 8, 0.313f, 5.00f, 4.6f}};
