@@ -18,6 +18,7 @@
 #include "cg_common.cuh"
 #include "cg_internal.h"
 #include "tc_host.h"
+#include "tc_ptx.cuh"
 
 namespace {
 
@@ -40,7 +41,9 @@ __device__ __forceinline__ double widen(float f) {   // (double) f
 constexpr int BN_ONE_PASS = 1024;
 template <int PLANES, class OUT>
 __global__ void __launch_bounds__(256) bn_stats_pass1(const float *__restrict__ part, int ngroups, int chunk, int kn,
-                                                      OUT *__restrict__ out) {
+        OUT *__restrict__ out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     __shared__ double red[PLANES][32][9];
     const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
     const int c = blockIdx.x * 8 + tx;
@@ -97,6 +100,8 @@ __device__ __forceinline__ double chunk_total(const double *__restrict__ chunks,
 }
 // stats[0][c] = sum, stats[1][c] = sum of squares.
 __global__ void __launch_bounds__(256) bn_stats_pass2(const double *__restrict__ chunks, int nchunks, int kn, double *__restrict__ stats) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const int i = blockIdx.x * 32 + (threadIdx.x & 31);
     const double a = chunk_total(chunks, nchunks, 2 * kn, i, i < 2 * kn);
     if (threadIdx.x < 32 && i < 2 * kn) stats[i] = a;
@@ -104,6 +109,8 @@ __global__ void __launch_bounds__(256) bn_stats_pass2(const double *__restrict__
 
 // Column sums in FP32: out[c] = sum over the chunks of the first statistics plane.
 __global__ void __launch_bounds__(256) colsum_pass2_f32(const double *__restrict__ chunks, int nchunks, int kn, float *__restrict__ out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const int c = blockIdx.x * 32 + (threadIdx.x & 31);
     const double a = chunk_total(chunks, nchunks, 2 * kn, c, c < kn);
     if (threadIdx.x < 32 && c < kn) out[c] = (float) a;
@@ -112,6 +119,8 @@ __global__ void __launch_bounds__(256) colsum_pass2_f32(const double *__restrict
 __global__ void bn_fold_kernel(int kn, const double *__restrict__ stats, double inv_count, const float *gamma,
                                const float *beta, float eps, float *scale, float *shift, float *mean_out,
                                float *var_out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= kn) return;
     const double mean = stats[c] * inv_count;
@@ -128,7 +137,9 @@ __global__ void bn_fold_kernel(int kn, const double *__restrict__ stats, double 
 // channels (the number of threads is a multiple of k8 = kn / 8) and has four loads in flight; with a 64-bit division
 // and the tables read at each step, 103 MB in and 103 out took 37 us, 31 so (30 at the rate of a copy).
 __global__ void __launch_bounds__(256) bn_apply_kernel(long long n8, int k8, const uint4 *z, const float *__restrict__ scale,
-                                                       const float *__restrict__ shift, int relu, uint4 *y) {
+        const float *__restrict__ shift, int relu, uint4 *y) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const long long step = (long long) gridDim.x * blockDim.x;
     long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x;
     const int c0 = (int) (i % k8) * 8;
@@ -169,6 +180,8 @@ __global__ void __launch_bounds__(256) bn_apply_kernel(long long n8, int k8, con
 // an infinity under the mask and the sign of a zero stay what they were.
 __global__ void epilogue_grad_kernel(uint32_t n8, uint32_t k8, const uint4 *__restrict__ gy, const uint4 *__restrict__ y,
                                      const float *__restrict__ scale, uint4 *__restrict__ dz) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += gridDim.x * blockDim.x) {
         const uint4 ug = gy[i], uy = y ? y[i] : ug;
         const uint32_t wg[4] = {ug.x, ug.y, ug.z, ug.w}, wy[4] = {uy.x, uy.y, uy.z, uy.w};
@@ -222,15 +235,14 @@ cudaError_t cg_colsum_reduce(void *workspace, int ngroups, int kn, float *out, c
     double *chunks = (double *) workspace;
     const float *part = (const float *) ((uint8_t *) workspace + (size_t) nchunks * 2 * kn * 8);
     if (ngroups <= BN_ONE_PASS) {
-        bn_stats_pass1<1, float><<<(kn + 7) / 8, 256, 0, st>>>(part, ngroups, BN_ONE_PASS, kn, out);
-        cg_note_launch();
+        cg_launch_pdl(bn_stats_pass1<1, float>, dim3((kn + 7) / 8), dim3(256), 0, st, part, ngroups, BN_ONE_PASS, kn, out);
         return cudaGetLastError();
     }
     dim3 g1((kn + 7) / 8, nchunks);
-    bn_stats_pass1<1, double><<<g1, 256, 0, st>>>(part, ngroups, BN_CHUNK, kn, chunks);
-    cg_note_launch();
-    colsum_pass2_f32<<<(kn + 31) / 32, 256, 0, st>>>(chunks, nchunks, kn, out);
-    cg_note_launch();
+    // launched plainly: 56 x 56, 256-channel block 258 us a step, 268 with its blocks launched during the tail of the
+    // kernel that writes the groups
+    cg_launch_ex(CG_PDL_OFF, bn_stats_pass1<1, double>, g1, dim3(256), 0, st, part, ngroups, BN_CHUNK, kn, chunks);
+    cg_launch_pdl(colsum_pass2_f32, dim3((kn + 31) / 32), dim3(256), 0, st, chunks, nchunks, kn, out);
     return cudaGetLastError();
 }
 
@@ -241,9 +253,9 @@ extern "C" size_t convgemm_fwd_bf16_stats_workspace_size(const convgemm_shape_t 
 }
 
 extern "C" convgemm_status_t convgemm_fwd_bf16_stats(const convgemm_shape_t *shape, const void *x,
-                                                     const void *wpacked, void *y, const float *scale,
-                                                     const float *shift, int relu, double *stats, void *workspace,
-                                                     size_t workspace_bytes, void *stream) {
+        const void *wpacked, void *y, const float *scale,
+        const float *shift, int relu, double *stats, void *workspace,
+        size_t workspace_bytes, void *stream) {
     const char *fn = "convgemm_fwd_bf16_stats";
     if (!shape || !x || !wpacked || !y || !stats || !workspace)
         return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "%s: NULL argument", fn);
@@ -274,31 +286,27 @@ extern "C" convgemm_status_t convgemm_fwd_bf16_stats(const convgemm_shape_t *sha
     }
     if (e) return e;
     if (ng <= BN_ONE_PASS) {
-        bn_stats_pass1<2, double><<<(s.kn + 7) / 8, 256, 0, st>>>(part, ng, BN_ONE_PASS, s.kn, stats);
-        cg_note_launch();
+        cg_launch_pdl(bn_stats_pass1<2, double>, dim3((s.kn + 7) / 8), dim3(256), 0, st, part, ng, BN_ONE_PASS, s.kn, stats);
     } else {
         dim3 g1((s.kn + 7) / 8, nchunks);
-        bn_stats_pass1<2, double><<<g1, 256, 0, st>>>(part, ng, BN_CHUNK, s.kn, chunks);
-        cg_note_launch();
-        bn_stats_pass2<<<(2 * s.kn + 31) / 32, 256, 0, st>>>(chunks, nchunks, s.kn, stats);
-        cg_note_launch();
+        cg_launch_pdl(bn_stats_pass1<2, double>, g1, dim3(256), 0, st, part, ng, BN_CHUNK, s.kn, chunks);
+        cg_launch_pdl(bn_stats_pass2, dim3((2 * s.kn + 31) / 32), dim3(256), 0, st, chunks, nchunks, s.kn, stats);
     }
     return cg_cuda_check(cudaGetLastError(), "batch statistics reduction");
 }
 
 extern "C" convgemm_status_t convgemm_bn_stats_fold(int kn, const double *stats, long long count, const float *gamma,
-                                                    const float *beta, float eps, float *scale, float *shift,
-                                                    float *batch_mean, float *batch_var, void *stream) {
+        const float *beta, float eps, float *scale, float *shift,
+        float *batch_mean, float *batch_var, void *stream) {
     if (kn < 1 || !stats || count < 1 || !scale || !shift || !(eps >= 0.0f))
         return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "convgemm_bn_stats_fold: bad arguments");
-    bn_fold_kernel<<<(kn + 127) / 128, 128, 0, (cudaStream_t) stream>>>(kn, stats, 1.0 / (double) count, gamma, beta,
-                                                                        eps, scale, shift, batch_mean, batch_var);
-    cg_note_launch();
+    cg_launch_pdl(bn_fold_kernel, dim3((kn + 127) / 128), dim3(128), 0, (cudaStream_t) stream, kn, stats, 1.0 / (double) count, gamma, beta,
+        eps, scale, shift, batch_mean, batch_var);
     return cg_cuda_check(cudaGetLastError(), "convgemm_bn_stats_fold");
 }
 
 extern "C" convgemm_status_t convgemm_bn_apply_bf16(long long npix, int kn, const void *z, const float *scale,
-                                                    const float *shift, int relu, void *y, void *stream) {
+        const float *shift, int relu, void *y, void *stream) {
     if (npix < 1 || kn < 8 || kn % 8 || !z || !scale || !shift || !y)
         return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "convgemm_bn_apply_bf16: bad arguments (kn % 8 == 0)");
     if (((uintptr_t) z & 15) || ((uintptr_t) y & 15))
@@ -310,21 +318,19 @@ extern "C" convgemm_status_t convgemm_bn_apply_bf16(long long npix, int kn, cons
     if (blocks > 152 * 8) blocks = 152 * 8;
     const int unit = k8 / std::gcd(k8, 256);
     blocks = (blocks + unit - 1) / unit * unit;
-    bn_apply_kernel<<<(int) blocks, 256, 0, (cudaStream_t) stream>>>(n8, k8, (const uint4 *) z, scale, shift, relu,
-                                                                     (uint4 *) y);
-    cg_note_launch();
+    cg_launch_pdl(bn_apply_kernel, dim3((int) blocks), dim3(256), 0, (cudaStream_t) stream, n8, k8, (const uint4 *) z, scale, shift, relu,
+        (uint4 *) y);
     return cg_cuda_check(cudaGetLastError(), "convgemm_bn_apply_bf16");
 }
 
 extern "C" convgemm_status_t convgemm_epilogue_grad_bf16(long long npix, int kn, const void *gy, const void *y,
-                                                         const float *scale, void *dz, void *stream) {
+        const float *scale, void *dz, void *stream) {
     if (npix < 1 || kn < 8 || kn % 8 || !gy || !dz || npix > ((1LL << 31) - 1) / kn)
         return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "convgemm_epilogue_grad_bf16: bad arguments (kn %% 8 == 0)");
     if (((uintptr_t) gy & 15) || ((uintptr_t) y & 15) || ((uintptr_t) dz & 15))
         return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "convgemm_epilogue_grad_bf16: tensors must be 16-byte aligned");
     const uint32_t n8 = (uint32_t) (npix * (kn / 8)), blocks = (n8 + 255) / 256;
-    epilogue_grad_kernel<<<blocks < 152 * 16 ? blocks : 152 * 16, 256, 0, (cudaStream_t) stream>>>(
+    cg_launch_pdl(epilogue_grad_kernel, dim3(blocks < 152 * 16 ? blocks : 152 * 16), dim3(256), 0, (cudaStream_t) stream,
         n8, (uint32_t) kn / 8, (const uint4 *) gy, (const uint4 *) y, scale, (uint4 *) dz);
-    cg_note_launch();
     return cg_cuda_check(cudaGetLastError(), "convgemm_epilogue_grad_bf16");
 }

@@ -65,8 +65,8 @@ bool cg_pdl_env_enabled();   // false when the environment sets CONVGEMM_NO_PDL=
 
 // Programmatic dependent launch modes of cg_launch_ex.
 enum CgPdl {
-    CG_PDL_OFF = 0,      // plain launch (the weight-gradient kernels and their reductions)
-    CG_PDL_THREAD = 1,   // as the calling thread's setting says (the persistent chain kernels)
+    CG_PDL_OFF = 0,      // plain launch (the weight-gradient kernels)
+    CG_PDL_THREAD = 1,   // as the calling thread's setting says (the persistent chain kernels, and the small ones around them)
 };
 
 // Launch, with programmatic stream serialization per `pdl` (CgPdl): the kernel must call

@@ -28,6 +28,8 @@ __device__ __forceinline__ float wref(const float *w, int nchw, int C, int kh, i
 // writes along ci (contiguous in the packed row) through shared memory.
 __global__ void pack_fwd_tiled_kernel(const float *__restrict__ w, int C, int khw, int kn, int Cp, int Kpad,
                                       bf16 *__restrict__ out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     __shared__ float tile[32][33];
     const int tap = blockIdx.z, ci0 = blockIdx.x * 32, co0 = blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -44,6 +46,8 @@ __global__ void pack_fwd_tiled_kernel(const float *__restrict__ w, int C, int kh
 
 // zero of the K padding columns [khw*Cp, Kpad) of every row
 __global__ void pack_fwd_tail_kernel(int kn, int Kbeg, int Kpad, bf16 *__restrict__ out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const int width = Kpad - Kbeg;
     const long long total = (long long) kn * width;
     for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < total;
@@ -53,6 +57,8 @@ __global__ void pack_fwd_tail_kernel(int kn, int Kbeg, int Kpad, bf16 *__restric
 
 __global__ void pack_fwd_kernel(const float *__restrict__ w, int nchw, int C, int kh, int kw, int kn, int Cp,
                                 int Kpad, bf16 *__restrict__ out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const long long total = (long long) kn * Kpad;
     for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < total;
          i += (long long) gridDim.x * blockDim.x) {
@@ -67,6 +73,8 @@ __global__ void pack_fwd_kernel(const float *__restrict__ w, int nchw, int C, in
 // Input-gradient operand: out[ci][kbeg_c + t*knp + co] = W(ci, kx_t, ky_t, co) for each class c.
 __global__ void pack_dgrad_kernel(const float *__restrict__ w, int nchw, int C, int kh, int kw, int kn, int knp,
                                   const PackDgradInfo info, bf16 *__restrict__ out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const long long total = (long long) C * info.Ktot;
     for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < total;
          i += (long long) gridDim.x * blockDim.x) {
@@ -85,6 +93,8 @@ __global__ void pack_dgrad_kernel(const float *__restrict__ w, int nchw, int C, 
 // besides the oracle where FP64 runs on the GPU).
 __global__ void fold_kernel(int kn, const float *bias, const float *mean, const float *inv_std, const float *gamma,
                             const float *beta, float *scale, float *shift) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= kn) return;
     double s = 1.0, t = bias ? (double) bias[n] : 0.0;
@@ -99,6 +109,8 @@ __global__ void fold_kernel(int kn, const float *bias, const float *mean, const 
 // FP32 NHWC or NCHW [B][C][H][W] -> BF16 NHWC [B][H][W][Cp] (padding channels zero).
 __global__ void to_bf16_nhwc_kernel(const float *__restrict__ in, int nchw, int B, int C, int H, int W, int Cp,
                                     bf16 *__restrict__ out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const long long total = (long long) B * H * W * Cp;
     for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < total;
          i += (long long) gridDim.x * blockDim.x) {
@@ -133,6 +145,8 @@ __device__ __forceinline__ uint4 bf16x8_of(const float (&v)[8]) {
 // NCHW with c <= 8: a thread reads its pixel from every plane (neighbouring lanes, neighbouring pixels).
 __global__ void __launch_bounds__(256) nchw_few_to_bf16_kernel(const float *__restrict__ in, int C, long long HW, long long P,
                                                                uint4 *__restrict__ out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     for (long long i = blockIdx.x * 256LL + threadIdx.x; i < P; i += gridDim.x * 256LL) {
         const float *src = in + i / HW * C * HW + i % HW;
         float v[8];
@@ -146,6 +160,8 @@ __global__ void __launch_bounds__(256) nchw_few_to_bf16_kernel(const float *__re
 // vectors when HW % 4 == 0 and the input is aligned), pixels written along the channels.
 __global__ void __launch_bounds__(256) nchw_tiled_to_bf16_kernel(const float *__restrict__ in, int C, int HW, int Cp, int vec,
                                                                  uint4 *__restrict__ out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     __shared__ float t[64][65];
     const int q0 = blockIdx.x * 64, c0 = blockIdx.y * 64, tid = threadIdx.x;
     const float *src = in + (size_t) blockIdx.z * C * HW;
@@ -190,6 +206,8 @@ __global__ void __launch_bounds__(256) nchw_tiled_to_bf16_kernel(const float *__
 // NHWC: eight channels of a pixel per thread.
 __global__ void __launch_bounds__(256) nhwc_to_bf16_kernel(const float *__restrict__ in, int C, int Cp, long long n8, int vec,
                                                            uint4 *__restrict__ out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const int k8 = Cp / 8;
     for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n8; i += gridDim.x * 256LL) {
         float v[8];
@@ -239,6 +257,8 @@ __device__ __forceinline__ float load1(const void *in, long long i) {
 // n8: groups of eight read as vectors (0 when `in` is not 16-byte aligned).
 template <bool BF>
 __global__ void __launch_bounds__(256) amax_kernel(const void *__restrict__ in, long long n8, long long n, unsigned *amax_bits) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     __shared__ float red[8];
     const long long step = gridDim.x * 256LL, i0 = blockIdx.x * 256LL + threadIdx.x;
     float m = 0.0f;
@@ -274,6 +294,8 @@ __global__ void __launch_bounds__(256) amax_kernel(const void *__restrict__ in, 
 template <bool BF>
 __global__ void __launch_bounds__(256) quant_e4m3_kernel(const void *__restrict__ in, long long n8, long long n,
                                                          const unsigned *amax_bits, uint8_t *__restrict__ out, float *scale_out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const float amax = __uint_as_float(*amax_bits);
     const float sc = amax > 0.0f ? amax / E4M3_MAX : 1.0f;
     const float inv = 1.0f / sc;
@@ -293,6 +315,8 @@ __global__ void __launch_bounds__(256) quant_e4m3_kernel(const void *__restrict_
 
 // per-output-channel weight scale (NHWC-API weights [K][kn]: threads along co, loop over K)
 __global__ void wscale_kernel(const float *__restrict__ w, int nchw, int K, int kn, float *wscale) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const int co = blockIdx.x * blockDim.x + threadIdx.x;
     if (co >= kn) return;
     float m = 0.0f;
@@ -303,6 +327,8 @@ __global__ void wscale_kernel(const float *__restrict__ w, int nchw, int K, int 
 // E4M3 operand [co][tap*Cp + ci] = w / wscale[co]
 __global__ void pack_fp8_kernel(const float *__restrict__ w, int nchw, int C, int kh, int kw, int kn, int Cp, int Kpad,
                                 const float *__restrict__ wscale, uint8_t *__restrict__ out) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const long long total = (long long) kn * Kpad;
     for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < total;
          i += (long long) gridDim.x * blockDim.x) {
@@ -317,6 +343,8 @@ __global__ void pack_fp8_kernel(const float *__restrict__ w, int nchw, int C, in
 // scale' = scale * wscale * xscale (the two quantisation scales folded into the epilogue)
 __global__ void fp8_scales_kernel(int kn, const float *scale, const float *shift, const float *wscale,
                                   const float *xscale, float *out_scale, float *out_shift) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= kn) return;
     out_scale[n] = (scale ? scale[n] : 1.0f) * wscale[n] * xscale[0];
@@ -327,6 +355,8 @@ __global__ void fp8_scales_kernel(int kn, const float *scale, const float *shift
 // tensor is not 16-byte aligned).
 __global__ void __launch_bounds__(256) split_kernel(const float *__restrict__ in, long long n8, long long n, bf16 *__restrict__ hi,
                                                     bf16 *__restrict__ lo) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const long long step = gridDim.x * 256LL, i0 = blockIdx.x * 256LL + threadIdx.x;
     for (long long i = i0; i < n8; i += step) {
         float v[8], r[8];
@@ -346,6 +376,8 @@ __global__ void __launch_bounds__(256) split_kernel(const float *__restrict__ in
 
 __global__ void pack_split_kernel(const float *__restrict__ w, int nchw, int C, int kh, int kw, int kn, int Cp, int Kpad,
                                   bf16 *__restrict__ hi, bf16 *__restrict__ lo) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const long long total = (long long) kn * Kpad;
     for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < total;
          i += (long long) gridDim.x * blockDim.x) {
@@ -625,29 +657,26 @@ int grid_for(long long n) {
 cudaError_t prep_pack_fwd(const float *w, int nchw, int C, int kh, int kw, int kn, int Cp, int Kpad, void *out,
                           cudaStream_t st) {
     if (nchw) {
-        pack_fwd_kernel<<<grid_for((long long) kn * Kpad), 256, 0, st>>>(w, nchw, C, kh, kw, kn, Cp, Kpad,
-                                                                        (bf16 *) out); cg_note_launch();
+        cg_launch_pdl(pack_fwd_kernel, dim3(grid_for((long long) kn * Kpad)), dim3(256), 0, st, w, nchw, C, kh, kw, kn, Cp, Kpad, (bf16 *) out);
         return cudaGetLastError();
     }
     const int khw = kh * kw;
     dim3 grid((Cp + 31) / 32, (kn + 31) / 32, khw), block(32, 8);
-    pack_fwd_tiled_kernel<<<grid, block, 0, st>>>(w, C, khw, kn, Cp, Kpad, (bf16 *) out); cg_note_launch();
+    cg_launch_pdl(pack_fwd_tiled_kernel, grid, block, 0, st, w, C, khw, kn, Cp, Kpad, (bf16 *) out);
     if (Kpad > khw * Cp)
-        pack_fwd_tail_kernel<<<grid_for((long long) kn * (Kpad - khw * Cp)), 256, 0, st>>>(kn, khw * Cp, Kpad,
-                                                                                          (bf16 *) out); cg_note_launch();
+        cg_launch_pdl(pack_fwd_tail_kernel, dim3(grid_for((long long) kn * (Kpad - khw * Cp))), dim3(256), 0, st, kn, khw * Cp, Kpad, (bf16 *) out);
     return cudaGetLastError();
 }
 
 cudaError_t prep_pack_dgrad(const float *w, int nchw, int C, int kh, int kw, int kn, int knp,
                             const PackDgradInfo &info, void *out, cudaStream_t st) {
-    pack_dgrad_kernel<<<grid_for((long long) C * info.Ktot), 256, 0, st>>>(w, nchw, C, kh, kw, kn, knp, info,
-                                                                          (bf16 *) out); cg_note_launch();
+    cg_launch_pdl(pack_dgrad_kernel, dim3(grid_for((long long) C * info.Ktot)), dim3(256), 0, st, w, nchw, C, kh, kw, kn, knp, info, (bf16 *) out);
     return cudaGetLastError();
 }
 
 cudaError_t prep_fold(int kn, const float *bias, const float *mean, const float *inv_std, const float *gamma,
                       const float *beta, float *scale, float *shift, cudaStream_t st) {
-    fold_kernel<<<(kn + 127) / 128, 128, 0, st>>>(kn, bias, mean, inv_std, gamma, beta, scale, shift); cg_note_launch();
+    cg_launch_pdl(fold_kernel, dim3((kn + 127) / 128), dim3(128), 0, st, kn, bias, mean, inv_std, gamma, beta, scale, shift);
     return cudaGetLastError();
 }
 
@@ -656,16 +685,15 @@ cudaError_t prep_to_bf16_nhwc(const float *in, int nchw, int B, int C, int H, in
     const long long HW = (long long) H * W, P = B * HW;
     const bool vin = ((uintptr_t) in & 15) == 0;
     if ((uintptr_t) out & 15 || HW > (1LL << 30) || B > 65535 || Cp > 64 * 65535) {
-        to_bf16_nhwc_kernel<<<grid_for(P * Cp), 256, 0, st>>>(in, nchw, B, C, H, W, Cp, (bf16 *) out);
+        cg_launch_pdl(to_bf16_nhwc_kernel, dim3(grid_for(P * Cp)), dim3(256), 0, st, in, nchw, B, C, H, W, Cp, (bf16 *) out);
     } else if (!nchw) {
-        nhwc_to_bf16_kernel<<<grid_for(P * (Cp / 8)), 256, 0, st>>>(in, C, Cp, P * (Cp / 8), vin && C == Cp, (uint4 *) out);
+        cg_launch_pdl(nhwc_to_bf16_kernel, dim3(grid_for(P * (Cp / 8))), dim3(256), 0, st, in, C, Cp, P * (Cp / 8), vin && C == Cp, (uint4 *) out);
     } else if (C <= 8) {
-        nchw_few_to_bf16_kernel<<<grid_for(P), 256, 0, st>>>(in, C, HW, P, (uint4 *) out);
+        cg_launch_pdl(nchw_few_to_bf16_kernel, dim3(grid_for(P)), dim3(256), 0, st, in, C, HW, P, (uint4 *) out);
     } else {
         const dim3 grid((unsigned) ((HW + 63) / 64), (unsigned) ((Cp + 63) / 64), (unsigned) B);
-        nchw_tiled_to_bf16_kernel<<<grid, 256, 0, st>>>(in, C, (int) HW, Cp, vin && HW % 4 == 0, (uint4 *) out);
+        cg_launch_pdl(nchw_tiled_to_bf16_kernel, grid, dim3(256), 0, st, in, C, (int) HW, Cp, vin && HW % 4 == 0, (uint4 *) out);
     }
-    cg_note_launch();
     return cudaGetLastError();
 }
 
@@ -676,39 +704,37 @@ cudaError_t prep_fp8_quantize(long long n, int in_bf16, const void *in, void *ou
     const long long na = ((uintptr_t) in & 15) == 0 ? n / 8 : 0, nq = ((uintptr_t) out & 7) == 0 ? na : 0;
     const int ga = (int) std::min<long long>(grid_for(na ? na : n), 152 * 8), gq = grid_for(nq ? nq : n);
     if (in_bf16) {
-        amax_kernel<true><<<ga, 256, 0, st>>>(in, na, n, amax_tmp); cg_note_launch();
-        quant_e4m3_kernel<true><<<gq, 256, 0, st>>>(in, nq, n, amax_tmp, (uint8_t *) out, scale); cg_note_launch();
+        cg_launch_pdl(amax_kernel<true>, dim3(ga), dim3(256), 0, st, in, na, n, amax_tmp);
+        cg_launch_pdl(quant_e4m3_kernel<true>, dim3(gq), dim3(256), 0, st, in, nq, n, amax_tmp, (uint8_t *) out, scale);
     } else {
-        amax_kernel<false><<<ga, 256, 0, st>>>(in, na, n, amax_tmp); cg_note_launch();
-        quant_e4m3_kernel<false><<<gq, 256, 0, st>>>(in, nq, n, amax_tmp, (uint8_t *) out, scale); cg_note_launch();
+        cg_launch_pdl(amax_kernel<false>, dim3(ga), dim3(256), 0, st, in, na, n, amax_tmp);
+        cg_launch_pdl(quant_e4m3_kernel<false>, dim3(gq), dim3(256), 0, st, in, nq, n, amax_tmp, (uint8_t *) out, scale);
     }
     return cudaGetLastError();
 }
 
 cudaError_t prep_pack_fp8(const float *w, int nchw, int C, int kh, int kw, int kn, int Cp, int Kpad, void *out,
                           float *wscale, cudaStream_t st) {
-    wscale_kernel<<<(kn + 127) / 128, 128, 0, st>>>(w, nchw, C * kh * kw, kn, wscale); cg_note_launch();
-    pack_fp8_kernel<<<grid_for((long long) kn * Kpad), 256, 0, st>>>(w, nchw, C, kh, kw, kn, Cp, Kpad, wscale,
-                                                                    (uint8_t *) out); cg_note_launch();
+    cg_launch_pdl(wscale_kernel, dim3((kn + 127) / 128), dim3(128), 0, st, w, nchw, C * kh * kw, kn, wscale);
+    cg_launch_pdl(pack_fp8_kernel, dim3(grid_for((long long) kn * Kpad)), dim3(256), 0, st, w, nchw, C, kh, kw, kn, Cp, Kpad, wscale, (uint8_t *) out);
     return cudaGetLastError();
 }
 
 cudaError_t prep_fp8_scales(int kn, const float *scale, const float *shift, const float *wscale, const float *xscale,
                             float *out_scale, float *out_shift, cudaStream_t st) {
-    fp8_scales_kernel<<<(kn + 127) / 128, 128, 0, st>>>(kn, scale, shift, wscale, xscale, out_scale, out_shift); cg_note_launch();
+    cg_launch_pdl(fp8_scales_kernel, dim3((kn + 127) / 128), dim3(128), 0, st, kn, scale, shift, wscale, xscale, out_scale, out_shift);
     return cudaGetLastError();
 }
 
 cudaError_t prep_split(long long n, const float *in, void *hi, void *lo, cudaStream_t st) {
     const long long n8 = (((uintptr_t) in | (uintptr_t) hi | (uintptr_t) lo) & 15) == 0 ? n / 8 : 0;
-    split_kernel<<<grid_for(n8 ? n8 : n), 256, 0, st>>>(in, n8, n, (bf16 *) hi, (bf16 *) lo); cg_note_launch();
+    cg_launch_pdl(split_kernel, dim3(grid_for(n8 ? n8 : n)), dim3(256), 0, st, in, n8, n, (bf16 *) hi, (bf16 *) lo);
     return cudaGetLastError();
 }
 
 cudaError_t prep_pack_split(const float *w, int nchw, int C, int kh, int kw, int kn, int Cp, int Kpad, void *hi,
                             void *lo, cudaStream_t st) {
-    pack_split_kernel<<<grid_for((long long) kn * Kpad), 256, 0, st>>>(w, nchw, C, kh, kw, kn, Cp, Kpad, (bf16 *) hi,
-                                                                      (bf16 *) lo); cg_note_launch();
+    cg_launch_pdl(pack_split_kernel, dim3(grid_for((long long) kn * Kpad)), dim3(256), 0, st, w, nchw, C, kh, kw, kn, Cp, Kpad, (bf16 *) hi, (bf16 *) lo);
     return cudaGetLastError();
 }
 

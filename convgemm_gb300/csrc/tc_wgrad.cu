@@ -1128,12 +1128,12 @@ cudaError_t tc_wgrad_reduce(float *ws, float *dw, int splits, int xa, int Nx, in
     const int groups = tc_wgrad_groups(splits);
     if (groups) {
         const int rows = xa ? Nx : kn, cols = xa ? kn : Nx;
-        return cg_launch_ex(CG_PDL_OFF, wgrad_reduce_groups_kernel, dim3((rows + 3) / 4, (cols + 31) / 32),
+        return cg_launch_ex(CG_PDL_THREAD, wgrad_reduce_groups_kernel, dim3((rows + 3) / 4, (cols + 31) / 32),
                             dim3(32, WG_RED_WARPS), 0, st, (const float *) ws, dw, splits, groups,
                             (splits + groups - 1) / groups, xa, Nx, kn, C, Cp, kh * kw, layout);
     }
     dim3 grid((kn + 31) / 32, (Nx + 31) / 32), block(32, 8);
-    return cg_launch_ex(CG_PDL_OFF, wgrad_reduce_kernel, grid, block, 0, st, (const float *) ws, dw, splits, xa, Nx, kn, C, Cp, kh * kw, layout);
+    return cg_launch_ex(CG_PDL_THREAD, wgrad_reduce_kernel, grid, block, 0, st, (const float *) ws, dw, splits, xa, Nx, kn, C, Cp, kh * kw, layout);
 }
 
 // ------------------------------------------------------------ bias gradient
@@ -1148,6 +1148,8 @@ namespace {
 // ld % 8 == 0).
 __global__ void __launch_bounds__(256) bias_grad_pass1(const __nv_bfloat16 *__restrict__ dy, int P, int kn, int ld,
                                                        int rows, int vec, float *__restrict__ part) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     __shared__ float acc[32][65];
     const int r = threadIdx.x >> 3, c8 = (threadIdx.x & 7) * 8, ch = blockIdx.x * 64 + c8;
     const int p0 = blockIdx.y * rows, p1 = min(P, p0 + rows);
@@ -1184,6 +1186,8 @@ __global__ void __launch_bounds__(256) bias_grad_pass1(const __nv_bfloat16 *__re
 }
 
 __global__ void bias_grad_pass2(const float *__restrict__ part, int groups, int kn, float *__restrict__ db) {
+    tc::pdl_wait();
+    tc::pdl_trigger();
     const int ch = blockIdx.x * blockDim.x + threadIdx.x;
     if (ch >= kn) return;
     float sacc = 0.0f;
@@ -1210,8 +1214,8 @@ cudaError_t tc_bias_grad(const void *dy, long long P, int kn, int ld, float *db,
     const int groups = tc_bias_grad_groups(P);
     const int rows = (int) ((P + groups - 1) / groups);
     dim3 g1((kn + 63) / 64, groups);
-    bias_grad_pass1<<<g1, 256, 0, st>>>((const __nv_bfloat16 *) dy, (int) P, kn, ld, rows, ((uintptr_t) dy & 15) == 0, part); cg_note_launch();
-    bias_grad_pass2<<<(kn + 127) / 128, 128, 0, st>>>(part, groups, kn, db); cg_note_launch();
+    cg_launch_pdl(bias_grad_pass1, g1, dim3(256), 0, st, (const __nv_bfloat16 *) dy, (int) P, kn, ld, rows, ((uintptr_t) dy & 15) == 0, part);
+    cg_launch_pdl(bias_grad_pass2, dim3((kn + 127) / 128), dim3(128), 0, st, part, groups, kn, db);
     return cudaGetLastError();
 }
 
