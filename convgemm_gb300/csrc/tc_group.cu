@@ -52,13 +52,23 @@ struct alignas(64) GroupProblem {
 };
 
 constexpr int GBN = 256;
-constexpr int GSTAGES = 3, GEW = 8;
+constexpr int GEW = 8;
 constexpr int GTHREADS = 32 * (4 + GEW);
 constexpr uint32_t A_BYTES = 128 * 128;
-constexpr uint32_t B_MAX = GBN * 128;
-constexpr uint32_t STAGE_BYTES = A_BYTES + B_MAX;
-constexpr uint32_t EPI_BYTES = GEW * 4096;   // one 32 x 64 staging chunk per epilogue warp; two buffers
-constexpr size_t GSMEM = 1024 + GSTAGES * STAGE_BYTES + 2 * EPI_BYTES + 256 + 2 * GBN * 4;
+// The ring's 192 KB hold four, six or eight stages by the width of the problem's tiles (up to 256, 128, 64
+// channels), so that narrow tiles have as many bytes in flight as wide ones: 22 convolutions led by 5 x 5, 400 -> 96
+// took 472 us with three stages for all widths, 347 so. The table lists the problems by ring class, and the producer
+// lets the ring run empty between two classes.
+constexpr uint32_t RING_BYTES = 192 * 1024;
+constexpr int GCLS = 3, GMAXSTAGES = 8;
+__host__ __device__ constexpr int ring_class(int nn) { return nn > 128 ? 0 : (nn > 64 ? 1 : 2); }
+__host__ __device__ constexpr int ring_stages(int c) { return 4 + 2 * c; }
+__host__ __device__ constexpr uint32_t ring_stage_bytes(int c) { return A_BYTES + (c == 0 ? 256u : (c == 1 ? 128u : 64u)) * 128u; }
+static_assert(ring_stages(0) * ring_stage_bytes(0) <= RING_BYTES && ring_stages(1) * ring_stage_bytes(1) <= RING_BYTES &&
+                  ring_stages(2) * ring_stage_bytes(2) <= RING_BYTES && ring_stages(GCLS - 1) <= GMAXSTAGES,
+              "ring");
+constexpr uint32_t EPI_BYTES = GEW * 4096;   // one 32 x 64 staging chunk per epilogue warp
+constexpr size_t GSMEM = RING_BYTES + EPI_BYTES + 512 + 2 * GBN * 4;
 static_assert(GSMEM <= 232448, "shared memory above the 227 KB per-block limit");
 
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(32 * GEW) : "memory"); }
@@ -75,27 +85,27 @@ __device__ __forceinline__ bool advance(const GroupProblem *probs, int nprob, in
 
 __global__ void __launch_bounds__(GTHREADS, 1)
     tc_group_kernel(const GroupProblem *__restrict__ probs, int nprob, int total, int *err) {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t *base = (uint8_t *) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023);
-    uint8_t *epi = base + GSTAGES * STAGE_BYTES;
-    uint64_t *full = (uint64_t *) (epi + 2 * EPI_BYTES);
-    uint64_t *empty = full + GSTAGES;
-    uint64_t *acc_full = empty + GSTAGES;
+    extern __shared__ __align__(1024) uint8_t base[];
+    uint8_t *epi = base + RING_BYTES;
+    uint64_t *full = (uint64_t *) (epi + EPI_BYTES);    // [ring class][stage]
+    uint64_t *empty = full + GCLS * GMAXSTAGES;
+    uint64_t *acc_full = empty + GCLS * GMAXSTAGES;
     uint64_t *acc_empty = acc_full + 2;
     uint32_t *tmem_holder = (uint32_t *) (acc_empty + 2);
-    float *sc_tab = (float *) (epi + 2 * EPI_BYTES + 256);
+    static_assert((2 * GCLS * GMAXSTAGES + 5) * 8 <= 512, "mbarriers");
+    float *sc_tab = (float *) (epi + EPI_BYTES + 512);
     float *sh_tab = sc_tab + GBN;
 
     const int warp = tc::w::warp_index(), lane = threadIdx.x & 31;
     tc::pdl_wait();   // pdl_trigger: when the producer starts this CTA's last tile
-    // a table prepared for another count, or a tile count beyond the table: run nothing
-    if (__ldg(&probs[0].count) != nprob) {
+    // a table prepared for another count (or tiles that would not lie on the swizzle's 1024-byte grid): run nothing
+    if (__ldg(&probs[0].count) != nprob || (tc::smem_u32(base) & 1023)) {
         if (threadIdx.x == 0) atomicCAS(err, 0, 25);
         return;
     }
     total = min(total, __ldg(&probs[nprob - 1].tile_end));
     if (threadIdx.x == 0) {
-        for (int s = 0; s < GSTAGES; s++) {
+        for (int s = 0; s < GCLS * GMAXSTAGES; s++) {
             tc::mbar_init(&full[s], 1);
             tc::mbar_init(&empty[s], 1);
         }
@@ -118,7 +128,9 @@ __global__ void __launch_bounds__(GTHREADS, 1)
 
     if (warp == 0) {
         // ---------------------------------------------- producer
-        uint32_t it = 0, tx_bytes = 0;
+        uint32_t it = 0, ph = 0, tx_bytes = 0;   // K blocks of this ring class so far, parity of the ring's turn
+        int rc = -1, S = 1, s = 0;                // ring class, its stages, the next stage
+        uint64_t *fullc = full, *emptyc = empty;
         const GroupProblem *P = nullptr;
         int tile0 = 0, ntn = 1, nn = 0, ktiles = 0, cpb = 1, isy = 0, isx = 0, lo_y = 0, lo_x = 0;
         FastDiv dwg, dhg;
@@ -138,6 +150,18 @@ __global__ void __launch_bounds__(GTHREADS, 1)
                 dwg = P->dwg;
                 dhg = P->dhg;
                 tx_bytes = A_BYTES + (uint32_t) nn * 128;
+                const int c = __shfl_sync(0xFFFFFFFFu, ring_class(nn), 0);
+                if (c != rc) {
+                    for (uint32_t j = it > (uint32_t) S ? it - S : 0; j < it && ok; j++)
+                        ok = tc::w::mbar_wait(&emptyc[j % S], (j / S) & 1, err, 21);
+                    if (!ok) break;
+                    rc = c;
+                    S = ring_stages(c);
+                    fullc = full + c * GMAXSTAGES;
+                    emptyc = empty + c * GMAXSTAGES;
+                    it = ph = 0;
+                    s = 0;
+                }
             }
             const int local = tile - tile0, mt = local / ntn, n0 = (local - mt * ntn) * nn;
             uint32_t q, jw, j, b;
@@ -147,14 +171,16 @@ __global__ void __launch_bounds__(GTHREADS, 1)
             int tap = 0, cc = 0;
             int32_t to = __ldg(&P->taps[0]), to_next = __ldg(&P->taps[1]);   // the next tap's offsets, loaded ahead
             for (int kt = 0; kt < ktiles; kt++, it++) {
-                const int s = it % GSTAGES;
-                const uint32_t ph = (it / GSTAGES) & 1;
-                if (it >= (uint32_t) GSTAGES && !(ok = tc::w::mbar_wait(&empty[s], ph ^ 1, err, 21))) break;
-                const uint32_t sa = tc::smem_u32(base + s * STAGE_BYTES);
-                tc::w::mbar_arrive_expect_tx(&full[s], tx_bytes);
+                if (it >= (uint32_t) S && !(ok = tc::w::mbar_wait(&emptyc[s], ph ^ 1, err, 21))) break;
+                const uint32_t sa = tc::smem_u32(base + s * ring_stage_bytes(rc));
+                tc::w::mbar_arrive_expect_tx(&fullc[s], tx_bytes);
                 tc::w::tma_load_im2col_4d(sa, &P->amap, cc * 64, w0, h0, (int) b, (uint16_t) (to & 0xFFFF),
-                                          (uint16_t) (to >> 16), &full[s]);
-                tc::w::tma_load_2d(sa + A_BYTES, &P->wmap, kt * 64, n0, &full[s]);
+                                          (uint16_t) (to >> 16), &fullc[s]);
+                tc::w::tma_load_2d(sa + A_BYTES, &P->wmap, kt * 64, n0, &fullc[s]);
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1;
+                }
                 if (++cc == cpb) {
                     cc = 0;
                     tap++;
@@ -167,7 +193,7 @@ __global__ void __launch_bounds__(GTHREADS, 1)
         // -------------------------------------------------- epilogue
         const int ew = (warp - 4) & 3, half = (warp - 4) >> 2, et = threadIdx.x - 128;
         uint32_t lt = 0;
-        int ebuf = 0;
+        uint8_t *stg = epi + (warp - 4) * 4096;
         const GroupProblem *P = nullptr;
         int tile0 = 0, ntn = 1, nn = 0, Cout = 0, relu = 0, M = 0;
         const float *scale = nullptr, *shift = nullptr;
@@ -213,9 +239,8 @@ __global__ void __launch_bounds__(GTHREADS, 1)
                 uint32_t pk[32];
                 tc::frag_pack(v, relu != 0, pk);
                 // each warp stages its 32 rows and stores them itself: no barrier across warps
-                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                 __syncwarp();
-                uint8_t *stg = epi + ebuf * EPI_BYTES + (warp - 4) * 4096;
                 tc::frag_stage(stg, pk);
                 tc::fence_proxy_async_smem();
                 __syncwarp();
@@ -226,20 +251,29 @@ __global__ void __launch_bounds__(GTHREADS, 1)
                                 (uint64_t) &P->omap),
                             "r"(tc::smem_u32(stg)), "r"(n0 + c0), "r"(m0 + ew * 32)
                             : "memory");
-                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");   // a group per chunk: the waits count them
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
-                ebuf ^= 1;
             }
         }
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else if (warp == 1) {
         // -------------------------------------------------- MMA issuer
-        uint32_t it = 0, lt = 0, idesc = 0;
-        int ktiles = 0;
+        uint32_t ph = 0, lt = 0, idesc = 0;
+        int ktiles = 0, rc = -1, S = 1, s = 0;
+        uint64_t *fullc = full, *emptyc = empty;
         for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, lt++) {
             if (advance(probs, nprob, tile, pi, pend)) {
                 ktiles = __shfl_sync(0xFFFFFFFFu, __ldg(&probs[pi].ktiles), 0);
                 idesc = __shfl_sync(0xFFFFFFFFu, __ldg(&probs[pi].idesc), 0);
+                const int c = __shfl_sync(0xFFFFFFFFu, ring_class(__ldg(&probs[pi].nn)), 0);
+                if (c != rc) {
+                    rc = c;
+                    S = ring_stages(c);
+                    fullc = full + c * GMAXSTAGES;
+                    emptyc = empty + c * GMAXSTAGES;
+                    ph = 0;
+                    s = 0;
+                }
             }
             const int buf = lt & 1;
             if (lt >= 2) {
@@ -248,20 +282,22 @@ __global__ void __launch_bounds__(GTHREADS, 1)
                 tc::tc_fence_after();
             }
             const uint32_t dt = tmem + (uint32_t) (buf * GBN);
-            for (int kt = 0; kt < ktiles; kt++, it++) {
-                const int s = it % GSTAGES;
-                const uint32_t ph = (it / GSTAGES) & 1;
-                if (!tc::w::mbar_wait(&full[s], ph, err, 22)) {
+            for (int kt = 0; kt < ktiles; kt++) {
+                if (!tc::w::mbar_wait(&fullc[s], ph, err, 22)) {
                     ok = false;
                     break;
                 }
                 tc::tc_fence_after();
                 // descriptors built once per stage; a 32-byte K step adds 2 to the start field
-                const uint64_t ad = tc::sw128_desc(tc::smem_u32(base + s * STAGE_BYTES), 16, 1024);
+                const uint64_t ad = tc::sw128_desc(tc::smem_u32(base + s * ring_stage_bytes(rc)), 16, 1024);
                 const uint64_t bd = ad + (A_BYTES >> 4);
 #pragma unroll
                 for (int k = 0; k < 4; k++) tc::w::mma_f16(dt, ad + 2 * k, bd + 2 * k, idesc, (kt | k) != 0);
-                tc::w::mma_commit(&empty[s]);
+                tc::w::mma_commit(&emptyc[s]);
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1;
+                }
             }
             tc::w::mma_commit(&acc_full[buf]);
         }
@@ -316,8 +352,8 @@ extern "C" convgemm_status_t convgemm_group_prepare(int n, const convgemm_group_
         return cg_set_error(CONVGEMM_ERROR_WORKSPACE, "%s: table needs %zu bytes, 64-byte aligned", fn,
                             convgemm_group_table_size(n));
     // Tiles go to the persistent CTAs round-robin, so the table lists the
-    // convolutions by decreasing K length (the cost of one of their tiles):
-    // every CTA then gets a similar mix of long and short tiles.
+    // convolutions of a ring class (below) by decreasing K length (the cost of one of
+    // their tiles): every CTA then gets a similar mix of long and short tiles.
     std::vector<int> order(n);
     for (int i = 0; i < n; i++) order[i] = i;
     auto klen = [&](int i) {
@@ -334,6 +370,14 @@ extern "C" convgemm_status_t convgemm_group_prepare(int n, const convgemm_group_
         wide += (make_geom(cg_from_public(s)).P + 127) / 128 * ((s.kn + 255) / 256);
     }
     const bool wide_ok = wide >= 2LL * tc_num_sms();
+    // equal tiles of whole 16-column widths; two tiles never share a 64-column chunk
+    auto tile_width = [&](const convgemm_group_conv_t &cv) {
+        const int kn = cv.shape.kn > 0 ? cv.shape.kn : 8;
+        const int bn = cv.bn == 64 || cv.bn == 128 || cv.bn == 256 ? cv.bn : (kn >= 256 || wide_ok ? 256 : (kn > 64 ? 128 : 64));
+        const int ntn = (kn + bn - 1) / bn, nn = rup((kn + ntn - 1) / ntn, 16);
+        return nn < 64 && ntn > 1 ? 64 : nn;
+    };
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return ring_class(tile_width(convs[a])) < ring_class(tile_width(convs[b])); });
     std::vector<GroupProblem> host(n);
     int t0 = 0;
     for (int oi = 0; oi < n; oi++) {
@@ -343,10 +387,7 @@ extern "C" convgemm_status_t convgemm_group_prepare(int n, const convgemm_group_
         if (!cv.x || !cv.w || !cv.y) return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "%s: conv %d has a NULL tensor", fn, i);
         const cg_shape s = cg_from_public(cv.shape);
         const ConvGeom g = make_geom(s);
-        const int bn = cv.bn == 64 || cv.bn == 128 || cv.bn == 256 ? cv.bn : (s.kn >= 256 || wide_ok ? 256 : (s.kn > 64 ? 128 : 64));
-        const int ntn = (s.kn + bn - 1) / bn;
-        int nn = rup((s.kn + ntn - 1) / ntn, 16);   // equal tiles; two tiles never share a 64-column chunk
-        if (nn < 64 && ntn > 1) nn = 64;
+        const int nn = tile_width(cv), ntn = (s.kn + nn - 1) / nn;
         const int c64 = rup(s.c, 64);
         GroupProblem &P = host[oi];
         memset(&P, 0, sizeof(P));

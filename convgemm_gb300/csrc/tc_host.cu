@@ -313,7 +313,7 @@ constexpr TileForm FORMS_SUMS[] = {{64, 1, 8, 0.190f, 1.30f, 3.2f}, {128, 1, 8, 
 constexpr TileForm FORMS_GATHER[] = {{64, 1, 4, 0.58f, 1.95f, 3.2f}, {128, 1, 4, 0.61f, 2.10f, 3.8f}, {256, 1, 4, 0.75f, 3.00f, 4.6f}};
 constexpr TileForm FORMS_FP8[] = {{64, 1, 4, 0.107f, 0.92f, 3.2f}, {128, 1, 4, 0.130f, 1.50f, 3.6f}, {256, 1, 4, 0.185f, 2.75f, 4.6f}};
 constexpr TileForm FORMS_FP8W[] = {{64, 1, 4, 0.150f, 0.92f, 3.2f}, {128, 1, 4, 0.200f, 1.50f, 3.6f}, {256, 1, 4, 0.306f, 2.75f, 4.6f}};
-constexpr TileForm FORMS_X3[] = {{64, 1, 4, 0.335f, 1.43f, 3.2f}, {128, 1, 4, 0.440f, 2.60f, 3.6f}, {256, 1, 4, 0.870f, 4.90f, 4.6f}};
+constexpr TileForm FORMS_X3[] = {{64, 1, 4, 0.335f, 1.22f, 3.2f}, {128, 1, 4, 0.440f, 2.10f, 3.6f}, {256, 1, 4, 0.870f, 4.50f, 4.6f}};
 
 // The plan's K blocks hold `kdiv` blocks of 64 channels each; *cost_out: the form's estimate.
 template <int N>

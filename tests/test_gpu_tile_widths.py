@@ -86,3 +86,29 @@ def test_input_gradient_widths(cglib, c, stride):
     torch.cuda.synchronize()
     cg.check_device()
     assert nmax(masked, torch.where(x > 0, want, torch.zeros_like(want))) <= 6e-3
+
+
+def test_group_of_every_ring_class(cglib):
+    """More tiles than CTAs in each class of widths (up to 64, 128, 256), long and short reductions, in one launch."""
+    from convgemm_gb300 import tc
+    cg = cglib
+    g = torch.Generator(device="cuda").manual_seed(9)
+    items, want = [], []
+    for b, hw, c, kn, k in [(40, 28, 64, 48, 3), (64, 28, 40, 96, 1), (33, 27, 72, 144, 3), (90, 14, 128, 264, 1),
+                            (64, 28, 24, 16, 1), (21, 30, 200, 128, 3), (2, 9, 8, 512, 5), (50, 28, 64, 64, 1)]:
+        s = cg.Shape.of(b, hw, hw, c, kn, k, k, k // 2, k // 2, 1, 1)
+        x = torch.randn(b, hw, hw, c, device="cuda", generator=g).to(torch.bfloat16)
+        wt = (torch.randn(c, k, k, kn, device="cuda", generator=g) * (2 / (c * k * k)) ** 0.5).to(torch.bfloat16).float()
+        wp = torch.empty(tc.group_weights_size(s) // 2, dtype=torch.bfloat16, device="cuda")
+        tc.group_pack_weights(cg.NHWC, s, wt, wp)
+        y = torch.full((b, hw, hw, kn), float("nan"), dtype=torch.bfloat16, device="cuda")
+        items.append({"shape": s, "x": x, "w": wp, "y": y, "bn": 0})
+        want.append(torch.nn.functional.conv2d(x.double().permute(0, 3, 1, 2), wt.double().permute(3, 0, 1, 2),
+                                               padding=k // 2).permute(0, 2, 3, 1))
+    grp = tc.Group(items)
+    for _ in range(2):
+        grp.launch()
+    torch.cuda.synchronize()
+    cg.check_device()
+    for it, z in zip(items, want):
+        assert nmax(it["y"], z) <= 6e-3
