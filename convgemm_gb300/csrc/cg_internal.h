@@ -88,6 +88,27 @@ cudaError_t cg_launch_ex(int pdl, void (*kernel)(KArgs...), dim3 grid, dim3 bloc
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args &&>(args)...);
 }
 
+// The same with clusters of `csize` adjacent blocks.
+template <typename... KArgs, typename... Args>
+cudaError_t cg_launch_pdl_cluster(int csize, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                  Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned) csize;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cg_pdl_enabled() ? 2 : 1;
+    cg_note_launch();
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args &&>(args)...);
+}
+
 // Launch with programmatic stream serialization (the kernel must call
 // tc::pdl_wait() before its first global memory access); plain launch when the
 // environment sets CONVGEMM_NO_PDL=1.  Counts the launch.

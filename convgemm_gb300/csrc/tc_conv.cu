@@ -21,16 +21,23 @@
 // (channel, tap, Cout) boxes where a tap's last K block is partly zeros).  The
 // FP32 accumulator lives in TMEM.
 //
-// The kernel is persistent: each CTA walks tiles blockIdx.x, +gridDim.x, ...
-// with two TMEM accumulators, so the epilogue of one tile runs while the MMAs
-// of the next accumulate.  Warp roles (288 threads):
-//   warps 0-3  load A (one thread issuing the im2col TMA, or all four warps
-//              gathering), thread 0 also issues the B TMA; stage ring of STAGES;
-//   warps 4-7  epilogue: TMEM -> registers (tcgen05.ld), scale/shift/ReLU,
-//              BF16, then either a 128-byte-swizzled shared-memory tile and a
-//              TMA store (pixels contiguous in the output), or direct stores
-//              (the strided pixels of an input-gradient class);
-//   warp 8     allocates TMEM; one lane issues tcgen05.mma and the commits.
+// The kernel is persistent: each CTA walks tiles blockIdx.x, +gridDim.x, ... (launches of few tiles: a
+// cluster of 2 or 4 CTAs per tile, see TcConvParams::split)
+// with two to four TMEM accumulators, so the epilogue of one tile runs while the
+// MMAs of the next accumulate.  Warp roles (288 threads, 384 with EW = 8):
+//   warps 0-3   load A and B (warp 0 by TMA; or all four warps gathering A);
+//               stage ring of STAGES;
+//   warps 4-    epilogue (EW = 4 or 8 warps): TMEM -> registers (tcgen05.ld),
+//               scale/shift/ReLU, BF16, then either a 128-byte-swizzled
+//               shared-memory tile and a TMA store (pixels contiguous in the
+//               output), or whole rows (the strided pixels of a class);
+//   warp 8 / 1  allocates TMEM, issues tcgen05.mma and the commits.
+// The producer and MMA loops run by whole warps, an elected lane issuing each
+// instruction, so that its operands are in uniform registers: issued by a single
+// thread, every operand was moved there first, and that, not the tensor core or the
+// loads, bounded the short K blocks (64-wide tiles 0.27 us per block, 0.18 so).
+// What bounds it now: the tensor core at its operand-read rate on long reductions,
+// the loads of x on short ones, and waves of tiles that do not fill the SMs.
 #include <cuda_bf16.h>
 
 #include "cg_common.cuh"
@@ -91,6 +98,7 @@ struct TcCfg {
     static constexpr size_t SMEM = 1024 + (size_t) STAGES * STAGE_BYTES + EPI_BUFS * EPI_BYTES + BAR_BYTES + TAB_BYTES;
     static_assert(SMEM <= 232448, "shared memory above the 227 KB per-block limit");
     static_assert(EW == 4 || EW == 8, "four or eight epilogue warps");
+    static_assert(BN != 64 || MT != 1 || (size_t) STAGES * STAGE_BYTES >= 3 * 128 * BN * 4, "a split tile's shares in the ring");
     // warps: 0 producer (0-3 on the cp.async path), 4..4+EW-1 epilogue, the MMA issuer in
     // warp 8 (EW = 4) or in the otherwise idle warp 1 (EW = 8)
     static constexpr int THREADS = EW == 8 ? 384 : 288;
@@ -240,13 +248,18 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
     tc::tc_fence_after();
     const uint32_t tmem = *tmem_holder;
     bool ok = true;
+    // split reductions: CTA `krank` of the tile's cluster takes its share of the K blocks
+    constexpr bool SPLITS = IM2C && MT == 1 && BN == 64;
+    const int split = SPLITS ? p.split : 1, krank = split > 1 ? (int) blockIdx.x % split : 0;
+    const int cta = split > 1 ? (int) blockIdx.x / split : (int) blockIdx.x;   // the first tile
+    bool met = false;   // this thread has passed the cluster's two meetings
 
     if (IM2C && warp < 4 && warp != C::MMA_WARP) {
         // ------------------------------------------------ producer: one warp, im2col TMA for A, TMA for B
         if (warp == 0) {
             uint32_t it = 0;
             const uint32_t b_bytes = (uint32_t) (C::NOPS * nn * C::ROWB);
-            for (int tile = blockIdx.x; tile < p.ntiles_total && ok; tile += gridDim.x) {
+            for (int tile = cta; tile < p.ntiles_total && ok; tile += gridDim.x) {
                 if (tile + (int) gridDim.x >= p.ntiles_total) tc::pdl_trigger();   // this CTA's last tile
                 const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, nn, tile, MT);
                 const ClsS &cl = cls_tab[tl.cls];
@@ -264,11 +277,19 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                 }
                 const CUtensorMap *am = &amaps.a[tl.cls];
                 int tap = 0, ci0 = 0;   // k = tap*Cin + ci0, walked incrementally
-                for (int kt = 0; kt < ktiles; kt += KB, it++) {
+                int k0 = 0, k1 = ktiles;
+                if (split > 1) {
+                    const int cpb = (p.Cin + C::BK - 1) / C::BK;
+                    k0 = ktiles * krank / split;
+                    k1 = ktiles * (krank + 1) / split;
+                    tap = k0 / cpb;
+                    ci0 = (k0 - tap * cpb) * C::BK;
+                }
+                for (int kt = k0; kt < k1; kt += KB, it++) {
                     const int s = it % STAGES;
                     const uint32_t ph = (it / STAGES) & 1;
                     if (it >= (uint32_t) STAGES && !(ok = tc::w::mbar_wait(&empty[s], ph ^ 1, p.err, 1))) break;
-                    const int nkb = min(KB, ktiles - kt);
+                    const int nkb = min(KB, k1 - kt);
                     const uint32_t sa = tc::smem_u32(base + s * C::STAGE_BYTES);
                     tc::w::mbar_arrive_expect_tx(&full[s], nkb * (MT * C::A_BLOCK + b_bytes));
                     for (int kb = 0; kb < nkb; kb++) {
@@ -415,10 +436,10 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
         bool by_tma = false;       // this item's mask arrives at mbar[ebuf]
         uint32_t mphase = 0;       // bit b: parity of the next arrival at mbar[b]
         if constexpr (MASKED) {
-            const int t0 = blockIdx.x + (int) (lt * gridDim.x);
-            if (p.mask && t0 < p.ntiles_total && first_item < NIT) by_tma = prefetch_mask(t0, first_item, 0);
+            const int t0 = cta + (int) (lt * gridDim.x);
+            if (p.mask && t0 < p.ntiles_total && first_item < NIT && krank == 0) by_tma = prefetch_mask(t0, first_item, 0);
         }
-        for (int tile = blockIdx.x + (int) (lt * gridDim.x); tile < p.ntiles_total && ok; tile += TSTEP * gridDim.x, lt += TSTEP) {
+        for (int tile = cta + (int) (lt * gridDim.x); tile < p.ntiles_total && ok; tile += TSTEP * gridDim.x, lt += TSTEP) {
             const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, nn, tile, MT);
             const ClsS &cl = cls_tab[tl.cls];
             const int M = p.B * cl.Hg * cl.Wg;
@@ -444,8 +465,33 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                 shp = sh;
             }
             ok = tc::mbar_wait(&acc_full[buf], (lt / C::ACC_BUFS) & 1, p.err, 3);
-            if (!ok) break;
             tc::tc_fence_after();
+            if constexpr (SPLITS) {
+                if (split > 1) {
+                    // the tile's only pass: the other CTAs' accumulators go to the first one's ring, which nothing uses
+                    // any more, as [chunk][warp][four registers][lane]
+                    met = true;
+                    tc::cluster_meet();
+                    if (krank > 0) {
+                        const uint32_t dst = tc::mapa_shared(tc::smem_u32(base) + (uint32_t) ((krank - 1) * C::NCH * 4 * C::CW * 128), 0);
+                        for (int ch = 0; ch < nch && ok; ch++) {
+                            uint32_t v[2][C::CW / 2];
+                            tc::frag_load<C::CW / 8>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * BN + chunk_col(ch)), v);
+#pragma unroll
+                            for (int j = 0; j < C::CW / 4; j++) {
+                                const uint32_t *w = &v[j / (C::CW / 8)][j % (C::CW / 8) * 4];
+                                asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
+                                                 dst + (uint32_t) (((ch * 4 + ew) * (C::CW / 4) + j) * 512 + lane * 16)),
+                                             "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+                                             : "memory");
+                            }
+                        }
+                    }
+                    tc::cluster_meet();
+                    if (krank > 0) break;
+                }
+            }
+            if (!ok) break;
             if (first_item >= NIT) {   // nothing for this warp in the tile: its share of the buffer is free
                 tc::tc_fence_before();
                 tc::mbar_arrive(&acc_empty[buf]);
@@ -467,6 +513,20 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                 constexpr int NQ = C::CW / 8;
                 uint32_t v[2][4 * NQ];
                 tc::frag_load<NQ>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) ((buf * MT + mt) * BN + c0), v);
+                if constexpr (SPLITS) {
+                    for (int o = 0; o < split - 1; o++) {   // the other shares of the sum, in order
+                        const uint8_t *src = base + o * C::NCH * 4 * C::CW * 128 + (item * 4 + ew) * (C::CW / 4) * 512 + lane * 16;
+#pragma unroll
+                        for (int j = 0; j < C::CW / 4; j++) {
+                            const uint4 u = *reinterpret_cast<const uint4 *>(src + j * 512);
+                            uint32_t *w = &v[j / (C::CW / 8)][j % (C::CW / 8) * 4];
+                            w[0] = __float_as_uint(__uint_as_float(w[0]) + __uint_as_float(u.x));
+                            w[1] = __float_as_uint(__uint_as_float(w[1]) + __uint_as_float(u.y));
+                            w[2] = __float_as_uint(__uint_as_float(w[2]) + __uint_as_float(u.z));
+                            w[3] = __float_as_uint(__uint_as_float(w[3]) + __uint_as_float(u.w));
+                        }
+                    }
+                }
                 if (item + STEP >= NIT) {
                     // this warp's last read of the accumulator: its share of the TMEM buffer
                     // goes back to the MMA warp
@@ -656,9 +716,10 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
             constexpr bool F8 = MODE == MODE_FP8 || MODE == MODE_FP8W;
             const uint32_t idesc = (F8 ? tc::idesc_e4m3(128, 0) : tc::idesc_bf16(128, 0, 0, 0)) | (uint32_t) (nn >> 3) << 17;
             uint32_t it = 0, lt = 0;
-            for (int tile = blockIdx.x; tile < p.ntiles_total && ok; tile += gridDim.x, lt++) {
+            for (int tile = cta; tile < p.ntiles_total && ok; tile += gridDim.x, lt++) {
                 const Tile tl = decode_tile(cls_tab, p.ncls, p.ntiles, nn, tile, MT);
-                const int KT = __shfl_sync(0xFFFFFFFFu, cls_tab[tl.cls].ktiles, 0);   // warp-uniform loop bounds
+                int KT = __shfl_sync(0xFFFFFFFFu, cls_tab[tl.cls].ktiles, 0);   // warp-uniform loop bounds
+                if (split > 1) KT = KT * (krank + 1) / split - KT * krank / split;
                 const int buf = lt % C::ACC_BUFS;
                 if (lt >= (uint32_t) C::ACC_BUFS) {
                     ok = tc::w::mbar_wait(&acc_empty[buf], ((lt / C::ACC_BUFS) - 1) & 1, p.err, 4);
@@ -713,6 +774,10 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
         }
         __syncwarp();
     }
+    if (split > 1 && !met) {   // the threads without a share in the exchange
+        tc::cluster_meet();
+        tc::cluster_meet();
+    }
 
     tc::tc_fence_before();
     __syncthreads();
@@ -731,6 +796,7 @@ cudaError_t launch_bn(const TcConvParams &p, const CUtensorMap &wmap, const CUte
         if (e != cudaSuccess) return e;
         attr = true;
     }
+    if (p.split > 1) return cg_launch_pdl_cluster(p.split, kern, dim3(grid), dim3(C::THREADS), C::SMEM, st, p, wmap, omap, amaps);
     return cg_launch_pdl(kern, dim3(grid), dim3(C::THREADS), C::SMEM, st, p, wmap, omap, amaps);
 }
 

@@ -47,6 +47,8 @@ struct TcConvParams {
     int bn;                    // output channels per tile (64, 128, 256)
     int ntiles;                // tiles along the output channels
     int nn;                    // output channels per tile in use: Cout / ntiles rounded up to 16, at most bn
+    int split;                 // CTAs (a cluster of 1, 2 or 4) that share each tile's K blocks: im2col, bn 64, one M tile, at
+                               // most one tile per cluster; the first adds the others' FP32 accumulators to its own
     int ntiles_total;          // all tiles of all classes; tile t of a class: m = t / ntiles, n = t % ntiles
     int epi_tma;               // output pixels are the GEMM rows in order: stage in SMEM, TMA store
     int im2col;                // A loaded by im2col-mode TMA, else gathered by cp.async

@@ -377,6 +377,31 @@ TileForm tc_pick_form(const TcPlan &pl, int mode, bool im2col, bool mask, bool s
     return mask ? cheapest_form(FORMS_MASK, pl, 1, sms) : cheapest_form(FORMS_BF16, pl, 1, sms);
 }
 
+// CTAs per tile where the tiles leave most SMs idle: the K blocks of a 64-channel tile shared by a cluster of 2 or 4,
+// where the blocks fewer in each CTA's chain (0.153 us each) save more than the cluster costs (its launch and the
+// exchange: 2.0 us for two, 3.2 for four; 16 shapes with each forced). Worth it from 27 blocks on: 14 x 14, 256 -> 256
+// 3 x 3 at batch 1 (8 tiles of 36 blocks) 8.9 -> 7.7 us, 7 x 7, 512 -> 512 (72 blocks) 14.4 -> 9.0; 28 x 28,
+// 128 -> 128 (18 blocks) 6.1 alone, 6.5 shared by two. The rule depends on the plan alone, and leaves out the slab
+// kernel's shapes, so that every form of a layer adds its products in the same order.
+int tc_pick_split(const TcPlan &pl, int kdiv, int sms) {
+    long long tiles = 0;
+    int kmax = 0;
+    for (int c = 0; c < pl.ncls; c++) {
+        tiles += (long long) pl.cls[c].mtiles * ((pl.Cout + 63) / 64);
+        kmax = pl.cls[c].ktiles / kdiv > kmax ? pl.cls[c].ktiles / kdiv : kmax;
+    }
+    int best = 1;
+    float best_cost = (float) kmax * 0.153f;
+    for (int sp = 2; sp <= 4 && tiles * sp <= sms; sp *= 2) {
+        const float cost = (float) ((kmax + sp - 1) / sp) * 0.153f + (sp == 2 ? 2.0f : 3.2f);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = sp;
+        }
+    }
+    return best;
+}
+
 // Epilogue warps of tc_conv_kernel: eight where asked for (`by_k`: where every class has at most 8 K
 // blocks) and the form exists.
 int tc_epilogue_warps(const TcPlan &pl, bool eight, bool by_k, int bn, int mt, bool bf16_im2col) {
@@ -413,7 +438,9 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     for (int c = 0; f8w && c < pi.ncls; c++)
         if (pi.cls[c].kbeg % 128 || pi.cls[c].ktiles % 2) f8w = false;
     const TileForm form = tc_pick_form(pi, f8w ? 3 : mode, p.im2col, mask != nullptr, stats != nullptr, sms);
-    p.bn = bn_override ? bn_override : form.bn;
+    // (a tuning entry names a form without the split, for all of the operation's forms)
+    p.split = p.im2col && !bn_override && !aux_override && !(mode == 0 && tc_slab_applicable(pl)) ? tc_pick_split(pi, f8w ? 2 : 1, sms) : 1;
+    p.bn = bn_override ? bn_override : (p.split > 1 ? 64 : form.bn);
     p.ntiles = (pl.Cout + p.bn - 1) / p.bn;
     // equal tiles of whole 16-column MMA widths; a single chunk of 64 columns is never shared by two tiles,
     // and an accumulating call, which must not add a repeated column twice, keeps whole chunks
@@ -500,7 +527,8 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     // eight epilogue warps, bit 3 (above) the general kernel instead of the slab kernel. Without bits 0-2:
     // the cheapest form's, or for a width that was set, one M tile and eight epilogue warps when every
     // class has at most 8 K blocks per tile (the epilogue, not the MMA, bounds such tiles)
-    const bool by_form = !bn_override && (aux_override & 7) == 0;
+    if (p.split > 1) aux_override = 1;   // one M tile, four epilogue warps
+    const bool by_form = p.split == 1 && !bn_override && (aux_override & 7) == 0;
     p.mt = (by_form ? form.mt == 2 : (aux_override & 3) == 2) && mode == 0 && p.im2col ? 2 : 1;
     p.ew = tc_epilogue_warps(pi, by_form ? form.ew == 8 : (aux_override & 4) != 0, !by_form && (aux_override & 7) == 0, p.bn,
                              p.mt, mode == 0 && p.im2col);
@@ -522,7 +550,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
         g0 += (int) (((long long) s.b * pl.cls[c].Hg * pl.cls[c].Wg + 31) / 32);
     }
     p.ntiles_total = t0;
-    const int grid = t0 < sms ? t0 : sms;
+    const int grid = p.split > 1 ? t0 * p.split : (t0 < sms ? t0 : sms);   // split: at most one tile per cluster
     return cg_cuda_check(tc_conv_launch(p, wmap, omap, amaps, grid, st), "tensor-core conv launch");
 }
 
@@ -1109,8 +1137,11 @@ extern "C" convgemm_status_t convgemm_tune_describe(int op, const convgemm_shape
         *bn = 64;
         return CONVGEMM_SUCCESS;
     }
+    const bool slab = tc_slab_applicable(pl);
     const int im2col = tc_use_im2col(pl, tc_num_sms());
     const TileForm form = tc_pick_form(pl, 0, im2col, false, false, tc_num_sms());
+    *cluster = im2col && !slab && !t.bn && !t.splits ? tc_pick_split(pl, 1, tc_num_sms()) : 1;
+    if (*cluster > 1) t = TcTune{64, 1};   // as tc_run
     const bool by_form = !t.bn && (t.splits & 7) == 0;
     *bn = t.bn ? t.bn : form.bn;
     const int mt = (by_form ? form.mt == 2 : (t.splits & 3) == 2) && im2col ? 2 : 1;

@@ -50,7 +50,7 @@ struct SlabParams {
     int kbeg;                    // first K column of the class in the packed weights
     int nbuf;                    // slab buffers
     int nstage;                  // output staging buffers (1 or 2)
-    int niss;                    // MMA-issuing threads (2..4): issuer k takes the CTA's tiles k, k + niss, ...
+    int niss;                    // MMA-issuing warps (2..4): issuer k takes the CTA's tiles k, k + niss, ...
     uint32_t buf_bytes;          // one slab buffer (1024-aligned)
     uint32_t slab_tx;            // bytes one slab load delivers
     uint32_t w_bytes;            // resident weights of one N tile
@@ -186,8 +186,7 @@ __global__ void __launch_bounds__(288, 1)
     } else if (warp == 8 || (warp >= 1 && warp < p.niss)) {
         // ------------------------------------------------ MMA issuers: warp 8 (issuer 0) and warps
         // 1 .. niss-1; issuer k takes this CTA's tiles k, k + niss, ..., each into its own
-        // accumulator buffer (one thread's instruction stream cannot issue N = 64 MMAs as fast as
-        // the tensor core runs them)
+        // accumulator buffer, so that the waits of one tile overlap the MMAs of another
         {
             const uint32_t me = warp == 8 ? 0u : (uint32_t) warp;
             constexpr uint32_t idesc = tc::idesc_bf16(128, SLAB_BN, 0, 0);

@@ -17,8 +17,8 @@
 //     8 channels x 8 pixels each, no swizzle) of pair m start at slab row 4*r and are one
 //     slab row apart (SBO = the row pitch), 8-pixel K groups 128 bytes apart (LBO): one
 //     M=128 MMA per pair and 16-pixel K step, four TMEM accumulators of 64 columns;
-//   * slab stages are double-buffered across bands; one MMA-issuing thread per tap pair
-//     (one thread's loop overhead between MMAs bounds its issue rate);
+//   * slab stages are double-buffered across bands; one MMA-issuing warp per tap pair
+//     (its loop overhead between MMAs bounds its issue rate);
 //   * dY arrives per output row (64 channels x Wpad pixels, 128-byte swizzle, pixels past
 //     Wo zero-filled) through a ring of SW_DYB buffers filled by a second producer warp;
 //   * kernel rows >= kh (their slab rows are not loaded: stale data) and taps kx >= kw
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(320, 1)
         __syncwarp();
     } else if (warp == 1 || warp >= 7) {
         // ------------------------------------------------ MMA issuers: one per tap pair, warp 1 pair 0,
-        // warps 7-9 pairs 1-3 (one thread's loop overhead between MMAs bounds its issue rate)
+        // warps 7-9 pairs 1-3 (a warp's loop overhead between MMAs bounds its issue rate)
         {
             const int m = warp == 1 ? 0 : warp - 6;
             constexpr uint32_t idesc = tc::idesc_bf16(128, 64, 1, 1);

@@ -104,13 +104,12 @@ struct WgCfg {
     static constexpr size_t SMEM = 1024 + (size_t) STAGES * STAGE_BYTES + 256;
 };
 
-// Warps: the gather warps (one TMA-issuing thread on the im2col path; eight warps of
+// Warps: the gather warps (one TMA-issuing warp on the im2col path; eight warps of
 // cp.async gathers otherwise, whose issue rate bounds that path), then the MMA warp;
 // warps 0-3 run the epilogue.
 // ISS2: a second MMA-issuing warp (warp GW + 1).  Each issuer takes alternate chunks of every
-// two-chunk stage into its own accumulator and the epilogue adds the two: one thread's tcgen05
-// issue, barrier wait and commit cost tens of cycles each, which bounds a single issuer of the
-// eight 128-wide MMAs of a stage.
+// two-chunk stage into its own accumulator and the epilogue adds the two (a tuning option: the barrier
+// waits and commits of one issuer overlap the other's MMAs).
 template <bool IM2C, bool ISS2 = false>
 struct WgWarps {
     static constexpr int GW = IM2C ? 4 : 8, THREADS = 32 * (GW + 1 + (ISS2 ? 1 : 0));

@@ -48,7 +48,7 @@ struct WsParams {
     int ncp, nct;              // input-block pairs, output-channel tiles
     int ksteps;                // 16-row K steps per band
     int stages;
-    int niss;                  // MMA-issuing threads (lane 0 of warps 1..niss), min(kw, 3)
+    int niss;                  // MMA-issuing warps (1..niss), min(kw, 3)
     uint32_t x_bytes, dy_bytes, stage_bytes;   // one slab / one dY atom buffer, one stage
     uint32_t x_box_rows;       // rows one TMA box writes (R * Wp)
     int *err;
@@ -132,8 +132,7 @@ __global__ void __launch_bounds__(128, 2)
     } else if (warp >= 1 && warp <= p.niss) {
         // MMA issuers (warps 1..niss): issuer j takes the accumulators dx = j, j + niss, ...;
         // each waits for the band, issues its MMAs and commits once to the band's empty barrier
-        // (count niss).  One thread's tcgen05 issue, barrier wait and commit cost tens of cycles
-        // each, so a single issuer cannot keep kw accumulators of short bands busy.
+        // (count niss), so that one's barrier waits and commits overlap the others' MMAs.
         constexpr uint32_t idesc = tc::idesc_bf16(128, BN, 1, 1);
         const int j = warp - 1;
         for (int i = 0; i < nb; i++) {

@@ -68,8 +68,8 @@ convgemm_status_t convgemm_selftest_wait_timeout(unsigned budget_ms, void *strea
 /* Number of GPU kernels the library has launched (or recorded into a stream
  * capture) in this process: a diagnostic for counting launches per step. */
 unsigned long long convgemm_launch_count(void);
-/* Programmatic dependent launch of the persistent forward / input-gradient kernels
- * (a kernel's prologue overlaps the previous kernel's tail on the same stream), for
+/* Programmatic dependent launch of the persistent forward / input-gradient kernels and of the
+ * casts, packings, reductions and normalisations around them (a kernel's prologue overlaps the previous kernel's tail on the same stream), for
  * the calling host thread: 1 on, 0 off, -1 back to the default (on unless the
  * environment sets CONVGEMM_NO_PDL=1).  Returns the previous setting (0 / 1).
  * Turn it off while other streams run work beside the chain: the early-launched
@@ -302,8 +302,9 @@ void convgemm_tune_clear(void);
  * gradient on one shape: *kernel 0 the general implicit GEMM, 1 a slab kernel, 2 the
  * small-channel kernel; *bn the tile width; *stages the ring stages of the general kernels (0 for
  * the slab and small-channel kernels, which size their buffers at run time); *cluster 1, or the
- * thread-block cluster size of a weight gradient whose splits are reduced in a cluster.  The
- * reference chooses its blocking once, from the BLIS context (src/gemm_blis.h:181-188). */
+ * thread-block cluster size of a weight gradient whose splits are reduced in a cluster, or of a
+ * forward / input gradient of few tiles whose K blocks are shared by a cluster (no tuning entry).
+ * The reference chooses its blocking once, from the BLIS context (src/gemm_blis.h:181-188). */
 convgemm_status_t convgemm_tune_describe(int op, const convgemm_shape_t *shape, int *kernel, int *bn, int *stages,
                                          int *cluster);
 
@@ -312,7 +313,7 @@ convgemm_status_t convgemm_tune_describe(int op, const convgemm_shape_t *shape, 
 /* One convolution of a grouped launch: BF16 NHWC x [b][h][w][c] (c % 8 == 0),
  * weights packed by convgemm_group_pack_weights, BF16 NHWC y [b][ho][wo][kn] =
  * relu?(acc*scale + shift) (scale/shift may be NULL); bn = output channels per
- * tile (64, 128 or 256; 0 = chosen from kn), e.g. from the autotuner. */
+ * tile at most (64, 128 or 256; 0 = chosen from kn and the number of tiles), e.g. from the autotuner. */
 typedef struct {
     convgemm_shape_t shape;
     const void *x;
