@@ -306,7 +306,7 @@ struct TileForm {
     float block, epi, launch;
 };
 constexpr TileForm FORMS_BF16[] = {{64, 1, 4, 0.178f, 1.01f, 3.1f}, {128, 1, 4, 0.210f, 1.45f, 3.7f}, {128, 1, 8, 0.231f, 1.11f, 3.5f},
-                                   {128, 2, 8, 0.335f, 1.86f, 4.1f}, {256, 1, 8, 0.315f, 1.77f, 4.1f}};
+                                   {64, 2, 8, 0.320f, 1.20f, 3.5f}, {128, 2, 8, 0.335f, 1.86f, 4.1f}, {256, 1, 8, 0.315f, 1.77f, 4.1f}};
 // with a ReLU mask, or with column sums (batch statistics, a fused bias gradient) in the epilogue
 constexpr TileForm FORMS_MASK[] = {{64, 1, 8, 0.190f, 0.95f, 3.2f}, {128, 1, 8, 0.230f, 1.85f, 3.8f}, {256, 1, 8, 0.313f, 3.50f, 4.6f}};
 constexpr TileForm FORMS_SUMS[] = {{64, 1, 8, 0.190f, 1.30f, 3.2f}, {128, 1, 8, 0.230f, 2.80f, 3.8f}, {256, 1, 8, 0.313f, 5.00f, 4.6f}};
