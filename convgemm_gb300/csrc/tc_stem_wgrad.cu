@@ -36,11 +36,13 @@
 
 namespace {
 
-constexpr int SW_R = 8;                          // output rows per band
+// Bands of 6 rows leave room for four dY rows in flight: the 224 x 224 stem's step 190 us, 194 with 8 rows and three
+// (which reload fewer input rows), 192 with 7 and four, 194 with 4 and seven.
+constexpr int SW_R = 6;                          // output rows per band
 constexpr int SW_NY = 2 * SW_R + 6;              // slab rows per stream and stage (kernel rows 0..7)
 constexpr int SW_MAXPAIRS = 4;                   // kw <= 8
-constexpr uint32_t SW_SLAB_MAX = 83 * 1024;      // 2 * SW_NY slab rows of one stage
-constexpr int SW_DYB = 3;                        // dY row buffers
+constexpr uint32_t SW_SLAB_MAX = 68 * 1024;      // 2 * SW_NY slab rows of one stage
+constexpr int SW_DYB = 4;                        // dY row buffers
 constexpr uint32_t SW_DY_MAX = 16 * 1024;        // one output row of dY: Wpad pixels x 128 B
 constexpr size_t SW_SMEM = 1024 + 2 * (size_t) SW_SLAB_MAX + SW_DYB * (size_t) SW_DY_MAX + 256;
 static_assert(SW_SMEM <= 232448, "shared memory");
