@@ -142,18 +142,24 @@ __device__ __forceinline__ uint4 bf16x8_of(const float (&v)[8]) {
 // 16-byte groups of eight channels; the element form above divides per element, reads NCHW planes with
 // one value per lane and line, and ran at 1.0 TB/s (64 x 3 x 224 x 224: 87 us) to 1.5 TB/s.
 //
-// NCHW with c <= 8: a thread reads its pixel from every plane (neighbouring lanes, neighbouring pixels).
-__global__ void __launch_bounds__(256) nchw_few_to_bf16_kernel(const float *__restrict__ in, int C, long long HW, long long P,
-                                                               uint4 *__restrict__ out) {
+// NCHW with c <= 8: a thread reads its pixels from every plane (neighbouring lanes, neighbouring pixels), four
+// pixels at a time, an image per blockIdx.y: 64 x 3 x 224 x 224 in 14.9 us (18.7 with one pixel at a time, found by
+// 64-bit division; 13.3 at the rate of a copy).
+__global__ void __launch_bounds__(256) nchw_few_to_bf16_kernel(const float *__restrict__ in, int C, int HW, uint4 *__restrict__ out) {
     tc::pdl_wait();
     tc::pdl_trigger();
-    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < P; i += gridDim.x * 256LL) {
-        const float *src = in + i / HW * C * HW + i % HW;
-        float v[8];
+    const float *src = in + (size_t) blockIdx.y * C * HW;
+    uint4 *dst = out + (size_t) blockIdx.y * HW;
+    const int p0 = blockIdx.x * 1024 + threadIdx.x;
+    float v[4][8];
 #pragma unroll
-        for (int c = 0; c < 8; c++) v[c] = c < C ? __ldg(src + c * HW) : 0.0f;
-        out[i] = bf16x8_of(v);
-    }
+    for (int k = 0; k < 4; k++)
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+            v[k][c] = c < C && p0 + 256 * k < HW ? __ldg(src + (size_t) c * HW + p0 + 256 * k) : 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (p0 + 256 * k < HW) dst[p0 + 256 * k] = bf16x8_of(v[k]);
 }
 
 // NCHW: 64 channels x 64 pixels per block through shared memory; planes read along the pixels (16-byte
@@ -697,7 +703,7 @@ cudaError_t prep_to_bf16_nhwc(const float *in, int nchw, int B, int C, int H, in
     } else if (!nchw) {
         cg_launch_pdl(nhwc_to_bf16_kernel, dim3(grid_for(P * (Cp / 8))), dim3(256), 0, st, in, C, Cp, P * (Cp / 8), vin && C == Cp, (uint4 *) out);
     } else if (C <= 8) {
-        cg_launch_pdl(nchw_few_to_bf16_kernel, dim3(grid_for(P)), dim3(256), 0, st, in, C, HW, P, (uint4 *) out);
+        cg_launch_pdl(nchw_few_to_bf16_kernel, dim3((unsigned) ((HW + 1023) / 1024), (unsigned) B), dim3(256), 0, st, in, C, (int) HW, (uint4 *) out);
     } else {
         const dim3 grid((unsigned) ((HW + 63) / 64), (unsigned) ((Cp + 63) / 64), (unsigned) B);
         cg_launch_pdl(nchw_tiled_to_bf16_kernel, grid, dim3(256), 0, st, in, C, (int) HW, Cp, vin && HW % 4 == 0, (uint4 *) out);

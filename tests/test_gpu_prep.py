@@ -97,3 +97,15 @@ def test_column_sums(cglib, b, h, w, c, kn):
     # the sums are of the FP32 accumulators, dx of their BF16 rounding: 2^-8 of each term
     ref = dx.double().sum((0, 1, 2))
     assert ((dbx.double() - ref).abs() <= (2.0 ** -8 + tol) * dx.double().abs().sum((0, 1, 2))).all()
+
+
+@pytest.mark.parametrize("b,c,h,w", [(3, 3, 33, 31), (2, 1, 32, 32), (2, 8, 41, 25), (5, 4, 64, 64), (1, 7, 129, 127)])
+def test_few_channel_cast_blocks_of_pixels(cglib, b, c, h, w):
+    """NCHW with c <= 8: 1024 pixels of an image per block (1023 to 16383 pixels), the values rounded as by torch."""
+    from convgemm_gb300 import tc
+    x = torch.randn(b, c, h, w, device="cuda")
+    out = torch.full((b, h, w, 8), float("nan"), dtype=torch.bfloat16, device="cuda")
+    tc.to_bf16_nhwc(cglib.NCHW, b, c, h, w, x, out)
+    want = torch.zeros_like(out)
+    want[..., :c] = x.permute(0, 2, 3, 1).to(torch.bfloat16)
+    assert torch.equal(out, want)
