@@ -178,6 +178,7 @@ struct FwdOp {
     // Single-tap NHWC: the row's reduction indices are its input pixel's channels, contiguous.
     __device__ const float *vrow(const Row &rw) const { return (~rw.a & tap_bits(0, 0)) == 0 ? rw.p : nullptr; }
     __device__ bool bin(const Col &cl, long long bd) const { return cl.valid && bd >= 0; }
+    __device__ const float *bbase() const { return w; }   // 16-byte aligned where B is read as vectors
     __host__ __device__ int segments() const { return (g.K + KC - 1) / KC; }
     __host__ __device__ long long rlen() const { return g.K; }
     __device__ void range(int m0, int z, int &rbeg, int &rend) const {
@@ -309,6 +310,7 @@ struct WgradOp {
     }
     __device__ const float *vrow(const Row &) const { return nullptr; }
     __device__ bool bin(const Col &cl, long long bd) const { return cl.valid && bd >= 0; }
+    __device__ const float *bbase() const { return dy; }   // 16-byte aligned where B is read as vectors
     __device__ bool by_rows() const { return false; }
     __device__ bool by_column() const { return false; }
     __device__ void finish(int, int, float) const {}
@@ -427,6 +429,7 @@ struct DgradOp {
     // Single-tap NHWC: the row's reduction indices are its output pixel's channels, contiguous.
     __device__ const float *vrow(const Row &rw) const { return (~rw.a & tap_bits(0, 0)) == 0 ? rw.p : nullptr; }
     __device__ bool bin(const Col &cl, long long bd) const { return cl.valid && bd >= 0; }
+    __device__ const float *bbase() const { return w; }   // 16-byte aligned where B is read as vectors
     __host__ __device__ int segments() const { return g.kh * g.kw * ((g.kn + KC - 1) / KC); }
     __host__ __device__ long long rlen() const { return (long long) g.kh * g.kw * g.kn; }
     __device__ void range(int m0, int z, int &rbeg, int &rend) const {
@@ -587,6 +590,7 @@ struct DgradPhaseOp {
         return in;
     }
     __device__ bool bin(const Col &cl, long long bd) const { return cl.valid && bd >= 0; }
+    __device__ const float *bbase() const { return w; }   // 16-byte aligned where B is read as vectors
     __device__ bool by_rows() const { return false; }
     __device__ bool by_column() const { return nchw && !ws; }
     __device__ void finish_m4(int, int, const float (&)[4]) const {}
@@ -679,7 +683,8 @@ __device__ __forceinline__ unsigned long long both(float v) {
     asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
     return d;
 }
-// Asynchronous copies into shared memory; `in` false: zeros, and the source is not read.
+// Asynchronous copies into shared memory; `in` false: zeros, and the source is not read. It has to lie on the copy's
+// own grid (4 or 16 bytes) all the same.
 __device__ __forceinline__ void copy4(uint32_t dst, const float *src, bool in) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(in ? 4 : 0) : "memory");
 }
@@ -822,8 +827,9 @@ __global__ void __launch_bounds__(T::NT, T::CTAS) fp32_igemm_kernel(const __grid
 #pragma unroll
             for (int i = 0; i < BI; i++) {
                 const int kk = (tid + NT * i) / QB;
-                const auto bd = rt[kk].bd;
-                copy16(b0 + 4 * (kk * T::BN + 4 * (tid % QB)), bcol[0].p + bd, op.bin(bcol[0], bd));
+                const auto bd = rt[kk].bd;   // -1 past the range
+                const bool in = op.bin(bcol[0], bd);
+                copy16(b0 + 4 * (kk * T::BN + 4 * (tid % QB)), in ? bcol[0].p + bd : op.bbase(), in);
             }
         } else {
 #pragma unroll

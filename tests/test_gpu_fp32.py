@@ -327,3 +327,42 @@ def test_tiles_and_tap_forms_follow_reference_order(cglib, oracle_lib, b, h, w, 
         assert errors(got, want)[0] <= FP32_TOL, layout
         again = dropin(cglib, "dgrad", layout, g, inp, inp["dx0"].copy(), to_dev=True)
         assert bitexact(got, again), layout
+
+
+@pytest.mark.parametrize("b,h,w,c,kn,k,stride,pad", [
+    (1, 11, 9, 3, 64, 7, 2, 3),     # 147 reduction indices: 3 of the last slice's 16
+    (2, 9, 7, 20, 36, 1, 1, 0),     # 20, one column group past the 64-wide tile's half
+    (1, 7, 5, 12, 68, 3, 1, 1),     # 108, one vector of columns past a tile; 35 pixels in the weight gradient
+])
+def test_masked_vector_copies_leave_the_neighbours_alone(cglib, oracle_lib, b, h, w, c, kn, k, stride, pad):
+    """The 16-byte copies of reduction indices and columns that do not exist take their zeros without an address of
+    their own: tensors on the 16-byte grid, NaN directly before and behind each, give the reference order's bits."""
+    g = C.geom(b, h, w, c, kn, k, k, vpad=pad, hpad=pad, vstr=stride, hstr=stride)
+    ho, wo = C.out_hw(g)
+    K = c * k * k
+    rng = np.random.default_rng(K + kn)
+    inp = {"x": rng.uniform(-1, 1, b * h * w * c).astype(np.float32),
+           "w": (rng.standard_normal(K * kn) * np.sqrt(2 / K)).astype(np.float32),
+           "dy": rng.uniform(-1, 1, b * ho * wo * kn).astype(np.float32),
+           "dx0": rng.uniform(-1, 1, b * h * w * c).astype(np.float32), "epi": {}}
+
+    def fenced(a):
+        buf = torch.full((a.size + 8,), float("nan"), device="cuda")
+        buf[4:4 + a.size] = torch.from_numpy(a)
+        return buf[4:4 + a.size]
+
+    geo = (kn, k, k, pad, pad, stride, stride, 1, 1)
+    for layout in (C.NHWC, C.NCHW):
+        nhwc = layout == C.NHWC
+        conv = cglib.sconvGemmNHWC if nhwc else cglib.sconvGemmNCHW
+        back = cglib.sconvGemmNHWC_back if nhwc else cglib.sconvGemmNCHW_back
+        dims = (b, h, w, c) if nhwc else (b, c, h, w)
+        x, wt, dy = (fenced(inp[n]) for n in ("x", "w", "dy"))
+        y, dw, dx = torch.empty(b * ho * wo * kn, device="cuda"), torch.empty(K * kn, device="cuda"), fenced(inp["dx0"])
+        conv("N", *dims, *geo, wt, x, y)
+        conv("T", *dims, *geo, dy, x, dw)
+        back(*dims, kn, k, k, stride, stride, pad, pad, 1, 1, wt, dy, dx)
+        torch.cuda.synchronize()
+        assert bitexact(y.cpu().numpy(), port(oracle_lib, "fwd", layout, g, inp, y.numel())), layout
+        assert bitexact(dw.cpu().numpy(), port(oracle_lib, "wgrad", layout, g, inp, dw.numel())), layout
+        assert errors(dx.cpu().numpy(), port(oracle_lib, "dgrad", layout, g, inp, None))[0] <= FP32_TOL, layout
