@@ -443,8 +443,9 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     p.bn = bn_override ? bn_override : (p.split > 1 ? 64 : form.bn);
     p.ntiles = (pl.Cout + p.bn - 1) / p.bn;
     // equal tiles of whole 16-column MMA widths; a single chunk of 64 columns is never shared by two tiles,
-    // and an accumulating call, which must not add a repeated column twice, keeps whole chunks
-    p.nn = round_up((pl.Cout + p.ntiles - 1) / p.ntiles, accum ? 64 : 16);
+    // and whole chunks are kept where a column must not be repeated: by an accumulating call, which would add it
+    // twice, and by a call in place of its mask, which would mask it by what it has just stored
+    p.nn = round_up((pl.Cout + p.ntiles - 1) / p.ntiles, accum || mask == out ? 64 : 16);
     if (p.nn < 64 && p.ntiles > 1) p.nn = 64;
     const int eb = mode == 1 ? 1 : 2;   // operand element bytes
     CUtensorMap wmap, omap;

@@ -348,7 +348,10 @@ convgemm_status_t convgemm_wgrad_bf16_plan(const convgemm_shape_t *shape, int *b
 
 /* Input gradient followed by the backward of the ReLU that produced the layer's
  * input x: dx = dgrad(dy, w) where x > 0, else 0 (x: the BF16 NHWC input of the
- * forward pass, [b][h][w][c]).  The masking is fused into the kernel's epilogue. */
+ * forward pass, [b][h][w][c]).  The masking is fused into the kernel's epilogue.
+ * In place: here and in the two forms below dx may be the mask itself (the same address) if
+ * some tap reaches every input pixel (a filter at least as wide and high as its strides, without
+ * dilation) or dx accumulates; otherwise dx must not overlap the mask. */
 convgemm_status_t convgemm_dgrad_bf16_relu(const convgemm_shape_t *shape, const void *dy, const void *wpacked, void *dx,
                                            const void *x, void *stream);
 

@@ -112,3 +112,31 @@ def test_group_of_every_ring_class(cglib):
     cg.check_device()
     for it, z in zip(items, want):
         assert nmax(it["y"], z) <= 6e-3
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+@pytest.mark.parametrize("b,c", [(3, 64), (3, 72), (40, 72), (3, 144), (40, 144), (3, 272)])
+def test_masked_input_gradient_in_place(cglib, b, c, stride):
+    """dx == relu_x, widths that are and are not whole 64-column chunks, one to several tiles per CTA: the bits of the
+    call with a separate dx, for the masked, the accumulating and the bias-gradient form."""
+    from convgemm_gb300 import tc
+    cg = cglib
+    s = cg.Shape.of(b, 15, 13, c, 64, 3, 3, 1, 1, stride, stride)
+    g = torch.Generator(device="cuda").manual_seed(c + stride)
+    x = torch.randn(b, 15, 13, c, device="cuda", generator=g).to(torch.bfloat16)
+    wt = torch.randn(c, 3, 3, 64, device="cuda", generator=g) * (2 / 576) ** 0.5
+    dy = torch.randn(b, s.ho, s.wo, 64, device="cuda", generator=g).to(torch.bfloat16)
+    wpd = torch.empty(tc.weights_size(s, tc.OPERAND_DGRAD) // 2, dtype=torch.bfloat16, device="cuda")
+    tc.pack_weights(cg.NHWC, s, tc.OPERAND_DGRAD, wt, wpd)
+    want, want_acc, db, db_in = torch.empty_like(x), x.clone(), torch.empty(c, device="cuda"), torch.empty(c, device="cuda")
+    tc.dgrad_bf16_bias_grad(s, dy, wpd, want, db, relu_x=x)
+    tc.dgrad_bf16_ex(s, dy, wpd, want_acc, relu_x=x, accumulate=True)
+    for _ in range(5):
+        dx, dx_sum, dx_acc = x.clone(), x.clone(), x.clone()
+        tc.dgrad_bf16_relu(s, dy, wpd, dx, dx)
+        tc.dgrad_bf16_bias_grad(s, dy, wpd, dx_sum, db_in, relu_x=dx_sum)
+        tc.dgrad_bf16_ex(s, dy, wpd, dx_acc, relu_x=dx_acc, accumulate=True)
+        assert torch.equal(dx, want) and torch.equal(dx_sum, want) and torch.equal(dx_acc, want_acc)
+        assert torch.equal(db_in, db)
+    torch.cuda.synchronize()
+    cg.check_device()
