@@ -217,3 +217,27 @@ def test_shipped_tuning_table_entries_parse():
             assert e["stages"] >= 2, k
         shape = [int(v) for v in k.split("|")[1].split("x")]
         assert len(shape) == 13 and min(shape[:7]) >= 1, k
+
+
+@pytest.mark.parametrize("private", ["there", "absent", "raising", "different"])
+def test_default_stream_is_torchs_current_one(cglib, monkeypatch, private):
+    """stream=None means torch's current stream, with or without the private lookups that make it cheap."""
+    import sys
+    import types
+    current = [0x1000]
+
+    def fail(*_):
+        raise RuntimeError("no such lookup")
+
+    c = {"there": {"_cuda_getCurrentRawStream": lambda d: current[0] + d, "_cuda_getDevice": lambda: 0}, "absent": {},
+         "raising": {"_cuda_getCurrentRawStream": fail, "_cuda_getDevice": lambda: 0},
+         "different": {"_cuda_getCurrentRawStream": lambda d: 7, "_cuda_getDevice": lambda: 0}}[private]
+    fake = types.SimpleNamespace(
+        cuda=types.SimpleNamespace(current_stream=lambda: types.SimpleNamespace(cuda_stream=current[0])),
+        _C=types.SimpleNamespace(**c))
+    monkeypatch.setitem(sys.modules, "torch", fake)
+    monkeypatch.setattr(cglib, "_raw_stream", None)
+    assert cglib._stream(None) == 0x1000
+    current[0] = 0x2000   # the program switches streams
+    assert cglib._stream(None) == 0x2000
+    assert cglib._stream(64) == 64
