@@ -955,7 +955,7 @@ extern "C" convgemm_status_t convgemm_wgrad_bf16_plan(const convgemm_shape_t *sh
     const WgPlan w = plan_wgrad(*shape);
     if (bn) *bn = w.bn;
     if (splits) *splits = w.splits;
-    if (max_splits) *max_splits = w.nchunks;
+    if (max_splits) *max_splits = (int) ((make_geom(cg_from_public(*shape)).P + 63) / 64);   // whatever the plan's own chunks
     return CONVGEMM_SUCCESS;
 }
 

@@ -241,3 +241,19 @@ def test_default_stream_is_torchs_current_one(cglib, monkeypatch, private):
     current[0] = 0x2000   # the program switches streams
     assert cglib._stream(None) == 0x2000
     assert cglib._stream(64) == 64
+
+
+def test_weight_gradient_plan_counts_64_pixel_chunks(cglib):
+    """max_splits of convgemm_wgrad_bf16_plan is the number of 64-pixel chunks, whatever the plan's own chunks hold."""
+    from convgemm_gb300 import tc
+    shapes = [(32, 28, 28, 512, 512, 3, 3, 1, 1), (1, 7, 7, 64, 64, 3, 3, 1, 1), (3, 23, 25, 24, 304, 1, 1),
+              (64, 224, 224, 3, 64, 7, 7, 3, 3, 2, 2), (4, 30, 30, 8, 48, 3, 3, 1, 1)]
+    try:
+        for args in shapes:
+            s = cglib.Shape.of(*args)
+            chunks = -(-s.b * s.ho * s.wo // 64)
+            for bn, aux in ((0, 0), (128, 2), (128, 2 | tc.WGRAD_WIDE_CHUNKS), (128, tc.WGRAD_PAIR)):
+                tc.tune_set(tc.TUNE_WGRAD, s, bn, aux)
+                assert tc.wgrad_bf16_plan(s)[2] == chunks, (args, bn, aux)
+    finally:
+        tc.tune_clear()
