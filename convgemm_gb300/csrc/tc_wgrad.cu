@@ -1137,49 +1137,66 @@ cudaError_t tc_wgrad_reduce(float *ws, float *dw, int splits, int xa, int Nx, in
 
 // ------------------------------------------------------------ bias gradient
 // db[co] = sum over the P pixels of dY[p][co] (dY BF16 [P][ld]), FP32, in a fixed
-// order: pass 1 sums `rows` consecutive pixels per (group, 64-channel chunk) with
-// four interleaved row streams combined in order; pass 2 adds the groups in order.
+// order: pass 1 sums `rows` consecutive pixels per (group, 64-channel chunk); pass 2
+// adds the groups in order.
 namespace {
 
-// Block = 64 channels of a group of pixels: thread (row r of 32, eight channels) adds the pixels r, r + 32,
-// ... in order from 16-byte loads, then the 32 rows are added in order. HBM-bound; one channel per
-// thread with 2-byte loads took 20 us for 25088 x 512 (1.3 TB/s). vec: dy 16-byte aligned (rows are:
-// ld % 8 == 0).
-__global__ void __launch_bounds__(256) bias_grad_pass1(const __nv_bfloat16 *__restrict__ dy, int P, int kn, int ld,
-                                                       int rows, int vec, float *__restrict__ part) {
+// Block = 64 channels of a group of pixels: thread (row r of 128, eight channels) adds the pixels r, r + 128,
+// ... in order from 16-byte loads, eight in flight; then the rows are added in order, eight and then sixteen. HBM-bound:
+// both passes, dy in HBM, 25088 x 512 11.4 us, 200704 x 64 13.8 (one load in flight in blocks of 32 rows, and four times
+// the groups: 13.1 and 21.8). vec: dy 16-byte aligned (rows are: ld % 8 == 0).
+constexpr int BG_ROWS = 128, BG_BATCH = 8;
+__global__ void __launch_bounds__(8 * BG_ROWS) bias_grad_pass1(const __nv_bfloat16 *__restrict__ dy, int P, int kn, int ld,
+                                                               int rows, int vec, float *__restrict__ part) {
     tc::pdl_wait();
     tc::pdl_trigger();
-    __shared__ float acc[32][65];
+    __shared__ float acc[BG_ROWS][65], sum[16][64];
     const int r = threadIdx.x >> 3, c8 = (threadIdx.x & 7) * 8, ch = blockIdx.x * 64 + c8;
     const int p0 = blockIdx.y * rows, p1 = min(P, p0 + rows);
     float s[8] = {};
     if (ch < ld) {
-        for (int p = p0 + r; p < p1; p += 32) {
-            const __nv_bfloat16 *src = dy + (size_t) p * ld + ch;
-            uint32_t w[4];
-            if (vec) {
-                const uint4 u = __ldg(reinterpret_cast<const uint4 *>(src));
-                w[0] = u.x, w[1] = u.y, w[2] = u.z, w[3] = u.w;
-            } else {
+        for (int p = p0 + r; p < p1; p += BG_ROWS * BG_BATCH) {
+            uint4 u[BG_BATCH];
 #pragma unroll
-                for (int j = 0; j < 4; j++)
-                    w[j] = __bfloat16_as_ushort(src[2 * j]) | (uint32_t) __bfloat16_as_ushort(src[2 * j + 1]) << 16;
+            for (int k = 0; k < BG_BATCH; k++) {
+                u[k] = make_uint4(0, 0, 0, 0);
+                if (p + BG_ROWS * k >= p1) continue;
+                const __nv_bfloat16 *src = dy + (size_t) (p + BG_ROWS * k) * ld + ch;
+                if (vec) {
+                    u[k] = __ldg(reinterpret_cast<const uint4 *>(src));
+                } else {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        w[j] = __bfloat16_as_ushort(src[2 * j]) | (uint32_t) __bfloat16_as_ushort(src[2 * j + 1]) << 16;
+                    u[k] = make_uint4(w[0], w[1], w[2], w[3]);
+                }
             }
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                s[2 * j] = __fadd_rn(s[2 * j], __uint_as_float(w[j] << 16));
-                s[2 * j + 1] = __fadd_rn(s[2 * j + 1], __uint_as_float(w[j] & 0xFFFF0000u));
+            for (int k = 0; k < BG_BATCH; k++) {   // zeros past the group's last pixel
+                const uint32_t w[4] = {u[k].x, u[k].y, u[k].z, u[k].w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    s[2 * j] = __fadd_rn(s[2 * j], __uint_as_float(w[j] << 16));
+                    s[2 * j + 1] = __fadd_rn(s[2 * j + 1], __uint_as_float(w[j] & 0xFFFF0000u));
+                }
             }
         }
     }
 #pragma unroll
     for (int j = 0; j < 8; j++) acc[r][c8 + j] = s[j];
     __syncthreads();
+    const int col = threadIdx.x & 63, part8 = threadIdx.x >> 6;
+    float v = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; j++) v = __fadd_rn(v, acc[8 * part8 + j][col]);
+    sum[part8][col] = v;
+    __syncthreads();
     const int co = blockIdx.x * 64 + threadIdx.x;
     if (threadIdx.x < 64 && co < kn) {
-        float v = 0.0f;
+        v = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 32; j++) v = __fadd_rn(v, acc[j][threadIdx.x]);
+        for (int j = 0; j < 16; j++) v = __fadd_rn(v, sum[j][threadIdx.x]);
         part[(size_t) blockIdx.y * kn + co] = v;
     }
 }
@@ -1205,7 +1222,7 @@ __global__ void bias_grad_pass2(const float *__restrict__ part, int groups, int 
 }  // namespace
 
 int tc_bias_grad_groups(long long P) {
-    long long g = (P + 255) / 256;   // about 256 pixels per group
+    long long g = (P + 1023) / 1024;   // about 1024 pixels per group: the callers' workspace has a plane for each
     return (int) (g > 256 ? 256 : (g < 1 ? 1 : g));
 }
 
@@ -1213,7 +1230,7 @@ cudaError_t tc_bias_grad(const void *dy, long long P, int kn, int ld, float *db,
     const int groups = tc_bias_grad_groups(P);
     const int rows = (int) ((P + groups - 1) / groups);
     dim3 g1((kn + 63) / 64, groups);
-    cg_launch_pdl(bias_grad_pass1, g1, dim3(256), 0, st, (const __nv_bfloat16 *) dy, (int) P, kn, ld, rows, ((uintptr_t) dy & 15) == 0, part);
+    cg_launch_pdl(bias_grad_pass1, g1, dim3(8 * BG_ROWS), 0, st, (const __nv_bfloat16 *) dy, (int) P, kn, ld, rows, ((uintptr_t) dy & 15) == 0, part);
     cg_launch_pdl(bias_grad_pass2, dim3((kn + 127) / 128), dim3(128), 0, st, part, groups, kn, db);
     return cudaGetLastError();
 }

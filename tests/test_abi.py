@@ -257,3 +257,12 @@ def test_weight_gradient_plan_counts_64_pixel_chunks(cglib):
                 assert tc.wgrad_bf16_plan(s)[2] == chunks, (args, bn, aux)
     finally:
         tc.tune_clear()
+
+
+def test_bias_gradient_workspace_is_one_plane_per_1024_pixels(cglib):
+    """The size that callers allocate: kn FP32 sums for each 1024 pixels, at most 256 planes."""
+    L = cglib.lib()
+    for b, hw, kn in ((1, 28, 64), (2, 28, 72), (32, 28, 512), (400, 28, 64)):
+        s = cglib.Shape.of(b, hw, hw, 64, kn, 3, 3, 1, 1)
+        planes = min(256, -(-b * hw * hw // 1024))
+        assert L.convgemm_bias_grad_bf16_workspace_size(ctypes.byref(s)) == 4 * kn * planes

@@ -109,3 +109,20 @@ def test_few_channel_cast_blocks_of_pixels(cglib, b, c, h, w):
     want = torch.zeros_like(out)
     want[..., :c] = x.permute(0, 2, 3, 1).to(torch.bfloat16)
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("b,h,w,kn", [(1, 1, 1, 8), (1, 1, 129, 72), (1, 1, 1025, 64), (1, 45, 46, 136), (2, 420, 317, 24)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_bias_gradient_groups(cglib, b, h, w, kn, off):
+    """One pixel, one more than a block's rows, one more than a group, ragged groups, groups of more than 1024 pixels. Of a
+    sum of n terms in groups of at most 1041 pixels, each term passes at most 9 + 8 + 16 + 256 FP32 additions."""
+    from convgemm_gb300 import tc
+    s = cglib.Shape.of(b, h, w, 64, kn, 1, 1)
+    g = torch.Generator(device="cuda").manual_seed(w)
+    dy = torch.randn(b, h, w, kn, device="cuda", generator=g).add_(0.25).to(torch.bfloat16)
+    db, db2 = (torch.full((kn,), float("nan"), device="cuda") for _ in range(2))
+    tc.bias_grad_bf16(s, offset(dy, off), db)
+    tc.bias_grad_bf16(s, offset(dy, off), db2)
+    ref, mag = dy.double().sum((0, 1, 2)), dy.double().abs().sum((0, 1, 2))
+    assert torch.equal(db, db2)
+    assert ((db.double() - ref).abs() <= 289 * 2.0 ** -24 * mag).all()
