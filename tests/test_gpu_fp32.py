@@ -366,3 +366,29 @@ def test_masked_vector_copies_leave_the_neighbours_alone(cglib, oracle_lib, b, h
         assert bitexact(y.cpu().numpy(), port(oracle_lib, "fwd", layout, g, inp, y.numel())), layout
         assert bitexact(dw.cpu().numpy(), port(oracle_lib, "wgrad", layout, g, inp, dw.numel())), layout
         assert errors(dx.cpu().numpy(), port(oracle_lib, "dgrad", layout, g, inp, None))[0] <= FP32_TOL, layout
+
+
+@pytest.mark.parametrize("b,h,w,c,kn,kh,kw,stride,pad", [
+    (1, 30, 9, 36, 72, 17, 1, 1, 3),      # 64 x 64 tiles, B as vectors, a second column tile of 8
+    (2, 22, 20, 4, 32, 16, 16, 2, 7),     # 128 x 32 tiles; more taps than the phase table of the strided input gradient
+    (1, 4, 60, 8, 20, 1, 31, 2, 15),      # strided input gradient by phases
+    (4, 40, 33, 5, 130, 18, 3, 1, 4),     # element loads of B (kn, c no multiples of 4), three column tiles
+])
+def test_filters_beyond_the_tap_masks(cglib, oracle_lib, b, h, w, c, kn, kh, kw, stride, pad):
+    """Filters of more than 15 rows or columns run in every tile shape, with and without vector loads of B: the reference
+    order's bits (forward, weight gradient), the input gradient within FP32 tolerance and reproducible."""
+    g = C.geom(b, h, w, c, kn, kh, kw, vpad=pad, hpad=pad, vstr=stride, hstr=stride)
+    ho, wo = C.out_hw(g)
+    K = c * kh * kw
+    rng = np.random.default_rng(K)
+    inp = {"x": rng.uniform(-1, 1, b * h * w * c).astype(np.float32),
+           "w": (rng.standard_normal(K * kn) * np.sqrt(2 / K)).astype(np.float32),
+           "dy": rng.uniform(-1, 1, b * ho * wo * kn).astype(np.float32),
+           "dx0": rng.uniform(-1, 1, b * h * w * c).astype(np.float32), "epi": {}}
+    for layout in (C.NHWC, C.NCHW):
+        for op, n in (("fwd", b * ho * wo * kn), ("wgrad", K * kn)):
+            got = dropin(cglib, op, layout, g, inp, np.zeros(n, np.float32), to_dev=True)
+            assert bitexact(got, port(oracle_lib, op, layout, g, inp, n)), (layout, op)
+        got = dropin(cglib, "dgrad", layout, g, inp, inp["dx0"].copy(), to_dev=True)
+        assert errors(got, port(oracle_lib, "dgrad", layout, g, inp, None))[0] <= FP32_TOL, layout
+        assert bitexact(got, dropin(cglib, "dgrad", layout, g, inp, inp["dx0"].copy(), to_dev=True)), layout
