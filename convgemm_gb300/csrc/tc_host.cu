@@ -377,6 +377,11 @@ TileForm tc_pick_form(const TcPlan &pl, int mode, bool im2col, bool mask, bool s
     return mask ? cheapest_form(FORMS_MASK, pl, 1, sms) : cheapest_form(FORMS_BF16, pl, 1, sms);
 }
 
+// CTAs in clusters of 2 or 4 that run at once, one per SM. Of 152 SMs, 36 clusters of four fit (what is left of each GPC
+// takes none): 37 tiles shared by four run in two rounds, 18.0 us where 36 take 12.7 and whole tiles 14.7 (1 x 8 x 8, 512 ->
+// 2368 and 2304, 3 x 3).
+inline int tc_cluster_ctas(int sms, int csize) { return csize == 4 ? sms - 8 : sms; }
+
 // CTAs per tile where the tiles leave most SMs idle: the K blocks of a 64-channel tile shared by a cluster of 2 or 4,
 // where the blocks fewer in each CTA's chain (0.153 us each) save more than the cluster costs (its launch and the
 // exchange: 2.0 us for two, 3.2 for four; 16 shapes with each forced). Worth it from 27 blocks on: 14 x 14, 256 -> 256
@@ -392,7 +397,7 @@ int tc_pick_split(const TcPlan &pl, int kdiv, int sms) {
     }
     int best = 1;
     float best_cost = (float) kmax * 0.153f;
-    for (int sp = 2; sp <= 4 && tiles * sp <= sms; sp *= 2) {
+    for (int sp = 2; sp <= 4 && tiles * sp <= tc_cluster_ctas(sms, sp); sp *= 2) {
         const float cost = (float) ((kmax + sp - 1) / sp) * 0.153f + (sp == 2 ? 2.0f : 3.2f);
         if (cost < best_cost) {
             best_cost = cost;
@@ -840,7 +845,8 @@ TcTune pick_wgrad(const cg_shape &s, const ConvGeom &g) {
                 if (sp > nch) continue;
                 const int cps = (nch + sp - 1) / sp, n = (nch + cps - 1) / cps;
                 if (!f.pair && n > 1 && n <= 8 && n != 2 && n != 4 && !(n == 8 && tiles * n <= 96)) continue;
-                float cost = f.launch + (float) ((tiles * n + sms - 1) / sms) * ((float) cps * f.chunk + f.tile);
+                const int at_once = tc_cluster_ctas(sms, f.pair ? 2 : n);
+                float cost = f.launch + (float) ((tiles * n + at_once - 1) / at_once) * ((float) cps * f.chunk + f.tile);
                 if (n > 1) cost += !f.pair && n <= 8 ? 2.4f : 5.6f + (float) n * (float) Nx * (float) s.kn * 4.0f / 4.5e6f;
                 if (best_cost < 0.0f || cost < best_cost) {
                     best_cost = cost;

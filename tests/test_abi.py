@@ -266,3 +266,23 @@ def test_bias_gradient_workspace_is_one_plane_per_1024_pixels(cglib):
         s = cglib.Shape.of(b, hw, hw, 64, kn, 3, 3, 1, 1)
         planes = min(256, -(-b * hw * hw // 1024))
         assert L.convgemm_bias_grad_bf16_workspace_size(ctypes.byref(s)) == 4 * kn * planes
+
+
+def test_clusters_of_four_are_chosen_where_they_run_at_once(cglib):
+    """A tile shared by a cluster of four only where all clusters are resident together: eight SMs (two of 152 / 4
+    clusters) find no place in one."""
+    import torch
+    from convgemm_gb300 import tc
+    sms = torch.cuda.get_device_properties(0).multi_processor_count if torch.cuda.is_available() else 148
+    seen = set()
+    for tiles in range(sms // 4 - 6, sms // 4 + 3):
+        s = cglib.Shape.of(1, 8, 8, 512, 64 * tiles, 3, 3, 1, 1)
+        cluster = tc.tune_describe(tc.TUNE_FWD, s)[3]
+        seen.add(cluster)
+        assert cluster <= 2 or tiles * cluster <= sms - 8, (tiles, cluster)
+    assert 4 in seen
+    tiles = sms // 4 // 2 * 2   # weight gradient, kn = 64: 4 taps of 32 * tiles channels are `tiles` tiles of 128 rows
+    s = cglib.Shape.of(16, 28, 28, 32 * tiles, 64, 2, 2)
+    assert tc.wgrad_bf16_plan(s)[1] != 4
+    s = cglib.Shape.of(16, 28, 28, 32 * (tiles - 2), 64, 2, 2)
+    assert tc.wgrad_bf16_plan(s)[1] == 4
