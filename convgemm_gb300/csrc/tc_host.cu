@@ -434,6 +434,8 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     p.mode = mode;
     TcPlan pi = pl;
     p.im2col = mode == 0 ? tc_use_im2col(pi, sms) : pl.Cin % 64 == 0 && tc_plan_im2col(pi);
+    if (!p.im2col && ((uintptr_t) in & 15))   // the gathers' 16-byte copies, as the maps of the other loads
+        return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "gathered operand not 16-byte aligned");
     if (mode != 0 && !p.im2col)
         return cg_set_error(CONVGEMM_ERROR_NOT_SUPPORTED,
                             "FP8 / 3xBF16 forms need channels a multiple of 64 (im2col-mode TMA)");
@@ -992,6 +994,8 @@ extern "C" convgemm_status_t convgemm_wgrad_bf16(convgemm_layout_t layout, const
         return tc_wgrad_slab_run(s, t.splits & 0xffff, t.bn, dy, x, (float *) workspace, dw,
                                  layout == CONVGEMM_NCHW, (cudaStream_t) stream);
     }
+    if (!wgrad_im2col_ok(s, g) && ((uintptr_t) x & 15))
+        return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "convgemm_wgrad_bf16: x not 16-byte aligned");
     CUtensorMap map;
     if (convgemm_status_t e = tc_make_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dy, g.P, w.kn8, 64, w.bk))
         return e;

@@ -89,6 +89,7 @@ extern "C" convgemm_status_t convgemm_wgrad_bf16_noalloc(convgemm_layout_t layou
                             "%s: kh*kw*c8*kn = %lld FP32 partials exceed the fixed scratch of %u (16 MiB); "
                             "use convgemm_wgrad_bf16 with a workspace",
                             fn, tile, CONVGEMM_NOALLOC_SCRATCH_FLOATS);
+    if ((uintptr_t) x & 15) return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "%s: x not 16-byte aligned", fn);
     NoallocDevice *d = nullptr;
     if (convgemm_status_t e = noalloc_setup(&d)) return e;
 

@@ -286,3 +286,20 @@ def test_clusters_of_four_are_chosen_where_they_run_at_once(cglib):
     assert tc.wgrad_bf16_plan(s)[1] != 4
     s = cglib.Shape.of(16, 28, 28, 32 * (tiles - 2), 64, 2, 2)
     assert tc.wgrad_bf16_plan(s)[1] == 4
+
+
+def test_gathered_operands_off_the_16_byte_grid_are_refused(cglib):
+    """Few or ragged channels are gathered by 16-byte copies: a tensor off their grid is an error before any launch, as it
+    is where TMA loads it (addresses only: nothing is read)."""
+    L = cglib.lib()
+    s = cglib.Shape.of(2, 10, 9, 8, 48, 3, 3, 1, 1)      # forward (y off the grid: not the small-channel kernel), weight gradient
+    d = cglib.Shape.of(2, 10, 9, 48, 8, 3, 3, 1, 1)      # input gradient: dy has 8 channels
+    base = 1 << 20
+    assert L.convgemm_fwd_bf16(ctypes.byref(s), base + 2, base, base + 2, None, None, 0, None) == 1
+    assert "16-byte" in cglib.last_error()[1]
+    assert L.convgemm_dgrad_bf16(ctypes.byref(d), base + 8, base, base, None) == 1 and "16-byte" in cglib.last_error()[1]
+    n = L.convgemm_wgrad_bf16_workspace_size(ctypes.byref(s))
+    assert L.convgemm_wgrad_bf16(0, ctypes.byref(s), base, base + 2, base, base, n, None) == 1
+    assert "16-byte" in cglib.last_error()[1]
+    assert L.convgemm_wgrad_bf16_noalloc(0, ctypes.byref(s), base, base + 2, base, None) == 1
+    assert "16-byte" in cglib.last_error()[1]
