@@ -377,10 +377,10 @@ TileForm tc_pick_form(const TcPlan &pl, int mode, bool im2col, bool mask, bool s
     return mask ? cheapest_form(FORMS_MASK, pl, 1, sms) : cheapest_form(FORMS_BF16, pl, 1, sms);
 }
 
-// CTAs in clusters of 2, 3 or 4 that run at once, one per SM. Of 152 SMs, 46 clusters of three and 36 of four fit (what is
-// left of each GPC takes none): 37 tiles shared by four run in two rounds, 18.0 us where 36 take 12.7 and whole tiles 14.7 (1 x 8 x 8, 512 ->
+// CTAs in clusters of 2 or 4 that run at once, one per SM. Of 152 SMs, 36 clusters of four fit (what is left of each GPC
+// takes none): 37 tiles shared by four run in two rounds, 18.0 us where 36 take 12.7 and whole tiles 14.7 (1 x 8 x 8, 512 ->
 // 2368 and 2304, 3 x 3).
-inline int tc_cluster_ctas(int sms, int csize) { return csize == 4 ? sms - 8 : (csize == 3 ? sms - 14 : sms); }
+inline int tc_cluster_ctas(int sms, int csize) { return csize == 4 ? sms - 8 : sms; }
 
 // CTAs per tile where the tiles leave most SMs idle: the K blocks of a 64-channel tile shared by a cluster of 2 or 4,
 // where the blocks fewer in each CTA's chain (0.153 us each) save more than the cluster costs (its launch and the
@@ -841,13 +841,15 @@ TcTune pick_wgrad(const cg_shape &s, const ConvGeom &g) {
             long long tiles = (M + 127) / 128;
             if (f.pair) tiles += tiles & 1;
             tiles *= (N + f.bn - 1) / f.bn;
-            // splits: 1, 2, 3, 4, 8, and those that fill one wave and half of one (three in one round, where clusters of four do not fit:
-            // 192 -> 64 5 x 5, 28 x 28, batch 64, 38 tiles: 37 us, 51 with two, 56 with four)
+            // splits: 1, 2, 4, 8, and those that fill one wave and half of one; three for the tile counts whose clusters of
+            // four would fill the SMs but do not all fit (192 -> 64 5 x 5, 28 x 28, batch 64, 38 tiles: 37 us, 51 with two,
+            // 56 with four)
             const int wave = (int) (sms / tiles > 0 ? sms / tiles : 1);
-            for (int sp : {1, 2, 3, 4, 8, wave, (wave + 1) / 2}) {
+            const int three = !f.pair && tiles * 4 > tc_cluster_ctas(sms, 4) && tiles * 4 <= sms ? 3 : 1;
+            for (int sp : {1, 2, three, 4, 8, wave, (wave + 1) / 2}) {
                 if (sp > nch) continue;
                 const int cps = (nch + sp - 1) / sp, n = (nch + cps - 1) / cps;
-                if (!f.pair && n > 2 && n != 4 && n <= 8 && !(n == 3 && tiles * n <= tc_cluster_ctas(sms, 3)) && !(n == 8 && tiles * n <= 96)) continue;
+                if (!f.pair && n > 1 && n <= 8 && n != 2 && n != 4 && n != three && !(n == 8 && tiles * n <= 96)) continue;
                 const int at_once = tc_cluster_ctas(sms, f.pair ? 2 : n);
                 float cost = f.launch + (float) ((tiles * n + at_once - 1) / at_once) * ((float) cps * f.chunk + f.tile);
                 if (n > 1) cost += !f.pair && n <= 8 ? 2.4f : 5.6f + (float) n * (float) Nx * (float) s.kn * 4.0f / 4.5e6f;
