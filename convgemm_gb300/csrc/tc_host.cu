@@ -788,6 +788,7 @@ namespace {
 struct WgPlan {
     int xa, bn, x2d, stem, mtiles, ntiles, splits, cps, nchunks, Nx, Cp, kn8;
     int csize, groups;   // grouped cluster reduction (groups > 1): splits = groups * csize
+    int im2col;          // X by TMA, else gathered by threads
     int slab;            // the slab kernel (tc_wgrad_slab.cu) with `splits` partials
     int kb1;             // im2col path: one chunk per ring stage (twice the stages)
     int iss2;            // im2col path, two chunks per stage: two MMA-issuing warps
@@ -797,11 +798,8 @@ struct WgPlan {
     size_t ws_bytes;
 };
 
-// Whether the weight gradient gathers X with im2col TMA (padding and far-edge offsets within the im2col map's
-// signed 8-bit corners). Channels that are no multiple of 64 are padded to one with zeros by the loads; up to
-// 8 channels, nearly all padding, the cp.async gathers run instead. 14 x 14, 200 -> 328 3 x 3, batch 32: 52 us
-// gathered, 26 padded; 23 x 25, 24 -> 304, batch 1: 20 and 7 us; 37 x 45, 72 -> 136 stride 2, batch 12: 20 and 13 us
-// (28 x 28, 72 -> 72, batch 64, where the second block of every tap is nearly empty: 37.5 and 39.6).
+// Whether TMA can load the weight gradient's X (padding and far-edge offsets within the im2col map's
+// signed 8-bit corners); up to 8 channels a 64-channel box would be nearly all padding.
 bool wgrad_im2col_ok(const cg_shape &s, const ConvGeom &g) {
     const int up_h = -s.vpad + (g.ho - 1) * s.vstride - (s.h - 1), up_w = -s.hpad + (g.wo - 1) * s.hstride - (s.w - 1);
     return s.c > 8 && s.vpad <= 128 && s.hpad <= 128 && up_h >= -128 && up_h <= 127 &&
@@ -826,9 +824,20 @@ struct WgForm {
 };
 constexpr WgForm WG_FORMS[] = {{64, 0, 0.257f, 4.34f, -0.7f}, {128, 0, 0.375f, 5.67f, -1.8f}, {128, 1, 0.347f, 4.89f, -0.7f}, {256, 1, 0.584f, 6.46f, -1.1f}};
 
-TcTune pick_wgrad(const cg_shape &s, const ConvGeom &g) {
+// Adding n splits up outside a cluster: the reduction kernel, the planes of partials.
+inline float wgrad_planes_cost(int n, int Nx, int kn) { return 5.6f + (float) n * (float) Nx * (float) kn * 4.0f / 4.5e6f; }
+
+struct WgPick {
+    WgForm f;
+    int xa, splits, cps;   // X on the 128-row side, pixel splits, chunks of each
+    long long rounds;      // CTAs that an SM runs one after the other
+    float reduce;
+    float cost(float chunk) const { return f.launch + (float) rounds * ((float) cps * chunk + f.tile) + reduce; }
+};
+
+WgPick pick_wgrad(const cg_shape &s, const ConvGeom &g) {
     const int sms = tc_num_sms(), Nx = s.kh * s.kw * round_up(s.c, 64), nch = (int) ((g.P + 127) / 128);
-    TcTune best{0, 0};
+    WgPick best{};
     float best_cost = -1.0f;
     for (const WgForm &f : WG_FORMS)
         // X on the 128-row side: always for narrow layers, else tried second (several taps: first, the
@@ -851,16 +860,59 @@ TcTune pick_wgrad(const cg_shape &s, const ConvGeom &g) {
                 const int cps = (nch + sp - 1) / sp, n = (nch + cps - 1) / cps;
                 if (!f.pair && n > 1 && n <= 8 && n != 2 && n != 4 && n != three && !(n == 8 && tiles * n <= 96)) continue;
                 const int at_once = tc_cluster_ctas(sms, f.pair ? 2 : n);
-                float cost = f.launch + (float) ((tiles * n + at_once - 1) / at_once) * ((float) cps * f.chunk + f.tile);
-                if (n > 1) cost += !f.pair && n <= 8 ? 2.4f : 5.6f + (float) n * (float) Nx * (float) s.kn * 4.0f / 4.5e6f;
+                const WgPick k{f, xa, n, cps, (tiles * n + at_once - 1) / at_once,
+                               n == 1 ? 0.0f : (!f.pair && n <= 8 ? 2.4f : wgrad_planes_cost(n, Nx, s.kn))};
+                const float cost = k.cost(f.chunk);
                 if (best_cost < 0.0f || cost < best_cost) {
                     best_cost = cost;
-                    best.bn = f.bn;
-                    best.splits = n | (f.pair ? CONVGEMM_WGRAD_PAIR : CONVGEMM_WGRAD_WIDE_CHUNKS) | (s.kn >= 128 && xa ? CONVGEMM_WGRAD_X_ON_A : 0);
+                    best = k;
                 }
             }
         }
     return best;
+}
+
+// Tiles and splits of the kernel that gathers X (and of table entries that name none): one wave of CTAs, no partial
+// second one, at least 512 pixels per split.
+int wgrad_wide_bn(int kn, int Nx) { return kn < 128 ? (kn <= 64 ? 64 : 128) : (Nx >= 256 ? 256 : (Nx > 64 ? 128 : 64)); }
+int wgrad_wave_splits(int tiles, int bn, long long P) {
+    const long long wave = tc_num_sms() * (bn == 256 ? 1 : 2) / tiles, most = (P + 511) / 512;
+    return (int) (wave < 1 ? 1 : (wave < most ? wave : most));
+}
+
+// Whether X whose channels are no multiple of 64 is loaded by TMA, each tap padded to whole 64-channel boxes, or gathered
+// by threads, which take packed channels. Boxes cost by what they hold: TMA_TAIL (microseconds per 128 pixels) by the
+// channels past the last multiple of 64, in eights; a whole box before it TMA_EVEN / TMA_ODD by whether rows start on
+// 32 bytes; dY's TMA_DY by its own channels. Fitted to 575 shapes run both ways (16 to 470 channels, 1 x 1 to 7 x 7, 49 to
+// 400k pixels; the two estimates err by 16 and 21%). Gathered up to 128 channels (two boxes per tap) where that is
+// estimated a tenth cheaper: 45 of the 575, 3% off all together; by TMA 36 of them ran slower than they had with gathers
+// for all such channels. 56 x 56, 24 -> 96 3 x 3, batch 64: 43 us gathered, 76 by TMA; 112 x 112, 40 -> 24 5 x 5, batch 16:
+// 113 and 219; 28 x 28, 40 -> 384, batch 64: 41 and 65; by TMA 14 x 14, 200 -> 328, batch 32: 52 and 26; 23 x 25, 24 -> 304,
+// batch 1: 20 and 7. The rule depends on the shape alone, not on the tuning table.
+constexpr float TMA_EVEN = 0.169f, TMA_ODD = 0.220f;
+constexpr float TMA_TAIL[8] = {0.0f, 0.303f, 0.152f, 0.420f, 0.173f, 0.467f, 0.216f, 0.250f};
+constexpr float TMA_DY[3] = {0.16f, 0.27f, 0.32f};   // rows on 32 bytes; else 8 or 56 channels past a multiple of 64; else
+constexpr float GATHER_CHUNK[3] = {1.15f, 1.07f, 0.76f}, GATHER_TILE[3] = {8.1f, 10.2f, 16.0f};   // 64, 128, 256 columns
+bool wgrad_by_tma(const cg_shape &s, const ConvGeom &g, const WgPick &k) {
+    const int c8 = round_up(s.c, 8), kn8 = round_up(s.kn, 8), tail = c8 % 64 / 8, ktail = kn8 % 64;
+    if (tail == 0 || c8 > 128) return true;
+    const float box = ((float) (c8 / 64) * (c8 % 16 ? TMA_ODD : TMA_EVEN) + TMA_TAIL[tail]) / (float) (c8 / 64 + 1);
+    const float dy_box = TMA_DY[kn8 % 16 == 0 ? 0 : (ktail == 8 || ktail == 56 ? 1 : 2)];
+    const int bn64 = k.f.bn / (k.f.pair && k.f.bn > 64 ? 128 : 64);   // 64-column boxes of the N side that a CTA loads
+    const float loads = (float) (k.xa ? 2 : bn64) * box + (float) (k.xa ? bn64 : 2) * dy_box;
+    const float by_tma = k.cost(loads > k.f.chunk ? loads : k.f.chunk);
+
+    const int Nx = s.kh * s.kw * c8, bn = wgrad_wide_bn(s.kn, Nx), q = bn == 64 ? 0 : (bn == 128 ? 1 : 2);
+    const int M = s.kn < 128 ? Nx : s.kn, N = s.kn < 128 ? s.kn : Nx, tiles = ((M + 127) / 128) * ((N + bn - 1) / bn);
+    const int nch = (int) ((g.P + 63) / 64), cps = (nch + wgrad_wave_splits(tiles, bn, g.P) - 1) / wgrad_wave_splits(tiles, bn, g.P);
+    const int n = (nch + cps - 1) / cps, sms = tc_num_sms(), per_sm = bn == 256 ? 1 : 2;
+    const long long ctas = (long long) tiles * n;
+    const float alone = per_sm == 2 && ctas <= sms ? 0.2f : 1.0f;   // a chunk's time with the SM to itself, against two CTAs'
+    const float slow = (ctas > 96 && (n == 3 || (n >= 5 && n <= 8)) ? 1.6f : 1.0f) *   // clusters that leave SMs without a place
+                       (q == 2 && s.kh * s.kw > 9 ? 1.2f : 1.0f);                      // more taps re-read more than L1 holds
+    const float gathered = slow * (float) ((ctas + sms * per_sm - 1) / (sms * per_sm)) * ((float) cps * GATHER_CHUNK[q] * alone + GATHER_TILE[q]) +
+                           (n == 1 ? 0.0f : (n <= 8 ? 5.3f : wgrad_planes_cost(n, Nx, s.kn)));
+    return gathered * 1.1f >= by_tma;
 }
 
 WgPlan plan_wgrad(const convgemm_shape_t &ps) {
@@ -868,9 +920,19 @@ WgPlan plan_wgrad(const convgemm_shape_t &ps) {
     const ConvGeom g = make_geom(s);
     TcTune t{0, 0};
     tc_tune_get(CONVGEMM_TUNE_WGRAD, ps, &t);
-    if (t.bn == 0 && t.splits == 0 && wgrad_im2col_ok(s, g) && !tc_stem_wgrad_applicable(s)) t = pick_wgrad(s, g);
+    const bool set = t.bn != 0 || t.splits != 0;
     WgPlan w;
-    const bool im2col = wgrad_im2col_ok(s, g);
+    w.stem = tc_stem_wgrad_applicable(s);
+    w.im2col = wgrad_im2col_ok(s, g);
+    if (w.im2col && !w.stem && (!set || round_up(s.c, 8) % 64)) {
+        const WgPick k = pick_wgrad(s, g);
+        w.im2col = wgrad_by_tma(s, g, k);
+        if (w.im2col && !set) {
+            t.bn = k.f.bn;
+            t.splits = k.splits | (k.f.pair ? CONVGEMM_WGRAD_PAIR : CONVGEMM_WGRAD_WIDE_CHUNKS) | (s.kn >= 128 && k.xa ? CONVGEMM_WGRAD_X_ON_A : 0);
+        }
+    }
+    const bool im2col = w.im2col != 0;
     w.Cp = round_up(s.c, im2col ? 64 : 8);
     w.kn8 = round_up(s.kn, 8);
     w.Nx = s.kh * s.kw * w.Cp;
@@ -895,7 +957,7 @@ WgPlan plan_wgrad(const convgemm_shape_t &ps) {
     } else {
         Mext = s.kn;
         Next = w.Nx;
-        w.bn = w.Nx >= 256 ? 256 : (w.Nx > 64 ? 128 : 64);
+        w.bn = wgrad_wide_bn(s.kn, w.Nx);
         if (t.bn) w.bn = t.bn;
     }
     if (w.pair) w.bn = t.bn == 128 ? 128 : 256;   // pair tiles: 256 x 128 or 256 x 256
@@ -903,16 +965,11 @@ WgPlan plan_wgrad(const convgemm_shape_t &ps) {
     if (w.pair) w.mtiles += w.mtiles & 1;   // the two CTAs of a pair take adjacent M tiles
     w.ntiles = (Next + w.bn - 1) / w.bn;
     w.nchunks = (int) ((g.P + w.bk - 1) / w.bk);
-    const int base = w.mtiles * w.ntiles;
-    const int per_sm = w.bn == 256 ? 1 : 2;
-    int splits = tc_num_sms() * per_sm / base;   // one wave: no partial second wave
-    const int max_splits = (int) ((g.P + 511) / 512);   // at least 512 pixels per split
-    if (splits > max_splits) splits = max_splits;
+    int splits = wgrad_wave_splits(w.mtiles * w.ntiles, w.bn, g.P);
     if (aux_splits) splits = aux_splits < w.nchunks ? aux_splits : w.nchunks;
     if (splits < 1) splits = 1;
     w.cps = (w.nchunks + splits - 1) / splits;
     w.splits = (w.nchunks + w.cps - 1) / w.cps;
-    w.stem = tc_stem_wgrad_applicable(s);
     if (w.stem) {   // the slab kernel: one partial per CTA, tile settings do not apply
         w.bn = 64;
         w.splits = tc_stem_wgrad_splits(s);
@@ -997,7 +1054,7 @@ extern "C" convgemm_status_t convgemm_wgrad_bf16(convgemm_layout_t layout, const
         return tc_wgrad_slab_run(s, t.splits & 0xffff, t.bn, dy, x, (float *) workspace, dw,
                                  layout == CONVGEMM_NCHW, (cudaStream_t) stream);
     }
-    if (!wgrad_im2col_ok(s, g) && ((uintptr_t) x & 15))
+    if (!w.im2col && ((uintptr_t) x & 15))
         return cg_set_error(CONVGEMM_ERROR_INVALID_VALUE, "convgemm_wgrad_bf16: x not 16-byte aligned");
     CUtensorMap map;
     if (convgemm_status_t e = tc_make_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dy, g.P, w.kn8, 64, w.bk))
@@ -1032,7 +1089,7 @@ extern "C" convgemm_status_t convgemm_wgrad_bf16(convgemm_layout_t layout, const
     memset(&xmap, 0, sizeof(xmap));
     {
         const int up_h = -s.vpad + (g.ho - 1) * s.vstride - (s.h - 1), up_w = -s.hpad + (g.wo - 1) * s.hstride - (s.w - 1);
-        p.im2col = wgrad_im2col_ok(s, g);
+        p.im2col = w.im2col;
         p.x2d = w.x2d;
         if (p.x2d) {
             if (convgemm_status_t e = tc_make_map_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, g.P, round_up(s.c, 8), 64, w.bk))
@@ -1124,12 +1181,10 @@ extern "C" convgemm_status_t convgemm_tune_describe(int op, const convgemm_shape
             *kernel = w.stem ? 2 : 1;
             return CONVGEMM_SUCCESS;
         }
-        const ConvGeom g = make_geom(s);
-        const int im2col = wgrad_im2col_ok(s, g);
-        *stages = tc_wgrad_stages(w.bn, im2col, w.kb1, w.wide, w.pair);
+        *stages = tc_wgrad_stages(w.bn, w.im2col, w.kb1, w.wide, w.pair);
         if (w.pair) *cluster = 2;
         else if (w.groups > 1) *cluster = w.csize;
-        else if (tc_wgrad_cluster_ok(w.bn, w.xa, im2col, w.splits, w.kb1, w.iss2, w.wide)) *cluster = w.splits;
+        else if (tc_wgrad_cluster_ok(w.bn, w.xa, w.im2col, w.splits, w.kb1, w.iss2, w.wide)) *cluster = w.splits;
         return CONVGEMM_SUCCESS;
     }
     if (op != CONVGEMM_TUNE_FWD && op != CONVGEMM_TUNE_DGRAD)

@@ -75,3 +75,39 @@ def test_ragged_channels_against_fp64(cglib, shape):
     torch.cuda.synchronize()
     cg.check_device()
     assert nmax(dwc, want) <= 1e-4
+
+
+@pytest.mark.parametrize("shape,gathered", [
+    ((64, 28, 28, 24, 384, 3, 1, 1, 1), True),     # dY on the 128-row side, 256 columns of taps and channels
+    ((16, 56, 56, 40, 24, 5, 2, 1, 1), True),      # X on the 128-row side, 64 columns
+    ((32, 28, 28, 104, 72, 3, 1, 2, 1), False),    # the same channels past 64, few pixels: by TMA
+    ((4, 57, 55, 120, 128, 3, 1, 1, 1), False),    # the last of two boxes nearly full
+], ids=str)
+def test_weight_gradient_of_many_pixels(cglib, shape, gathered):
+    """Both ways of loading ragged channels at the sizes where the estimates decide between them, with and without a tuning
+    entry (which names tiles and splits, not the way). FP32 accumulation over at most 57600 pixels of unit-variance
+    products: 1e-4 of the largest value."""
+    from convgemm_gb300 import tc
+    cg = cglib
+    b, h, w, c, kn, k, pad, stride, dil = shape
+    s = cg.Shape.of(b, h, w, c, kn, k, k, pad, pad, stride, stride, dil, dil)
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    x = torch.randn(b, h, w, c, device="cuda", generator=g).to(torch.bfloat16)
+    dy = torch.randn(b, s.ho, s.wo, kn, device="cuda", generator=g).to(torch.bfloat16)
+    want = torch.nn.grad.conv2d_weight(x.double().permute(0, 3, 1, 2), (kn, c, k, k), dy.double().permute(0, 3, 1, 2),
+                                       stride=stride, padding=pad, dilation=dil)
+    try:
+        for bn, aux in ((0, 0), (128, 12 | tc.WGRAD_STAGES1)):
+            tc.tune_set(tc.TUNE_WGRAD, s, bn, aux)
+            if bn:   # ring stages: a flag of the TMA form, which the gathering one has not
+                assert tc.tune_describe(tc.TUNE_WGRAD, s)[2] == (3 if gathered else 6)
+            n = tc.wgrad_bf16_workspace_size(s)
+            ws = torch.full((n // 4 + 4,), float("nan"), device="cuda")
+            dw, dw2 = torch.empty(c, k, k, kn, device="cuda"), torch.empty(kn, c, k, k, device="cuda")
+            tc.wgrad_bf16(cg.NHWC, s, dy, x, dw, ws)
+            tc.wgrad_bf16(cg.NCHW, s, dy, x, dw2, ws)
+            torch.cuda.synchronize()
+            cg.check_device()
+            assert nmax(dw, want.permute(1, 2, 3, 0)) <= 1e-4 and nmax(dw2, want) <= 1e-4
+    finally:
+        tc.tune_set(tc.TUNE_WGRAD, s, 0, 0)
