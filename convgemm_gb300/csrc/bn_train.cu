@@ -35,10 +35,11 @@ __device__ __forceinline__ double widen(float f) {   // (double) f
     if (e - 1u < 254u) return __hiloint2double((int) ((u & 0x80000000u) | ((u & 0x7FFFFFFFu) >> 3) + 0x38000000u), (int) (u << 29));
     return (u << 1) == 0 ? __hiloint2double((int) u, 0) : (double) f;   // zero; subnormal, infinite, NaN
 }
-// With one chunk of all groups (at most BN_ONE_PASS: a few batches of loads per thread) its sums are the
-// result, and the second kernel is not needed: OUT double writes them like the chunk sums, OUT float the
-// first plane's.
-constexpr int BN_ONE_PASS = 1024;
+// With one chunk of all groups its sums are the result, and the second kernel is not needed: OUT double writes them like
+// the chunk sums, OUT float the first plane's. That leaves one block per 8 channels, so it is for what one chunk holds, and
+// up to two chunks of few channels (500 groups of 64 channels with their forward 10.4 us, 10.3 in two passes, with the input
+// gradient 8.9 and 11.8; 1000 groups 30 and 17, 26 and 13; 375 groups of 256 channels 25 and 19, 22 and 13).
+inline bool one_pass(long long ngroups, int kn) { return ngroups <= BN_CHUNK || (ngroups <= 2 * BN_CHUNK && ngroups * kn <= 36864); }
 template <int PLANES, class OUT>
 __global__ void __launch_bounds__(256) bn_stats_pass1(const float *__restrict__ part, int ngroups, int chunk, int kn,
         OUT *__restrict__ out) {
@@ -234,13 +235,16 @@ cudaError_t cg_colsum_reduce(void *workspace, int ngroups, int kn, float *out, c
     const int nchunks = (ngroups + BN_CHUNK - 1) / BN_CHUNK;
     double *chunks = (double *) workspace;
     const float *part = (const float *) ((uint8_t *) workspace + (size_t) nchunks * 2 * kn * 8);
-    if (ngroups <= BN_ONE_PASS) {
-        cg_launch_pdl(bn_stats_pass1<1, float>, dim3((kn + 7) / 8), dim3(256), 0, st, part, ngroups, BN_ONE_PASS, kn, out);
+    if (one_pass(ngroups, kn)) {
+        // many blocks: launched plainly, as the first of two passes (125 groups of 512 channels: 16.6 us otherwise)
+        cg_launch_ex(kn > 256 ? CG_PDL_OFF : CG_PDL_THREAD, bn_stats_pass1<1, float>, dim3((kn + 7) / 8), dim3(256), 0, st, part, ngroups,
+                     ngroups, kn, out);
         return cudaGetLastError();
     }
     dim3 g1((kn + 7) / 8, nchunks);
-    // launched plainly: 56 x 56, 256-channel block 258 us a step, 268 with its blocks launched during the tail of the
-    // kernel that writes the groups
+    // launched plainly: with its blocks launched during the tail of the kernel that writes the groups, 9 of 10 input
+    // gradients took longer by 2 to 5 us (56 x 56, 256 -> 64 1 x 1, batch 64: 64 us, 66; 28 x 28, 128 -> 512: 20.6, 25), none
+    // less
     cg_launch_ex(CG_PDL_OFF, bn_stats_pass1<1, double>, g1, dim3(256), 0, st, part, ngroups, BN_CHUNK, kn, chunks);
     cg_launch_pdl(colsum_pass2_f32, dim3((kn + 31) / 32), dim3(256), 0, st, chunks, nchunks, kn, out);
     return cudaGetLastError();
@@ -285,8 +289,8 @@ extern "C" convgemm_status_t convgemm_fwd_bf16_stats(const convgemm_shape_t *sha
         e = tc_run(pl, s, x, wpacked, y, scale, shift, relu, st, 0, nullptr, nullptr, t.bn, t.splits, nullptr, part);
     }
     if (e) return e;
-    if (ng <= BN_ONE_PASS) {
-        cg_launch_pdl(bn_stats_pass1<2, double>, dim3((s.kn + 7) / 8), dim3(256), 0, st, part, ng, BN_ONE_PASS, s.kn, stats);
+    if (one_pass(ng, s.kn)) {
+        cg_launch_pdl(bn_stats_pass1<2, double>, dim3((s.kn + 7) / 8), dim3(256), 0, st, part, ng, ng, s.kn, stats);
     } else {
         dim3 g1((s.kn + 7) / 8, nchunks);
         cg_launch_pdl(bn_stats_pass1<2, double>, g1, dim3(256), 0, st, part, ng, BN_CHUNK, s.kn, chunks);
