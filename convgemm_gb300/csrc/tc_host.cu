@@ -340,28 +340,79 @@ TileForm cheapest_form(const TileForm (&forms)[N], const TcPlan &pl, int kdiv, i
     return best;
 }
 
+// CTAs in clusters of 2 or 4 that run at once, one per SM. Of 152 SMs, 36 clusters of four fit (what is left of each GPC
+// takes none): 37 tiles shared by four run in two rounds, 18.0 us where 36 take 12.7 and whole tiles 14.7 (1 x 8 x 8, 512 ->
+// 2368 and 2304, 3 x 3).
+inline int tc_cluster_ctas(int sms, int csize) { return csize == 4 ? sms - 8 : sms; }
+
+// CTAs per tile where the tiles leave most SMs idle: the K blocks of a 64-channel tile shared by a cluster of 2 or 4,
+// where the blocks fewer in each CTA's chain (0.153 us each) save more than the cluster costs (its launch and the
+// exchange: 2.0 us for two, 3.2 for four; 16 shapes with each forced). Worth it from 27 blocks on: 14 x 14, 256 -> 256
+// 3 x 3 at batch 1 (8 tiles of 36 blocks) 8.9 -> 7.7 us, 7 x 7, 512 -> 512 (72 blocks) 14.4 -> 9.0; 28 x 28,
+// 128 -> 128 (18 blocks) 6.1 alone, 6.5 shared by two. The rule depends on the plan (its batch, too) and the SM count, and leaves
+// out the slab kernel's shapes, so that every form of a layer adds its products in the same order. Every stride-phase class
+// has a block for each CTA: at most four classes split, whose tap counts differ by a factor of four at most, and a split
+// pays from 27 blocks on. *kblocks: the longest class's.
+constexpr float SPLIT_BLOCK = 0.153f;
+inline float split_cost(int sp) { return sp == 2 ? 2.0f : 3.2f; }
+int tc_pick_split(const TcPlan &pl, int kdiv, int sms, int *kblocks = nullptr) {
+    long long tiles = 0;
+    int kmax = 0;
+    for (int c = 0; c < pl.ncls; c++) {
+        tiles += (long long) pl.cls[c].mtiles * ((pl.Cout + 63) / 64);
+        kmax = pl.cls[c].ktiles / kdiv > kmax ? pl.cls[c].ktiles / kdiv : kmax;
+    }
+    if (kblocks) *kblocks = kmax;
+    int best = 1;
+    float best_cost = (float) kmax * SPLIT_BLOCK;
+    for (int sp = 2; sp <= 4 && tiles * sp <= tc_cluster_ctas(sms, sp); sp *= 2) {
+        const float cost = (float) ((kmax + sp - 1) / sp) * SPLIT_BLOCK + split_cost(sp);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = sp;
+        }
+    }
+    return best;
+}
+
 // Whether the BF16 kernel loads the gathered operand by im2col TMA (pl's classes then count whole 64-channel K
-// blocks per tap). With channels in blocks of 64 always. Else each tap's last block is padded with zeros and
-// rows straddle cache lines, which makes a block TAIL_COST times as expensive, but still cheaper than one gathered
-// by threads (0.6 us against 0.36 for 64-wide tiles): it pays unless the blocks are mostly padding.
-// 14 x 14, 328 -> 200 3 x 3, batch 32 (54 blocks for 47): 31.7 -> 23.1 us; 56 x 56, 104 -> 312 1 x 1, batch 24 (2 for 2):
-// 44 -> 20 us; 28 x 28, 72 -> 72 3 x 3, batch 64 (18 for 11): 26.4 gathered, 42.8 by TMA. The rule depends on the
-// plan alone, so that every form of a layer adds its products in the same order.
-constexpr float TAIL_COST = 2.0f;
+// blocks per tap). With channels in blocks of 64 always. Else each tap's last block is padded with zeros, and a box costs
+// by what it holds, in blocks of whole aligned rows: TAIL_BOX by the channels past the last multiple of 64, in eights, a
+// whole box before it EVEN_BOX / ODD_BOX by whether rows start on 32 bytes (fitted to 330 shapes, forward and input gradient
+// run both ways; the two estimates err by 18 and 11%), at most FEW_BOX where half of the SMs have no tile. Blocks gathered by threads cost more (0.6 us against 0.18 for 64-wide
+// tiles) but hold packed channels. The cheaper estimate is 0.6% off the better way on average (2.0% with twice an
+// aligned block for every box). 14 x 14, 328 -> 200 3 x 3, batch 32: 31.7 us gathered, 23.1 by TMA; 56 x 56, 104 -> 312
+// 1 x 1, batch 24: 44 and 20; 107 x 107, 32 -> 64 7 x 7, batch 17: 149 and 104; 100 x 100, 40 -> 96 3 x 3, batch 40: 90 and 150;
+// 35 x 35, 72 -> 32 3 x 3, batch 43: 22 and 31. The rule depends on the plan (its batch, too) and the SM count, so that every
+// form of a layer adds its products in the same order.
+constexpr float EVEN_BOX = 1.1f, ODD_BOX = 1.6f, FEW_BOX = 1.5f;
+constexpr float TAIL_BOX[8] = {0.0f, 2.85f, 1.25f, 3.35f, 1.35f, 3.7f, 1.75f, 2.15f};
 bool tc_use_im2col(TcPlan &pl, int sms) {
     TcPlan pi = pl;
     if (!tc_plan_im2col(pi)) return false;
     if (pl.Cin % 64) {
-        TileForm forms[sizeof(FORMS_BF16) / sizeof(FORMS_BF16[0])];
-        for (size_t i = 0; i < sizeof(forms) / sizeof(forms[0]); i++) {
-            forms[i] = FORMS_BF16[i];
-            forms[i].block *= TAIL_COST;
+        const int whole = pl.Cin / 64;
+        float box = ((float) whole * (pl.Cin % 16 ? ODD_BOX : EVEN_BOX) + TAIL_BOX[pl.Cin % 64 / 8]) / (float) (whole + 1);
+        long long tiles = 0;
+        for (int c = 0; c < pi.ncls; c++) {
+            pi.cls[c].ktiles = pi.cls[c].ntaps * (whole + 1);
+            tiles += (long long) pi.cls[c].mtiles * ((pl.Cout + 63) / 64);
         }
-        for (int c = 0; c < pi.ncls; c++) pi.cls[c].ktiles = pi.cls[c].ntaps * ((pl.Cin + 63) / 64);
+        if (2 * tiles <= sms && box > FEW_BOX) box = FEW_BOX;
         float by_tma, gathered;
-        cheapest_form(forms, pi, 1, sms, &by_tma);
+        int kblocks;
+        if (const int sp = tc_pick_split(pi, 1, sms, &kblocks); sp > 1) {
+            by_tma = 4.1f + (float) ((kblocks + sp - 1) / sp) * SPLIT_BLOCK * box + split_cost(sp);
+        } else {
+            TileForm forms[sizeof(FORMS_BF16) / sizeof(FORMS_BF16[0])];
+            for (size_t i = 0; i < sizeof(forms) / sizeof(forms[0]); i++) {
+                forms[i] = FORMS_BF16[i];
+                forms[i].block *= box;
+            }
+            cheapest_form(forms, pi, 1, sms, &by_tma);
+        }
         cheapest_form(FORMS_GATHER, pl, 1, sms, &gathered);
-        if (gathered < by_tma) return false;
+        if (gathered * 0.95f < by_tma) return false;
     }
     pl = pi;
     return true;
@@ -375,36 +426,6 @@ TileForm tc_pick_form(const TcPlan &pl, int mode, bool im2col, bool mask, bool s
     if (!im2col) return cheapest_form(FORMS_GATHER, pl, 1, sms);
     if (sums) return cheapest_form(FORMS_SUMS, pl, 1, sms);
     return mask ? cheapest_form(FORMS_MASK, pl, 1, sms) : cheapest_form(FORMS_BF16, pl, 1, sms);
-}
-
-// CTAs in clusters of 2 or 4 that run at once, one per SM. Of 152 SMs, 36 clusters of four fit (what is left of each GPC
-// takes none): 37 tiles shared by four run in two rounds, 18.0 us where 36 take 12.7 and whole tiles 14.7 (1 x 8 x 8, 512 ->
-// 2368 and 2304, 3 x 3).
-inline int tc_cluster_ctas(int sms, int csize) { return csize == 4 ? sms - 8 : sms; }
-
-// CTAs per tile where the tiles leave most SMs idle: the K blocks of a 64-channel tile shared by a cluster of 2 or 4,
-// where the blocks fewer in each CTA's chain (0.153 us each) save more than the cluster costs (its launch and the
-// exchange: 2.0 us for two, 3.2 for four; 16 shapes with each forced). Worth it from 27 blocks on: 14 x 14, 256 -> 256
-// 3 x 3 at batch 1 (8 tiles of 36 blocks) 8.9 -> 7.7 us, 7 x 7, 512 -> 512 (72 blocks) 14.4 -> 9.0; 28 x 28,
-// 128 -> 128 (18 blocks) 6.1 alone, 6.5 shared by two. The rule depends on the plan alone, and leaves out the slab
-// kernel's shapes, so that every form of a layer adds its products in the same order.
-int tc_pick_split(const TcPlan &pl, int kdiv, int sms) {
-    long long tiles = 0;
-    int kmax = 0;
-    for (int c = 0; c < pl.ncls; c++) {
-        tiles += (long long) pl.cls[c].mtiles * ((pl.Cout + 63) / 64);
-        kmax = pl.cls[c].ktiles / kdiv > kmax ? pl.cls[c].ktiles / kdiv : kmax;
-    }
-    int best = 1;
-    float best_cost = (float) kmax * 0.153f;
-    for (int sp = 2; sp <= 4 && tiles * sp <= tc_cluster_ctas(sms, sp); sp *= 2) {
-        const float cost = (float) ((kmax + sp - 1) / sp) * 0.153f + (sp == 2 ? 2.0f : 3.2f);
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = sp;
-        }
-    }
-    return best;
 }
 
 // Epilogue warps of tc_conv_kernel: eight where asked for (`by_k`: where every class has at most 8 K

@@ -111,3 +111,20 @@ def test_weight_gradient_of_many_pixels(cglib, shape, gathered):
             assert nmax(dw, want.permute(1, 2, 3, 0)) <= 1e-4 and nmax(dw2, want) <= 1e-4
     finally:
         tc.tune_set(tc.TUNE_WGRAD, s, 0, 0)
+
+
+@pytest.mark.parametrize("shape,gathered", [
+    ((16, 28, 28, 40, 96, 3, 1, 1, 1), (True, False)),     # boxes off the 32-byte grid with a short tail
+    ((16, 28, 28, 96, 40, 3, 1, 1, 1), (False, True)),     # the same for the input gradient's dY
+    ((8, 31, 29, 32, 64, 7, 3, 1, 1), (False, False)),     # aligned rows, half a box
+    ((4, 9, 7, 72, 32, 3, 1, 1, 1), (False, False)),       # few tiles
+], ids=str)
+def test_both_ways_of_loading_ragged_channels(cglib, shape, gathered):
+    """Sizes on either side of the estimates' line, every form of each operation (equal bits) against FP64."""
+    from convgemm_gb300 import tc
+    b, h, w, c, kn, k, pad, stride, dil = shape
+    s = cglib.Shape.of(b, h, w, c, kn, k, k, pad, pad, stride, stride, dil, dil)
+    for op, by_threads in zip((tc.TUNE_FWD, tc.TUNE_DGRAD), gathered):
+        _, bn, stages, _ = tc.tune_describe(op, s)
+        assert (stages == {64: 8, 128: 6, 256: 4}[bn]) == by_threads, (op, bn, stages)   # the gathering ring
+    test_ragged_channels_against_fp64(cglib, shape)
