@@ -49,10 +49,11 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 
-// What the epilogue does beside scale, shift and ReLU (BF16 forms): nothing (or adding into the output);
-// masking by the activation of a ReLU; column sums of its output, masked when a mask is given (input
-// gradient); column sums of its output and of the squares (forward).
-constexpr int EXTRA_NONE = 0, EXTRA_MASK = 1, EXTRA_SUMS = 2, EXTRA_STATS = 3;
+// What the epilogue does beside scale, shift and ReLU (BF16 forms): nothing; masking by the activation of a ReLU (and
+// adding the output's old values first); column sums of its output, masked when a mask is given (input
+// gradient); column sums of its output and of the squares (forward); adding the output's old values, which take
+// the mask's place in the parameters and its way into the staging buffer.
+constexpr int EXTRA_NONE = 0, EXTRA_MASK = 1, EXTRA_SUMS = 2, EXTRA_STATS = 3, EXTRA_ACC = 4;
 
 // Operand forms of the kernel.
 constexpr int MODE_BF16 = 0;  // BF16 x BF16, kind::f16
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
             tc::mbar_init(&full[s], IM2C ? 1 : 128 + 1);
             tc::mbar_init(&empty[s], 1);
         }
-        if (EXTRA == EXTRA_MASK || EXTRA == EXTRA_SUMS)
+        if (EXTRA == EXTRA_MASK || EXTRA == EXTRA_SUMS || EXTRA == EXTRA_ACC)
             for (int b = 0; b < 2 * EW; b++) tc::mbar_init(&mask_full[b], 1);
         for (int b = 0; b < C::ACC_BUFS; b++) {
             tc::mbar_init(&acc_full[b], 1);
@@ -395,7 +396,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
         const bool affine = p.scale || p.shift;
         uint32_t lt = ALT ? half : 0;     // local tile count
         int ebuf = 0;                     // staging buffer toggle
-        // The mask's 32 x 64 values of an item, loaded into the staging buffer the item will use: by TMA, or where
+        // The mask's (or the output's old) 32 x 64 values of an item, loaded into the staging buffer the item will use: by TMA, or where
         // the rows are scattered (stride-phase classes) by 16-byte pieces, eight lanes to a row. (Read by
         // their own lanes, one cache line of another row per lane, the masked form of 56 x 56, 256 -> 64 took 60 us,
         // 27 without a mask.) The load is issued during the item before, off the critical path. Returns whether
@@ -432,7 +433,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
             tc::cp_async_commit();
             return false;
         };
-        constexpr bool MASKED = EXTRA == EXTRA_MASK || EXTRA == EXTRA_SUMS;
+        constexpr bool MASKED = EXTRA == EXTRA_MASK || EXTRA == EXTRA_SUMS || EXTRA == EXTRA_ACC;
         bool by_tma = false;       // this item's mask arrives at mbar[ebuf]
         uint32_t mphase = 0;       // bit b: parity of the next arrival at mbar[b]
         if constexpr (MASKED) {
@@ -571,8 +572,21 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                             }
                     }
                 }
-                if ((EXTRA == EXTRA_NONE || EXTRA == EXTRA_MASK) && !C::OUTF32 && p.accum) {
-                    // accumulate (the reference's dx += ...): add the output's current values in FP32
+                if constexpr (EXTRA == EXTRA_ACC) {
+                    // accumulate (the reference's dx += ...): add the output's old values in FP32
+                    uint8_t *stg = stg_warp + ebuf * C::EPI_BYTES;
+#pragma unroll
+                    for (int q = 0; q < NQ; q++)
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const uint32_t old = *reinterpret_cast<const uint32_t *>(tc::frag_word(stg, q, k));
+                            uint32_t *w = &v[k >> 1][4 * q + 2 * (k & 1)];
+                            w[0] = __float_as_uint(__uint_as_float(w[0]) + __uint_as_float(old << 16));
+                            w[1] = __float_as_uint(__uint_as_float(w[1]) + __uint_as_float(old & 0xFFFF0000u));
+                        }
+                }
+                if (EXTRA == EXTRA_MASK && p.accum == TC_ACCUM_DIRECT) {
+                    // the same beside a mask, which has the staging buffer: from the output
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
                         const int mr = m0 + ew * 32 + (lane >> 2) + 8 * k;
@@ -866,6 +880,7 @@ cudaError_t tc_conv_launch(const TcConvParams &p, const CUtensorMap &wmap, const
     }
     if (p.stats && p.sums_only) return launch_extra<EXTRA_SUMS>(p, wmap, omap, amaps, grid, st);
     if (p.stats) return launch_extra<EXTRA_STATS>(p, wmap, omap, amaps, grid, st);
+    if (p.accum == TC_ACCUM_STAGED) return launch_extra<EXTRA_ACC>(p, wmap, omap, amaps, grid, st);
     if (p.mask) return launch_extra<EXTRA_MASK>(p, wmap, omap, amaps, grid, st);
     if (p.im2col && p.ew == 8) {
         // eight epilogue warps (short-K tiles): one K block per stage, two staging buffers

@@ -29,6 +29,7 @@ struct TcClass {
     FastDiv dwg, dhg;
 };
 
+enum { TC_ACCUM_DIRECT = 1, TC_ACCUM_STAGED = 2 };   // the old values read by the epilogue's lanes; loaded as a mask is
 struct TcConvParams {
     const __nv_bfloat16 *in;   // gathered activation, NHWC [B][Hin][Win][Cin]
     __nv_bfloat16 *out;        // NHWC [B][Hout][Wout][Cout]
@@ -37,7 +38,8 @@ struct TcConvParams {
     int relu;
     const __nv_bfloat16 *mask;   // BF16 tensor laid out like out, or NULL: out = 0 where mask <= 0 (ReLU backward)
     int accum;                 // BF16 input gradient: out = out + acc (the old value read first; FP32 sum, one
-                               // rounding), then the mask; 0: out overwritten
+                               // rounding), then the mask: TC_ACCUM_STAGED with `mask` = out, beside a mask
+                               // TC_ACCUM_DIRECT; 0: out overwritten
     float *stats;              // BF16 forward: per 32-row group g of the output pixels, [g][0][Cout] the sum
                                // and [g][1][Cout] the sum of squares of z = acc * scale + shift; or NULL
     int sums_only;             // stats without the squares (bias gradient)

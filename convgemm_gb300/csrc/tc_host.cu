@@ -465,7 +465,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     bool f8w = mode == 1 && p.im2col && pl.Cin % 128 == 0 && pl.Ktot % 128 == 0;
     for (int c = 0; f8w && c < pi.ncls; c++)
         if (pi.cls[c].kbeg % 128 || pi.cls[c].ktiles % 2) f8w = false;
-    const TileForm form = tc_pick_form(pi, f8w ? 3 : mode, p.im2col, mask != nullptr, stats != nullptr, sms);
+    const TileForm form = tc_pick_form(pi, f8w ? 3 : mode, p.im2col, mask || accum, stats != nullptr, sms);
     // (a tuning entry names a form without the split, for all of the operation's forms)
     p.split = p.im2col && !bn_override && !aux_override && !(mode == 0 && tc_slab_applicable(pl)) ? tc_pick_split(pi, f8w ? 2 : 1, sms) : 1;
     p.bn = bn_override ? bn_override : (p.split > 1 ? 64 : form.bn);
@@ -498,8 +498,9 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     p.scale = scale;
     p.shift = shift;
     p.relu = relu;
-    p.mask = (const __nv_bfloat16 *) mask;
-    p.accum = accum;
+    p.mask = (const __nv_bfloat16 *) (mask ? mask : (accum ? out : nullptr));
+    p.accum = !accum ? 0 : (mask ? TC_ACCUM_DIRECT : TC_ACCUM_STAGED);
+    const bool staged = mask || accum;   // a tensor laid out as the output goes through the epilogue's staging buffers
     p.stats = stats;
     p.sums_only = sums_only;
     p.B = s.b;
@@ -517,8 +518,8 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     memcpy(p.tox, pl.tox, sizeof(p.tox));
     TcMaps amaps;
     memset(&amaps, 0, sizeof(amaps));
-    if (mask && p.epi_tma)
-        if (convgemm_status_t e = tc_make_map_2d(&amaps.mask, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, mask,
+    if (staged && p.epi_tma)
+        if (convgemm_status_t e = tc_make_map_2d(&amaps.mask, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.mask,
                                                  (long long) s.b * pl.Hout * pl.Wout, pl.Cout, 64, 32))
             return e;
     if (f8w) {
@@ -561,7 +562,7 @@ convgemm_status_t tc_run(const TcPlan &pl, const cg_shape &s, const void *in, co
     p.mt = (by_form ? form.mt == 2 : (aux_override & 3) == 2) && mode == 0 && p.im2col ? 2 : 1;
     p.ew = tc_epilogue_warps(pi, by_form ? form.ew == 8 : (aux_override & 4) != 0, !by_form && (aux_override & 7) == 0, p.bn,
                              p.mt, mode == 0 && p.im2col);
-    if (stats || mask) {   // the forms with column sums or a mask: one M tile, eight epilogue warps beside TMA loads
+    if (stats || staged) {   // the forms with column sums or a staged tensor: one M tile, eight epilogue warps beside TMA loads
         p.mt = 1;
         p.ew = p.im2col ? 8 : 4;
     }
