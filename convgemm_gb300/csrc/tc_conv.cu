@@ -122,6 +122,19 @@ __device__ __forceinline__ uint32_t positive_mask(uint32_t v) {
     return __hgt2_mask(*reinterpret_cast<const __nv_bfloat162 *>(&v), __floats2bfloat162_rn(0.0f, 0.0f));
 }
 
+// A chunk of the warp's 32 accumulator rows: 64 columns as fragments (tc_epi.cuh), 32 columns of an FP32 output as a row per
+// lane, whose 16-byte staging stores meet no bank twice as often as need be (8-byte ones of fragments do: 3xBF16, 54 x 54,
+// 64 -> 256 1 x 1, batch 15: 15.1 us as fragments, 14.2 so).
+template <bool F32>
+__device__ __forceinline__ void acc_load(uint32_t ta, uint32_t (&v)[F32 ? 1 : 2][32]) {
+    if constexpr (F32) {
+        tc::tmem_ld_32x32b_x32(ta, v[0]);
+        tc::tmem_ld_wait();
+    } else {
+        tc::frag_load<8>(ta, v);
+    }
+}
+
 template <int N>
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(N) : "memory"); }
 
@@ -476,11 +489,11 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                     if (krank > 0) {
                         const uint32_t dst = tc::mapa_shared(tc::smem_u32(base) + (uint32_t) ((krank - 1) * C::NCH * 4 * C::CW * 128), 0);
                         for (int ch = 0; ch < nch && ok; ch++) {
-                            uint32_t v[2][C::CW / 2];
-                            tc::frag_load<C::CW / 8>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * BN + chunk_col(ch)), v);
+                            uint32_t v[C::CW / 32][32];
+                            acc_load<C::OUTF32>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * BN + chunk_col(ch)), v);
 #pragma unroll
                             for (int j = 0; j < C::CW / 4; j++) {
-                                const uint32_t *w = &v[j / (C::CW / 8)][j % (C::CW / 8) * 4];
+                                const uint32_t *w = &v[j / 8][j % 8 * 4];
                                 asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
                                                  dst + (uint32_t) (((ch * 4 + ew) * (C::CW / 4) + j) * 512 + lane * 16)),
                                              "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
@@ -512,15 +525,15 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                            ((((size_t) b * p.Hout + oy) * p.Wout + ox) * p.Cout) * (C::OUTF32 ? 4 : 2);
                 }
                 constexpr int NQ = C::CW / 8;
-                uint32_t v[2][4 * NQ];
-                tc::frag_load<NQ>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) ((buf * MT + mt) * BN + c0), v);
+                uint32_t v[C::CW / 32][32];
+                acc_load<C::OUTF32>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) ((buf * MT + mt) * BN + c0), v);
                 if constexpr (SPLITS) {
                     for (int o = 0; o < split - 1; o++) {   // the other shares of the sum, in order
                         const uint8_t *src = base + o * C::NCH * 4 * C::CW * 128 + (item * 4 + ew) * (C::CW / 4) * 512 + lane * 16;
 #pragma unroll
                         for (int j = 0; j < C::CW / 4; j++) {
                             const uint4 u = *reinterpret_cast<const uint4 *>(src + j * 512);
-                            uint32_t *w = &v[j / (C::CW / 8)][j % (C::CW / 8) * 4];
+                            uint32_t *w = &v[j / 8][j % 8 * 4];
                             w[0] = __float_as_uint(__uint_as_float(w[0]) + __uint_as_float(u.x));
                             w[1] = __float_as_uint(__uint_as_float(w[1]) + __uint_as_float(u.y));
                             w[2] = __float_as_uint(__uint_as_float(w[2]) + __uint_as_float(u.z));
@@ -610,7 +623,23 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                         }
                     }
                 }
-                tc::frag_affine<NQ>(v, affine, scp + c0, shp + c0);
+                if constexpr (C::OUTF32) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        float4 sc = make_float4(1.0f, 1.0f, 1.0f, 1.0f), sh = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        if (affine) {
+                            sc = *reinterpret_cast<const float4 *>(scp + c0 + 4 * j);
+                            sh = *reinterpret_cast<const float4 *>(shp + c0 + 4 * j);
+                        }
+                        uint32_t *w = &v[0][4 * j];
+                        w[0] = __float_as_uint(fmaf(__uint_as_float(w[0]), sc.x, sh.x));
+                        w[1] = __float_as_uint(fmaf(__uint_as_float(w[1]), sc.y, sh.y));
+                        w[2] = __float_as_uint(fmaf(__uint_as_float(w[2]), sc.z, sh.z));
+                        w[3] = __float_as_uint(fmaf(__uint_as_float(w[3]), sc.w, sh.w));
+                    }
+                } else {
+                    tc::frag_affine<NQ>(v, affine, scp + c0, shp + c0);
+                }
                 if constexpr (EXTRA == EXTRA_SUMS || EXTRA == EXTRA_STATS) {
                     // Column sums of this item's 64 columns over the warp's 32 rows, to group
                     // gbase + m0 / 32 + ew of the class (the classes' groups are concatenated): the forward's
@@ -631,10 +660,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                 uint32_t pk[32];   // 128 bytes of each of the 32 rows, over the warp
                 if constexpr (C::OUTF32) {
 #pragma unroll
-                    for (int h = 0; h < 2; h++)
-#pragma unroll
-                        for (int j = 0; j < 16; j++)
-                            pk[16 * h + j] = p.relu ? __float_as_uint(fmaxf(__uint_as_float(v[h][j]), 0.0f)) : v[h][j];
+                    for (int j = 0; j < 32; j++) pk[j] = p.relu ? __float_as_uint(fmaxf(__uint_as_float(v[0][j]), 0.0f)) : v[0][j];
                 } else {
                     tc::frag_pack(v, p.relu != 0, pk);
                 }
@@ -651,16 +677,10 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                 // to the staging buffer of the warp
                 auto stage = [&](uint8_t *stg) {
                     if constexpr (C::OUTF32) {
-                        const int fr = lane >> 2, fc = lane & 3;
 #pragma unroll
-                        for (int h = 0; h < 2; h++)
-#pragma unroll
-                            for (int q = 0; q < 4; q++)
-#pragma unroll
-                                for (int k = 0; k < 2; k++)
-                                    *reinterpret_cast<uint2 *>(stg + (16 * h + 8 * k + fr) * 128 +
-                                                               (((2 * q + (fc >> 1)) ^ fr) << 4) + (fc & 1) * 8) =
-                                        make_uint2(pk[16 * h + 4 * q + 2 * k], pk[16 * h + 4 * q + 2 * k + 1]);
+                        for (int q = 0; q < 8; q++)
+                            *reinterpret_cast<uint4 *>(stg + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+                                make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
                     } else {
                         tc::frag_stage(stg, pk);
                     }
