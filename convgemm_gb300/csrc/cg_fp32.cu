@@ -182,6 +182,7 @@ struct FwdOp {
     __device__ bool bin(const Col &cl, long long bd) const { return cl.valid && bd >= 0; }
     __device__ const float *bbase() const { return w; }   // 16-byte aligned where B is read as vectors
     __host__ __device__ int segments() const { return (g.K + KC - 1) / KC; }
+    bool phased() const { return false; }
     __host__ __device__ long long rlen() const { return g.K; }
     __device__ void range(int m0, int z, int &rbeg, int &rend) const {
         if (ws) {
@@ -228,6 +229,17 @@ struct FwdOp {
 #pragma unroll
         for (int i = 0; i < 4; i++) v[i] = fwd_epilogue(s[i], n, e);
         store4(y + ((size_t) bb * g.kn + n) * g.ho * g.wo + (size_t) ox * g.wo + oy, v, true, 4);
+    }
+    // NCHW y: channel 0 of row m, or NULL past the last
+    __device__ float *out_row(int m) const {
+        if (m >= (int) g.P) return nullptr;
+        uint32_t q, oy, ox, bb;
+        dwo.divmod(m, q, oy);
+        dho.divmod(q, bb, ox);
+        return y + ((size_t) bb * g.kn * g.ho + ox) * g.wo + oy;
+    }
+    __device__ void put(float *row, int n, float s) const {
+        if (row && n < g.kn) row[(size_t) n * g.ho * g.wo] = fwd_epilogue(s, n, e);
     }
     __device__ void finish(int m, int n, float s) const {
         if (m >= (int) g.P || n >= g.kn) return;
@@ -315,8 +327,9 @@ struct WgradOp {
     __device__ const float *bbase() const { return dy; }   // 16-byte aligned where B is read as vectors
     __device__ bool by_rows() const { return false; }
     __device__ bool by_column() const { return false; }
-    __device__ void finish(int, int, float) const {}
     __device__ void finish_m4(int, int, const float (&)[4]) const {}
+    __device__ float *out_row(int) const { return nullptr; }
+    __device__ void put(float *, int, float) const {}
     __device__ void range(int m0, int z, int &rbeg, int &rend) const {
         rbeg = z * KC;
         rend = min((long long) (z + 1) * KC, g.P);
@@ -433,6 +446,7 @@ struct DgradOp {
     __device__ bool bin(const Col &cl, long long bd) const { return cl.valid && bd >= 0; }
     __device__ const float *bbase() const { return w; }   // 16-byte aligned where B is read as vectors
     __host__ __device__ int segments() const { return g.kh * g.kw * ((g.kn + KC - 1) / KC); }
+    bool phased() const { return false; }
     __host__ __device__ long long rlen() const { return (long long) g.kh * g.kw * g.kn; }
     __device__ void range(int m0, int z, int &rbeg, int &rend) const {
         if (ws) {
@@ -479,6 +493,10 @@ struct DgradOp {
     __device__ bool by_column() const { return nchw && !ws; }
     __device__ void finish_m4(int m, int n, const float (&s)[4]) const {
         if (m < M() && n < g.c) store4(dx + out_index(m, n), s, true, 4);
+    }
+    __device__ float *out_row(int m) const { return m < M() ? dx + out_index(m, 0) : nullptr; }   // NCHW dx: channel 0
+    __device__ void put(float *row, int n, float s) const {
+        if (row && n < g.c) row[(size_t) n * g.h * g.w] = s;
     }
     __device__ void finish(int m, int n, float s) const {
         if (m >= M() || n >= g.c) return;
@@ -596,6 +614,7 @@ struct DgradPhaseOp {
     __device__ bool by_rows() const { return false; }
     __device__ bool by_column() const { return nchw && !ws; }
     __device__ void finish_m4(int, int, const float (&)[4]) const {}
+    bool phased() const { return true; }
     __host__ __device__ int segments() const {
         int nt = 0;
         for (int i = 0; i < ncls; i++) nt = ph[i].ntaps > nt ? ph[i].ntaps : nt;
@@ -647,9 +666,18 @@ struct DgradPhaseOp {
     }
     __device__ void finish_n4(int m, int n, const float (&s)[4]) const {
         size_t o;
-        if (ov && out_index(m, n, o)) return store4(dx + o, s, true, g.c - n);
+        if (!out_index(m, n, o)) return;
+        if (!nchw) return store4(dx + o, s, ov, g.c - n);
 #pragma unroll
-        for (int j = 0; j < 4; j++) finish(m, n + j, s[j]);
+        for (int j = 0; j < 4; j++)
+            if (n + j < g.c) dx[o + (size_t) j * g.h * g.w] = s[j];
+    }
+    __device__ float *out_row(int m) const {   // NCHW dx: channel 0
+        size_t o;
+        return out_index(m, 0, o) ? dx + o : nullptr;
+    }
+    __device__ void put(float *row, int n, float s) const {
+        if (row && n < g.c) row[(size_t) n * g.h * g.w] = s;
     }
     __device__ void finish(int m, int n, float s) const {
         size_t o;
@@ -768,9 +796,15 @@ __global__ void __launch_bounds__(T::NT, T::CTAS) fp32_igemm_kernel(const __grid
     // over it are rolled: unrolled 128 times they are tens of KB of code run once per CTA, and
     // short reductions then spend their time on instruction fetches.
     bool none = !op.starts();
-    if (!none) {
+    if (!none) {   // eight loads in flight (one by one, a 64 x 64 tile's 32 per thread took 9 us)
 #pragma unroll 1
-        for (int e = 0; e < TM * TN; e++) Ssm[e * NT + tid] = op.s_init(mrow(e / TN), ncol(e % TN));
+        for (int e = 0; e < TM * TN; e += 8) {
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[j] = op.s_init(mrow((e + j) / TN), ncol((e + j) % TN));
+#pragma unroll
+            for (int j = 0; j < 8; j++) Ssm[(e + j) * NT + tid] = v[j];
+        }
     }
 
     unsigned long long acc[TM / 2][TN];   // rows 2i, 2i + 1
@@ -936,14 +970,17 @@ __global__ void __launch_bounds__(T::NT, T::CTAS) fp32_igemm_kernel(const __grid
     }
     if (op.by_column()) {   // NCHW rows that are no vectors: a warp stores 32 rows of one column at a time
         __syncthreads();
+        constexpr int RG = T::BM / GM, CG = T::BN / GN;   // rows / columns between a thread's runs of four
 #pragma unroll 1
-        for (int e = warp; e < T::BN * (T::BM / 32); e += NW) {
-            const int col = e % T::BN, row = e / T::BN * 32 + lane;
-            constexpr int RG = T::BM / GM, CG = T::BN / GN;   // rows / columns between a thread's runs of four
-            const int i = row / RG * 4 + row % 4, ry = row % RG / 4;
-            const int j = col / CG * 4 + col % 4, cx = col % CG / 4;
-            const int t = (ry / 4 * WX + cx / 8) * 32 + ry % 4 * 8 + cx % 8;   // the thread that holds it
-            op.finish(m0 + row, n0 + col, Ssm[(i * TN + j) * NT + t]);
+        for (int rb = 0; rb < T::BM / 32; rb++) {
+            const int row = 32 * rb + lane, i = row / RG * 4 + row % 4, ry = row % RG / 4;
+            float *out = op.out_row(m0 + row);   // the row's place is found once
+#pragma unroll 4
+            for (int col = warp; col < T::BN; col += NW) {
+                const int j = col / CG * 4 + col % 4, cx = col % CG / 4;
+                const int t = (ry / 4 * WX + cx / 8) * 32 + ry % 4 * 8 + cx % 8;   // the thread that holds it
+                op.put(out, n0 + col, Ssm[(i * TN + j) * NT + t]);
+            }
         }
         return;
     }
@@ -1188,33 +1225,38 @@ inline int num_sms() {
 
 // Estimated seconds of n tiles of R reduction steps each on the SM with the most of them. It runs `ctas`
 // at a time; fewer resident CTAs leave latencies uncovered, so they run at eff[resident - 1] of the FMA
-// rate. A tile's start and end cost about `ov` more steps. Fitted to 20 shapes (0.01 to 118 GFLOP) with
-// each tile forced: 128 x 128 takes 2.10 ms where 64 x 64 takes 2.35 (56 x 56, 256 -> 256, 3 x 3, batch 32),
+// rate. A tile's start and end cost about `ov` more steps and `begin` microseconds a round, adding a segment to the
+// running sum `fold`, the rows of a stride-phase tile, whose places are found one by one, `phase`. Fitted to 20 shapes
+// (0.01 to 118 GFLOP) with each tile forced, the microseconds to 170 forwards and input gradients with every tile, fused
+// and split (0.5% off the best on average; 5% for input gradients without them: 14 x 14, 34 -> 22 5 x 5 stride 2, batch 34
+// fused 55 us, split 41). 128 x 128 takes 2.10 ms where 64 x 64 takes 2.35 (56 x 56, 256 -> 256, 3 x 3, batch 32),
 // 223 us against 206 (56 x 56, 64 -> 256, 1 x 1, batch 64), 68 us against 28 (28 x 28, 64 -> 64, batch 8).
 struct TileCost {
     int bm, bn, ctas, ov;
     double eff[4];
+    double begin, fold, phase;
 };
-constexpr TileCost TILE_COST[3] = {{128, 128, 2, 60, {0.58, 0.74, 0, 0}},
-                                   {64, 64, 4, 40, {0.38, 0.50, 0.57, 0.63}},
-                                   {128, 32, 4, 40, {0.38, 0.50, 0.57, 0.63}}};
+constexpr TileCost TILE_COST[3] = {{128, 128, 2, 60, {0.58, 0.74, 0, 0}, 1.9, 1.7, 37.0},
+                                   {64, 64, 4, 40, {0.38, 0.50, 0.57, 0.63}, 0.7, 1.0, 12.0},
+                                   {128, 32, 4, 40, {0.38, 0.50, 0.57, 0.63}, 2.3, 1.1, 13.0}};
 
-inline double tile_time(const TileCost &c, long long n, double R, int sms) {
+inline double tile_time(const TileCost &c, long long n, double R, int segs, bool phased, int sms) {
     const long long per_sm = (n + sms - 1) / sms;
     const double one = (double) c.bm * c.bn * (R + c.ov) / 128 / 2.0e9;   // 128 multiply-adds per cycle, about 2 GHz
     const long long rounds = per_sm / c.ctas, rest = per_sm % c.ctas;
-    return one * (rounds * c.ctas / c.eff[c.ctas - 1] + (rest ? rest / c.eff[rest - 1] : 0.0));
+    const double adds = (double) (rounds + (rest > 0)) * (c.begin + c.fold * (segs - 1) + (phased ? c.phase : 0.0)) * 1e-6;
+    return one * (rounds * c.ctas / c.eff[c.ctas - 1] + (rest ? rest / c.eff[rest - 1] : 0.0)) + adds;
 }
 
-// The cheapest tile shape for M x N outputs, nz chains of R steps per output; *cost: its estimate.
-inline int pick_tile(long long M, long long N, int nz, double R, double *cost) {
+// The cheapest tile shape for M x N outputs, nz chains of `segs` segments, R steps in all, per output; *cost: its estimate.
+inline int pick_tile(long long M, long long N, int nz, double R, int segs, bool phased, double *cost) {
     const int sms = num_sms();
     int best = TILE_SQUARE;
     *cost = -1.0;
     for (int t = 0; t < 3; t++) {
         if (t == TILE_NARROW && N > 32) continue;
         const TileCost &c = TILE_COST[t];
-        const double v = tile_time(c, ((M + c.bm - 1) / c.bm) * ((N + c.bn - 1) / c.bn) * nz, R, sms);
+        const double v = tile_time(c, ((M + c.bm - 1) / c.bm) * ((N + c.bn - 1) / c.bn) * nz, R, segs, phased, sms);
         if (*cost < 0 || v < *cost) {
             *cost = v;
             best = t;
@@ -1233,11 +1275,11 @@ cudaError_t launch_split_or_fused(Op op, int M, int N, bool vec, bool bv, cudaSt
     const double R = (double) op.rlen();
     op.ws = nullptr;
     double cost;
-    int tile = pick_tile(M, N, 1, R, &cost);
+    int tile = pick_tile(M, N, 1, R, nz, op.phased(), &cost);
     if (nz > 1) {
         double c2;
-        const int t2 = pick_tile(M, N, nz, R / nz, &c2);
-        if (c2 + 2.0 * (double) bytes / 4e12 + 3e-6 < cost) {
+        const int t2 = pick_tile(M, N, nz, R / nz, 1, false, &c2);
+        if (c2 + 2.0 * (double) bytes / 4e12 + 10e-6 < cost) {
             op.ws = scratch(SLOT_SPLIT, bytes, st);
             if (op.ws) tile = t2;
         }
@@ -1332,7 +1374,7 @@ cudaError_t wgrad_call(int nchw, const cg_shape &s, const float *dy, const float
     }
     const int nblocks = (int) ((op.g.P + KC - 1) / KC);
     double cost;
-    const int tile = pick_tile(op.g.K, s.kn, nblocks, KC, &cost);
+    const int tile = pick_tile(op.g.K, s.kn, nblocks, KC, 1, false, &cost);
     op.ov = s.kn % 4 == 0 && aligned16(ws);
     cudaError_t e = launch(op, tile, nblocks, false, op.yl == 0 && s.kn % 4 == 0 && aligned16(op.dy), st);
     if (e != cudaSuccess) return e;
