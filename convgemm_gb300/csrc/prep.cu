@@ -421,11 +421,12 @@ __device__ __forceinline__ void batched(int n, Load load, Store store) {
 
 // Grouped preparation: every block finds its job by binary search over the jobs'
 // first blocks and runs that job's body for its block (256 threads).
-// What bounds it is the chain of latencies within a block: the jobs' first blocks (b0, njobs ints) are staged in
-// shared memory, so the search costs one global round trip, then the job itself (read field by field from memory,
-// each access a round trip again behind the stores), and the weights are read several at a time. Both operands of
-// 512 x 512 x 3 x 3 (NCHW) 20.6 us, 14.4 so; of a 1024 / 256-channel bottleneck 12.9, 10.4.
-__global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restrict__ jobs, const int *__restrict__ b0,
+// What bounds it is the chain of latencies within a block, and how many blocks share an SM: the jobs' first blocks (b0,
+// njobs ints) are staged in shared memory, so the search costs one global round trip, then the job itself (read field by
+// field from memory, each access a round trip again behind the stores), and the weights are read several at a time, as far
+// as six blocks per SM leave registers (40: with eight loads in flight and 64 registers, four blocks, 262 x 688 x 7 x 7 NHWC
+// took 118 us a round of six, 94 so). Both operands of 512 x 512 x 3 x 3 (NCHW): 47 us value by value, 11.5 staged.
+__global__ void __launch_bounds__(256, 6) prep_group_kernel(const PrepJob *__restrict__ jobs, const int *__restrict__ b0,
                                                          int njobs) {
     __shared__ float tile[64][65];
     extern __shared__ int s_b0[];
@@ -524,8 +525,14 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
             float *buf = &tile[0][0];
             const float *src = J.w + ((size_t) co * J.C + ci0) * khw;
             const int have = max(0, min(n, J.C - ci0)) * khw;
+            if (khw == 1) {   // one tap: the row as it is
+                bf16 *row = (bf16 *) J.out + (size_t) co * Kpad + ci0;
+                const int end = ci0 + n == Cp ? Kpad - ci0 : n;   // with the K padding after the last chunk
+                batched<2, float>(end, [&](int i) { return i < have ? __ldg(src + i) : 0.0f; }, [&](int i, float v) { row[i] = __float2bfloat16_rn(v); });
+                return;
+            }
             if (((uintptr_t) src & 15) == 0 && (have & 3) == 0 && (n * khw & 3) == 0)
-                batched<4, float4>(
+                batched<2, float4>(
                     n * khw >> 2,
                     [&](int i) { return 4 * i < have ? __ldg(reinterpret_cast<const float4 *>(src) + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f); },
                     [&](int i, float4 v) {
@@ -535,7 +542,7 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
                         buf[4 * i + 3] = v.w;
                     });
             else
-                batched<8, float>(n * khw, [&](int i) { return i < have ? __ldg(src + i) : 0.0f; }, [&](int i, float v) { buf[i] = v; });
+                batched<4, float>(n * khw, [&](int i) { return i < have ? __ldg(src + i) : 0.0f; }, [&](int i, float v) { buf[i] = v; });
             __syncthreads();
             // a warp per tap, two channels per store where the chunk's ends are even
             bf16 *row = (bf16 *) J.out + (size_t) co * Kpad;
@@ -563,22 +570,20 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
             return;
         }
         case PREP_DGRAD_NCHW: {
-            // NCHW-API weights [co][ci][tap]: block = (4 input channels, one class, a run of output
-            // channels): the run's 4 x taps values, contiguous per output channel, staged through shared
-            // memory (odd pitch) and written along co
+            // NCHW-API weights [co][ci][tap], one class: block = (4 input channels, a run of output channels): the run's
+            // 4 x taps values, contiguous per output channel, staged through shared memory (odd pitch) and written along co
             const int khw = J.kh * J.kw, Ktot = J.info.Ktot, knp = J.knp, C = J.C;
             const int run = prep_nchw_run(khw), nrun = (knp + run - 1) / run;
-            const int c = (lb / nrun) % J.info.ncls, ci0 = lb / nrun / J.info.ncls * 4, co0 = lb % nrun * run;
-            const int beg = J.info.kbeg[c], end = c + 1 < J.info.ncls ? J.info.kbeg[c + 1] : Ktot;
-            const int nt = J.info.ntaps[c], nci = min(4, C - ci0), w4 = nci * khw, pitch = (4 * khw) | 1, nco = min(run, knp - co0);
+            const int ci0 = lb / nrun * 4, co0 = lb % nrun * run;
+            const int nci = min(4, C - ci0), w4 = nci * khw, pitch = (4 * khw) | 1, nco = min(run, knp - co0);
             float *buf = &tile[0][0];
-            if (t < nt) taps[t] = J.info.kx[J.info.tap0[c] + t] * J.kw + J.info.ky[J.info.tap0[c] + t];
+            if (t < khw) taps[t] = J.info.kx[t] * J.kw + J.info.ky[t];
             const float *src = J.w + ((size_t) co0 * C + ci0) * khw;
             const int have = J.kn - co0;
             const int lane = t & 31;
             if ((w4 & 3) == 0 && (C * khw & 3) == 0 && ((uintptr_t) src & 15) == 0) {
                 // 16 lanes per output channel
-#pragma unroll 4
+#pragma unroll 2
                 for (int co = t >> 4; co < nco; co += 16)
                     for (int k = 4 * (t & 15); k < w4; k += 64) {
                         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -590,16 +595,25 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
                         d[3] = v.w;
                     }
             } else {
-                for (int co = t >> 5; co < nco; co += 8)
-                    for (int k = lane; k < w4; k += 32)
-                        buf[co * pitch + k] = co < have ? __ldg(src + (size_t) co * C * khw + k) : 0.0f;
+                // several output channels' values at a time
+                const uint32_t inv = 0xFFFFFFFFu / (uint32_t) w4 + 1;   // i / w4 (w4 > 1) by its high product: i * w4 is far below 2^32
+                batched<4, float>(
+                    nco * w4,
+                    [&](int i) {
+                        const int co = (int) __umulhi((uint32_t) i, inv);
+                        return co < have ? __ldg(src + (size_t) co * C * khw + (i - co * w4)) : 0.0f;
+                    },
+                    [&](int i, float v) {
+                        const int co = (int) __umulhi((uint32_t) i, inv);
+                        buf[co * pitch + (i - co * w4)] = v;
+                    });
             }
             __syncthreads();
             // a warp per (input channel, tap), two output channels per store
-            bf16 *dst = (bf16 *) J.out + (size_t) ci0 * Ktot + beg + co0;
+            bf16 *dst = (bf16 *) J.out + (size_t) ci0 * Ktot + co0;
             const bool two = (nco & 1) == 0 && (knp & 1) == 0 && (Ktot & 1) == 0 && ((uintptr_t) dst & 3) == 0;
-            for (int q = t >> 5; q < nci * nt; q += 8) {
-                const int r = q / nt, g = q - r * nt;
+            for (int q = t >> 5; q < nci * khw; q += 8) {
+                const int r = q / khw, g = q - r * khw;
                 const float *v = buf + r * khw + taps[g];
                 bf16 *o = dst + (size_t) r * Ktot + g * knp;
                 if (two)
@@ -608,9 +622,9 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
                 else
                     for (int co = lane; co < nco; co += 32) o[co] = __float2bfloat16_rn(v[co * pitch]);
             }
-            if (co0 == 0)   // the K padding after the class's taps
+            if (co0 == 0)   // the K padding after the taps
                 for (int r = 0; r < nci; r++)
-                    for (int k = nt * knp + t; k < end - beg; k += 256) dst[(size_t) r * Ktot + k] = __float2bfloat16_rn(0.0f);
+                    for (int k = khw * knp + t; k < Ktot; k += 256) dst[(size_t) r * Ktot + k] = __float2bfloat16_rn(0.0f);
             return;
         }
         default: {   // PREP_DGRAD: block = (4 input channels, one stride-phase class): the class's
@@ -621,29 +635,36 @@ __global__ void __launch_bounds__(256) prep_group_kernel(const PrepJob *__restri
             if (!J.nchw && (J.kn & 3) == 0 && (J.knp & 3) == 0 && ((beg | end | J.info.Ktot) & 3) == 0 &&
                 ((uintptr_t) J.w & 15) == 0 && ((uintptr_t) J.out & 7) == 0) {
                 // NHWC-API weights: four consecutive output channels per 16-byte load and 8-byte
-                // store, four loads in flight
+                // store; long rows one after the other (to find its row by a division per value took 470 x 664 x 3 x 3 from
+                // 15 us to 21 a round of six; 13 so)
                 if (t < nt) taps[t] = J.info.kx[J.info.tap0[c] + t] * J.kw + J.info.ky[J.info.tap0[c] + t];
                 __syncthreads();
                 const int nq = (end - beg) >> 2, khw = J.kh * J.kw, kn = J.kn, knp = J.knp, Ktot = J.info.Ktot;
                 const FastDiv dknp = J.dknp;
                 const float *w = J.w + (size_t) ci0 * khw * kn;
                 bf16 *out = (bf16 *) J.out + (size_t) ci0 * Ktot + beg;
-                batched<4, float4>(
-                    min(4, J.C - ci0) * nq,
-                    [&](int i) {
-                        const int r = i / nq, idx = (i - r * nq) * 4;
-                        const int g = (int) dknp.div((uint32_t) idx), co = idx - g * knp;
-                        if (g >= nt || co >= kn) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        return __ldg(reinterpret_cast<const float4 *>(w + ((size_t) r * khw + taps[g]) * kn + co));
-                    },
-                    [&](int i, float4 v) {
-                        const int r = i / nq, idx = (i - r * nq) * 4;
-                        __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-                        uint2 u;
-                        u.x = *reinterpret_cast<uint32_t *>(&lo);
-                        u.y = *reinterpret_cast<uint32_t *>(&hi);
-                        *reinterpret_cast<uint2 *>(out + (size_t) r * Ktot + idx) = u;
-                    });
+                const int nci = min(4, J.C - ci0);
+                auto load = [&](int r, int idx) {
+                    const int g = (int) dknp.div((uint32_t) idx), co = idx - g * knp;
+                    if (g >= nt || co >= kn) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    return __ldg(reinterpret_cast<const float4 *>(w + ((size_t) r * khw + taps[g]) * kn + co));
+                };
+                auto store = [&](int r, int idx, float4 v) {
+                    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+                    uint2 u;
+                    u.x = *reinterpret_cast<uint32_t *>(&lo);
+                    u.y = *reinterpret_cast<uint32_t *>(&hi);
+                    *reinterpret_cast<uint2 *>(out + (size_t) r * Ktot + idx) = u;
+                };
+                if (nq <= 128) {   // short rows side by side
+                    batched<2, float4>(
+                        4 * nq, [&](int i) { return (i & 3) < nci ? load(i & 3, i & ~3) : make_float4(0.0f, 0.0f, 0.0f, 0.0f); },
+                        [&](int i, float4 v) { if ((i & 3) < nci) store(i & 3, i & ~3, v); });
+                } else {
+                    for (int r = 0; r < nci; r++)
+#pragma unroll 4
+                        for (int q = t; q < nq; q += 256) store(r, 4 * q, load(r, 4 * q));
+                }
                 return;
             }
             for (int r = 0; r < 4; r++) {

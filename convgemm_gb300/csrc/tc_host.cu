@@ -1329,13 +1329,16 @@ extern "C" convgemm_status_t convgemm_prep_prepare(int n, const convgemm_prep_it
                 return cg_set_error(CONVGEMM_ERROR_NOT_SUPPORTED, "%s: item %d: more than 16 stride-phase classes", fn, i);
             if (pl.Ktot > 0) {
                 PrepJob f = j;
-                f.type = j.nchw ? PREP_DGRAD_NCHW : PREP_DGRAD;
+                // NCHW weights staged where one class has several taps (a block reads all taps of its channels for each class,
+                // and one tap of four channels fills half a sector), else gathered
+                const bool staged = j.nchw && pl.ncls == 1 && s.kh * s.kw > 1;
+                f.type = staged ? PREP_DGRAD_NCHW : PREP_DGRAD;
                 f.knp = pl.Cin;
                 f.info = tc_pack_info(pl);
                 f.dknp = FastDiv((uint32_t) f.knp);
                 f.out = it.packed_dgrad;
                 const int run = prep_nchw_run(s.kh * s.kw);
-                add(f, (long long) ((s.c + 3) / 4) * f.info.ncls * (j.nchw ? (f.knp + run - 1) / run : 1));
+                add(f, (long long) ((s.c + 3) / 4) * f.info.ncls * (staged ? (f.knp + run - 1) / run : 1));
             }
         }
         if (blocks > (1LL << 31) - 1) return cg_set_error(CONVGEMM_ERROR_NOT_SUPPORTED, "%s: too many blocks", fn);
