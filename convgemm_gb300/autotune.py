@@ -15,10 +15,9 @@ package (autotune_gb300.json) and are used when the user cache has no entry.
 
 Other choices of the design are fixed and not tuned: one CTA per cluster (no
 operand is shared between the CTAs of a group, whose tiles belong to unrelated
-convolutions), four pipeline stages (the largest ring that holds a 256-wide
-stage of 48 KB beside the output staging buffer), and no split-K in the
-forward (the grouped table spreads small-M / long-K convolutions across SMs
-instead; split-K is used by the weight gradient, whose K is the pixel count).
+convolutions), four, six or eight pipeline stages by the tile width (what the
+ring of 192 KB holds), and no split of a grouped convolution's reduction (the
+table spreads small-M / long-K convolutions across SMs instead).
 """
 from __future__ import annotations
 
@@ -200,6 +199,8 @@ def op_candidates(op: int, s):
         return [(w, 0) for w in candidate_widths(s.kn)]
     tc.tune_set(op, s, 0, 0)
     bn0, s0, mx = tc.wgrad_bf16_plan(s)
+    # Ragged channels: widths and splits of the library's own load path alone. The pairs, 128-pixel chunks and X on
+    # the 128-row side that its estimate may use for them are in the (0, 0) candidate of tune_ops.
     widths = [64, 128] if s.kn < 128 else candidate_widths(s.kh * s.kw * tc.c8(s.c))
     # around the heuristic, plus the cluster-reduced split counts (2..8) that fit
     splits = sorted({max(1, s0 // 4), max(1, s0 // 2), s0, min(mx, 2 * s0)} | {x for x in (2, 4, 8) if x <= mx})

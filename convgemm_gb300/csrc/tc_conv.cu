@@ -131,7 +131,7 @@ __device__ __forceinline__ void acc_load(uint32_t ta, uint32_t (&v)[F32 ? 1 : 2]
         tc::tmem_ld_32x32b_x32(ta, v[0]);
         tc::tmem_ld_wait();
     } else {
-        tc::frag_load<8>(ta, v);
+        tc::frag_load(ta, v);
     }
 }
 
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(EW == 8 ? 384 : 288, 1)
                         w[3] = __float_as_uint(fmaf(__uint_as_float(w[3]), sc.w, sh.w));
                     }
                 } else {
-                    tc::frag_affine<NQ>(v, affine, scp + c0, shp + c0);
+                    tc::frag_affine(v, affine, scp + c0, shp + c0);
                 }
                 if constexpr (EXTRA == EXTRA_SUMS || EXTRA == EXTRA_STATS) {
                     // Column sums of this item's 64 columns over the warp's 32 rows, to group

@@ -25,27 +25,19 @@ __device__ __forceinline__ uint32_t cvt_bf16x2(float lo, float hi) {
     return d;
 }
 
-// 32 rows x 8 * NQ columns of FP32 accumulators; ta: the warp's lane quarter and the first column.
-template <int NQ>
-__device__ __forceinline__ void frag_load(uint32_t ta, uint32_t (&v)[2][4 * NQ]) {
-    static_assert(NQ == 8 || NQ == 4, "64 or 32 columns");
-    if constexpr (NQ == 8) {
-        tmem_ld_16x256b_x8(ta, v[0]);
-        tmem_ld_16x256b_x8(ta + (16u << 16), v[1]);
-    } else {
-        tmem_ld_16x256b_x4(ta, v[0]);
-        tmem_ld_16x256b_x4(ta + (16u << 16), v[1]);
-    }
+// 32 rows x 64 columns of FP32 accumulators; ta: the warp's lane quarter and the first column.
+__device__ __forceinline__ void frag_load(uint32_t ta, uint32_t (&v)[2][32]) {
+    tmem_ld_16x256b_x8(ta, v[0]);
+    tmem_ld_16x256b_x8(ta + (16u << 16), v[1]);
     tmem_ld_wait();
 }
 
 // v = v * sc + sh (sc, sh: the first column's, 8-byte aligned); without either v + 0, which is the same for 1 and 0.
-template <int NQ>
-__device__ __forceinline__ void frag_affine(uint32_t (&v)[2][4 * NQ], bool affine, const float *__restrict__ sc,
+__device__ __forceinline__ void frag_affine(uint32_t (&v)[2][32], bool affine, const float *__restrict__ sc,
                                             const float *__restrict__ sh) {
     const int fc = 2 * (threadIdx.x & 3);
 #pragma unroll
-    for (int q = 0; q < NQ; q++) {
+    for (int q = 0; q < 8; q++) {
         float2 s = make_float2(1.0f, 1.0f), t = make_float2(0.0f, 0.0f);
         if (affine) {
             s = *reinterpret_cast<const float2 *>(sc + 8 * q + fc);

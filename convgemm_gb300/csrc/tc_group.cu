@@ -230,12 +230,12 @@ __global__ void __launch_bounds__(GTHREADS, 1)
             for (int ch = half; ch < nch; ch += 2) {
                 const int c0 = max(0, min(ch * 64, nn - 64));   // the last chunk repeats columns of the one before
                 uint32_t v[2][32];
-                tc::frag_load<8>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * GBN + c0), v);
+                tc::frag_load(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * GBN + c0), v);
                 if (ch + 2 >= nch) {
                     tc::tc_fence_before();
                     tc::mbar_arrive(&acc_empty[buf]);
                 }
-                tc::frag_affine<8>(v, scale || shift, sc_tab + c0, sh_tab + c0);
+                tc::frag_affine(v, scale || shift, sc_tab + c0, sh_tab + c0);
                 uint32_t pk[32];
                 tc::frag_pack(v, relu != 0, pk);
                 // each warp stages its 32 rows and stores them itself: no barrier across warps

@@ -33,8 +33,6 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-int pick_bn(int cout) { return cout >= 256 ? 256 : (cout > 64 ? 128 : 64); }
-
 typedef CUresult (*EncodeIm2colFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                    const cuuint64_t *, const int *, const int *, cuuint32_t, cuuint32_t,
                                    const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -56,8 +54,7 @@ EncodeIm2colFn encode_im2col_fn() {
 
 }  // namespace
 
-// im2col-mode map of a BF16 NHWC tensor [B][H][W][C]: `pixels` pixels x 64 channels per load,
-// bounding box [lo, dim-1+up] per spatial dimension, traversal strides (sh, sw), 128-byte swizzle.
+// Tiled maps of rank 3 to 5 (dimension 0 innermost; strides of the others in bytes).
 convgemm_status_t tc_make_map_nd(CUtensorMap *map, int rank, const void *ptr, const unsigned long long *dims,
                                   const unsigned long long *strides_bytes, const unsigned *box, const unsigned *estr,
                                   int swizzle128) {
@@ -88,6 +85,8 @@ convgemm_status_t tc_make_map_nd_dt(CUtensorMap *map, CUtensorMapDataType dt, in
     return CONVGEMM_SUCCESS;
 }
 
+// im2col-mode map of a BF16 NHWC tensor [B][H][W][C]: `pixels` pixels x `chans` channels per load,
+// bounding box [lo, dim-1+up] per spatial dimension, traversal strides (sh, sw), 128-byte swizzle.
 convgemm_status_t tc_make_im2col_map(CUtensorMap *map, const void *ptr, int B, int H, int W, int C, int lo_h,
                                      int lo_w, int up_h, int up_w, int sh, int sw, int pixels, int elem_bytes,
                                      int chans) {
@@ -197,9 +196,7 @@ bool tc_plan_fwd(const cg_shape &s, TcPlan &pl) {
     c.dwg = FastDiv(c.Wg);
     c.dhg = FastDiv(c.Hg);
     pl.Ktot = c.ktiles * 64;
-    pl.mtiles_max = c.mtiles;
     pl.has_empty_class = false;
-    pl.bn = pick_bn(pl.Cout);
     return true;
 }
 
@@ -217,7 +214,6 @@ bool tc_plan_dgrad(const cg_shape &s, TcPlan &pl) {
     memset(pl.toy, 0, sizeof(pl.toy));
     memset(pl.tox, 0, sizeof(pl.tox));
     pl.has_empty_class = false;
-    pl.mtiles_max = 0;
     int kb = 0, tap0 = 0;
     for (int cy = 0; cy < sy; cy++)
         for (int cx = 0; cx < sx; cx++) {
@@ -261,11 +257,9 @@ bool tc_plan_dgrad(const cg_shape &s, TcPlan &pl) {
             c.mtiles = (int) (((long long) s.b * Hg * Wg + 127) / 128);
             c.dwg = FastDiv(Wg);
             c.dhg = FastDiv(Hg);
-            if (c.mtiles > pl.mtiles_max) pl.mtiles_max = c.mtiles;
             pl.ncls++;
         }
     pl.Ktot = kb;
-    pl.bn = pick_bn(pl.Cout);
     return true;
 }
 
@@ -1007,6 +1001,7 @@ WgPlan plan_wgrad(const convgemm_shape_t &ps) {
             w.xa = 1;
         }
     }
+    // (the groups' planes are not written: see tc_wgrad_groups)
     w.ws_bytes = sizeof(float) * (size_t) (w.splits + tc_wgrad_groups(w.splits)) * (size_t) w.Nx * (size_t) s.kn;
     w.csize = w.groups = 0;
     if (w.slab) return w;

@@ -10,7 +10,7 @@
 // A planned tensor-core convolution: its classes, and the packed-operand geometry.
 struct TcPlan {
     int Cin, Cout, Hin, Win, Hout, Wout;
-    int ncls, Ktot, mtiles_max, bn;
+    int ncls, Ktot;
     bool has_empty_class;
     TcClass cls[TC_MAXCLS];
     int16_t toy[TC_MAXTAPS], tox[TC_MAXTAPS];   // taps of all classes (TcClass::tap0): offsets in the gathered tensor

@@ -10,8 +10,8 @@
 //
 // Limits and sharing:
 //   * the scratch holds CONVGEMM_NOALLOC_SCRATCH_FLOATS FP32 values (16 MiB);
-//     the number of pixel splits is capped so the partials (and the group sums
-//     of the two-pass reduction) fit, and a layer
+//     the number of pixel splits is capped so the partials fit (with room for as many
+//     planes as the reduction has groups of splits, which it does not use), and a layer
 //     whose single partial tile (Nx*kn, Nx = kh*kw*c8) does not fit is
 //     rejected with CONVGEMM_ERROR_NOT_SUPPORTED;
 //   * every GPU that loads the library holds the 16 MiB until the process exits;
@@ -93,15 +93,15 @@ extern "C" convgemm_status_t convgemm_wgrad_bf16_noalloc(convgemm_layout_t layou
     NoallocDevice *d = nullptr;
     if (convgemm_status_t e = noalloc_setup(&d)) return e;
 
-    // the same tiling as the workspace form, with the pixel splits capped by the scratch
+    // 64-pixel chunks, no pairs or operand exchange (the workspace form's tuned and estimated plans may differ), X
+    // gathered unless its channels are a multiple of 64, the pixel splits capped by the scratch
     const int xa = s.kn < 128;
     const int Mext = xa ? Nx : s.kn, Next = xa ? s.kn : Nx;
     const int bn = xa ? (s.kn <= 64 ? 64 : 128) : (Nx >= 256 ? 256 : (Nx > 64 ? 128 : 64));
     const int mtiles = (Mext + 127) / 128, ntiles = (Next + bn - 1) / bn;
     const int nchunks = (int) ((g.P + 63) / 64);
     const int base = mtiles * ntiles;
-    // the workspace form's default: one wave of CTAs (no partial second wave), at least 8
-    // chunks (512 pixels) per split
+    // one wave of CTAs (no partial second wave), at least 8 chunks (512 pixels) per split
     int splits = tc_num_sms() * (bn == 256 ? 1 : 2) / base;
     splits = splits > (nchunks + 7) / 8 ? (nchunks + 7) / 8 : splits;
     const int fit = (int) ((long long) CONVGEMM_NOALLOC_SCRATCH_FLOATS / tile);
@@ -109,7 +109,7 @@ extern "C" convgemm_status_t convgemm_wgrad_bf16_noalloc(convgemm_layout_t layou
     if (splits < 1) splits = 1;
     int cps = (nchunks + splits - 1) / splits;
     splits = (nchunks + cps - 1) / cps;
-    // the reduction's group planes follow the split planes in the scratch
+    // room for the reduction's groups as well: not written, but the split count, and with it the bits, stay what they were
     while (splits > 1 && (long long) (splits + tc_wgrad_groups(splits)) * tile > (long long) CONVGEMM_NOALLOC_SCRATCH_FLOATS) {
         splits--;
         cps = (nchunks + splits - 1) / splits;

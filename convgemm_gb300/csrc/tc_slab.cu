@@ -155,10 +155,10 @@ __global__ void __launch_bounds__(288, 1)
             if (!(ok = tc::mbar_wait(&acc_full[buf], (lt / SLAB_ACC) & 1, p.err, 53))) break;
             tc::tc_fence_after();
             uint32_t v[2][32];
-            tc::frag_load<8>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * SLAB_BN), v);
+            tc::frag_load(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * SLAB_BN), v);
             tc::tc_fence_before();
             tc::mbar_arrive(&acc_empty[buf]);
-            tc::frag_affine<8>(v, p.scale || p.shift, sc_tab, sh_tab);
+            tc::frag_affine(v, p.scale || p.shift, sc_tab, sh_tab);
             uint32_t pk[32];
             tc::frag_pack(v, p.relu != 0, pk);
             uint8_t *stg = stage + (size_t) (p.nstage == 2 ? (lt & 1) : 0) * SLAB_STAGE;

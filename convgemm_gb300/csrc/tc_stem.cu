@@ -206,12 +206,12 @@ __global__ void __launch_bounds__(STEM_THREADS, 1)
                 tc::tc_fence_after();
                 for (int c0 = 0; c0 < BN; c0 += 64) {
                     uint32_t v[2][32];
-                    tc::frag_load<8>(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * BN + c0), v);
+                    tc::frag_load(tmem + ((uint32_t) (ew * 32) << 16) + (uint32_t) (buf * BN + c0), v);
                     if (c0 + 64 >= BN) {
                         tc::tc_fence_before();
                         tc::mbar_arrive(&acc_empty[buf]);
                     }
-                    tc::frag_affine<8>(v, p.scale || p.shift, sc_tab + c0, sh_tab + c0);
+                    tc::frag_affine(v, p.scale || p.shift, sc_tab + c0, sh_tab + c0);
                     if (p.stats) {
                         // batch-norm statistics of the 64 columns over this warp's 32 pixels
                         if (ox0 + 32 > p.Wo) tc::frag_clear_rows(v, p.Wo - ox0);

@@ -2,7 +2,7 @@
 // sconvGemmNHWC('T') (src/convGemm.c:71-76),
 //     dW[co][n] = sum_p dY[p][co] * X_im2row[p][n],  n = tap*Cp + ci,
 // whose reduction runs over all b*ho*wo output pixels.  The pixels are cut
-// into 64-pixel chunks and the chunks into `splits` contiguous ranges, one per
+// into chunks of 64 or 128 pixels and the chunks into `splits` contiguous ranges, one per
 // blockIdx.z; each CTA writes its FP32 partial tile to a workspace and
 // the reduction adds the splits in a fixed order (in increasing split order,
 // or, with many splits, in fixed contiguous groups whose sums are then added in
@@ -10,12 +10,14 @@
 //
 // Both operands reach the tensor core MN-major (the pixel index is the slow,
 // K dimension in memory):
-//   dY side: TMA boxes of 64 channels x 64 pixels from dY viewed as [P][kn8];
-//   X side:  im2col-mode TMA boxes of 64 channels of one tap x 64 pixels when the
-//            channels are multiples of 64 (tiled boxes of the [P][Cp] matrix for a
-//            1x1 stride-1 unpadded convolution), else 16-byte cp.async gathers of
-//            8 channels of one tap for each pixel, zero-filled for padding, written
-//            in the 128-byte-swizzled layout.
+//   dY side: TMA boxes of 64 channels x 64 or 128 pixels from dY viewed as [P][kn8];
+//   X side:  im2col-mode TMA boxes of 64 channels of one tap x 64 or 128 pixels (tiled
+//            boxes of the [P][Cp] matrix for a 1x1 stride-1 unpadded convolution),
+//            channels that are no multiple of 64 padded to one with zeros by the
+//            loads; up to 8 channels, and for ragged ones up to 128 where it is
+//            estimated cheaper, 16-byte cp.async gathers of 8 channels of one tap
+//            for each pixel, zero-filled for padding, written in the
+//            128-byte-swizzled layout.
 // The X side is the 128-row A operand when kn < 128 (template XA), else dY is,
 // so narrow layers do not waste half of each MMA; a tuned configuration may put
 // the X side on A for wide layers too (measured faster on 3x3 layers at the same

@@ -10,10 +10,10 @@ struct TcWgradParams {
     float *ws;                // [splits][Mext][Next] FP32 partial tiles
     int B, H, W, Cp, kh, kw, kn, Nx, P;
     int vstr, hstr, vpad, hpad, vdil, hdil;
-    int nchunks, chunks_per_split;  // 64-pixel chunks of the reduction, per split
+    int nchunks, chunks_per_split;  // chunks of the reduction (64 pixels; `wide` 128), per split
     FastDiv dcp, dwo, dho;
     int *err;
-    int im2col;               // X by im2col-mode TMA (Cp % 64 == 0), else by cp.async gathers
+    int im2col;               // X by im2col-mode TMA (Cp: the channels rounded up to 64), else by cp.async gathers (to 8)
     int x2d;                  // with im2col: X of a 1x1 stride-1 unpadded convolution is the matrix
                               // [P][Cp], loaded by tiled TMA (xmap 2-D, 64 x 64 boxes) instead
     // one split: the epilogue writes dW itself (no workspace, no reduction) in the
@@ -66,11 +66,12 @@ int tc_wgrad_stages(int bn, int im2col, int kb1, int wide = 0, int pair = 0);
 // Tile counters of the grouped cluster reduction on the current device: `n` consecutive
 // zero words for one launch (a rotating range of a fixed device array; NULL if unavailable).
 unsigned *tc_wgrad_counters(int n);
-// Split groups of the two-pass reduction (0: one pass).  With many splits, the
-// first pass sums each of G contiguous split ranges into planes that follow the
-// split planes in the workspace, so the workspace holds splits + G planes.
+// Split groups of the reduction (0: the splits are added in order).  With many splits, each of G
+// contiguous split ranges is summed in order, then the G sums (in shared memory).  The workspace
+// size and the fixed scratch's split count still count G planes behind the splits', which are not
+// written: both are what callers and their bits have known.
 int tc_wgrad_groups(int splits);
-// ws: [splits + tc_wgrad_groups(splits)][Nx * kn] FP32.
+// ws: [splits][Nx * kn] FP32.
 cudaError_t tc_wgrad_reduce(float *ws, float *dw, int splits, int xa, int Nx, int kn, int C, int Cp, int kh, int kw,
                             int layout, cudaStream_t st);
 

@@ -139,7 +139,15 @@ convgemm_status_t convgemm_to_bf16_nhwc(convgemm_layout_t layout, int b, int c, 
 /* Forward, BF16 tensor cores (tcgen05, FP32 accumulation in TMEM): generalises
  * sconvGemmNHWC('N') (src/convGemm.c:65-70).  x: BF16 NHWC [b][h][w][c8];
  * y: BF16 NHWC [b][ho][wo][kn] = relu?(acc*scale + shift); scale/shift may be NULL.
- * Needs kn % 8 == 0. */
+ * Needs kn % 8 == 0.
+ *
+ * Order of the FP32 additions, here, in the input gradients and in the FP8 and 3xBF16 forwards: the
+ * same for every form of an operation on a shape (with and without mask, sums or accumulation) and
+ * from run to run. It depends on the shape with its batch, on the number of SMs and on whether the
+ * shape has a tuning entry: launches of few tiles share a tile's reduction between CTAs, and channels
+ * that are no multiple of 64 come in the order of the cheaper of two load paths. One image may
+ * therefore round differently alone and within a larger batch. (The FP32 plain form adds in the
+ * reference's order throughout.) */
 convgemm_status_t convgemm_fwd_bf16(const convgemm_shape_t *shape, const void *x, const void *wpacked, void *y,
                                     const float *scale, const float *shift, int relu, void *stream);
 
@@ -258,11 +266,13 @@ enum {
  * form with eight epilogue warps (short-K layers; 0 = heuristic), plus 8 for the general
  * kernel instead of a slab kernel, plus 16 for one K block per ring stage and twice the
  * stages (64 / 128-wide tiles, one M tile, four epilogue warps).
- * bn = aux = 0 removes the entry.  Set the weight-gradient entry before querying
+ * bn = aux = 0 removes the entry.  A forward / input-gradient entry also keeps the launch from sharing a
+ * tile's reduction between CTAs (see below), which changes the order of its FP32 additions.  Set the weight-gradient entry before querying
  * its workspace size.  Thread-safe. */
 convgemm_status_t convgemm_tune_set(int op, const convgemm_shape_t *shape, int bn, int aux);
-/* Weight-gradient flags (channels that are multiples of 64): X, not dY, as the
- * 128-row A operand of a layer with kn >= 128 (N widths 64 / 128 / 256 of kn);
+/* Weight-gradient flags (where X is loaded by TMA: channels that are multiples of 64, and the others above 8
+ * except where gathers of up to 128 packed channels are estimated cheaper; ignored by the gathers):
+ * X, not dY, as the 128-row A operand of a layer with kn >= 128 (N widths 64 / 128 / 256 of kn);
  * X of a 1x1 stride-1 unpadded convolution by im2col boxes instead of tiled
  * boxes of the [pixels][channels] matrix.  Results equal the default's within
  * the BF16 bound (the tiled / im2col choice gives the same bits). */
@@ -289,7 +299,8 @@ convgemm_status_t convgemm_tune_set(int op, const convgemm_shape_t *shape, int b
 #define CONVGEMM_WGRAD_TWO_ISSUERS 0x800000
 /* Weight gradient (im2col path): chunks of 128 pixels, one per ring stage, so that every TMA
  * box carries twice the bytes (the per-box cost, not the bytes, bounds a TMA stream of 8 KB
- * boxes); the MMAs run in the same order, so dW is bit-identical to the default's. */
+ * boxes); the MMAs run in the same order, so dW is bit-identical to that of 64-pixel chunks with
+ * the same tiles and split boundaries. */
 #define CONVGEMM_WGRAD_WIDE_CHUNKS 0x1000000
 /* im2col path: CTA pairs (thread-block clusters of two) share 256 x 256 (bn 256, the default) or
  * 256 x 128 (bn 128) tiles through cta_group::2 MMAs, each CTA loading its A rows and half of the
@@ -379,7 +390,8 @@ convgemm_status_t convgemm_dgrad_bf16_bias_grad(const convgemm_shape_t *shape, c
 
 /* Bias gradient of the convolution: db[co] = sum over the b*ho*wo output pixels of
  * dy[p][co] (dy BF16 NHWC with kn rounded up to 8 channels, as for
- * convgemm_wgrad_bf16), FP32 in a fixed order (bit-reproducible). */
+ * convgemm_wgrad_bf16), FP32 in a fixed order (bit-reproducible).  workspace: kn floats for each
+ * 1024 pixels, at most 256 times. */
 size_t convgemm_bias_grad_bf16_workspace_size(const convgemm_shape_t *shape);
 convgemm_status_t convgemm_bias_grad_bf16(const convgemm_shape_t *shape, const void *dy, float *db, void *workspace,
                                           size_t workspace_bytes, void *stream);
