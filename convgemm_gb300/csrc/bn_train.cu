@@ -37,8 +37,8 @@ __device__ __forceinline__ double widen(float f) {   // (double) f
 }
 // With one chunk of all groups its sums are the result, and the second kernel is not needed: OUT double writes them like
 // the chunk sums, OUT float the first plane's. That leaves one block per 8 channels, so it is for what one chunk holds, and
-// up to two chunks of few channels (500 groups of 64 channels with their forward 10.4 us, 10.3 in two passes, with the input
-// gradient 8.9 and 11.8; 1000 groups 30 and 17, 26 and 13; 375 groups of 256 channels 25 and 19, 22 and 13).
+// up to two chunks of few channels (500 groups of 64 channels with their forward 10.4 us, 10.3 in two passes; 1000 groups 30
+// and 17; 375 groups of 256 channels 25 and 19). The column sums, half the loads, have a line of their own.
 inline bool one_pass(long long ngroups, int kn) { return ngroups <= BN_CHUNK || (ngroups <= 2 * BN_CHUNK && ngroups * kn <= 36864); }
 template <int PLANES, class OUT>
 __global__ void __launch_bounds__(256) bn_stats_pass1(const float *__restrict__ part, int ngroups, int chunk, int kn,
@@ -235,10 +235,15 @@ cudaError_t cg_colsum_reduce(void *workspace, int ngroups, int kn, float *out, c
     const int nchunks = (ngroups + BN_CHUNK - 1) / BN_CHUNK;
     double *chunks = (double *) workspace;
     const float *part = (const float *) ((uint8_t *) workspace + (size_t) nchunks * 2 * kn * 8);
-    if (one_pass(ngroups, kn)) {
-        // many blocks: launched plainly, as the first of two passes (125 groups of 512 channels: 16.6 us otherwise)
-        cg_launch_ex(kn > 256 ? CG_PDL_OFF : CG_PDL_THREAD, bn_stats_pass1<1, float>, dim3((kn + 7) / 8), dim3(256), 0, st, part, ngroups,
-                     ngroups, kn, out);
+    // One pass up to two chunks of groups, of any width: never behind two on 36 input gradients of 263 to 500 groups (392 groups of
+    // 256 channels with their 3 x 3: 32.8 us, 34.8 in two; 512 -> 512: 69.6, 71.7). Its blocks are launched during the tail of the
+    // kernel that writes the groups where there are few of them or their chains are short; otherwise they keep its last
+    // tiles waiting (392 groups of 128 channels from 512: 30.7 us, 20.5 launched plainly; 125 groups of 512: 16.6, 10.7; but
+    // 392 of 64: 16.4, 18.4).
+    if (ngroups <= 2 * BN_CHUNK) {
+        const bool early = kn <= 64 || (ngroups <= BN_CHUNK && kn <= 256);
+        cg_launch_ex(early ? CG_PDL_THREAD : CG_PDL_OFF, bn_stats_pass1<1, float>, dim3((kn + 7) / 8), dim3(256), 0, st, part,
+                     ngroups, ngroups, kn, out);
         return cudaGetLastError();
     }
     dim3 g1((kn + 7) / 8, nchunks);
