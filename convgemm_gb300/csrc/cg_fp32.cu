@@ -756,6 +756,9 @@ __global__ void __launch_bounds__(T::NT, T::CTAS) fp32_igemm_kernel(const __grid
     const int z = blockIdx.z;
     int rbeg, rend;
     op.range(m0, z, rbeg, rend);
+    // Pixels of a stride phase that no tap reaches: an accumulating call leaves them as they are (56 x 56, 256 -> 512 1 x 1
+    // stride 2, batch 64: 848 -> 477 us; 256 -> 128: 530 -> 180)
+    if (op.starts() && rbeg >= rend) return;
     Rt[0][tid] = op.rent(rbeg + tid, rend);
     Rt[1][tid] = op.rent(rbeg + NT + tid, rend);
 

@@ -392,3 +392,38 @@ def test_filters_beyond_the_tap_masks(cglib, oracle_lib, b, h, w, c, kn, kh, kw,
         got = dropin(cglib, "dgrad", layout, g, inp, inp["dx0"].copy(), to_dev=True)
         assert errors(got, port(oracle_lib, "dgrad", layout, g, inp, None))[0] <= FP32_TOL, layout
         assert bitexact(got, dropin(cglib, "dgrad", layout, g, inp, inp["dx0"].copy(), to_dev=True)), layout
+
+
+@pytest.mark.parametrize("b,h,w,c,kn,k,stride,pad", [
+    (2, 23, 17, 36, 40, 1, 2, 0),     # 1 x 1: three of four phases have no tap
+    (1, 14, 14, 5, 12, 2, 3, 0),      # five of nine, c no multiple of 4
+    (40, 28, 28, 64, 64, 1, 2, 0),    # several tiles per phase
+])
+def test_accumulating_input_gradient_leaves_unreached_pixels(cglib, oracle_lib, b, h, w, c, kn, k, stride, pad):
+    """Pixels of a stride phase without taps keep dx's bits, -0, infinities and NaN with them; the others are the reference's
+    sums within FP32 tolerance. An overwriting call writes zeros there."""
+    g = C.geom(b, h, w, c, kn, k, k, vpad=pad, hpad=pad, vstr=stride, hstr=stride)
+    ho, wo = C.out_hw(g)
+    rng = np.random.default_rng(b * h + k)
+    iy, ix = np.meshgrid(np.arange(h), np.arange(w), indexing="ij")
+    out = ((iy + pad) % stride >= k) | ((ix + pad) % stride >= k)   # taps reach residues 0 .. k - 1 only
+    s = cglib.Shape.of(b, h, w, c, kn, k, k, pad, pad, stride, stride)
+    for layout in (C.NHWC, C.NCHW):
+        shape = (b, h, w, c) if layout == C.NHWC else (b, c, h, w)
+        inp = {"w": (rng.standard_normal(c * k * k * kn) * np.sqrt(2 / c)).astype(np.float32), "x": None, "epi": {},
+               "dy": rng.uniform(-1, 1, b * ho * wo * kn).astype(np.float32),
+               "dx0": rng.uniform(-1, 1, b * h * w * c).astype(np.float32)}
+        ref = port(oracle_lib, "dgrad", layout, g, inp, None).reshape(shape)
+        odd = inp["dx0"].copy().reshape(shape)
+        mask = np.broadcast_to(out[None, :, :, None] if layout == C.NHWC else out[None, None], shape)
+        odd[mask] = np.resize(np.array([-0.0, np.inf, np.nan, -np.inf, 1e-42, 3.0], np.float32), mask.sum())
+        wd, dyd = torch.from_numpy(inp["w"]).cuda(), torch.from_numpy(inp["dy"]).cuda()
+        dx = torch.from_numpy(odd.copy()).cuda()
+        cglib.dgrad_f32(layout, s, wd, dyd, dx)
+        got = dx.cpu().numpy()
+        assert bitexact(got[mask], odd[mask]), layout
+        assert errors(got[~mask], ref[~mask])[0] <= FP32_TOL, layout
+        dx.fill_(float("nan"))
+        cglib.dgrad_f32(layout, s, wd, dyd, dx, accumulate=False)
+        got = dx.cpu().numpy()
+        assert (got[mask] == 0).all() and errors(got[~mask], (ref - inp["dx0"].reshape(shape))[~mask])[0] <= 2 * FP32_TOL, layout
