@@ -904,7 +904,7 @@ int wgrad_wave_splits(int tiles, int bn, long long P) {
 // estimated a tenth cheaper: 45 of the 575, 3% off all together; by TMA 36 of them ran slower than they had with gathers
 // for all such channels. 56 x 56, 24 -> 96 3 x 3, batch 64: 43 us gathered, 76 by TMA; 112 x 112, 40 -> 24 5 x 5, batch 16:
 // 113 and 219; 28 x 28, 40 -> 384, batch 64: 41 and 65; by TMA 14 x 14, 200 -> 328, batch 32: 52 and 26; 23 x 25, 24 -> 304,
-// batch 1: 20 and 7. The rule depends on the shape alone, not on the tuning table.
+// batch 1: 20 and 7. The rule depends on the shape (its batch, too) and the SM count, not on the tuning table.
 constexpr float TMA_EVEN = 0.169f, TMA_ODD = 0.220f;
 constexpr float TMA_TAIL[8] = {0.0f, 0.303f, 0.152f, 0.420f, 0.173f, 0.467f, 0.216f, 0.250f};
 constexpr float TMA_DY[3] = {0.16f, 0.27f, 0.32f};   // rows on 32 bytes; else 8 or 56 channels past a multiple of 64; else
