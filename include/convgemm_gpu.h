@@ -371,8 +371,7 @@ convgemm_status_t convgemm_dgrad_bf16_relu(const convgemm_shape_t *shape, const 
  * dx = dx + dgrad(dy, w), the old BF16 value read in the epilogue and added in FP32
  * before one rounding; accumulate == 0: dx overwritten, as convgemm_dgrad_bf16.
  * relu_x (optional, as for convgemm_dgrad_bf16_relu): the result is then zeroed
- * where relu_x <= 0, after the sum.  dx must be 16-byte aligned when accumulating.
- * relu_x may be dx itself (without accumulate): the mask is read before its values are overwritten. */
+ * where relu_x <= 0, after the sum.  dx must be 16-byte aligned when accumulating. */
 convgemm_status_t convgemm_dgrad_bf16_ex(const convgemm_shape_t *shape, const void *dy, const void *wpacked, void *dx,
                                          const void *relu_x, int accumulate, void *stream);
 
